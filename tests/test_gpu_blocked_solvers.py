@@ -1,0 +1,83 @@
+"""Blocked FP64 tensor-core solvers at the sizes where their tiling can go wrong (needs a B200):
+the Gauss-Jordan inversion (panels of 4 columns, blocks of 8), the pair sums over its Green
+functions and the Dyson LU (panels of 8, blocks of 64)."""
+import numpy as np
+import pytest
+
+from oracle import titan_oracle as O
+from titan_b200.host import synthetic
+from titan_b200.host.system import initial_state
+
+from gg_numpy import fermi_column_numpy, gg_tensor_numpy
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(float).eps
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    from titan_b200.native import GreenGPU
+    g = GreenGPU(0)
+    yield g
+    g.close()
+
+
+@pytest.mark.parametrize("shape,scale", [("bcc1", 0.0), ("sq2", 0.0), ("slab3", 1.0), ("slab3", 0.0), ("bcc4", 0.0),
+                                         ("slab5", 0.0)])
+def test_inversion_needs_its_pivots(gpu, shape, scale):
+    """z - H with H = scale * model + a permutation-like Hermitian matrix: every diagonal entry
+    is tiny, so elimination without row exchanges loses all digits.  Each entry within 1e-12 n
+    of the largest one of LAPACK's inverse (the bound of the plain inversion test)."""
+    deck = synthetic.make_deck(shape, mesh=False)
+    s = deck.system
+    n = s.dimH
+    rng = np.random.default_rng(7)
+    gpu.set_system(s)
+    p = rng.permutation(n)
+    h0 = np.zeros((n, n), complex)
+    for a, b in zip(p[0::2], p[1::2]):
+        t = np.exp(2j * np.pi * rng.uniform()) * rng.uniform(0.5, 2.0)
+        h0[a, b], h0[b, a] = t, np.conj(t)
+    gpu.set_h0(h0)
+    kp = rng.uniform(-2, 2, size=(5, 3))
+    Hk = gpu.hamiltk_batch(kp)
+    if scale == 0.0:   # remove the hoppings: h0 - H_nl(k) at each k in turn
+        zs, out, ref = [], [], []
+        for k in range(5):
+            gpu.set_h0(2.0 * h0 - Hk[k])
+            z = np.array([1e-9j + 1e-7 * k])
+            out.append(gpu.green_batch(z, kp[k:k + 1])[0])
+            ref.append(np.linalg.inv(z[0] * np.eye(n) - h0))
+    else:
+        z = 1e-3j + 0.01 * np.arange(5)
+        out = gpu.green_batch(z, kp)
+        ref = [np.linalg.inv(z[k] * np.eye(n) - Hk[k]) for k in range(5)]
+    for a, b in zip(out, ref):
+        assert np.max(np.abs(a - b)) <= 1e-12 * n * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("shape,nk", [("slab3", (2, 2, 1)), ("bcc4", (2, 2, 2)), ("slab5", (2, 3, 1))])
+def test_pair_sums_of_larger_cells(gpu, shape, nk):
+    """GG tensor (orbital-resolved and summed), Fermi column and J_ij against numpy: products of
+    two Green functions, each within 1e-12 n of its largest entry."""
+    deck = synthetic.make_deck(shape, nk=nk, n1gl=5, parts=1, n3gl=4)
+    s = deck.system
+    h0 = s.h0(initial_state(s))
+    gpu.setup(deck, h0)
+    m = O.Model(s, h0)
+    ek = deck.ek
+    tol = 2e-12 * s.dimH
+    G = m.green(s.Ef + 1j * (ek.point_energy() + s.eta), ek.kp)
+    for resolved in (True, False):
+        T = gpu.gg_tensor(s.Ef, s.eta, resolved)
+        Tr = gg_tensor_numpy(s, G, ek.weight, resolved)
+        assert np.max(np.abs(T - Tr)) <= tol * np.max(np.abs(Tr))
+    Gr = m.green(np.full(deck.real_kp.shape[0], s.Ef + 1j * s.eta), deck.real_kp)
+    D, Dr = gpu.fermi_column(s.Ef, s.eta), fermi_column_numpy(s, Gr, deck.real_w)
+    assert np.max(np.abs(D - Dr)) <= tol * np.max(np.abs(Dr))
+    ev = np.random.default_rng(2).standard_normal((s.n_atoms, 3))
+    ev /= np.linalg.norm(ev, axis=1)[:, None]
+    q = np.array([0.1, -0.05, 0.0])
+    J, Jr = gpu.jij(q, s.Ef, s.eta, ev, s.Um()), O.jij(m, ek, q, s.Ef, s.eta, ev, s.Um(), s.dorbs)
+    assert np.max(np.abs(J - Jr)) <= tol * np.max(np.abs(Jr))

@@ -155,7 +155,6 @@ struct tg_ctx {
   int kind_n[4] = {0, 0, 0, 0};
   int64_t launches = 0;   // kernels launched by the last chi0 call
   int64_t pass_points = 0;     // points per pass (bounded workspace)
-  int gg_blocks = 0, gg_nrow = 0, gg_ncol = 0, gg_mode = -1;
   // spectral Green functions: eigendecomposition of each H(k) table, inverse output map
   int green_method = 0;   // TG_GREEN_AUTO / TG_GREEN_GAUSS_JORDAN / TG_GREEN_SPECTRAL
   DevArray<double2> d_eigU[4];
@@ -165,9 +164,6 @@ struct tg_ctx {
   DevArray<double> d_ldos_e, d_ldos;
   // linear SOC: V, G V G of both Green functions, four operands, chi_lsoc partials
   DevArray<double2> d_vsoc, d_lsb[6], d_Cl, d_Dl;
-  // exchange coupling: d-orbital tables and per-CTA tensor slices
-  DevArray<int> d_jij_tab;
-  DevArray<double2> d_jij_part, d_jij_sum;
   // disturbance response (eintshe)
   DevArray<int> d_she_tab, d_ia, d_she_ztiles, d_she_rowoff;
   DevArray<double2> d_she_part, d_she_sum, d_she_pref, d_she_out;
@@ -1085,7 +1081,6 @@ int tg_set_system(tg_ctx* c, int n_atoms, const int* norb, int norb_max, int n_n
   TG_CHECK(c, cudaStreamSynchronize(s), "sync");
   c->sys_set = true;
   c->h0_set = false;
-  c->gg_mode = -1;
   return TG_OK;
 }
 
@@ -1916,6 +1911,142 @@ int tg_profile(tg_ctx* c, int enable) {
   return TG_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+struct PairRef {
+  int block;   // output block of an orbital pair
+};
+
+// the imaginary-axis points at Ef + i (y + eta); on a uniform mesh (and when `table`) with the
+// H(k) table of its k list in slot 0
+int imag_points(tg_ctx* c, double Ef, double eta, bool table, GreenArgs& a) {
+  a = base_args(c);
+  a.pts.kind = 0;
+  a.pts.y = c->d_y.p;
+  a.pts.kp = c->d_kp.p;
+  a.pts.w = c->d_w.p;
+  a.zr = Ef;
+  a.zi = eta;
+  if (table && c->imag_uniform && (int64_t)c->nk_u * c->dimH * c->dimH * 16 <= ((int64_t)8 << 30)) {
+    const double zero3[3] = {0.0, 0.0, 0.0};
+    int rc = build_htab(c, 0, c->d_klist_u.p, c->nk_u, zero3);
+    if (rc) return rc;
+    a.htab = c->d_htab[0].p;
+    a.n_e = c->n_e_u;
+    a.nk_tab = c->nk_u;
+    a.ylist = c->d_ylist.p;
+  }
+  return TG_OK;
+}
+
+// out[e] = sum over the np points of a of w G(ent[e].x, ent[e].y): raw Green functions of at
+// most 1 GiB per pass, summed by the entry kernel
+int entry_sums(tg_ctx* c, GreenArgs a, int64_t np, const std::vector<int2>& ent, std::vector<double2>& out,
+               const char* what) {
+  cudaStream_t s = c->stream;
+  const int64_t nn = (int64_t)c->dimH * c->dimH;
+  const int ne = (int)ent.size();
+  out.assign(ent.size(), make_double2(0.0, 0.0));
+  const int64_t P = pass_size(c, np, (int64_t)1 << 30);
+  const int parts = entry_partials(P, c->num_sms);
+  TG_CHECK(c, c->d_gg_desc.upload(reinterpret_cast<const int*>(ent.data()), 2 * ent.size(), s), "upload");
+  TG_CHECK(c, c->d_graw.ensure((size_t)P * nn), "alloc G");
+  TG_CHECK(c, c->d_acc.ensure((size_t)parts * ne), "alloc acc");
+  TG_CHECK(c, c->d_acc_red.ensure(ne), "alloc acc");
+  TG_CHECK(c, cudaMemsetAsync(c->d_acc.p, 0, sizeof(double2) * (size_t)parts * ne, s), "memset");
+  int rc = reset_status(c);
+  if (rc) return rc;
+  a.mode = MODE_RAW;
+  a.out = c->d_graw.p;
+  for (int64_t p0 = 0; p0 < np; p0 += P) {
+    a.p0 = p0;
+    a.np = std::min<int64_t>(P, np - p0);
+    TG_CHECK(c, launch_green(a, c->num_sms, s, nullptr), what);
+    TG_CHECK(c, launch_entries(a, c->d_graw.p, reinterpret_cast<const int2*>(c->d_gg_desc.p), ne, c->num_sms,
+                               c->d_acc.p, s),
+             "entry sums");
+  }
+  TG_CHECK(c, launch_reduce_blocks(c->d_acc.p, parts, ne, c->d_acc_red.p, s), "reduce");
+  TG_CHECK(c, cudaMemcpyAsync(out.data(), c->d_acc_red.p, sizeof(double2) * ne, cudaMemcpyDeviceToHost, s), "copy");
+  return read_status(c);
+}
+
+// h[16 b + q]: the 16 spin products of orbital pair b summed over the imaginary axis, with
+// G(k) in both factors, or (q not null) with G(k) in the first and G(k - q) in the second one,
+// and then hs[..] with the two exchanged
+int imag_pairs(tg_ctx* c, double Ef, double eta, const double* q, const std::vector<int4>& pairs,
+               std::vector<double2>& h, std::vector<double2>* hs) {
+  cudaStream_t s = c->stream;
+  const int64_t nn = (int64_t)c->dimH * c->dimH;
+  const int npairs = (int)pairs.size(), len = 16 * npairs, sets = q ? 2 : 1;
+  h.assign(len, make_double2(0.0, 0.0));
+  if (hs) hs->assign(len, make_double2(0.0, 0.0));
+  if (npairs == 0) return TG_OK;
+  GreenArgs a;
+  int rc = imag_points(c, Ef, eta, true, a);
+  if (rc) return rc;
+  GreenArgs b = a;   // the points of G(k - q)
+  if (q) {
+    const double mq[3] = {-q[0], -q[1], -q[2]};
+    if (a.htab) {
+      if ((rc = build_htab(c, 1, c->d_klist_u.p, c->nk_u, mq))) return rc;
+      b.htab = c->d_htab[1].p;
+    } else {
+      for (int i = 0; i < 3; ++i) b.q[i] = mq[i];
+    }
+  }
+  const int64_t P = pass_size(c, c->n_imag, (int64_t)1 << 30);
+  const size_t parts = pair_partials(c->dimH, npairs, q != nullptr, c->num_sms, P);
+  TG_CHECK(c, c->d_gg_desc.upload(reinterpret_cast<const int*>(pairs.data()), 4 * pairs.size(), s), "upload pairs");
+  const int4* dp = reinterpret_cast<const int4*>(c->d_gg_desc.p);
+  TG_CHECK(c, c->d_A.ensure((size_t)P * nn), "alloc G");
+  if (q) TG_CHECK(c, c->d_B.ensure((size_t)P * nn), "alloc G");
+  TG_CHECK(c, c->d_acc.ensure(sets * parts * len), "alloc acc");
+  TG_CHECK(c, c->d_acc_red.ensure((size_t)sets * len), "alloc acc");
+  TG_CHECK(c, cudaMemsetAsync(c->d_acc.p, 0, sizeof(double2) * sets * parts * len, s), "memset");
+  if ((rc = reset_status(c))) return rc;
+  profile_begin(c);
+  a.mode = b.mode = MODE_RAW;
+  a.out = c->d_A.p;
+  b.out = q ? c->d_B.p : c->d_A.p;
+  for (int64_t p0 = 0; p0 < c->n_imag; p0 += P) {
+    a.p0 = b.p0 = p0;
+    a.np = b.np = std::min<int64_t>(P, c->n_imag - p0);
+    {
+      KindTimer kt(c, 0);
+      TG_CHECK(c, launch_green(a, c->num_sms, s, nullptr), "green (k)");
+    }
+    if (q) {
+      KindTimer kt(c, 0);
+      TG_CHECK(c, launch_green(b, c->num_sms, s, nullptr), "green (k - q)");
+    }
+    KindTimer kt(c, 1);
+    for (int x = 0; x < sets; ++x) {
+      c->launches += 1;
+      TG_CHECK(c, launch_pairs(a, x ? b.out : a.out, x ? a.out : b.out, dp, npairs, c->num_sms,
+                               c->d_acc.p + x * parts * len, s),
+               "pair sums");
+    }
+  }
+  for (int x = 0; x < sets; ++x) {
+    KindTimer kt(c, 2);
+    TG_CHECK(c, launch_reduce_blocks(c->d_acc.p + x * parts * len, (int)parts, len, c->d_acc_red.p + (size_t)x * len, s),
+             "reduce");
+  }
+  TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_acc_red.p, sizeof(double2) * len, cudaMemcpyDeviceToHost, s), "copy");
+  if (hs && q)
+    TG_CHECK(c, cudaMemcpyAsync(hs->data(), c->d_acc_red.p + len, sizeof(double2) * len, cudaMemcpyDeviceToHost, s),
+             "copy");
+  profile_end(c);
+  return read_status(c);
+}
+
+}  // namespace
+
+extern "C" {
+
 int tg_expectation(tg_ctx* c, double Ef, double eta, double* rho, double* mx, double* my, double* mz, double* mp) {
   int rc = check_ready(c, true, false);
   if (rc) return rc;
@@ -1935,7 +2066,7 @@ int tg_expectation(tg_ctx* c, double Ef, double eta, double* rho, double* mx, do
   a.zr = Ef;
   a.zi = eta;
   a.mode = MODE_EXPECT;
-  a.gg_desc = c->d_exp_rows.p;
+  a.exp_rows = c->d_exp_rows.p;
   if (c->imag_uniform && (int64_t)c->nk_u * c->dimH * c->dimH * 16 <= ((int64_t)8 << 30)) {
     const double zero3[3] = {0.0, 0.0, 0.0};
     if ((rc = build_htab(c, 0, c->d_klist_u.p, c->nk_u, zero3))) return rc;
@@ -1944,11 +2075,10 @@ int tg_expectation(tg_ctx* c, double Ef, double eta, double* rho, double* mx, do
     a.nk_tab = c->nk_u;
     a.ylist = c->d_ylist.p;
   }
-  const int maxgrid = c->num_sms * 8;
+  const int maxgrid = c->num_sms * (kGreenMaxCtas + 1);
   TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * len), "alloc acc");
   TG_CHECK(c, c->d_acc_red.ensure(len), "alloc acc");
   a.acc = c->d_acc.p;
-  a.acc_len = 0;   // EXPECT keeps its sums in registers
   rc = reset_status(c);
   if (rc) return rc;
   int grid = 0;
@@ -2002,7 +2132,6 @@ int tg_gg_tensor(tg_ctx* c, double Ef, double eta, int orbital_resolved, const i
   if ((rc = require_native(c, "tg_gg_tensor"))) return rc;
   if (!T || (orbital_resolved && !dmask)) return set_err(c, TG_ERR_ARG, "tg_gg_tensor: null argument");
   cudaSetDevice(c->device);
-  cudaStream_t s = c->stream;
   const int nat = c->n_atoms;
   // groups per site
   std::vector<std::vector<std::vector<int>>> rowg(nat), colg(nat);
@@ -2030,79 +2159,29 @@ int tg_gg_tensor(tg_ctx* c, double Ef, double eta, int orbital_resolved, const i
     nrow = std::max<int>(nrow, (int)rowg[i].size());
     ncol = std::max<int>(ncol, (int)colg[i].size());
   }
-  // descriptors: per block (i, g, j, h) in output order T(16, ncol, nrow, j, i)
-  std::vector<int> desc, lists;
-  std::vector<int> block_of;   // output slot per descriptor block
-  int nblocks = 0;
-  std::vector<int> list_off;
-  auto add_list = [&](const std::vector<int>& l) {
-    const int off = (int)lists.size();
-    lists.push_back((int)l.size());
-    for (int x : l) lists.push_back(x);
-    return off;
-  };
+  // every orbital pair (row orbital of any site, column orbital of any site) is summed on the
+  // device; the groups of several orbitals are added up here
+  std::vector<PairRef> refs;
+  std::vector<int4> pairs;
   for (int i = 0; i < nat; ++i)
     for (int j = 0; j < nat; ++j)
-      for (int g = 0; g < (int)rowg[i].size(); ++g)
-        for (int h = 0; h < (int)colg[j].size(); ++h) {
-          desc.push_back(c->ia[i]);
-          desc.push_back(c->ia[i] + c->norb[i]);
-          desc.push_back(c->ia[j]);
-          desc.push_back(c->ia[j] + c->norb[j]);
-          desc.push_back(-1);
-          desc.push_back(-1);
-          block_of.push_back(((i * nat + j) * nrow + g) * ncol + h);
-          ++nblocks;
-        }
-  // list offsets (relative to the list area start)
-  {
-    int b = 0;
-    for (int i = 0; i < nat; ++i)
-      for (int j = 0; j < nat; ++j)
-        for (int g = 0; g < (int)rowg[i].size(); ++g)
-          for (int h = 0; h < (int)colg[j].size(); ++h) {
-            desc[6 * b + 4] = add_list(rowg[i][g]);
-            desc[6 * b + 5] = add_list(colg[j][h]);
-            ++b;
-          }
-  }
-  std::vector<int> all(desc);
-  all.insert(all.end(), lists.begin(), lists.end());
-  TG_CHECK(c, c->d_gg_desc.upload(all.data(), all.size(), s), "upload gg desc");
-  const int acc_len = 16 * nblocks;
-  GreenArgs a = base_args(c);
-  a.pts.kind = 0;
-  a.pts.y = c->d_y.p;
-  a.pts.kp = c->d_kp.p;
-  a.pts.w = c->d_w.p;
-  a.np = c->n_imag;
-  a.zr = Ef;
-  a.zi = eta;
-  a.mode = MODE_GG;
-  a.gg_desc = c->d_gg_desc.p;
-  a.acc_len = acc_len;
-  const int maxgrid = c->num_sms * 8;
-  TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * acc_len), "alloc acc");
-  TG_CHECK(c, c->d_acc_red.ensure(acc_len), "alloc acc");
-  a.acc = c->d_acc.p;
-  rc = reset_status(c);
-  if (rc) return rc;
-  int grid = 0;
-  cudaError_t e = launch_green(a, c->num_sms, s, &grid);
-  if (e == cudaErrorInvalidValue) return set_err(c, TG_ERR_ARG, "tg_gg_tensor: accumulator does not fit in shared memory");
-  TG_CHECK(c, e, "green (gg)");
-  TG_CHECK(c, launch_reduce_blocks(c->d_acc.p, grid, acc_len, c->d_acc_red.p, s), "reduce");
-  std::vector<double2> h(acc_len);
-  TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_acc_red.p, sizeof(double2) * acc_len, cudaMemcpyDeviceToHost, s), "copy");
-  rc = read_status(c);
-  if (rc) return rc;
+      for (int h = 0; h < (int)colg[j].size(); ++h)
+        for (int nu : colg[j][h])
+          for (int g = 0; g < (int)rowg[i].size(); ++g)
+            for (int mu : rowg[i][g]) {
+              pairs.push_back(make_int4(c->ia[i] + mu, c->ia[i] + c->norb[i] + mu, c->ia[j] + nu,
+                                        c->ia[j] + c->norb[j] + nu));
+              refs.push_back(PairRef{((i * nat + j) * nrow + g) * ncol + h});
+            }
+  std::vector<double2> h;
+  if ((rc = imag_pairs(c, Ef, eta, nullptr, pairs, h, nullptr))) return rc;
   const size_t total = (size_t)nat * nat * nrow * ncol * 16;
   std::memset(T, 0, sizeof(double) * 2 * total);
-  for (int b = 0; b < nblocks; ++b)
+  for (size_t b = 0; b < refs.size(); ++b)
     for (int q = 0; q < 16; ++q) {
-      const size_t dst = (size_t)block_of[b] * 16 + q;
-      T[2 * dst] = h[16 * b + q].x;
-      T[2 * dst + 1] = h[16 * b + q].y;
+      const size_t dst = (size_t)refs[b].block * 16 + q;
+      T[2 * dst] += h[16 * b + q].x;
+      T[2 * dst + 1] += h[16 * b + q].y;
     }
   return TG_OK;
 }
@@ -2114,23 +2193,19 @@ int tg_fermi_column(tg_ctx* c, double Ef, double eta, double* D) {
   if (!D) return set_err(c, TG_ERR_ARG, "tg_fermi_column: null output");
   cudaSetDevice(c->device);
   cudaStream_t s = c->stream;
-  const int n = c->dimH;
-  const int acc_len = 2 * n;   // 4 per orbital
   double one = 1.0, ef = Ef;
   TG_CHECK(c, c->d_x2.upload(&ef, 1, s), "upload");
   TG_CHECK(c, c->d_p2.upload(&one, 1, s), "upload");
-  TG_CHECK(c, c->d_gg_desc.upload(nullptr, 0, s), "upload");
-  std::vector<int> rows(n);
-  {
-    int o = 0;
-    for (int i = 0; i < c->n_atoms; ++i)
-      for (int mu = 0; mu < c->norb[i]; ++mu) {
-        rows[2 * o] = c->ia[i] + mu;
-        rows[2 * o + 1] = c->ia[i] + c->norb[i] + mu;
-        ++o;
-      }
-  }
-  TG_CHECK(c, c->d_gg_desc.upload(rows.data(), rows.size(), s), "upload");
+  // the spin blocks uu, dd, ud, du of every orbital's diagonal
+  std::vector<int2> ent;
+  for (int i = 0; i < c->n_atoms; ++i)
+    for (int mu = 0; mu < c->norb[i]; ++mu) {
+      const int u = c->ia[i] + mu, d = u + c->norb[i];
+      ent.push_back(make_int2(u, u));
+      ent.push_back(make_int2(d, d));
+      ent.push_back(make_int2(u, d));
+      ent.push_back(make_int2(d, u));
+    }
   GreenArgs a = base_args(c);
   a.pts.kind = 1;
   a.pts.kp = c->d_rkp.p;
@@ -2138,25 +2213,17 @@ int tg_fermi_column(tg_ctx* c, double Ef, double eta, double* D) {
   a.pts.x2 = c->d_x2.p;
   a.pts.p2 = c->d_p2.p;
   a.pts.nk = c->n_realk;
-  a.np = c->n_realk;
   a.zr = 0.0;
   a.zi = eta;
-  a.mode = MODE_DIAG4;
-  a.gg_desc = c->d_gg_desc.p;
-  a.acc_len = acc_len;
-  const int maxgrid = c->num_sms * 8;
-  TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * acc_len), "alloc acc");
-  TG_CHECK(c, c->d_acc_red.ensure(acc_len), "alloc acc");
-  a.acc = c->d_acc.p;
-  rc = reset_status(c);
-  if (rc) return rc;
-  int grid = 0;
-  TG_CHECK(c, launch_green(a, c->num_sms, s, &grid), "green (fermi column)");
-  TG_CHECK(c, launch_reduce_blocks(c->d_acc.p, grid, acc_len, c->d_acc_red.p, s), "reduce");
-  std::vector<double2> h(acc_len);
-  TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_acc_red.p, sizeof(double2) * acc_len, cudaMemcpyDeviceToHost, s), "copy");
-  rc = read_status(c);
-  if (rc) return rc;
+  std::vector<double2> g, h(ent.size());
+  if ((rc = entry_sums(c, a, c->n_realk, ent, g, "green (fermi column)"))) return rc;
+  for (size_t o = 0; o + 3 < g.size(); o += 4) {   // traces with 1, sigma_x, sigma_y, sigma_z
+    const double2 uu = g[o], dd = g[o + 1], ud = g[o + 2], du = g[o + 3];
+    h[o] = cadd(uu, dd);
+    h[o + 1] = cadd(du, ud);
+    h[o + 2] = cmul(make_double2(0.0, 1.0), csub(ud, du));
+    h[o + 3] = csub(uu, dd);
+  }
   // D(4, norb_max, n_atoms); orbital counter o runs over the sites' orbitals
   int o = 0;
   for (int i = 0; i < c->n_atoms; ++i) {
@@ -2401,70 +2468,27 @@ int tg_jij(tg_ctx* c, const double* q, double Ef, double eta, const double* evec
   if ((rc = require_native(c, "tg_jij"))) return rc;
   if (!q || !evec || !Um || !dmask || !J) return set_err(c, TG_ERR_ARG, "tg_jij: null argument");
   cudaSetDevice(c->device);
-  cudaStream_t s = c->stream;
-  const int n = c->dimH, nat = c->n_atoms, nmax = c->nmax;
-  const int64_t nn = (int64_t)n * n;
-  // d-orbital lists: tab = [dstart (nat + 1) | dlist]
-  std::vector<int> tab(nat + 1, 0);
-  for (int i = 0; i < nat; ++i) {
-    int cnt = 0;
-    for (int o = 0; o < c->norb[i]; ++o)
-      if (dmask[(size_t)i * nmax + o]) {
-        tab.push_back(o);
-        ++cnt;
-      }
-    tab[i + 1] = tab[i] + cnt;
-  }
-  TG_CHECK(c, c->d_jij_tab.upload(tab.data(), tab.size(), s), "upload d orbitals");
-  TG_CHECK(c, c->d_ia.upload(c->ia.data(), c->ia.size(), s), "upload ia");
-  const int len = nat * nat * 32;
-  const int grid = c->num_sms * 4;
-  TG_CHECK(c, c->d_jij_part.ensure((size_t)grid * len), "alloc partials");
-  TG_CHECK(c, c->d_jij_sum.ensure((size_t)len), "alloc");
-  TG_CHECK(c, cudaMemsetAsync(c->d_jij_part.p, 0, sizeof(double2) * (size_t)grid * len, s), "memset");
-  const int64_t P = pass_size(c, c->n_imag);
-  TG_CHECK(c, c->d_A.ensure((size_t)P * nn), "alloc");
-  TG_CHECK(c, c->d_B.ensure((size_t)P * nn), "alloc");
-  if ((rc = reset_status(c))) return rc;
-  profile_begin(c);
-  for (int64_t p0 = 0; p0 < c->n_imag; p0 += P) {
-    GreenArgs g = base_args(c);
-    g.pts.kind = 0;
-    g.pts.y = c->d_y.p;
-    g.pts.kp = c->d_kp.p;
-    g.pts.w = c->d_w.p;
-    g.p0 = p0;
-    g.np = std::min<int64_t>(P, c->n_imag - p0);
-    g.zr = Ef;
-    g.zi = eta;
-    g.mode = MODE_RAW;
-    g.out = c->d_A.p;
-    {
-      KindTimer kt(c, 0);
-      TG_CHECK(c, launch_green(g, c->num_sms, s, nullptr), "green (k)");
+  const int nat = c->n_atoms, nmax = c->nmax;
+  // pairs of d orbitals of every two sites
+  std::vector<int4> pairs;
+  std::vector<int> site;
+  for (int i = 0; i < nat; ++i)
+    for (int j = 0; j < nat; ++j)
+      for (int be = 0; be < c->norb[j]; ++be)
+        for (int al = 0; al < c->norb[i]; ++al) {
+          if (!dmask[(size_t)i * nmax + al] || !dmask[(size_t)j * nmax + be]) continue;
+          pairs.push_back(make_int4(c->ia[i] + al, c->ia[i] + c->norb[i] + al, c->ia[j] + be,
+                                    c->ia[j] + c->norb[j] + be));
+          site.push_back(i * nat + j);
+        }
+  std::vector<double2> hp, hq, h((size_t)nat * nat * 32, make_double2(0.0, 0.0));
+  if ((rc = imag_pairs(c, Ef, eta, q, pairs, hp, &hq))) return rc;
+  for (size_t b = 0; b < site.size(); ++b)
+    for (int x = 0; x < 16; ++x) {
+      double2* t = h.data() + (size_t)site[b] * 32;
+      t[x] = cadd(t[x], hp[16 * b + x]);
+      t[16 + x] = cadd(t[16 + x], hq[16 * b + x]);
     }
-    g.q[0] = -q[0];
-    g.q[1] = -q[1];
-    g.q[2] = -q[2];
-    g.out = c->d_B.p;
-    {
-      KindTimer kt(c, 0);
-      TG_CHECK(c, launch_green(g, c->num_sms, s, nullptr), "green (k - q)");
-    }
-    KindTimer kt(c, 1);
-    c->launches += 1;
-    TG_CHECK(c, launch_jij(c->d_A.p, c->d_B.p, p0, g.np, c->d_w.p, n, nat, c->d_ia.p, c->d_norb.p, c->d_jij_tab.p,
-                           c->d_jij_tab.p + (nat + 1), c->d_jij_part.p, grid, s),
-             "jij tensors");
-  }
-  {
-    KindTimer kt(c, 2);
-    TG_CHECK(c, launch_reduce_blocks(c->d_jij_part.p, grid, len, c->d_jij_sum.p, s), "reduce");
-  }
-  std::vector<double2> h(len);
-  TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_jij_sum.p, sizeof(double2) * len, cudaMemcpyDeviceToHost, s), "copy");
-  profile_end(c);
-  if ((rc = read_status(c))) return rc;
   // sigma_a[s][s'] (0 = up), a = x, y, z
   const double2 sig[3][2][2] = {{{{0, 0}, {1, 0}}, {{1, 0}, {0, 0}}},
                                 {{{0, 0}, {0, -1}}, {{0, 1}, {0, 0}}},
@@ -2512,9 +2536,7 @@ int tg_smunu(tg_ctx* c, double Ef, double eta, double* S) {
   if (rc) return rc;
   if ((rc = require_native(c, "tg_smunu"))) return rc;
   if (!S) return set_err(c, TG_ERR_ARG, "tg_smunu: null output");
-  if (!green_supported(c->dimH)) return set_err(c, TG_ERR_ARG, "tg_smunu: dimH has no accumulating kernel");
   cudaSetDevice(c->device);
-  cudaStream_t s = c->stream;
   const int nat = c->n_atoms, nmax = c->nmax;
   // entries (r, c) of every on-site block, site by site, row-major inside the 2n x 2n block
   std::vector<int> desc, site_off(nat + 1, 0);
@@ -2527,31 +2549,12 @@ int tg_smunu(tg_ctx* c, double Ef, double eta, double* S) {
       }
     site_off[i + 1] = site_off[i] + n2 * n2;
   }
-  const int acc_len = site_off[nat];
-  TG_CHECK(c, c->d_gg_desc.upload(desc.data(), desc.size(), s), "upload");
-  GreenArgs a = base_args(c);
-  a.pts.kind = 0;
-  a.pts.y = c->d_y.p;
-  a.pts.kp = c->d_kp.p;
-  a.pts.w = c->d_w.p;
-  a.np = c->n_imag;
-  a.zr = Ef;
-  a.zi = eta;
-  a.mode = MODE_ENTRIES;
-  a.gg_desc = c->d_gg_desc.p;
-  a.acc_len = acc_len;
-  const int maxgrid = green_acc_ctas(c->dimH, c->n_imag, c->num_sms);
-  TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * acc_len), "alloc acc");
-  TG_CHECK(c, c->d_acc_red.ensure(acc_len), "alloc acc");
-  a.acc = c->d_acc.p;
-  c->gg_mode = -1;   // the entry list replaced the GG descriptors
-  if ((rc = reset_status(c))) return rc;
-  int grid = 0;
-  TG_CHECK(c, launch_green(a, c->num_sms, s, &grid), "green (on-site blocks)");
-  TG_CHECK(c, launch_reduce_blocks(c->d_acc.p, grid, acc_len, c->d_acc_red.p, s), "reduce");
-  std::vector<double2> h(acc_len);
-  TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_acc_red.p, sizeof(double2) * acc_len, cudaMemcpyDeviceToHost, s), "copy");
-  if ((rc = read_status(c))) return rc;
+  std::vector<int2> ent;
+  for (size_t e = 0; e + 1 < desc.size(); e += 2) ent.push_back(make_int2(desc[e], desc[e + 1]));
+  GreenArgs a;
+  if ((rc = imag_points(c, Ef, eta, true, a))) return rc;
+  std::vector<double2> h;
+  if ((rc = entry_sums(c, a, c->n_imag, ent, h, "green (on-site blocks)"))) return rc;
   // calcSmunu: imgXY(mu, nu) = (A(nu X, mu Y) + conj(A(mu Y, nu X))) / 2 pi, 1/2 on the uu / dd diagonals
   const double tpi = 2.0 * kPi;
   std::fill(S, S + (size_t)2 * nmax * nmax * 3 * nat, 0.0);
@@ -2588,7 +2591,6 @@ int tg_gs_orbital(tg_ctx* c, double Ef, double eta, double* gupgd) {
   if ((rc = require_native(c, "tg_gs_orbital"))) return rc;
   if (!gupgd) return set_err(c, TG_ERR_ARG, "tg_gs_orbital: null output");
   cudaSetDevice(c->device);
-  cudaStream_t s = c->stream;
   const int nat = c->n_atoms, nmax = c->nmax;
   // entries (i mu s, i nu s) of the two spin-diagonal blocks of every site: s = up, then down
   std::vector<int> desc, site_off(nat + 1, 0);
@@ -2602,31 +2604,12 @@ int tg_gs_orbital(tg_ctx* c, double Ef, double eta, double* gupgd) {
         }
     site_off[i + 1] = site_off[i] + 2 * n * n;
   }
-  const int acc_len = site_off[nat];
-  TG_CHECK(c, c->d_gg_desc.upload(desc.data(), desc.size(), s), "upload");
-  GreenArgs a = base_args(c);
-  a.pts.kind = 0;
-  a.pts.y = c->d_y.p;
-  a.pts.kp = c->d_kp.p;
-  a.pts.w = c->d_w.p;
-  a.np = c->n_imag;
-  a.zr = Ef;
-  a.zi = eta;
-  a.mode = MODE_ENTRIES;
-  a.gg_desc = c->d_gg_desc.p;
-  a.acc_len = acc_len;
-  const int maxgrid = green_acc_ctas(c->dimH, c->n_imag, c->num_sms);
-  TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * acc_len), "alloc acc");
-  TG_CHECK(c, c->d_acc_red.ensure(acc_len), "alloc acc");
-  a.acc = c->d_acc.p;
-  c->gg_mode = -1;   // the entry list replaced the GG descriptors
-  if ((rc = reset_status(c))) return rc;
-  int grid = 0;
-  TG_CHECK(c, launch_green(a, c->num_sms, s, &grid), "green (on-site spin blocks)");
-  TG_CHECK(c, launch_reduce_blocks(c->d_acc.p, grid, acc_len, c->d_acc_red.p, s), "reduce");
-  std::vector<double2> h(acc_len);
-  TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_acc_red.p, sizeof(double2) * acc_len, cudaMemcpyDeviceToHost, s), "copy");
-  if ((rc = read_status(c))) return rc;
+  std::vector<int2> ent;
+  for (size_t e = 0; e + 1 < desc.size(); e += 2) ent.push_back(make_int2(desc[e], desc[e + 1]));
+  GreenArgs a;
+  if ((rc = imag_points(c, Ef, eta, true, a))) return rc;
+  std::vector<double2> h;
+  if ((rc = entry_sums(c, a, c->n_imag, ent, h, "green (on-site spin blocks)"))) return rc;
   // gupgd(nu, mu, i) = (1/pi) sum w (G(i mu up, i nu up) + G(i mu dn, i nu dn))  (mod_expectation.F90:957-975)
   std::fill(gupgd, gupgd + (size_t)2 * nmax * nmax * nat, 0.0);
   for (int i = 0; i < nat; ++i) {
@@ -2834,7 +2817,7 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
   // Im z >= 10 eta (its eps |H| / Im z error is negligible there; the nanoribbon goldens
   // hold with the split at 10 eta), the one-warp Gauss-Jordan kernel below and on the real axis
   const bool hybrid = !spec && c->green_method == TG_GREEN_AUTO && tab_imag && eig_supported(n) &&
-                      green_w1_supported(n, MODE_RAW);
+                      n == 36 && green_mma_supported(n, MODE_RAW);
   const double y_split = 10.0 * eta;
   if ((spec || hybrid) && (tab_imag || tab_real) && (rc = reset_eig_status(c))) return rc;
   auto tables = [&](int slot, const double* d_k, int64_t nk, bool shift) -> int {
@@ -3083,9 +3066,8 @@ extern "C" int tg_expectation_noalloc(tg_ctx* c, double Ef, double eta, double* 
   a.zr = Ef;
   a.zi = eta;
   a.mode = MODE_EXPECT;
-  a.gg_desc = c->d_exp_rows.p;
+  a.exp_rows = c->d_exp_rows.p;
   a.acc = partial;
-  a.acc_len = 0;
   rc = reset_status(c);
   if (rc) return rc;
   int grid = 0;

@@ -10,7 +10,7 @@
 // (eintshechi.F90:146-164).  The chi element is then picked out of C in the
 // epilogue (chi = C_ij + conj(C_ji) with permuted indices, Fint = -i D_ij).
 // This file holds the FP64 SIMT GEMM (the plain-precision GPU path), the
-// chi assembly epilogue and a block-partial reduction.
+// chi assembly epilogue.
 #include "tg_internal.cuh"
 
 #include <algorithm>
@@ -149,14 +149,6 @@ __global__ void chi_epilogue_kernel(const double2* __restrict__ Cpart, const dou
   }
 }
 
-__global__ void reduce_blocks_kernel(const double2* __restrict__ part, int nblocks, int len, double2* __restrict__ out) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < len; e += gridDim.x * blockDim.x) {
-    double2 s = make_double2(0, 0);
-    for (int b = 0; b < nblocks; ++b) s = cadd(s, part[(int64_t)b * len + e]);
-    out[e] = s;
-  }
-}
-
 }  // namespace
 
 cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit,
@@ -181,14 +173,6 @@ cudaError_t launch_chi_epilogue(const double2* Cpart, const double2* Dpart, int 
   int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
   chi_epilogue_kernel<<<blocks, 256, 0, s>>>(Cpart, Dpart, nsplit, cstride, dimens, decode, norb, pair_coff,
                                              n_atoms, scale, chi);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_reduce_blocks(const double2* part, int nblocks, int len, double2* out, cudaStream_t s) {
-  int blocks = (len + 255) / 256;
-  if (blocks > 1024) blocks = 1024;
-  if (blocks < 1) blocks = 1;
-  reduce_blocks_kernel<<<blocks, 256, 0, s>>>(part, nblocks, len, out);
   return cudaGetLastError();
 }
 

@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
       }
     } else if (OUT == 1) {
       for (int o = tl; o < N / 2; o += LANES) {
-        const int ru = a.gg_desc[2 * o], rd = a.gg_desc[2 * o + 1];
+        const int ru = a.exp_rows[2 * o], rd = a.exp_rows[2 * o + 1];
         eacc[4 * o + 0] = cadd(eacc[4 * o + 0], cscale(X[piv[ru] * N + pinv[ru]], w));
         eacc[4 * o + 1] = cadd(eacc[4 * o + 1], cscale(X[piv[rd] * N + pinv[rd]], w));
         eacc[4 * o + 2] = cadd(eacc[4 * o + 2], cscale(X[piv[ru] * N + pinv[rd]], w));
@@ -409,8 +409,7 @@ cudaError_t launch_t(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_
 
 // Team-per-matrix path: raw / operand / expectation / H(k) modes.
 int green_warp_supported(int n, int mode) {
-  const bool nok = (n == 4 || n == 8 || n == 16 || n == 18 || n == 20 || n == 36 || n == 40 || n == 54 ||
-                    n == 72 || n == 90);
+  const bool nok = n == 4 || n == 8 || n == 16 || n == 20;
   const bool mok = mode == MODE_RAW || mode == MODE_A_IMAG || mode == MODE_B_IMAG || mode == MODE_A_REAL ||
                    mode == MODE_B_REAL || mode == MODE_EXPECT || mode == MODE_HK;
   return nok && mok;
@@ -425,13 +424,7 @@ cudaError_t launch_green_warp(const GreenArgs& a, int num_sms, cudaStream_t s, i
     case 4: return launch_t<4, 1, 8>(a, num_sms, s, grid_used);
     case 8: return launch_t<8, 1, 8>(a, num_sms, s, grid_used);
     case 16: return launch_t<16, 1, 8>(a, num_sms, s, grid_used);
-    case 18: return launch_t<18, 1, 8>(a, num_sms, s, grid_used);
     case 20: return launch_t<20, 1, 8>(a, num_sms, s, grid_used);
-    case 36: return launch_t<36, 2, 8>(a, num_sms, s, grid_used);
-    case 40: return launch_t<40, 2, 8>(a, num_sms, s, grid_used);
-    case 54: return launch_t<54, 4, 16>(a, num_sms, s, grid_used);
-    case 72: return launch_t<72, 8, 16>(a, num_sms, s, grid_used);
-    case 90: return launch_t<90, 8, 16>(a, num_sms, s, grid_used);
   }
   return cudaErrorInvalidValue;
 }

@@ -80,10 +80,7 @@ enum GreenMode : int {
   MODE_A_REAL = 3,    // w * (G - G^dagger), pair-block layout
   MODE_B_REAL = 4,    // conj(G), pair-block layout
   MODE_EXPECT = 5,    // accumulate diagonal site blocks (occupations / moments)
-  MODE_GG = 6,        // accumulate the orbital-diagonal GG tensor (Jacobian)
-  MODE_DIAG4 = 7,     // accumulate w * sigma-traces of diagonal orbitals (Fermi column)
-  MODE_HK = 8,        // H(k) only (no inversion), column-major per point
-  MODE_ENTRIES = 9,   // accumulate w * G(r_e, c_e) for a list of entries (gg_desc pairs, acc_len of them)
+  MODE_HK = 6,        // H(k) only (no inversion), column-major per point
 };
 
 // A set of (k, z) points.  kind 0: flattened imaginary-axis list (y, kp, w per
@@ -124,9 +121,8 @@ struct GreenArgs {
   double2* out2 = nullptr;           // optional second operand from the same inverse
   int mode2 = MODE_RAW;
   const int* outmap = nullptr;       // [n*n] row*n + col of pair-block slot o
-  double2* acc = nullptr;            // per-CTA accumulators (EXPECT / GG / DIAG4)
-  int acc_len = 0;                   // complex entries per CTA
-  const int* gg_desc = nullptr;      // GG entry descriptors
+  double2* acc = nullptr;            // MODE_EXPECT: per-CTA sums, 2 n complex each
+  const int* exp_rows = nullptr;     // MODE_EXPECT: up / down row of every orbital
   int* status = nullptr;             // first singular point (1-based), atomicMin
   // optional precomputed H(k) table (row-major n x n per k) with a k-major
   // traversal: work item wi -> k index wi / n_e, energy index wi % n_e
@@ -153,7 +149,7 @@ struct GreenArgs {
   int16_t* eout = nullptr;
   int16_t* eout2 = nullptr;
   // energy split of a tabulated imaginary-axis pass: y_side = +1 keeps the points with
-  // Im z >= y_split (spectral kernel), -1 those below (one-warp Gauss-Jordan kernel); other
+  // Im z >= y_split (spectral kernel), -1 those below (blocked Gauss-Jordan kernel); other
   // kernels ignore it and evaluate every point
   double y_split = 0.0;
   int y_side = 0;
@@ -173,14 +169,38 @@ cudaError_t launch_green(const GreenArgs& a, int num_sms, cudaStream_t s, int* g
 int green_supported(int n);
 int green_warp_supported(int n, int mode);
 cudaError_t launch_green_warp(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used);
-int green_w1_supported(int n, int mode);
-cudaError_t launch_green_w1(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used);
-int green_acc_ctas(int n, int64_t np, int num_sms);
+// blocked Gauss-Jordan on the FP64 tensor cores (dimensions 18, 36, 40, 54, 72, 90): one CTA per
+// matrix, at most kGreenMaxCtas CTAs per SM (per-CTA partial sums of MODE_EXPECT)
+constexpr int kGreenMaxCtas = 15;
+int green_mma_supported(int n, int mode);
+cudaError_t launch_green_mma(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used);
 // any dimension up to 288, MODE_RAW only: one thread-block cluster per matrix
 int green_cluster_supported(int n, int mode);
 int green_cluster_size(int n);
 size_t green_cluster_ws_bytes(int n, int num_sms);
 cudaError_t launch_green_cluster(const GreenArgs& a, int num_sms, cudaStream_t s);
+
+// weight of point pl of a pass: k-major (an H(k) table or its decompositions) or mesh order
+__device__ __forceinline__ double point_weight(const GreenArgs& g, int64_t pl) {
+  const int64_t wi = g.p0 + pl;
+  if (g.htab || g.eigU || g.triQ) {
+    const int64_t ik = wi / g.n_e, ie = wi % g.n_e;
+    return g.pts.kind == 0 ? g.pts.w[ie * g.nk_tab + ik] : g.pts.p2[ie] * g.pts.w[ik];
+  }
+  if (g.pts.kind == 0) return g.pts.w[wi];
+  if (g.pts.kind == 1) return g.pts.p2[wi / g.pts.nk] * g.pts.w[wi % g.pts.nk];
+  return 1.0;
+}
+
+// Weighted sums over the column-major Green functions of a pass, added into per-CTA slices of
+// acc: products of the spin blocks of orbital pairs (16 sums each, rows (a up, a down, b up,
+// b down) per pair; pair_partials slices), and single entries (row, column) (entry_partials)
+size_t pair_partials(int n, int npairs, bool two, int num_sms, int64_t np);
+cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* Gb, const int4* pairs, int npairs,
+                         int num_sms, double2* acc, cudaStream_t s);
+int entry_partials(int64_t np, int num_sms);
+cudaError_t launch_entries(const GreenArgs& g, const double2* G, const int2* entries, int ne, int num_sms,
+                           double2* acc, cudaStream_t s);
 
 // FP64 pair-block contraction: Cpart[split][cpair_off + u*M + v] += sum_p A[p][off+u] B[p][off+v]
 struct PairTile { int pair; int u0; int v0; };
@@ -242,11 +262,6 @@ __device__ __forceinline__ int16_t exponent_code16(double2 v) {
   const int f = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
   return f == 0 ? (int16_t)-32768 : (int16_t)(f - 1022);
 }
-
-// Exchange coupling: d-orbital GG tensors T(G(k), G(k - q)) and T(G(k - q), G(k)) per site pair
-cudaError_t launch_jij(const double2* Ga, const double2* Gb, int64_t p0, int64_t np, const double* w, int n,
-                       int n_atoms, const int* ia, const int* norb, const int* dstart, const int* dlist,
-                       double2* partial, int grid, cudaStream_t s);
 
 // Disturbance-response vertex (eintshe): one launch per pass over RAW G1 / G2
 struct SheLaunch {

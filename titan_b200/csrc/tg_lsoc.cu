@@ -106,18 +106,7 @@ __global__ void gather_kernel(GreenArgs g, const double2* __restrict__ G, int mo
     const int rc = outmap[o];
     const int r = rc / n, c = rc - r * n;
     const double2* gp = G + pl * nn;
-    const int64_t wi = g.p0 + pl;
-    double w;
-    if (g.htab || g.eigU || g.triQ) {   // k-major: an H(k) table, or its decompositions
-      const int64_t ik = wi / g.n_e, ie = wi % g.n_e;
-      w = g.pts.kind == 0 ? g.pts.w[ie * g.nk_tab + ik] : g.pts.p2[ie] * g.pts.w[ik];
-    } else if (g.pts.kind == 0) {
-      w = g.pts.w[wi];
-    } else if (g.pts.kind == 1) {
-      w = g.pts.p2[wi / g.pts.nk] * g.pts.w[wi % g.pts.nk];
-    } else {
-      w = 1.0;
-    }
+    const double w = point_weight(g, pl);
     const double2 grc = gp[(int64_t)c * n + r];
     double2 v;
     if (mode == MODE_A_IMAG) {
