@@ -81,3 +81,25 @@ def test_pair_sums_of_larger_cells(gpu, shape, nk):
     q = np.array([0.1, -0.05, 0.0])
     J, Jr = gpu.jij(q, s.Ef, s.eta, ev, s.Um()), O.jij(m, ek, q, s.Ef, s.eta, ev, s.Um(), s.dorbs)
     assert np.max(np.abs(J - Jr)) <= tol * np.max(np.abs(Jr))
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 63, 64, 65, 72, 129])
+@pytest.mark.parametrize("order", ["C", "F"])
+def test_dyson_at_the_edges_of_its_panels(gpu, n, order):
+    """Random chi and U: 1 + chi U has no dominant diagonal, so rows are exchanged in every
+    panel.  Two backward-stable solves differ by at most ~ n eps cond."""
+    rng = np.random.default_rng(n)
+    x, u = (np.asarray(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)), order=order) for _ in range(2))
+    got = gpu.dyson(x, u)
+    M = np.eye(n) + x @ u
+    ref = np.linalg.solve(M, x)
+    assert np.linalg.norm(got - ref) <= 10.0 * n * EPS * np.linalg.cond(M) * np.linalg.norm(ref)
+
+
+def test_dyson_reports_a_singular_system(gpu):
+    from titan_b200.native import TitanGPUError
+    x = np.eye(70, dtype=complex)
+    u = -np.eye(70, dtype=complex)
+    with pytest.raises(TitanGPUError) as err:
+        gpu.dyson(x, 0.5 * u - 0.5 * np.diag(np.arange(70) == 66))
+    assert err.value.code == 67

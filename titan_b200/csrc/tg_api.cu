@@ -23,8 +23,8 @@
 using namespace tg;
 
 namespace tg {
-int dyson_device(int n, const double2* chi_hf, const double2* U, double2* work, double2* chi, int* piv, int* status,
-                 cudaStream_t s);
+cudaError_t dyson_device(int n, const double2* chi_hf, const double2* U, double2* work, double2* chi, int* piv,
+                         int* status, cudaStream_t s);
 }
 
 namespace {
@@ -2692,8 +2692,7 @@ int tg_dyson(tg_ctx* c, int dimens, const double* chi_hf, const double* umat, do
   TG_CHECK(c, cudaMemcpyAsync(U, umat, sizeof(double2) * nn, cudaMemcpyHostToDevice, s), "upload");
   int rc = reset_status(c);
   if (rc) return rc;
-  if (dyson_device(dimens, X, U, W, R, c->d_piv.p, c->d_status.p, s) != 0)
-    return cuda_err(c, cudaGetLastError(), "dyson");
+  TG_CHECK(c, dyson_device(dimens, X, U, W, R, c->d_piv.p, c->d_status.p, s), "dyson");
   TG_CHECK(c, cudaMemcpyAsync(chi, R, sizeof(double2) * nn, cudaMemcpyDeviceToHost, s), "copy");
   return read_status(c);
 }
