@@ -159,6 +159,7 @@ struct tg_ctx {
   int green_method = 0;   // TG_GREEN_AUTO / TG_GREEN_GAUSS_JORDAN / TG_GREEN_SPECTRAL
   DevArray<double2> d_eigU[4];
   DevArray<double> d_eigL[4];
+  DevArray<unsigned char> d_eigws;   // rotations and tridiagonal matrices of launch_eig
   DevArray<double2> d_hchunk;   // bounded H(k) scratch of eigendecompositions built chunk by chunk
   DevArray<int> d_outinv, d_eig_status;
   DevArray<double> d_ldos_e, d_ldos;
@@ -378,8 +379,9 @@ int build_eig(tg_ctx* c, int slot, int64_t nk) {
   TG_CHECK(c, c->d_eigU[slot].ensure((size_t)nk * nn), "alloc eigenvectors");
   TG_CHECK(c, c->d_eigL[slot].ensure((size_t)nk * c->dimH), "alloc eigenvalues");
   KindTimer kt(c, 0);
-  TG_CHECK(c, launch_eig(c->d_htab[slot].p, nk, c->dimH, c->d_eigU[slot].p, c->d_eigL[slot].p, c->d_eig_status.p,
-                         c->num_sms, c->stream),
+  TG_CHECK(c, c->d_eigws.ensure(eig_ws_bytes(c->dimH, nk)), "alloc rotations");
+  TG_CHECK(c, launch_eig(c->d_htab[slot].p, nk, c->dimH, c->d_eigU[slot].p, c->d_eigL[slot].p, c->d_eigws.p,
+                         c->d_eig_status.p, c->num_sms, c->stream),
            "eigendecomposition");
   return TG_OK;
 }
@@ -395,6 +397,7 @@ int build_eig_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
   TG_CHECK(c, c->d_hchunk.ensure((size_t)kc * nn), "alloc H chunk");
   TG_CHECK(c, c->d_hphase.ensure((size_t)kc * std::max(c->n_neigh, 1)), "alloc phases");
   TG_CHECK(c, c->d_qvec.upload(q, 3, c->stream), "upload q");
+  TG_CHECK(c, c->d_eigws.ensure(eig_ws_bytes((int)n, kc)), "alloc rotations");
   const GreenArgs a = base_args(c);
   KindTimer kt(c, 0);
   for (int64_t k0 = 0; k0 < nk; k0 += kc) {
@@ -402,9 +405,9 @@ int build_eig_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
     TG_CHECK(c, launch_hk_table(a, d_k + 3 * k0, m, c->d_qvec.p, c->d_hphase.p, c->d_hchunk.p, c->stream),
              "H table");
     TG_CHECK(c, launch_eig(c->d_hchunk.p, m, (int)n, c->d_eigU[slot].p + k0 * nn, c->d_eigL[slot].p + k0 * n,
-                           c->d_eig_status.p, c->num_sms, c->stream),
+                           c->d_eigws.p, c->d_eig_status.p, c->num_sms, c->stream),
              "eigendecomposition");
-    c->launches += 3;
+    c->launches += 5;
   }
   return TG_OK;
 }
@@ -425,6 +428,8 @@ bool eig_room(tg_ctx* c, int64_t nk, int s0, int s1) {
   const size_t kc = std::min<size_t>((size_t)nk, std::max<size_t>(1, ((size_t)2 << 30) / (nn * 16)));
   if (c->d_hchunk.n < kc * nn) need += (double)(kc * nn - c->d_hchunk.n) * sizeof(double2);
   return need <= 0.5 * (double)fr;
+  const size_t ws = eig_ws_bytes(c->dimH, kc);
+  if (c->d_eigws.n < ws) need += (double)(ws - c->d_eigws.n);
 }
 
 // Householder tridiagonalisation of H(k + q) for a k list into slot `slot`: T and the rows
@@ -485,7 +490,7 @@ int read_eig_status(tg_ctx* c) {
   TG_CHECK(c, cudaStreamSynchronize(c->stream), "sync");
   if (v != 0x7fffffff) {
     char b[128];
-    snprintf(b, sizeof b, "Jacobi eigensolver did not converge for table row %d", v - 1);
+    snprintf(b, sizeof b, "eigensolver did not converge for table row %d", v - 1);
     return set_err(c, TG_ERR_NUMERIC, b);
   }
   return TG_OK;
@@ -2326,7 +2331,7 @@ int tg_eig_batch(tg_ctx* c, int64_t nk, const double* kp, double* lam, double* U
   if ((rc = require_native(c, "tg_eig_batch"))) return rc;
   if (nk < 0 || (nk > 0 && (!kp || !lam || !U))) return set_err(c, TG_ERR_ARG, "tg_eig_batch: bad args");
   if (nk == 0) return TG_OK;
-  if (!eig_supported(c->dimH)) return set_err(c, TG_ERR_ARG, "tg_eig_batch: dimH too large for the Jacobi kernel");
+  if (!eig_supported(c->dimH)) return set_err(c, TG_ERR_ARG, "tg_eig_batch: dimH too large for the eigensolver");
   cudaSetDevice(c->device);
   cudaStream_t s = c->stream;
   const double zero3[3] = {0.0, 0.0, 0.0};

@@ -1,0 +1,590 @@
+// Eigendecompositions and tridiagonalisations of an H(k) table, one Hermitian matrix per k.
+//
+// Three kernels, each parallel over the k in its own way:
+//   1. hh_small_kernel: H = Q T Q^H, T real symmetric tridiagonal (the Householder reduction of
+//      LAPACK's zhetd2, lower form, with zlarfg's reflectors), one CTA per k with the matrix in
+//      shared memory; Q is accumulated backwards in place.  Also used for the resolvents of
+//      tg_tridiag.cu at dimensions up to 96.
+//   2. ql_kernel: T = Z diag(lambda) Z^T by the implicitly shifted QL iteration (Bowdler,
+//      Martin, Reinsch and Wilkinson, 1968), one thread per k with d and e in shared memory.
+//      The iteration is a serial chain of n^2 plane rotations, so only the number of k hides
+//      it; its rotations go to global memory.
+//   3. eig_finish_kernel: U = Q Z, one CTA per k with Q in shared memory and a thread per real
+//      row (rotations of columns act on every row alone, without any barrier), then one
+//      Newton-Schulz step U <- U (1 - (U^H U - 1) / 2) and Rayleigh quotients of H for the
+//      eigenvalues.
+// About 20 n^3 flops per matrix against the 10 sweeps of 24 n^3 of a cyclic Jacobi iteration,
+// whose rotations also need a CTA barrier per round.
+#include "tg_internal.cuh"
+
+#include <algorithm>
+
+namespace tg {
+
+namespace {
+
+constexpr int kHhMax = 96;          // largest dimension of hh_small_kernel (three rows per lane)
+constexpr int kHhThreads = 384;
+constexpr int kQlIterations = 60;   // per eigenvalue
+
+__host__ __device__ inline int odd_stride(int n) { return n | 1; }
+
+__device__ __forceinline__ double2 warp_sum2(double2 v) {
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
+
+// --------------------------------------------------------------------------- 1. tridiagonalisation
+// B holds A column by column with an odd stride (A(r, c) at c S + r), both triangles; PT
+// threads per row (or, for Q, per column) share its sums.  Per reflector: norm (every warp on
+// its own, no barrier), product A v, update
+//   A <- A - v p^H - q v^H,  p = tau A v, q = p - Re(tau p^H v) v,
+// three barriers; per reflector of Q one.  The loops read four entries before they write the
+// first (the compiler cannot tell the stores from the next loads apart).  Bound by the latency
+// of these steps where one matrix fills the SM (n = 90), by shared memory where several share
+// it (15 + 14 wavefronts per 32 entries and step, n^3 / 3 entries in all).
+constexpr int kHhBatch = 4;
+
+template <int PT>
+__device__ __forceinline__ double2 group_sum2(double2 v) {
+#pragma unroll
+  for (int o = 1; o < PT; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
+
+template <int PT>
+__global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __restrict__ H, int64_t nk, int n,
+                                                            const int* __restrict__ rows, int ns,
+                                                            double* __restrict__ D, double* __restrict__ E,
+                                                            double2* __restrict__ Q) {
+  extern __shared__ __align__(16) double2 hsm[];
+  const int S = odd_stride(n);
+  double2* B = hsm;
+  double2* v = B + n * S;
+  double2* p = v + n;
+  double2* taus = p + n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rt = tid / PT, h = tid % PT;
+  const double2 zero = make_double2(0.0, 0.0);
+  for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
+    const double2* Hk = H + k * (int64_t)n * n;
+#pragma unroll 4
+    for (int e = tid; e < n * n; e += blockDim.x) B[(e % n) * S + e / n] = Hk[e];
+    __syncthreads();
+    for (int j = 0; j + 1 < n; ++j) {
+      const int m = n - j - 1;
+      double2* col = B + j * S + j + 1;
+      double2 x[3];
+      double part = 0.0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const int r = lane + 32 * i;
+        x[i] = r < m ? col[r] : zero;
+        if (r > 0) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
+      }
+      const double2 alpha = col[0];
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      const bool refl = !(part == 0.0 && alpha.y == 0.0);
+      // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
+      const double beta =
+          refl ? -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, part))), alpha.x) : alpha.x;
+      double2 tau = zero;
+      if (refl) {
+        const double ib = 1.0 / beta;
+        tau = make_double2((beta - alpha.x) * ib, -alpha.y * ib);
+      }
+      if (warp == 0) {
+        if (lane == 0) {
+          D[k * n + j] = B[j * S + j].x;
+          E[k * n + j] = beta;
+          taus[j] = tau;
+        }
+        if (refl) {
+          const double dr = alpha.x - beta, di = alpha.y;
+          const double inv = 1.0 / fma(dr, dr, di * di);
+          const double2 sc = make_double2(dr * inv, -di * inv);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const int r = lane + 32 * i;
+            if (r < m) v[r] = r == 0 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
+          }
+        }
+      }
+      __syncthreads();
+      if (!refl) continue;   // (uniform: every thread took the same sums)
+      if (warp == 0)
+        for (int r = lane; r < m; r += 32) col[r] = v[r];   // kept for Q; the column is done with
+      double2* Ar = B + (j + 1) * S + j + 1 + rt;
+      double2 acc = zero, acc1 = zero;
+      if (rt < m) {
+        int c = h;
+        for (; c + 3 * PT < m; c += 4 * PT) {
+          acc = cfma(Ar[c * S], v[c], acc);
+          acc1 = cfma(Ar[(c + PT) * S], v[c + PT], acc1);
+          acc = cfma(Ar[(c + 2 * PT) * S], v[c + 2 * PT], acc);
+          acc1 = cfma(Ar[(c + 3 * PT) * S], v[c + 3 * PT], acc1);
+        }
+        for (; c < m; c += PT) acc = cfma(Ar[c * S], v[c], acc);
+      }
+      acc = group_sum2<PT>(cadd(acc, acc1));
+      const double2 pr = cmul(tau, acc);
+      if (rt < m && h == 0) p[rt] = pr;
+      __syncthreads();
+      double2 dot = zero;
+      for (int r = lane; r < m; r += 32) dot = cfma(cconj(p[r]), v[r], dot);
+      dot = warp_sum2(dot);
+      const double t2 = -cmul(tau, dot).x;   // 2 Re(-tau (p^H v) / 2)
+      if (rt < m) {
+        const double2 vr = v[rt], qr = make_double2(fma(t2, vr.x, pr.x), fma(t2, vr.y, pr.y));
+        for (int c0 = h; c0 < m; c0 += kHhBatch * PT) {
+          double2 a[kHhBatch];
+#pragma unroll
+          for (int u = 0; u < kHhBatch; ++u) {
+            const int c = c0 + u * PT;
+            a[u] = c < m ? cfms(qr, cconj(v[c]), cfms(vr, cconj(p[c]), Ar[c * S])) : zero;
+          }
+#pragma unroll
+          for (int u = 0; u < kHhBatch; ++u)
+            if (c0 + u * PT < m) Ar[(c0 + u * PT) * S] = a[u];
+        }
+      }
+      __syncthreads();
+    }
+    if (tid == 0) {
+      D[k * n + n - 1] = B[(n - 1) * S + n - 1].x;
+      E[k * n + n - 1] = 0.0;
+    }
+    // Q = H_0 H_1 .. H_{n-2} backwards: step j fills the block of rows and columns > j
+    for (int j = n - 2; j >= 0; --j) {
+      const int m = n - j - 1;
+      const double2 tau = taus[j];
+      const bool refl = tau.x != 0.0 || tau.y != 0.0;
+      const double2* vj = B + j * S + j + 1;
+      double2* col = B + (j + 1 + rt) * S + j + 1;   // this thread's column
+      double2 y = zero, y1 = zero;
+      if (refl && rt > 0 && rt < m) {
+        int r = 1 + h;
+        for (; r + 3 * PT < m; r += 4 * PT) {
+          y = cfma(cconj(vj[r]), col[r], y);
+          y1 = cfma(cconj(vj[r + PT]), col[r + PT], y1);
+          y = cfma(cconj(vj[r + 2 * PT]), col[r + 2 * PT], y);
+          y1 = cfma(cconj(vj[r + 3 * PT]), col[r + 3 * PT], y1);
+        }
+        for (; r < m; r += PT) y = cfma(cconj(vj[r]), col[r], y);
+      }
+      y = group_sum2<PT>(cadd(y, y1));
+      if (rt == 0) y = make_double2(1.0, 0.0);   // column j + 1 enters as a unit vector
+      const double2 ty = cmul(tau, y);
+      if (rt < m) {
+        if (refl || rt == 0)
+          for (int r0 = 1 + h; r0 < m; r0 += kHhBatch * PT) {
+            double2 a[kHhBatch];
+#pragma unroll
+            for (int u = 0; u < kHhBatch; ++u) {
+              const int r = r0 + u * PT;
+              const double2 vr = refl && r < m ? vj[r] : zero;   // (no reflector: the unit vector stays)
+              a[u] = cfms(ty, vr, rt > 0 && r < m ? col[r] : zero);
+            }
+#pragma unroll
+            for (int u = 0; u < kHhBatch; ++u)
+              if (r0 + u * PT < m) col[r0 + u * PT] = a[u];
+          }
+        if (h == 0) col[0] = make_double2((rt == 0 ? 1.0 : 0.0) - ty.x, -ty.y);
+      }
+      __syncthreads();
+    }
+    double2* Qk = Q + k * (int64_t)ns * n;
+#pragma unroll 2
+    for (int e = tid; e < ns * n; e += blockDim.x) {
+      const int s = e / n, c = e - s * n;
+      const int r = rows ? rows[s] : s;
+      Qk[e] = r == 0 || c == 0 ? make_double2(r == c ? 1.0 : 0.0, 0.0) : B[c * S + r];
+    }
+    __syncthreads();
+  }
+}
+
+// --------------------------------------------------------------------------- 2. QL iteration
+// d, e: [nk][n]; rot: [nk][cap] (c, s) in the order they act, sweep: [nk][scap] lowest column
+// l | top column m << 16 of each sweep (its rotations act on columns (i, i + 1), i = m - 1 .. l),
+// nsweep: [nk].  A lane whose lists would overflow, or an eigenvalue that does not settle, sets
+// status.  `lanes` matrices per warp: the warp runs as long as the longest sweep of its lanes, so
+// few matrices are spread over more warps.
+__global__ void __launch_bounds__(32) ql_kernel(const double* __restrict__ D, const double* __restrict__ E,
+                                                int64_t k0, int64_t nk, int n, double* __restrict__ lam,
+                                                double2* __restrict__ rot, int cap, int* __restrict__ sweep, int scap,
+                                                int* __restrict__ nsweep, int lanes, int* __restrict__ status) {
+  extern __shared__ __align__(16) double qsm[];
+  const int lane = threadIdx.x;
+  const int64_t kl = (int64_t)blockIdx.x * lanes + lane;
+  if (lane >= lanes || kl >= nk) return;   // (no barrier below)
+  const int64_t k = k0 + kl;
+  double* d = qsm + lane;            // d[32 i]
+  double* e = qsm + 32 * n + lane;   // e[32 i]
+  double an = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double di = D[k * n + i], ei = i + 1 < n ? E[k * n + i] : 0.0;
+    d[32 * i] = di;
+    e[32 * i] = ei;
+    an = fmax(an, fabs(di) + fabs(ei));
+  }
+  double2* rk = rot + kl * cap;
+  int* sk = sweep + kl * scap;
+  int nr = 0, nsw = 0;
+  bool ok = true;
+  const double tiny = 1e-17 * an;
+  for (int l = 0; l < n && ok; ++l) {
+    for (int it = 0;; ++it) {
+      int m = l;
+      for (; m + 1 < n; ++m)
+        if (fabs(e[32 * m]) <= 0x1p-53 * (fabs(d[32 * m]) + fabs(d[32 * (m + 1)])) + tiny) break;
+      if (m == l) break;
+      if (it == kQlIterations || nr + (m - l) > cap || nsw == scap) {
+        ok = false;
+        break;
+      }
+      // shift: the eigenvalue of the leading 2 x 2 block nearer d_l
+      const double dl = d[32 * l], el = e[32 * l];
+      double g = (d[32 * (l + 1)] - dl) / (2.0 * el);
+      g = d[32 * m] - dl + el / (g + copysign(sqrt(fma(g, g, 1.0)), g));
+      double s = 1.0, c = 1.0, pp = 0.0, dn = d[32 * m];
+      sk[nsw++] = l | m << 16;
+      for (int i = m - 1; i >= l; --i) {
+        const double ei = e[32 * i], di = d[32 * i];
+        const double f = s * ei, b = c * ei;
+        const double q = fma(f, f, g * g);
+        double ir, r;
+        if (q > 1e-280) {
+          ir = rsqrt(q);
+          r = q * ir;
+        } else {   // both below 1e-140: scaled
+          const double big = fmax(fabs(f), fabs(g));
+          const double fs = big > 0.0 ? f / big : 0.0, gs = big > 0.0 ? g / big : 1.0;
+          const double rs = sqrt(fma(fs, fs, gs * gs));
+          r = big * rs;
+          ir = 0.0;
+          s = fs / rs;
+          c = gs / rs;
+        }
+        e[32 * (i + 1)] = r;
+        if (ir != 0.0) {
+          s = f * ir;
+          c = g * ir;
+        }
+        // the pair (c, s) is a rotation to the last digit: s^2 + c^2 within rounding of 1
+        g = dn - pp;
+        const double t = fma(di - g, s, 2.0 * c * b);
+        pp = s * t;
+        d[32 * (i + 1)] = g + pp;
+        g = fma(c, t, -b);
+        dn = di;
+        rk[nr++] = make_double2(c, s);
+      }
+      d[32 * l] = dn - pp;
+      e[32 * l] = g;
+      e[32 * m] = 0.0;
+    }
+  }
+  nsweep[kl] = nsw;
+  for (int i = 0; i < n; ++i) lam[k * n + i] = d[32 * i];
+  if (!ok) atomicMin(status, (int)(k < 0x7ffffffe ? k + 1 : 0x7fffffff));
+}
+
+// --------------------------------------------------------------------------- 3. vectors
+// The Hermitian n x n scratch of the post-pass: the full array (odd stride), or (PACKED, where
+// it does not fit beside U) the upper triangle column by column.
+template <bool PACKED>
+struct HermA {
+  double2* a;
+  int n, S;
+  __device__ __forceinline__ double2 get(int i, int j) const {
+    if (!PACKED) return a[i * S + j];
+    return i <= j ? a[j * (j + 1) / 2 + i] : cconj(a[i * (i + 1) / 2 + j]);
+  }
+  __host__ __device__ static int entries(int n) { return PACKED ? n * (n + 1) / 2 : n * n; }
+  __host__ __device__ static size_t storage(int n) {
+    return PACKED ? (size_t)n * (n + 1) / 2 : (size_t)n * odd_stride(n);
+  }
+  __device__ __forceinline__ int at(int i, int j) const { return PACKED ? j * (j + 1) / 2 + i : i * S + j; }
+  // (i, j) of entry e (i <= j when PACKED)
+  __device__ __forceinline__ void ij(int e, int& i, int& j) const {
+    if (!PACKED) {
+      i = e / n;
+      j = e - i * n;
+      return;
+    }
+    j = (int)((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
+    while (j * (j + 1) / 2 > e) --j;
+    while ((j + 1) * (j + 2) / 2 <= e) ++j;
+    i = e - j * (j + 1) / 2;
+  }
+};
+
+constexpr int kEigCols = 3;   // columns per lane of the post-pass row products: n <= 96
+constexpr int kFinThreads = 256;
+
+// H: [nk][n][n] row-major; U: in Q (row-major), out the eigenvectors U[r][a]; lam: [nk][n]
+template <bool PACKED>
+__global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* __restrict__ H, int64_t nk, int n,
+                                                                 const double2* __restrict__ rot, int cap,
+                                                                 const int* __restrict__ sweep, int scap,
+                                                                 const int* __restrict__ nsweep,
+                                                                 double2* __restrict__ Uio, double* __restrict__ lam) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int S = odd_stride(n);
+  double2* U = reinterpret_cast<double2*>(smem);   // [n][S]
+  const HermA<PACKED> A{U + n * S, n, S};
+  const int na = HermA<PACKED>::entries(n);
+  const int room = (int)HermA<PACKED>::storage(n);   // rotations that the scratch holds
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+  for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
+    const double2* Hk = H + k * (int64_t)n * n;
+    double2* Uk = Uio + k * (int64_t)n * n;
+    for (int e = tid; e < n * n; e += blockDim.x) U[(e / n) * S + e % n] = Uk[e];
+    __syncthreads();
+    // U <- Q Z: real row 2 r + part of thread tid, the rotations in their order, staged through
+    // the scratch of the post-pass as many whole sweeps at a time as it holds
+    {
+      double* row = reinterpret_cast<double*>(U + (tid >> 1) * S) + (tid & 1);
+      const double2* rk = rot + k * cap;
+      const int* sk = sweep + k * scap;
+      const int nsw = nsweep[k];
+      for (int w0 = 0; w0 < nsw;) {
+        int w1 = w0, cnt = 0;
+        while (w1 < nsw) {
+          const int lm = sk[w1], len = (lm >> 16) - (lm & 0xffff);
+          if (w1 > w0 && cnt + len > room) break;   // (one sweep, n - 1 rotations, always fits)
+          cnt += len;
+          ++w1;
+        }
+#pragma unroll 4
+        for (int e = tid; e < cnt; e += blockDim.x) A.a[e] = rk[e];
+        __syncthreads();
+        if (tid < 2 * n) {
+          const double2* t = A.a;
+          for (int w = w0; w < w1; ++w) {
+            const int lm = sk[w], l = lm & 0xffff, m = lm >> 16;
+            double x = row[2 * m];
+            int i = m - 1;
+            for (; i >= l + 3; i -= 4, t += 4) {
+              const double f0 = row[2 * i], f1 = row[2 * i - 2], f2 = row[2 * i - 4], f3 = row[2 * i - 6];
+              const double2 r0 = t[0], r1 = t[1], r2 = t[2], r3 = t[3];
+              row[2 * i + 2] = fma(r0.y, f0, r0.x * x);
+              x = fma(r0.x, f0, -(r0.y * x));
+              row[2 * i] = fma(r1.y, f1, r1.x * x);
+              x = fma(r1.x, f1, -(r1.y * x));
+              row[2 * i - 2] = fma(r2.y, f2, r2.x * x);
+              x = fma(r2.x, f2, -(r2.y * x));
+              row[2 * i - 4] = fma(r3.y, f3, r3.x * x);
+              x = fma(r3.x, f3, -(r3.y * x));
+            }
+            for (; i >= l; --i, ++t) {
+              const double f = row[2 * i];
+              row[2 * i + 2] = fma(t->y, f, t->x * x);
+              x = fma(t->x, f, -(t->y * x));
+            }
+            row[2 * l] = x;
+          }
+        }
+        __syncthreads();
+        rk += cnt;
+        w0 = w1;
+      }
+    }
+    // Post-pass: re-orthonormalised vectors and Rayleigh-quotient eigenvalues.
+    //  (1) E = U^H U - 1 (Hermitian)
+    for (int e = tid; e < na; e += blockDim.x) {
+      int i, j;
+      A.ij(e, i, j);
+      double2 acc = make_double2(i == j ? -1.0 : 0.0, 0.0);
+      for (int r = 0; r < n; ++r) acc = cfma(cconj(U[r * S + i]), U[r * S + j], acc);
+      A.a[A.at(i, j)] = acc;
+    }
+    __syncthreads();
+    //  (2) one Newton-Schulz step U <- U (1 - E / 2): a warp per row, the row read before written
+    for (int r = warp; r < n; r += nwarps) {
+      double2 x[kEigCols];
+#pragma unroll
+      for (int m = 0; m < kEigCols; ++m) {
+        x[m] = make_double2(0.0, 0.0);
+        const int j = lane + 32 * m;
+        if (j < n)
+          for (int i = 0; i < n; ++i) x[m] = cfma(U[r * S + i], A.get(i, j), x[m]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int m = 0; m < kEigCols; ++m) {
+        const int j = lane + 32 * m;
+        if (j < n) U[r * S + j] = csub(U[r * S + j], cscale(x[m], 0.5));
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    //  (3) lambda_a = Re u_a^H Hs u_a with Hs = (H + H^H) / 2 from the table
+    for (int e = tid; e < na; e += blockDim.x) {
+      int r, c;
+      A.ij(e, r, c);
+      const double2 x = Hk[r * n + c], y = Hk[c * n + r];
+      A.a[A.at(r, c)] = r == c ? make_double2(x.x, 0.0) : make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
+    }
+    __syncthreads();
+    for (int e = tid; e < n * n; e += blockDim.x) Uk[e] = U[(e / n) * S + e % n];
+    if (!PACKED) {
+      // W = Hs U row by row in place (a warp per row), then one thread per eigenvalue
+      for (int r = warp; r < n; r += nwarps) {
+        double2 x[kEigCols];
+#pragma unroll
+        for (int m = 0; m < kEigCols; ++m) {
+          x[m] = make_double2(0.0, 0.0);
+          const int j = lane + 32 * m;
+          if (j < n)
+            for (int c = 0; c < n; ++c) x[m] = cfma(A.a[r * S + c], U[c * S + j], x[m]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < kEigCols; ++m) {
+          const int j = lane + 32 * m;
+          if (j < n) A.a[r * S + j] = x[m];
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+      for (int a = tid; a < n; a += blockDim.x) {
+        double l = 0.0;
+        for (int r = 0; r < n; ++r) {
+          const double2 u = U[r * S + a], w = A.a[r * S + a];
+          l = fma(u.x, w.x, fma(u.y, w.y, l));   // Re(conj(u) w)
+        }
+        lam[k * n + a] = l;
+      }
+    } else {
+      // no room for W: a warp per eigenvalue, lanes over the rows r of sum_r conj(u_r) (Hs u)_r
+      for (int a = warp; a < n; a += nwarps) {
+        double l = 0.0;
+        for (int r = lane; r < n; r += 32) {
+          double2 w = make_double2(0.0, 0.0);
+          for (int c = 0; c < n; ++c) w = cfma(A.get(r, c), U[c * S + a], w);
+          const double2 u = U[r * S + a];
+          l = fma(u.x, w.x, fma(u.y, w.y, l));
+        }
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (lane == 0) lam[k * n + a] = l;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+int optin_smem() {
+  int dev = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+  return optin;
+}
+
+size_t fin_smem(int n, bool packed) {
+  return sizeof(double2) *
+         ((size_t)n * odd_stride(n) + (packed ? HermA<true>::storage(n) : HermA<false>::storage(n)));
+}
+
+bool fin_packed(int n, int optin) { return fin_smem(n, false) > (size_t)optin; }
+
+size_t hh_smem(int n) { return sizeof(double2) * ((size_t)n * odd_stride(n) + 3 * (size_t)n); }
+
+// rotations and sweeps kept per k: the iteration takes about 1.3 n^2 rotations in 2.3 n sweeps
+int ql_cap(int n) { return 3 * n * n + 32; }
+int ql_sweeps(int n) { return 8 * n + 16; }
+
+// k per chunk: at most 1 GiB of rotations
+int64_t ql_chunk(int n, int64_t nk) {
+  return std::max<int64_t>(1, std::min<int64_t>(nk, ((int64_t)1 << 30) / ((int64_t)ql_cap(n) * 16)));
+}
+
+}  // namespace
+
+// the unpacked post-pass (U and its scratch both whole in shared memory): cheap enough to
+// diagonalise per k even where few energies share a k list
+int eig_fast(int n) {
+  if (n % 2 != 0 || n < 2 || n > 32 * kEigCols) return 0;
+  return !fin_packed(n, optin_smem());
+}
+
+int eig_supported(int n) {
+  if (n % 2 != 0 || n < 2 || n > 32 * kEigCols) return 0;
+  const int optin = optin_smem();
+  return fin_smem(n, fin_packed(n, optin)) <= (size_t)optin;
+}
+
+int hh_small_supported(int n) { return n >= 2 && n <= kHhMax && hh_smem(n) <= (size_t)optin_smem(); }
+
+cudaError_t launch_hh_small(const double2* H, int64_t nk, int n, const int* rows, int ns, double* D, double* E,
+                            double2* Q, int num_sms, cudaStream_t s) {
+  if (nk <= 0) return cudaSuccess;
+  if (!hh_small_supported(n) || ns <= 0 || ns > n) return cudaErrorInvalidValue;
+  const size_t smem = hh_smem(n);
+  // two threads per row where several matrices share an SM, four where one fills it
+  const bool wide = smem > (size_t)optin_smem() / 2;
+  const int threads = ((wide ? 4 : 2) * n + 31) / 32 * 32;
+  auto kernel = wide ? hh_small_kernel<4> : hh_small_kernel<2>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+  if (e != cudaSuccess) return e;
+  if (per_sm <= 0) return cudaErrorInvalidValue;
+  const int64_t grid = std::min<int64_t>(nk, (int64_t)num_sms * per_sm);
+  kernel<<<(unsigned)grid, threads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
+  return cudaGetLastError();
+}
+
+size_t eig_ws_bytes(int n, int64_t nk) {
+  const int64_t c = ql_chunk(n, nk);
+  return (size_t)c * ((size_t)ql_cap(n) * sizeof(double2) + (size_t)ql_sweeps(n) * sizeof(int) + sizeof(int)) +
+         (size_t)nk * n * 2 * sizeof(double) + 256;
+}
+
+cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int* status,
+                       int num_sms, cudaStream_t s) {
+  if (nk <= 0) return cudaSuccess;
+  if (!eig_supported(n)) return cudaErrorInvalidValue;
+  const int64_t chunk = ql_chunk(n, nk);
+  const int cap = ql_cap(n), scap = ql_sweeps(n);
+  double2* rot = static_cast<double2*>(ws);
+  double* D = reinterpret_cast<double*>(rot + chunk * cap);
+  double* E = D + nk * n;
+  int* sweep = reinterpret_cast<int*>(E + nk * n);
+  int* nsweep = sweep + chunk * scap;
+  cudaError_t e = launch_hh_small(H, nk, n, nullptr, n, D, E, U, num_sms, s);
+  if (e != cudaSuccess) return e;
+  const size_t qsmem = sizeof(double) * 64 * (size_t)n;
+  e = cudaFuncSetAttribute(ql_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsmem);
+  if (e != cudaSuccess) return e;
+  const bool packed = fin_packed(n, optin_smem());
+  const size_t fsmem = fin_smem(n, packed);
+  auto fin = packed ? eig_finish_kernel<true> : eig_finish_kernel<false>;
+  e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fin, kFinThreads, fsmem);
+  if (e != cudaSuccess) return e;
+  if (per_sm <= 0) return cudaErrorInvalidValue;
+  for (int64_t k0 = 0; k0 < nk; k0 += chunk) {
+    const int64_t m = std::min(chunk, nk - k0);
+    int lanes = 32;
+    while (lanes > 2 && (m + lanes - 1) / lanes < 4 * num_sms) lanes /= 2;
+    ql_kernel<<<(unsigned)((m + lanes - 1) / lanes), 32, qsmem, s>>>(D, E, k0, m, n, lam, rot, cap, sweep, scap,
+                                                                    nsweep, lanes, status);
+    const int64_t grid = std::min<int64_t>(m, (int64_t)num_sms * per_sm);
+    fin<<<(unsigned)grid, kFinThreads, fsmem, s>>>(H + k0 * (int64_t)n * n, m, n, rot, cap, sweep, scap, nsweep,
+                                                   U + k0 * (int64_t)n * n, lam + k0 * n);
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace tg

@@ -219,12 +219,18 @@ cudaError_t launch_hk_table(const GreenArgs& a, const double* kp, int64_t nk, co
                             double2* H, cudaStream_t s);
 cudaError_t launch_reduce_blocks(const double2* part, int nblocks, int len, double2* out, cudaStream_t s);
 
-// Spectral Green functions: Jacobi eigendecomposition of an H(k) table and G from (U, lambda)
-size_t eig_smem_bytes(int n);
+// Spectral Green functions: eigendecomposition of an H(k) table (ws: eig_ws_bytes of device
+// memory) and G from (U, lambda)
 int eig_supported(int n);
 int eig_fast(int n);
-cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, int* status, int num_sms,
-                       cudaStream_t s);
+size_t eig_ws_bytes(int n, int64_t nk);
+cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int* status,
+                       int num_sms, cudaStream_t s);
+// Householder tridiagonalisation of an H(k) table in shared memory, dimensions up to 96 (H is
+// kept; rows null: every row of Q)
+int hh_small_supported(int n);
+cudaError_t launch_hh_small(const double2* H, int64_t nk, int n, const int* rows, int ns, double* D, double* E,
+                            double2* Q, int num_sms, cudaStream_t s);
 int spectral_supported(int mode, int mode2, bool has_out2);
 // Resolvents from a Householder tridiagonalisation per k: H (an H(k) table, overwritten) ->
 // T (D, E) and the rows `rows` of Q; G over those rows per point of a k-major pass (MODE_RAW)

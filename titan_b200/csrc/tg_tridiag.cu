@@ -439,6 +439,8 @@ cudaError_t launch_tridiag(double2* H, int64_t nk, int n, const int* rows, int n
                            double2* Q, int num_sms, cudaStream_t s) {
   if (nk <= 0) return cudaSuccess;
   if (n < 2 || ns <= 0 || ns > n) return cudaErrorInvalidValue;
+  // the matrix in shared memory where it fits (no pass over it goes to L2)
+  if (hh_small_supported(n)) return launch_hh_small(H, nk, n, rows, ns, D, E, Q, num_sms, s);
   const size_t smem = sizeof(double2) * 2 * (size_t)n + sizeof(double) * 2 * (kTriThreads / 32);
   const int64_t grid = std::min<int64_t>(nk, (int64_t)num_sms * 4);
   hh_tridiag_kernel<<<(unsigned)grid, kTriThreads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
