@@ -209,47 +209,68 @@ __global__ void __launch_bounds__(THREADS, THREADS == kSpecThreads ? 5 : 1) spec
 }
 
 // --------------------------------------------------------------------------- LDOS from (U, lambda)
-constexpr int kLdosE = 32;   // energies per CTA
+constexpr int kLdosE = 64;   // energies per CTA: eight per warp
 
 // out[ie][r] += (eta / pi) sum_{k in this CTA's chunk} w_k sum_a |U[k][r][a]|^2 / ((e_ie - lambda_ka)^2 + eta^2),
-// i.e. -Im G_rr(k, e + i eta) / pi summed over the chunk (atomicAdd into out)
+// i.e. -Im G_rr(k, e + i eta) / pi summed over the chunk (atomicAdd into out): per k a real GEMM
+// [energies x n] x [n x n] on the FP64 tensor cores, the weighted |U|^2 and the Lorentzians
+// formed in shared memory.  Strides of 4 mod 16 doubles keep the 8-byte fragment reads (eight
+// rows, four columns) apart.  NF: column fragments of a warp (all n columns).
+__host__ __device__ inline int ldos_stride(int n) { return (n + 11) / 16 * 16 + 4; }
+
+template <int NF>
 __global__ void __launch_bounds__(256) spec_ldos_kernel(const double2* __restrict__ U, const double* __restrict__ lam,
                                                         const double* __restrict__ w, int64_t nk, int n,
                                                         const double* __restrict__ e, int n_e, double eta,
                                                         int64_t k_per_cta, double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double* P = reinterpret_cast<double*>(smem);   // [n][n] |U|^2
-  double* L = P + n * n;                          // [kLdosE][n]
-  double* acc = L + kLdosE * n;                   // [kLdosE][n]
+  const int S = ldos_stride(n);
+  double* P = reinterpret_cast<double*>(smem);   // [8 NF][S] w |U[r][a]|^2 (zero rows and columns past n)
+  double* L = P + 8 * NF * S;                     // [kLdosE][S]
   const int e0 = blockIdx.x * kLdosE;
   const int ne = min(kLdosE, n_e - e0);
   const int64_t k0 = (int64_t)blockIdx.y * k_per_cta, k1 = min(nk, k0 + k_per_cta);
-  for (int o = threadIdx.x; o < kLdosE * n; o += blockDim.x) acc[o] = 0.0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+  const int kp = (n + 3) / 4 * 4;
+  for (int o = threadIdx.x; o < (8 * NF + kLdosE) * S; o += blockDim.x) P[o] = 0.0;
+  double c[NF][2];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) c[f][0] = c[f][1] = 0.0;
   for (int64_t k = k0; k < k1; ++k) {
     __syncthreads();
     const double2* Uk = U + k * (int64_t)n * n;
+    const double wk = w[k];
+#pragma unroll 4
     for (int o = threadIdx.x; o < n * n; o += blockDim.x) {
       const double2 u = Uk[o];
-      P[o] = u.x * u.x + u.y * u.y;
+      P[(o / n) * S + o % n] = wk * fma(u.x, u.x, u.y * u.y);
     }
+#pragma unroll 2
     for (int o = threadIdx.x; o < ne * n; o += blockDim.x) {
-      const double x = e[e0 + o / n] - lam[k * n + o % n];
-      L[o] = 1.0 / (x * x + eta * eta);
+      const int ie = o / n, a = o % n;
+      const double x = e[e0 + ie] - lam[k * n + a];
+      L[ie * S + a] = 1.0 / fma(x, x, eta * eta);
     }
     __syncthreads();
-    const double wk = w[k];
-    for (int o = threadIdx.x; o < ne * n; o += blockDim.x) {
-      const int ie = o / n, r = o % n;
-      const double* pr = P + r * n;
-      const double* le = L + ie * n;
-      double s = 0.0;
-      for (int a = 0; a < n; ++a) s = fma(pr[a], le[a], s);
-      acc[o] = fma(wk, s, acc[o]);
+    const double* La = L + (8 * warp + g8) * S + t4;
+    const double* Pb = P + g8 * S + t4;
+    for (int a = 0; a < kp; a += 4) {
+      const double av = La[a];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) dmma(c[f][0], c[f][1], av, Pb[8 * f * S + a]);
     }
   }
-  __syncthreads();
-  const double f = eta / 3.141592653589793238462643383279502884;
-  for (int o = threadIdx.x; o < ne * n; o += blockDim.x) atomicAdd(out + (int64_t)(e0 + o / n) * n + o % n, f * acc[o]);
+  const double f0 = eta / 3.141592653589793238462643383279502884;
+  const int ie = 8 * warp + g8;
+  if (ie < ne) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = 8 * f + 2 * t4 + h;
+        if (r < n) atomicAdd(out + (int64_t)(e0 + ie) * n + r, f0 * c[f][h]);
+      }
+  }
 }
 
 // --------------------------------------------------------------------------- expectation sums from (U, lambda)
@@ -312,16 +333,26 @@ cudaError_t launch_spec_expect(const double2* U, const double* lam, int64_t nk, 
 cudaError_t launch_spec_ldos(const double2* U, const double* lam, const double* w, int64_t nk, int n,
                              const double* e, int n_e, double eta, double* out, int num_sms, cudaStream_t s) {
   if (nk <= 0 || n_e <= 0) return cudaSuccess;
-  const size_t smem = sizeof(double) * ((size_t)n * n + 2 * (size_t)kLdosE * n);
-  cudaError_t err = cudaFuncSetAttribute(spec_ldos_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (n > 96) return cudaErrorInvalidValue;
+  const int nf = (n + 7) / 8;
+  const size_t smem = sizeof(double) * (size_t)ldos_stride(n) * (8 * (nf <= 3 ? 3 : nf <= 6 ? 6 : nf <= 9 ? 9 : 12) + kLdosE);
+  auto kernel = nf <= 3   ? spec_ldos_kernel<3>
+                : nf <= 6 ? spec_ldos_kernel<6>
+                : nf <= 9 ? spec_ldos_kernel<9>
+                          : spec_ldos_kernel<12>;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return err;
   err = cudaMemsetAsync(out, 0, sizeof(double) * (size_t)n_e * n, s);
   if (err != cudaSuccess) return err;
+  int per_sm = 0;
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem);
+  if (err != cudaSuccess) return err;
+  if (per_sm <= 0) return cudaErrorInvalidValue;
   const int eb = (n_e + kLdosE - 1) / kLdosE;
-  const int64_t kchunks = std::max<int64_t>(1, std::min<int64_t>(nk, (int64_t)4 * num_sms / eb));
+  const int64_t kchunks = std::max<int64_t>(1, std::min<int64_t>(nk, (int64_t)per_sm * num_sms / eb));
   const int64_t kper = (nk + kchunks - 1) / kchunks;
   const dim3 grid((unsigned)eb, (unsigned)((nk + kper - 1) / kper));
-  spec_ldos_kernel<<<grid, 256, smem, s>>>(U, lam, w, nk, n, e, n_e, eta, kper, out);
+  kernel<<<grid, 256, smem, s>>>(U, lam, w, nk, n, e, n_e, eta, kper, out);
   return cudaGetLastError();
 }
 
