@@ -42,58 +42,56 @@ struct SpecArgs {
   int kp = 0;                   // K padded to a multiple of 4
 };
 
-__host__ __device__ inline size_t spec_smem(int n, int kp) {
-  return sizeof(double2) * ((size_t)n * kp + (size_t)kSpecZ * kp) + sizeof(double) * kSpecZ + sizeof(int) * kSpecZ;
-}
+// row stride of U and D in shared memory: 4 mod 8 complex, so that the fragment reads of a
+// quarter warp (two rows, four columns) fall into distinct banks
+__host__ __device__ inline int spec_stride(int kp) { return kp % 8 == 4 ? kp : kp + 4; }
 
-// (row, col) of G that lands in output slot o for a mode
-__device__ __forceinline__ void slot_rc(const SpecArgs& sa, int mode, int o, int& r, int& c) {
-  const int n = sa.g.n;
-  if (mode == MODE_RAW) {
-    r = o % n;
-    c = o / n;
-    return;
-  }
-  const int rc = sa.g.outmap[o];
-  if (mode == MODE_B_IMAG) {   // G^T
-    c = rc / n;
-    r = rc % n;
-  } else {
-    r = rc / n;
-    c = rc % n;
-  }
+__host__ __device__ inline size_t spec_smem(int n, int kp) {
+  const int S = spec_stride(kp);
+  const int tiles = ((n + 1) / 2) * ((n + 7) / 8 + 1);   // more than the tiles of the upper triangle
+  return sizeof(double2) * ((size_t)n * S + (size_t)kSpecZ * S) + sizeof(double) * kSpecZ + sizeof(int) * kSpecZ +
+         sizeof(int) * (size_t)tiles;
 }
 
 // frexp exponent of max(|Re|, |Im|) read from the bits (exponent field - 1022 for a
 // normal number); zero and subnormal values give -32768
-__device__ __forceinline__ int16_t exponent_code(double2 v) {
-  const double m = fmax(fabs(v.x), fabs(v.y));
-  const int f = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
-  return f == 0 ? (int16_t)-32768 : (int16_t)(f - 1022);
+__device__ __forceinline__ uint32_t exponent_pair(double2 a, double2 b) {
+  return (uint32_t)(uint16_t)exponent_code16(a) | (uint32_t)(uint16_t)exponent_code16(b) << 16;
 }
 
-// five CTAs per SM (the occupancy its ~30 KB of shared memory allows at n = 36): 48
-// registers with a 4-byte spill, measured faster than 64 registers at four CTAs
-// ANTI (MODE_A_REAL, w (G - G^+)): the diagonal -2i y / |z - lambda|^2 is purely
-// imaginary, so two of the four DMMAs per step would multiply by zero and are skipped
-// THREADS = 1024 (one CTA per SM) where the shared memory of U leaves room for one CTA only
-// (n > 72): 32 warps instead of 8 hide the DMMA and shared-memory latencies
-template <bool ANTI, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == kSpecThreads ? 5 : 1) spec_green_kernel(SpecArgs sa) {
+// G = X + i Y with X = sum_a Re(D_a) P_a and Y = sum_a Im(D_a) P_a, both Hermitian because every
+// P_a = u_a u_a^H is: only the entries r <= c are formed, G(r, c) = X + i Y and
+// G(c, r) = conj(X) + i conj(Y).  One task is a k and 16 energies; a warp takes tiles of two
+// rows (r, r + 1) and eight columns from r on, four real DMMAs per 8 pairs, 8 energies and 4
+// eigenvalues, and writes the four 2 x 2 blocks (32 bytes each) of both triangles.
+// Im(D) alone (ANTI: w (G - G^+) = w 2 i Y) takes half of them.  Bound by the FP64 tensor pipe
+// up to n = 36 or so by the G output as well (16 n^2 bytes per point).
+template <bool ANTI>
+__global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa) {
   extern __shared__ __align__(16) unsigned char smem[];
   const GreenArgs& a = sa.g;
-  const int n = a.n, kp = sa.kp, nn = n * n;
-  double2* Us = reinterpret_cast<double2*>(smem);          // [n][kp]
-  double2* Ds = Us + (size_t)n * kp;                        // [kSpecZ][kp]
-  double* ws = reinterpret_cast<double*>(Ds + (size_t)kSpecZ * kp);
+  const int n = a.n, kp = sa.kp, nn = n * n, S = spec_stride(kp);
+  double2* Us = reinterpret_cast<double2*>(smem);          // [n][S]
+  double2* Ds = Us + (size_t)n * S;                         // [kSpecZ][S]
+  double* ws = reinterpret_cast<double*>(Ds + (size_t)kSpecZ * S);
   int* item = reinterpret_cast<int*>(ws + kSpecZ);          // pass-local point of each row, -1 = none
+  int* tiles = item + kSpecZ;                               // r | c0 << 16
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarp = blockDim.x >> 5;
+  const int g8 = lane >> 2, t4 = lane & 3;
+  int ntile = 0;
+  for (int r = 0; r < n; r += 2)
+    for (int c0 = r; c0 < n; c0 += 8, ++ntile)
+      if (ntile % (int)blockDim.x == (int)threadIdx.x) tiles[ntile] = r | c0 << 16;
   const int64_t ne = a.n_e;
   const int64_t per_k = (ne + kSpecZ - 1) / kSpecZ;
   const int64_t ik0 = a.p0 / ne, ik1 = (a.p0 + a.np - 1) / ne;
   const int64_t ntask = (ik1 - ik0 + 1) * per_k;
-  const bool anti = ANTI;
+  // position (p, q) of the output holds G(p, q), or G(q, p) (G^T, and column-major raw G)
+  const bool swap = a.mode == MODE_B_IMAG || a.mode == MODE_RAW;
+  const bool swap2 = a.mode2 == MODE_B_IMAG;
+  const bool scaled = a.mode == MODE_A_IMAG || a.mode == MODE_A_REAL;
+  const bool conj = a.mode == MODE_B_REAL;
   for (int64_t t = blockIdx.x; t < ntask; t += gridDim.x) {
     const int64_t ik = ik0 + t / per_k;
     const int64_t ie0 = (t % per_k) * kSpecZ;
@@ -107,7 +105,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kSpecThreads ? 5 : 1) spec
     const double2* Uk = sa.U + ik * (int64_t)nn;
     for (int e = threadIdx.x; e < n * kp; e += blockDim.x) {
       const int r = e / kp, aa = e % kp;
-      Us[e] = aa < n ? Uk[r * n + aa] : make_double2(0.0, 0.0);
+      Us[r * S + aa] = aa < n ? Uk[r * n + aa] : make_double2(0.0, 0.0);
     }
     __syncthreads();
     // D[z][a] and the weights
@@ -134,10 +132,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == kSpecThreads ? 5 : 1) spec
           }
         } else {
           const double inv = 1.0 / s;
-          dv = anti ? make_double2(0.0, -2.0 * y * inv) : make_double2(x * inv, -y * inv);
+          dv = ANTI ? make_double2(0.0, -2.0 * y * inv) : make_double2(x * inv, -y * inv);
         }
       }
-      Ds[e] = dv;
+      Ds[zr * S + aa] = dv;
     }
     if (threadIdx.x < kSpecZ) {
       double w = 0.0;
@@ -148,60 +146,89 @@ __global__ void __launch_bounds__(THREADS, THREADS == kSpecThreads ? 5 : 1) spec
       ws[threadIdx.x] = w;
     }
     __syncthreads();
-    // G tiles: 16 energies x 8 output slots per warp step
-    const int g8 = lane >> 2, t4 = lane & 3;
-    const int nfrag = (nn + 7) / 8;
-    for (int nf = warp; nf < nfrag; nf += nwarp) {
-      int rb = 0, cb = 0;
-      const int ob = nf * 8 + g8;
-      if (ob < nn) slot_rc(sa, a.mode, ob, rb, cb);
-      const double2* ur = Us + (size_t)rb * kp;
-      const double2* uc = Us + (size_t)cb * kp;
-      double cr[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, ci[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-      for (int k0 = 0; k0 < kp; k0 += 4) {
-        const int ka = k0 + t4;
-        const double2 pv = cmul(ur[ka], cconj(uc[ka]));
+    for (int tl = warp; tl < ntile; tl += nwarp) {
+      const int r = tiles[tl] & 0xffff, c0 = tiles[tl] >> 16;
+      const double2* u0 = Us + (size_t)r * S + t4;
+      const double2* u1 = r + 1 < n ? u0 + S : u0;
+      const double2* uc = Us + (size_t)min(c0 + g8, n - 1) * S + t4;
+      const double2* dp = Ds + (size_t)g8 * S + t4;
+      double xr[2][2][2], xi[2][2][2], yr[2][2][2], yi[2][2][2];   // [row][energy block][column]
 #pragma unroll
-        for (int mf = 0; mf < 2; ++mf) {
-          const double2 dv = Ds[(mf * 8 + g8) * kp + ka];
-          if (!ANTI) dmma(cr[mf][0], cr[mf][1], dv.x, pv.x);
-          dmma(cr[mf][0], cr[mf][1], -dv.y, pv.y);
-          if (!ANTI) dmma(ci[mf][0], ci[mf][1], dv.x, pv.y);
-          dmma(ci[mf][0], ci[mf][1], dv.y, pv.x);
-        }
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) xr[i][m][h] = xi[i][m][h] = yr[i][m][h] = yi[i][m][h] = 0.0;
+      for (int k0 = 0; k0 < kp; k0 += 4) {
+        const double2 cc = cconj(uc[k0]);
+        const double2 pv[2] = {cmul(u0[k0], cc), cmul(u1[k0], cc)};
+        const double2 dv[2] = {dp[k0], dp[8 * S + k0]};
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if (!ANTI) dmma(xr[i][m][0], xr[i][m][1], dv[m].x, pv[i].x);
+            if (!ANTI) dmma(xi[i][m][0], xi[i][m][1], dv[m].x, pv[i].y);
+            dmma(yr[i][m][0], yr[i][m][1], dv[m].y, pv[i].x);
+            dmma(yi[i][m][0], yi[i][m][1], dv[m].y, pv[i].y);
+          }
+      }
+      // the lane's columns c, c + 1 (n is even, so they exist together) against rows r, r + 1
+      const int c = c0 + 2 * t4;
+      if (c >= n) continue;
+      int pu[2], pl_[2];   // positions (r + i, c) and (c + i, r): each starts a pair of adjacent ones
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        pu[i] = a.mode == MODE_RAW ? (r + i) * n + c : sa.outinv[(r + i) * n + c];
+        pl_[i] = a.mode == MODE_RAW ? (c + i) * n + r : sa.outinv[(c + i) * n + r];
       }
 #pragma unroll
-      for (int mf = 0; mf < 2; ++mf) {
-        const int zr = mf * 8 + g8;
-        const int pl = item[zr];
-        if (pl < 0) continue;
+      for (int m = 0; m < 2; ++m) {
+        const int zr = m * 8 + g8;
+        const int pt = item[zr];
+        if (pt < 0) continue;
         const double w = ws[zr];
-        // the lane's two slots are adjacent (nn is even): one 4-byte store of both exponents
-        const int o0 = nf * 8 + 2 * t4;
-        uint32_t codes = 0;
+        double2 up[2][2], lo[2][2];   // G(r + i, c + h), G(c + i, r + h)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int o = o0 + j;
-          if (o >= nn) continue;
-          const double2 v = make_double2(cr[mf][j], ci[mf][j]);
-          double2 v1 = v;
-          if (a.mode == MODE_A_IMAG || a.mode == MODE_A_REAL) v1 = cscale(v, w);
-          else if (a.mode == MODE_B_REAL) v1 = cconj(v);
-          a.out[(int64_t)pl * nn + o] = v1;
-          codes |= (uint32_t)(uint16_t)exponent_code(v1) << (16 * j);
-          if (a.out2) {
-            // the other imaginary-axis operand of the same G: v = G[r][c] goes to slot
-            // (c, r) of the G^T layout (mode2 B) or, times w, to slot (r, c) of the G layout (mode2 A)
-            int r, c;
-            slot_rc(sa, a.mode, o, r, c);
-            const bool tr = a.mode2 == MODE_B_IMAG;
-            const int64_t i2 = (int64_t)pl * nn + sa.outinv[tr ? c * n + r : r * n + c];
-            const double2 v2 = tr ? v : cscale(v, w);
-            a.out2[i2] = v2;
-            if (a.eout2) a.eout2[i2] = exponent_code(v2);
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            up[i][h] = make_double2(xr[i][m][h] - yi[i][m][h], xi[i][m][h] + yr[i][m][h]);
+            lo[h][i] = make_double2(xr[i][m][h] + yi[i][m][h], yr[i][m][h] - xi[i][m][h]);
+          }
+        auto put = [&](double2* out, int16_t* eout, int pos, double2 v0, double2 v1, bool sc) {
+          if (sc) {
+            v0 = cscale(v0, w);
+            v1 = cscale(v1, w);
+          } else if (conj) {
+            v0 = cconj(v0);
+            v1 = cconj(v1);
+          }
+          const int64_t o = (int64_t)pt * nn + pos;
+          out[o] = v0;
+          out[o + 1] = v1;
+          if (eout) *reinterpret_cast<uint32_t*>(eout + o) = exponent_pair(v0, v1);
+        };
+        if (c == r) {
+          // positions (r + i, r + h) hold G(r + i, r + h) = up, or its transpose
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            put(a.out, a.eout, pu[i], swap ? up[0][i] : up[i][0], swap ? up[1][i] : up[i][1], scaled);
+            if (a.out2)
+              put(a.out2, a.eout2, pu[i], swap2 ? up[0][i] : up[i][0], swap2 ? up[1][i] : up[i][1], !swap2);
+          }
+        } else {
+          // G(q, p) at position (p, q): rows r + i take G(c + h, r + i), rows c + i take G(r + h, c + i)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            put(a.out, a.eout, pu[i], swap ? lo[0][i] : up[i][0], swap ? lo[1][i] : up[i][1], scaled);
+            put(a.out, a.eout, pl_[i], swap ? up[0][i] : lo[i][0], swap ? up[1][i] : lo[i][1], scaled);
+            if (a.out2) {
+              put(a.out2, a.eout2, pu[i], swap2 ? lo[0][i] : up[i][0], swap2 ? lo[1][i] : up[i][1], !swap2);
+              put(a.out2, a.eout2, pl_[i], swap2 ? up[0][i] : lo[i][0], swap2 ? up[1][i] : lo[i][1], !swap2);
+            }
           }
         }
-        if (a.eout && o0 < nn) *reinterpret_cast<uint32_t*>(a.eout + (int64_t)pl * nn + o0) = codes;
       }
     }
     __syncthreads();
@@ -370,8 +397,7 @@ cudaError_t launch_green_spectral(const GreenArgs& g, const double2* U, const do
   if (g.np <= 0) return cudaSuccess;
   if (g.n_e <= 0 || !U || !lam) return cudaErrorInvalidValue;
   if (!spectral_supported(g.mode, g.mode2, g.out2 != nullptr)) return cudaErrorInvalidValue;
-  if (g.out2 && !outinv) return cudaErrorInvalidValue;
-  if ((g.eout || g.eout2) && g.n % 2) return cudaErrorInvalidValue;   // paired 4-byte exponent stores
+  if (g.n % 2 || (g.mode != MODE_RAW && !outinv)) return cudaErrorInvalidValue;   // entries leave in pairs
   SpecArgs sa;
   sa.g = g;
   sa.U = U;
@@ -379,28 +405,17 @@ cudaError_t launch_green_spectral(const GreenArgs& g, const double2* U, const do
   sa.outinv = outinv;
   sa.kp = (g.n + 3) / 4 * 4;
   const size_t smem = spec_smem(g.n, sa.kp);
-  const bool anti = g.mode == MODE_A_REAL;
-  auto kernel = anti ? spec_green_kernel<true, kSpecThreads> : spec_green_kernel<false, kSpecThreads>;
+  auto kernel = g.mode == MODE_A_REAL ? spec_green_kernel<true> : spec_green_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSpecThreads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm <= 0) return cudaErrorInvalidValue;
-  int threads = kSpecThreads;
-  if (per_sm == 1) {
-    kernel = anti ? spec_green_kernel<true, 1024> : spec_green_kernel<false, 1024>;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 1024, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm <= 0) return cudaErrorInvalidValue;
-    threads = 1024;
-  }
   const int64_t ne = g.n_e;
   const int64_t ntask = ((g.p0 + g.np - 1) / ne - g.p0 / ne + 1) * ((ne + kSpecZ - 1) / kSpecZ);
   const int64_t grid = std::min<int64_t>(ntask, (int64_t)num_sms * per_sm);
-  kernel<<<(unsigned)grid, threads, smem, s>>>(sa);
+  kernel<<<(unsigned)grid, kSpecThreads, smem, s>>>(sa);
   return cudaGetLastError();
 }
 
