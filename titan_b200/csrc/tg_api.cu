@@ -190,6 +190,7 @@ struct tg_ctx {
   // (slots 4 .. 4 + kTriQSlots - 1: one per wave vector of a q-batched real axis)
   DevArray<double> d_triD[4 + kTriQSlots], d_triE[4 + kTriQSlots];
   DevArray<double2> d_triQ[4 + kTriQSlots];
+  DevArray<double2> d_triws;   // factors of z - T of a pass's points
   DevArray<unsigned char> d_clws;   // workspace of the thread-block-cluster Gauss-Jordan kernel
   // tg_expectation_noalloc: device address of the library's fixed scratch array on this
   // context's device (looked up by the context's first no-alloc call)
@@ -870,6 +871,11 @@ int chi_green(tg_ctx* c, const ChiView& v, const GreenArgs& g, const char* what)
   r.out = c->d_graw.p;
   r.out2 = nullptr;
   r.eout = r.eout2 = nullptr;
+  if (g.triQ) {
+    TG_CHECK(c, c->d_triws.ensure(tri_ws_entries(c->dimH, g.np)), "alloc factors");
+    r.triws = c->d_triws.p;
+    c->launches += 1;
+  }
   TG_CHECK(c, launch_green(r, c->num_sms, c->stream, nullptr), what);
   TG_CHECK(c, launch_gather(g, c->d_graw.p, g.mode, v.outmap, v.ld, g.out, g.eout, c->num_sms, c->stream), what);
   if (g.out2)

@@ -143,6 +143,7 @@ struct GreenArgs {
   const double2* triQ = nullptr;
   const int* trirows = nullptr;
   int tri_ns = 0;
+  double2* triws = nullptr;          // factors of the pass's points (tri_ws_entries)
   const int* outinv = nullptr;
   // optional exponent sidecars of out / out2 (spectral G only): per stored value the
   // frexp exponent of max(|Re|, |Im|), -32768 for zero or subnormal
@@ -237,6 +238,7 @@ int spectral_supported(int mode, int mode2, bool has_out2);
 int tri_supported(int n);
 cudaError_t launch_tridiag(double2* H, int64_t nk, int n, const int* rows, int ns, double* D, double* E,
                            double2* Q, int num_sms, cudaStream_t s);
+size_t tri_ws_entries(int n, int64_t np);
 cudaError_t launch_green_tri(const GreenArgs& g, int num_sms, cudaStream_t s);
 // per-CTA slices [grid][2 n] of the energy-summed diagonal spin blocks (uu, dd, ud, du per orbital)
 cudaError_t launch_spec_expect(const double2* U, const double* lam, int64_t nk, int n, const double* ylist, int64_t n_e,

@@ -22,10 +22,6 @@ namespace tg {
 namespace {
 
 constexpr int kTriThreads = 256;
-// tri_green_kernel: blocks of COLS columns of G per solve; COLS = 16 lets two CTAs share an
-// SM at n = 288, COLS = 96 solves every column of a system up to 96 rows at once
-constexpr int kTriColsBig = 96;
-constexpr int kTriColsSmall = 16;
 
 __device__ __forceinline__ double2 warp_sum2(double2 v) {
   for (int o = 16; o > 0; o >>= 1) {
@@ -149,39 +145,19 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-struct TriArgs {
-  GreenArgs g;
-};
-
-template <int COLS>
-__host__ __device__ inline size_t tri_smem(int n) {
-  return sizeof(double) * 2 * (size_t)n + sizeof(double2) * 2 * (size_t)n + sizeof(double2) * (size_t)n * (COLS + 1);
-}
-
-// One CTA per point (k, z) of a k-major pass: the LU of z - T (thread 0), then per block of COLS
-// columns c of S the solves (z - T) x_c = conj(Q_S(c, :))^T (one thread per column) and
-// G(S, c) = Q_S x_c on the FP64 tensor cores: tiles of MB 8-row fragments of Q_S by one 8-column
-// fragment of the block, K = n in steps of 4, tiles dealt to the warps in turn.  With COLS = 16
-// two CTAs per SM overlap one's serial LU and solves with the other's GEMM.  Output MODE_RAW: G
-// column-major per point, entries (r, c) of S x S only.
-template <int COLS, int MB, int MINB>
-__global__ void __launch_bounds__(kTriThreads, MINB) tri_green_kernel(TriArgs ta) {
-  constexpr int STRIDE = COLS + 1;   // padded row of the block in shared memory
-  constexpr int NF = COLS / 8;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const GreenArgs& a = ta.g;
-  const int n = a.n, ns = a.tri_ns;
-  double* Dk = reinterpret_cast<double*>(smem);         // [n]
-  double* Ek = Dk + n;                                  // [n]
-  double2* invd = reinterpret_cast<double2*>(Ek + n);   // [n] 1 / pivot
-  double2* lm = invd + n;                               // [n] multipliers e_i / d_i
-  double2* X = lm + n;                                  // [n][STRIDE]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-  const int g8 = lane >> 2, t4 = lane & 3;
-  const int64_t nn = (int64_t)n * n;
-  const int nmf = (ns + 7) / 8;
-  const int ngroups = (nmf + MB - 1) / MB;
-  for (int64_t pl = blockIdx.x; pl < a.np; pl += gridDim.x) {
+// G of S x S per point (k, z) of a k-major pass.  z - T = L D L^T (complex symmetric, no pivoting),
+// so with Q_S(s, :) the rows of Q
+//   G(s, c) = sum_i w_i(s) d_i^-1 v_i(c),   w = L^-1 Q_S(s, :)^T,   v = L^-1 Q_S(c, :)^H:
+// both factors are forward sweeps y_i = b_i + l_{i-1} y_{i-1}, one thread per row and per column
+// with its state in registers, so the sum streams over i in chunks of 8 (two DMMA steps) and no
+// solved block is ever stored.  Neither factor is solved backwards, and its rounding errors are
+// those of the LU solve (the same pivots; measured on the slabs down to Im z = 1e-3).
+//
+// tri_lu_kernel: the serial recurrence of the pivots, one thread per point, to global memory
+// (l_{i-1} and 1 / d_i, 32 bytes per i).
+__global__ void __launch_bounds__(64) tri_lu_kernel(GreenArgs a, double2* __restrict__ ld) {
+  const int n = a.n;
+  for (int64_t pl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; pl < a.np; pl += (int64_t)gridDim.x * blockDim.x) {
     const int64_t wi = a.p0 + pl;
     const int64_t ik = wi / a.n_e, ie = wi % a.n_e;
     double zx, zy;
@@ -192,248 +168,198 @@ __global__ void __launch_bounds__(kTriThreads, MINB) tri_green_kernel(TriArgs ta
       zx = a.zr + a.pts.x2[ie];
       zy = a.zi;
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      Dk[i] = a.triD[ik * n + i];
-      Ek[i] = a.triE[ik * n + i];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      // z - T = L U: d_0 = z - D_0, l_i = -E_i / d_i, d_{i+1} = z - D_{i+1} - E_i^2 / d_i (lm stores +E_i / d_i)
-      double2 d = make_double2(zx - Dk[0], zy);
-      for (int i = 0; i < n; ++i) {
-        const double s2 = d.x * d.x + d.y * d.y;
-        if (s2 == 0.0 && a.status) {
-          const int64_t pidx = wi + 1;
-          atomicMin(a.status, (int)(pidx < 0x7fffffff ? pidx : 0x7fffffff));
-        }
-        // |d|^2 >= (Im z)^2 keeps the Newton reciprocal in its range; the division covers the rest
-        const double inv = s2 > 1e-300 ? rcp_newton(s2) : (s2 > 0.0 ? 1.0 / s2 : 0.0);
-        const double2 id = make_double2(d.x * inv, -d.y * inv);
-        invd[i] = id;
-        if (i + 1 < n) {
-          const double2 l = cscale(id, Ek[i]);
-          lm[i] = l;
-          d = make_double2(zx - Dk[i + 1] - Ek[i] * l.x, zy - Ek[i] * l.y);
-        }
+    const double* Dk = a.triD + ik * n;
+    const double* Ek = a.triE + ik * n;
+    double2* out = ld + pl * 2 * (int64_t)n;
+    // d_0 = z - D_0, l_i = E_i / d_i, d_{i+1} = z - D_{i+1} - E_i l_i
+    double2 d = make_double2(zx - Dk[0], zy), l = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) {
+      const double s2 = d.x * d.x + d.y * d.y;
+      if (s2 == 0.0 && a.status) {
+        const int64_t pidx = wi + 1;
+        atomicMin(a.status, (int)(pidx < 0x7fffffff ? pidx : 0x7fffffff));
       }
-    }
-    const double2* Qk = a.triQ + ik * (int64_t)ns * n;
-    double2* Gp = a.out + pl * nn;
-    for (int cb = 0; cb < ns; cb += COLS) {
-      const int ncols = min(COLS, ns - cb);
-      // right-hand sides conj(Q_S(c, :)) of the block's columns (zero past the last)
-      for (int e = threadIdx.x; e < n * COLS; e += blockDim.x) {
-        const int t = e / n, i = e % n;
-        X[i * STRIDE + t] = t < ncols ? cconj(Qk[(int64_t)(cb + t) * n + i]) : make_double2(0.0, 0.0);
+      // |d|^2 >= (Im z)^2 keeps the Newton reciprocal in its range; the division covers the rest
+      const double inv = s2 > 1e-300 ? rcp_newton(s2) : (s2 > 0.0 ? 1.0 / s2 : 0.0);
+      const double2 id = make_double2(d.x * inv, -d.y * inv);
+      out[2 * i] = l;
+      out[2 * i + 1] = id;
+      if (i + 1 < n) {
+        const double e = Ek[i];
+        l = cscale(id, e);
+        d = make_double2(zx - Dk[i + 1] - e * l.x, zy - e * l.y);
       }
-      __syncthreads();
-      if (threadIdx.x < ncols) {
-        double2* x = X + threadIdx.x;
-        double2 y = x[0];
-        for (int i = 1; i < n; ++i) {   // L y = b
-          y = cfma(lm[i - 1], y, x[i * STRIDE]);
-          x[i * STRIDE] = y;
-        }
-        double2 xi = cmul(y, invd[n - 1]);   // U x = y
-        x[(n - 1) * STRIDE] = xi;
-        for (int i = n - 2; i >= 0; --i) {
-          xi = cmul(cadd(x[i * STRIDE], cscale(xi, Ek[i])), invd[i]);
-          x[i * STRIDE] = xi;
-        }
-      }
-      __syncthreads();
-      // G(S, cb + t) = Q_S X: tile (M group mg, column fragment nf) -> warp (tile mod warps)
-      const int nfl = (ncols + 7) / 8;
-      for (int tile = warp; tile < ngroups * nfl; tile += nwarp) {
-        const int nf = tile % nfl, mg = tile / nfl;
-        double cr[MB][2], ci[MB][2];
-        const double2* qrow[MB];
-        bool live[MB];
-#pragma unroll
-        for (int u = 0; u < MB; ++u) {
-          cr[u][0] = cr[u][1] = ci[u][0] = ci[u][1] = 0.0;
-          const int row = (mg * MB + u) * 8 + g8;
-          live[u] = row < ns;
-          qrow[u] = Qk + (int64_t)(live[u] ? row : 0) * n;
-        }
-        for (int k0 = 0; k0 < n; k0 += 4) {
-          const int kk = k0 + t4;
-          const bool kin = kk < n;
-          const double2 b = kin ? X[kk * STRIDE + nf * 8 + g8] : make_double2(0.0, 0.0);
-#pragma unroll
-          for (int u = 0; u < MB; ++u) {
-            const double2 av = live[u] && kin ? qrow[u][kk] : make_double2(0.0, 0.0);
-            dmma(cr[u][0], cr[u][1], av.x, b.x);
-            dmma(cr[u][0], cr[u][1], -av.y, b.y);
-            dmma(ci[u][0], ci[u][1], av.x, b.y);
-            dmma(ci[u][0], ci[u][1], av.y, b.x);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < MB; ++u) {
-          const int row = (mg * MB + u) * 8 + g8;
-          if (row >= ns) continue;
-          const int r = a.trirows[row];
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const int t = nf * 8 + 2 * t4 + j;
-            if (t < ncols) Gp[(int64_t)a.trirows[cb + t] * n + r] = make_double2(cr[u][j], ci[u][j]);
-          }
-        }
-      }
-      __syncthreads();
     }
   }
 }
 
-// Systems of at most 96 rows: Q_S stays in shared memory for all the points of its k (each CTA
-// walks a contiguous range of the k-major pass), so the GEMM reads both operands from shared
-// memory.  Per point: the LU of z - T, then two blocks of 48 columns, each solved one thread per
-// column and multiplied on the FP64 tensor cores by a 4 x 2 grid of warps, each holding 3 x 3
-// fragments of 8 x 8.
-constexpr int kSmallRows = 96;
-constexpr int kSmallCols = 48;
+// One CTA per point and tile of G: eight warps in a 4 x 2 grid, FM x FN fragments of 8 x 8 each
+// (tile 32 FM x 16 FN).  Per chunk of 8 steps i every sweeping thread fetches its 8 entries of
+// Q_S two chunks ahead (cp.async, its own 128 bytes, so no barrier), advances its state and
+// leaves w_i / d_i or v_i in the double-buffered operand tiles; one barrier per chunk.  The
+// DMMAs bound it: 4 FM FN per warp and 4 steps against FM + FN shared-memory reads.
+constexpr int kTriK = 8, kTriStages = 3;
 
-__host__ __device__ inline size_t tri_small_smem(int n) {
-  return sizeof(double) * 2 * (size_t)n + sizeof(double2) * 2 * (size_t)n +
-         sizeof(double2) * (size_t)n * (kSmallCols + 1) + sizeof(double2) * (size_t)kSmallRows * (n + 1);
-}
+template <int FM, int FN>
+struct TriTile {
+  static constexpr int TM = 32 * FM, TN = 16 * FN;
+  static constexpr int SA = TM + 2, SB = TN + 2;   // 2 mod 8: four steps i and two rows apart
+  static constexpr int SQ = kTriK + 1;
+  static constexpr size_t smem =
+      sizeof(double2) * (kTriStages * ((size_t)(TM + TN) * SQ + 2 * kTriK) + 2 * kTriK * (size_t)(SA + SB));
+};
 
-__global__ void __launch_bounds__(kTriThreads, 1) tri_green_small_kernel(TriArgs ta) {
-  constexpr int XS = kSmallCols + 1;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const GreenArgs& a = ta.g;
-  const int n = a.n, ns = a.tri_ns, AS = n + 1;
-  double* Dk = reinterpret_cast<double*>(smem);         // [n]
-  double* Ek = Dk + n;                                  // [n]
-  double2* invd = reinterpret_cast<double2*>(Ek + n);   // [n]
-  double2* lm = invd + n;                               // [n]
-  double2* X = lm + n;                                  // [n][XS]
-  double2* As = X + (size_t)n * XS;                     // [ns][AS] = Q_S of the current k
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+template <int FM, int FN>
+__global__ void __launch_bounds__(kTriThreads, 1) tri_green_kernel(GreenArgs a, const double2* __restrict__ ld,
+                                                                  int tiles_m, int tiles_n) {
+  using TT = TriTile<FM, FN>;
+  constexpr int TM = TT::TM, TN = TT::TN, SA = TT::SA, SB = TT::SB, SQ = TT::SQ;
+  static_assert(TM + TN <= kTriThreads, "a thread per row and per column of the tile");
+  extern __shared__ __align__(16) double2 tsm[];
+  double2* qst = tsm;                                              // [stage][TM + TN][SQ]
+  double2* lst = qst + kTriStages * (size_t)(TM + TN) * SQ;        // [stage][2 kTriK]
+  double2* As = lst + kTriStages * 2 * kTriK;                      // [2][kTriK][SA]
+  double2* Bs = As + 2 * kTriK * SA;                               // [2][kTriK][SB]
+  const int n = a.n, ns = a.tri_ns;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g8 = lane >> 2, t4 = lane & 3;
-  const int wm = warp >> 1, wn = warp & 1;   // 4 x 2 warp grid: M fragments 3 wm.., N fragments 3 wn..
+  const int wm = (warp >> 1) * 8 * FM, wn = (warp & 1) * 8 * FN;
   const int64_t nn = (int64_t)n * n;
-  const int64_t per = (a.np + gridDim.x - 1) / gridDim.x;
-  const int64_t p_begin = blockIdx.x * per, p_end = min(a.np, p_begin + per);
-  int64_t k_loaded = -1;
-  for (int64_t pl = p_begin; pl < p_end; ++pl) {
-    const int64_t wi = a.p0 + pl;
-    const int64_t ik = wi / a.n_e, ie = wi % a.n_e;
-    double zx, zy;
-    if (a.pts.kind == 0) {
-      zx = a.zr;
-      zy = a.zi + a.ylist[ie];
-    } else {
-      zx = a.zr + a.pts.x2[ie];
-      zy = a.zi;
-    }
-    __syncthreads();   // the previous point is done with As, Dk, Ek
-    if (ik != k_loaded) {
-      const double2* Qk = a.triQ + ik * (int64_t)ns * n;
-      for (int e = threadIdx.x; e < ns * n; e += blockDim.x) As[(e / n) * AS + e % n] = Qk[e];
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        Dk[i] = a.triD[ik * n + i];
-        Ek[i] = a.triE[ik * n + i];
-      }
-      k_loaded = ik;
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      double2 d = make_double2(zx - Dk[0], zy);
-      for (int i = 0; i < n; ++i) {
-        const double s2 = d.x * d.x + d.y * d.y;
-        if (s2 == 0.0 && a.status) {
-          const int64_t pidx = wi + 1;
-          atomicMin(a.status, (int)(pidx < 0x7fffffff ? pidx : 0x7fffffff));
-        }
-        // |d|^2 >= (Im z)^2 keeps the Newton reciprocal in its range; the division covers the rest
-        const double inv = s2 > 1e-300 ? rcp_newton(s2) : (s2 > 0.0 ? 1.0 / s2 : 0.0);
-        const double2 id = make_double2(d.x * inv, -d.y * inv);
-        invd[i] = id;
-        if (i + 1 < n) {
-          const double2 l = cscale(id, Ek[i]);
-          lm[i] = l;
-          d = make_double2(zx - Dk[i + 1] - Ek[i] * l.x, zy - Ek[i] * l.y);
-        }
+  const int nch = (n + kTriK - 1) / kTriK;
+  const int tiles = tiles_m * tiles_n;
+  const int64_t items = a.np * tiles;
+  const bool sweeps = tid < TM + TN, isrow = tid < TM;
+  double2 state = make_double2(0.0, 0.0);
+
+  // this thread's row or column of the item's tile (null past the end), and its chunk loads
+  auto source = [&](int64_t item) -> const double2* {
+    const int64_t pl = item / tiles;
+    const int t = (int)(item - pl * tiles);
+    const int64_t ik = (a.p0 + pl) / a.n_e;
+    const int s = isrow ? (t % tiles_m) * TM + tid : (t / tiles_m) * TN + tid - TM;
+    return sweeps && s < ns ? a.triQ + (ik * ns + s) * (int64_t)n : nullptr;
+  };
+  auto fetch = [&](int64_t item, const double2* q, int ck) {
+    const int st = ck % kTriStages, i0 = ck * kTriK;
+    if (q) {
+      double2* dst = qst + ((size_t)st * (TM + TN) + tid) * SQ;
+#pragma unroll
+      for (int u = 0; u < kTriK; ++u) {
+        const bool in = i0 + u < n;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(dst + u)),
+                     "l"(in ? q + i0 + u : q), "r"(in ? 16 : 0));
       }
     }
+    if (tid < 2 * kTriK) {
+      const bool in = i0 + (tid >> 1) < n;
+      const double2* src = ld + (item / tiles) * 2 * (int64_t)n + (in ? 2 * i0 + tid : 0);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(lst + st * 2 * kTriK + tid)),
+                   "l"(src), "r"(in ? 16 : 0));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  auto advance = [&](bool live, int ck) {   // chunk ck of the sweep into operand buffer ck & 1
+    if (!sweeps) return;
+    const int st = ck % kTriStages;
+    const double2* q = qst + ((size_t)st * (TM + TN) + tid) * SQ;
+    const double2* l = lst + st * 2 * kTriK;
+    double2* dst = isrow ? As + (ck & 1) * kTriK * SA + tid : Bs + (ck & 1) * kTriK * SB + tid - TM;
+    const int step = isrow ? SA : SB;
+    double2 b[kTriK];
+#pragma unroll
+    for (int u = 0; u < kTriK; ++u) b[u] = live ? q[u] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < kTriK; ++u) {   // (past n: l, 1 / d and q are zero)
+      if (!isrow) b[u].y = -b[u].y;
+      state = cfma(l[2 * u], state, b[u]);
+      b[u] = isrow ? cmul(state, l[2 * u + 1]) : state;
+    }
+#pragma unroll
+    for (int u = 0; u < kTriK; ++u) dst[u * step] = b[u];
+  };
+
+  int64_t item = blockIdx.x;
+  const double2* q = item < items ? source(item) : nullptr;
+  if (item < items) {
+    fetch(item, q, 0);
+    if (nch > 1) fetch(item, q, 1);
+    else asm volatile("cp.async.commit_group;\n" ::);
+  }
+  for (; item < items; item += gridDim.x) {
+    double cr[FM][FN][2], ci[FM][FN][2];
+#pragma unroll
+    for (int u = 0; u < FM; ++u)
+#pragma unroll
+      for (int v = 0; v < FN; ++v) cr[u][v][0] = cr[u][v][1] = ci[u][v][0] = ci[u][v][1] = 0.0;
+    state = make_double2(0.0, 0.0);
+    // before chunk ck is multiplied, chunk ck + 1 is swept into the other operand buffer
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncthreads();
+    advance(q != nullptr, 0);
+    if (2 < nch) fetch(item, q, 2);
+    else asm volatile("cp.async.commit_group;\n" ::);
+    const int64_t nitem = item + gridDim.x;
+    const double2* nq = nitem < items ? source(nitem) : nullptr;
+    for (int ck = 0; ck < nch; ++ck) {
+      asm volatile("cp.async.wait_group 1;\n" ::);
+      __syncthreads();   // operands of chunk ck and the factors of chunk ck + 1 are in place
+      if (ck + 1 < nch) advance(q != nullptr, ck + 1);
+      if (ck + 3 < nch) fetch(item, q, ck + 3);
+      else asm volatile("cp.async.commit_group;\n" ::);
+      const double2* A = As + (ck & 1) * kTriK * SA;
+      const double2* B = Bs + (ck & 1) * kTriK * SB;
+#pragma unroll 1
+      for (int kk = 0; kk < kTriK; kk += 4) {
+        double2 bv[FN];
+#pragma unroll
+        for (int v = 0; v < FN; ++v) bv[v] = B[(kk + t4) * SB + wn + 8 * v + g8];
+#pragma unroll
+        for (int u = 0; u < FM; ++u) {
+          const double2 av = A[(kk + t4) * SA + wm + 8 * u + g8];
+#pragma unroll
+          for (int v = 0; v < FN; ++v) {
+            dmma(cr[u][v][0], cr[u][v][1], av.x, bv[v].x);
+            dmma(ci[u][v][0], ci[u][v][1], av.x, bv[v].y);
+            dmma(cr[u][v][0], cr[u][v][1], -av.y, bv[v].y);
+            dmma(ci[u][v][0], ci[u][v][1], av.y, bv[v].x);
+          }
+        }
+      }
+    }
+    // the next item's first chunks travel while this one's results leave
+    __syncthreads();
+    if (nitem < items) {
+      fetch(nitem, nq, 0);
+      if (nch > 1) fetch(nitem, nq, 1);
+      else asm volatile("cp.async.commit_group;\n" ::);
+    }
+    const int64_t pl = item / tiles;
+    const int t = (int)(item - pl * tiles);
+    const int rb = (t % tiles_m) * TM + wm, cb = (t / tiles_m) * TN + wn;
     double2* Gp = a.out + pl * nn;
-    for (int cb = 0; cb < ns; cb += kSmallCols) {
-      const int ncols = min(kSmallCols, ns - cb);
-      for (int e = threadIdx.x; e < n * kSmallCols; e += blockDim.x) {
-        const int t = e / n, i = e % n;
-        X[i * XS + t] = t < ncols ? cconj(As[(cb + t) * AS + i]) : make_double2(0.0, 0.0);
-      }
-      __syncthreads();
-      if (threadIdx.x < ncols) {
-        double2* x = X + threadIdx.x;
-        double2 y = x[0];
-        for (int i = 1; i < n; ++i) {
-          y = cfma(lm[i - 1], y, x[i * XS]);
-          x[i * XS] = y;
+#pragma unroll
+    for (int u = 0; u < FM; ++u) {
+      const int row = rb + 8 * u + g8;
+      if (row >= ns) continue;
+      const int r = a.trirows[row];
+#pragma unroll
+      for (int v = 0; v < FN; ++v)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = cb + 8 * v + 2 * t4 + h;
+          if (c < ns) Gp[(int64_t)a.trirows[c] * n + r] = make_double2(cr[u][v][h], ci[u][v][h]);
         }
-        double2 xi = cmul(y, invd[n - 1]);
-        x[(n - 1) * XS] = xi;
-        for (int i = n - 2; i >= 0; --i) {
-          xi = cmul(cadd(x[i * XS], cscale(xi, Ek[i])), invd[i]);
-          x[i * XS] = xi;
-        }
-      }
-      __syncthreads();
-      double cr[3][3][2], ci[3][3][2];
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-#pragma unroll
-        for (int v = 0; v < 3; ++v) cr[u][v][0] = cr[u][v][1] = ci[u][v][0] = ci[u][v][1] = 0.0;
-      for (int k0 = 0; k0 < n; k0 += 4) {
-        const int kk = k0 + t4;
-        const bool kin = kk < n;
-        double2 av[3], bv[3];
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-          const int row = (3 * wm + u) * 8 + g8;
-          av[u] = kin && row < ns ? As[row * AS + kk] : make_double2(0.0, 0.0);
-          bv[u] = kin ? X[kk * XS + (3 * wn + u) * 8 + g8] : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-#pragma unroll
-          for (int v = 0; v < 3; ++v) {
-            dmma(cr[u][v][0], cr[u][v][1], av[u].x, bv[v].x);
-            dmma(cr[u][v][0], cr[u][v][1], -av[u].y, bv[v].y);
-            dmma(ci[u][v][0], ci[u][v][1], av[u].x, bv[v].y);
-            dmma(ci[u][v][0], ci[u][v][1], av[u].y, bv[v].x);
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        const int row = (3 * wm + u) * 8 + g8;
-        if (row >= ns) continue;
-        const int r = a.trirows[row];
-#pragma unroll
-        for (int v = 0; v < 3; ++v)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const int t = (3 * wn + v) * 8 + 2 * t4 + j;
-            if (t < ncols) Gp[(int64_t)a.trirows[cb + t] * n + r] = make_double2(cr[u][v][j], ci[u][v][j]);
-          }
-      }
-      __syncthreads();
     }
+    q = nq;
   }
 }
 
 }  // namespace
 
-int tri_optin() {
-  int dev = 0, optin = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-  return optin;
-}
-
-int tri_supported(int n) { return n >= 2 && tri_smem<kTriColsSmall>(n) <= (size_t)tri_optin(); }
+int tri_supported(int n) { return n >= 2 && n <= 288; }
 
 cudaError_t launch_tridiag(double2* H, int64_t nk, int n, const int* rows, int ns, double* D, double* E,
                            double2* Q, int num_sms, cudaStream_t s) {
@@ -447,45 +373,60 @@ cudaError_t launch_tridiag(double2* H, int64_t nk, int n, const int* rows, int n
   return cudaGetLastError();
 }
 
-template <int COLS, int MB, int MINB>
-cudaError_t launch_tri_cols(const GreenArgs& g, int num_sms, cudaStream_t s) {
-  const size_t smem = tri_smem<COLS>(g.n);
-  auto kernel = tri_green_kernel<COLS, MB, MINB>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+namespace {
+
+template <int FM, int FN>
+cudaError_t launch_tri_tile(const GreenArgs& g, int num_sms, cudaStream_t s) {
+  using TT = TriTile<FM, FN>;
+  auto kernel = tri_green_kernel<FM, FN>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT::smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTriThreads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTriThreads, TT::smem);
   if (e != cudaSuccess) return e;
   if (per_sm <= 0) return cudaErrorInvalidValue;
-  TriArgs ta;
-  ta.g = g;
-  const int64_t grid = std::min<int64_t>(g.np, (int64_t)num_sms * per_sm);
-  kernel<<<(unsigned)grid, kTriThreads, smem, s>>>(ta);
+  const int tm = (g.tri_ns + TT::TM - 1) / TT::TM, tn = (g.tri_ns + TT::TN - 1) / TT::TN;
+  const int64_t grid = std::min<int64_t>(g.np * tm * tn, (int64_t)num_sms * per_sm);
+  kernel<<<(unsigned)grid, kTriThreads, TT::smem, s>>>(g, g.triws, tm, tn);
   return cudaGetLastError();
 }
 
+}  // namespace
+
+size_t tri_ws_entries(int n, int64_t np) { return (size_t)np * 2 * n; }
+
 cudaError_t launch_green_tri(const GreenArgs& g, int num_sms, cudaStream_t s) {
   if (g.np <= 0) return cudaSuccess;
-  if (g.mode != MODE_RAW || g.out2 || !g.triD || !g.triE || !g.triQ || !g.trirows || g.tri_ns <= 0 ||
+  if (g.mode != MODE_RAW || g.out2 || !g.triD || !g.triE || !g.triQ || !g.trirows || !g.triws || g.tri_ns <= 0 ||
       g.tri_ns > g.n || g.n_e <= 0)
     return cudaErrorInvalidValue;
   if (!tri_supported(g.n)) return cudaErrorInvalidValue;
-  // up to 96 rows: Q_S resident in shared memory per k
-  if (g.n <= kSmallRows && g.tri_ns <= kSmallRows && tri_small_smem(g.n) <= (size_t)tri_optin()) {
-    const size_t smem = tri_small_smem(g.n);
-    cudaError_t e = cudaFuncSetAttribute(tri_green_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    TriArgs ta;
-    ta.g = g;
-    const int64_t grid = std::min<int64_t>(g.np, (int64_t)num_sms);
-    tri_green_small_kernel<<<(unsigned)grid, kTriThreads, smem, s>>>(ta);
-    return cudaGetLastError();
+  const int64_t blocks = std::min<int64_t>((g.np + 63) / 64, (int64_t)num_sms * 16);
+  tri_lu_kernel<<<(unsigned)blocks, 64, 0, s>>>(g, g.triws);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // the tile shape whose tiles cover the fewest entries of G beyond ns x ns (the DMMAs of the
+  // padding cost as much as the others); larger ones first, for their operand reuse
+  struct Shape {
+    int m, n;
+  };
+  const Shape shapes[] = {{160, 80}, {96, 96}, {128, 64}, {64, 64}};
+  int best = 0;
+  int64_t least = 0;
+  for (int i = 0; i < 4; ++i) {
+    const int64_t area = (int64_t)((g.tri_ns + shapes[i].m - 1) / shapes[i].m * shapes[i].m) *
+                         ((g.tri_ns + shapes[i].n - 1) / shapes[i].n * shapes[i].n);
+    if (i == 0 || area < least) {
+      best = i;
+      least = area;
+    }
   }
-  // every column in one block where the rows of chi are few and the block fits
-  if (g.tri_ns <= kTriColsBig && tri_smem<kTriColsBig>(g.n) <= (size_t)tri_optin())
-    return launch_tri_cols<kTriColsBig, 6, 1>(g, num_sms, s);
-  return launch_tri_cols<kTriColsSmall, 5, 2>(g, num_sms, s);
+  switch (best) {
+    case 0: return launch_tri_tile<5, 5>(g, num_sms, s);
+    case 1: return launch_tri_tile<3, 6>(g, num_sms, s);
+    case 2: return launch_tri_tile<4, 4>(g, num_sms, s);
+    default: return launch_tri_tile<2, 4>(g, num_sms, s);
+  }
 }
 
 }  // namespace tg
