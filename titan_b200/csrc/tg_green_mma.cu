@@ -1,27 +1,24 @@
 // Blocked complex Gauss-Jordan inversion with FP64 tensor-core updates, fused with H(k).
 //
-// One CTA of W warps owns one (k, z) matrix in shared memory (row-major, stride = 1 mod 8
-// complex, so that the 16-byte accesses of a quarter warp to neighbouring rows or columns
-// fall into distinct banks).  Columns are eliminated in panels of four, the K of one DMMA
-// (mma.sync m8n8k4 .f64; tcgen05 has no FP64 kind):
+// One CTA of W warps owns one (k, z) matrix in shared memory (row-major, odd stride, so that
+// the 16-byte accesses of a quarter warp to neighbouring rows or columns fall into distinct
+// banks).  Columns are eliminated in panels of four, the K of one DMMA (mma.sync m8n8k4 .f64;
+// tcgen05 has no FP64 kind):
 //   * warp 0 factors the n x 4 panel in registers, a lane per row (two or three rows per
 //     lane beyond 32): per column the largest |Re| + |Im| of the rows not yet used, first
 //     row on ties (zgetrf's izamax choice; three integer warp reductions on the bits of the
 //     value), then the in-place Gauss-Jordan step on the four columns.  Its result X holds
 //     the inverse of the 4 x 4 pivot block P in the pivot rows, -A_r P^-1 in the others.
-//   * every other column block is updated as A <- A' + X A_P (A' = A with the pivot rows
-//     zeroed, A_P the four pivot rows before the update): 8 x 8 fragments, four real DMMAs
-//     each.  A warp owns whole column blocks, so A_P is read by the warp that overwrites it.
-//   * look-ahead: warp 0 updates the column block of the next panel and factors it while
-//     the other warps update the rest; one CTA barrier per panel.
+//   * every other column is updated as A <- A' + X A_P (A' = A with the pivot rows zeroed, A_P
+//     the four pivot rows before the update): 8 x 8 fragments, four real DMMAs each.  A warp
+//     owns whole blocks of 8 columns, so A_P is read by the warp that overwrites it.
+//   * look-ahead: warp 0 applies the update to the next panel's four columns itself, in
+//     registers, and factors it while the other warps update the rest; one CTA barrier per
+//     panel.
 // Rows are never swapped: G[r][s] = X[piv[r]][pinv[s]], applied by the output stage, which
 // writes the operand layouts (w G, G^T, w (G - G^+), conj G), raw G, H(k) or the
 // expectation sums.
 //
-// What bounds it: the serial panel (about 18 dependent FP64 operations and five warp
-// exchanges per column), overlapped with the updates of the other warps and of the other
-// CTAs of the SM; the update itself needs as many shared-memory as DMMA cycles (64 bytes
-// per lane and 8 x 8 fragment against four DMMAs of 16 cycles per sub-partition).
 #include "tg_internal.cuh"
 
 #include <algorithm>
@@ -41,9 +38,9 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
 template <int N>
 struct MmaDim {
   static constexpr int NB = (N + 7) / 8;        // row and column blocks of 8
-  static constexpr int ROWS = 8 * NB;           // padded with zero rows and columns
-  static constexpr int S = ROWS + 1;            // row stride, 1 mod 8
+  static constexpr int S = N + 1;               // row stride, odd (N is even)
   static constexpr int NP = (N + kPanel - 1) / kPanel;
+  static constexpr int X_SIZE = N * kPanel;
 };
 
 struct MmaSmem {
@@ -55,8 +52,8 @@ __host__ __device__ inline MmaSmem mma_smem(int n_neigh, bool expect) {
   using D = MmaDim<N>;
   MmaSmem L;
   size_t o = 0;
-  L.a = o;     o += sizeof(double2) * (size_t)D::ROWS * D::S;
-  L.x = o;     o += sizeof(double2) * 2 * (size_t)D::ROWS * kPanel;
+  L.a = o;     o += sizeof(double2) * (size_t)N * D::S;
+  L.x = o;     o += sizeof(double2) * 2 * (size_t)D::X_SIZE;
   L.prow = o;  o += sizeof(double2) * 2 * kPanel;
   L.phase = o; o += sizeof(double2) * (size_t)(n_neigh > 0 ? n_neigh : 1);
   L.acc = o;   o += expect ? sizeof(double2) * 2 * (size_t)N : 0;   // MODE_EXPECT sums (4 per orbital)
@@ -74,9 +71,11 @@ __device__ __forceinline__ void cta_sync() {
 
 // Factors panel t (columns 4 t ..): reads the columns from A, writes X to Xb and back into
 // A's columns, the pivot rows to piv.  One warp; `used` holds a bit per row slot of the lane.
-// Returns false when a column has no usable pivot.
-template <int N>
-__device__ __forceinline__ bool factor_panel(double2* A, double2* Xb, double2* prow, int* piv, int t, unsigned& used) {
+// PEND: the update of panel t - 1 (its X in Xp) has not reached these columns yet; it is applied
+// here to the rows in registers.  Returns false when a column has no usable pivot.
+template <int N, bool PEND>
+__device__ __forceinline__ bool factor_panel(double2* A, const double2* Xp, double2* Xb, double2* prow, int* piv, int t,
+                                             unsigned& used) {
   using D = MmaDim<N>;
   constexpr int RS = (N + 31) / 32;
   const int lane = threadIdx.x & 31;
@@ -87,8 +86,56 @@ __device__ __forceinline__ bool factor_panel(double2* A, double2* Xb, double2* p
   for (int s = 0; s < RS; ++s) {
     const int r = lane + 32 * s;
 #pragma unroll
-    for (int c = 0; c < kPanel; ++c) v[s][c] = r < N ? A[r * D::S + k0 + c] : make_double2(0.0, 0.0);
+    for (int c = 0; c < kPanel; ++c)
+      v[s][c] = r < N && (N % kPanel == 0 || k0 + c < N) ? A[r * D::S + k0 + c] : make_double2(0.0, 0.0);
   }
+  if (PEND) {
+    int q[kPanel];
+#pragma unroll
+    for (int k = 0; k < kPanel; ++k) q[k] = piv[k0 - kPanel + k];   // (panel t - 1 is a full one)
+#pragma unroll
+    for (int s = 0; s < RS; ++s) {
+      const int r = lane + 32 * s;
+      if (r == q[0] || r == q[1] || r == q[2] || r == q[3]) {
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) v[s][c] = make_double2(0.0, 0.0);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kPanel; ++k) {
+      double2 b[kPanel], x[RS];
+#pragma unroll
+      for (int c = 0; c < kPanel; ++c)
+        b[c] = N % kPanel == 0 || k0 + c < N ? A[q[k] * D::S + k0 + c] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int s = 0; s < RS; ++s) x[s] = lane + 32 * s < N ? Xp[(lane + 32 * s) * kPanel + k] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int s = 0; s < RS; ++s)
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) v[s][c] = cfma(x[s], b[c], v[s][c]);
+    }
+    __syncwarp();   // every lane has read the pivot rows' columns before they are overwritten
+  }
+  // pivot of column c: its row, or -1 past the last column
+  auto search = [&](int c, unsigned long long& key, int& row) {
+    key = 0ull;
+    row = 0x7fffffff;
+#pragma unroll
+    for (int s = 0; s < RS; ++s) {
+      const int r = lane + 32 * s;
+      const double m = fabs(v[s][c].x) + fabs(v[s][c].y);
+      const bool cand = r < N && !((used >> s) & 1u) && m > 0.0;
+      const unsigned long long b = cand ? (unsigned long long)__double_as_longlong(m) : 0ull;
+      if (cand && b > key) {   // bits of |Re| + |Im| (0: none, zero or NaN), first row on ties
+        key = b;
+        row = r;
+      }
+    }
+  };
+  unsigned long long key;
+  int row;
+  search(0, key, row);
+  unsigned mhi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
 #pragma unroll
   for (int c = 0; c < kPanel; ++c) {
     if (N % kPanel != 0 && k0 + c >= N) {   // past the last column: an inert step
@@ -97,22 +144,7 @@ __device__ __forceinline__ bool factor_panel(double2* A, double2* Xb, double2* p
       for (int s = 0; s < RS; ++s) v[s][c] = make_double2(0.0, 0.0);
       continue;
     }
-    // key: bits of |Re| + |Im| of the best unused row of the lane (0: none, zero or NaN)
-    unsigned long long key = 0ull;
-    int row = 0x7fffffff;
-#pragma unroll
-    for (int s = 0; s < RS; ++s) {
-      const int r = lane + 32 * s;
-      const double m = fabs(v[s][c].x) + fabs(v[s][c].y);
-      const bool cand = r < N && !((used >> s) & 1u) && m > 0.0;
-      const unsigned long long b = cand ? (unsigned long long)__double_as_longlong(m) : 0ull;
-      if (cand && b > key) {
-        key = b;
-        row = r;
-      }
-    }
     const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
     const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
     const bool any = (mhi | mlo) != 0u;
     int p = (int)__reduce_min_sync(0xffffffffu, any && hi == mhi && lo == mlo ? (unsigned)row : 0x7fffffffu);
@@ -126,29 +158,47 @@ __device__ __forceinline__ bool factor_panel(double2* A, double2* Xb, double2* p
       p = (int)__reduce_min_sync(0xffffffffu, (unsigned)fr);
     }
     double2* pr = prow + kPanel * (c & 1);
+    const bool owner = lane == (p & 31);
+    const int slot = p >> 5;   // the same in every lane
 #pragma unroll
     for (int s = 0; s < RS; ++s)
-      if (lane + 32 * s == p) {
+      if (slot == s && owner) {
 #pragma unroll
         for (int cc = 0; cc < kPanel; ++cc) pr[cc] = v[s][cc];
         used |= 1u << s;
+        piv[k0 + c] = p;
       }
-    if (lane == 0) piv[k0 + c] = p;
     __syncwarp();
-    const double2 d = crecip_fast(pr[c]);
     double2 pv[kPanel];
 #pragma unroll
-    for (int cc = 0; cc < kPanel; ++cc) pv[cc] = cc == c ? d : cmul(pr[cc], d);
+    for (int cc = 0; cc < kPanel; ++cc) pv[cc] = pr[cc];
+    const double2 d = crecip_fast(pv[c]);
 #pragma unroll
-    for (int s = 0; s < RS; ++s) {
-      const bool is_p = lane + 32 * s == p;
-      const double2 f = v[s][c];
+    for (int cc = 0; cc < kPanel; ++cc) pv[cc] = cc == c ? d : cmul(pv[cc], d);
+    double2 f[RS];
 #pragma unroll
-      for (int cc = 0; cc < kPanel; ++cc) {
-        const double2 u = cfms(f, pv[cc], cc == c ? make_double2(0.0, 0.0) : v[s][cc]);
-        v[s][cc] = is_p ? pv[cc] : u;
-      }
+    for (int s = 0; s < RS; ++s) f[s] = v[s][c];
+    // the next column first: its pivot search runs while the others are updated
+    const bool next = c + 1 < kPanel && (N % kPanel == 0 || k0 + c + 1 < N);
+    if (next) {
+      const int nc = c + 1 < kPanel ? c + 1 : c;
+#pragma unroll
+      for (int s = 0; s < RS; ++s) v[s][nc] = cfms(f[s], pv[nc], v[s][nc]);
+      search(nc, key, row);   // (the pivot row is marked used, so its stale value does not count)
+      mhi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
     }
+#pragma unroll
+    for (int cc = 0; cc < kPanel; ++cc) {
+      if (next && cc == c + 1) continue;
+#pragma unroll
+      for (int s = 0; s < RS; ++s) v[s][cc] = cfms(f[s], pv[cc], cc == c ? make_double2(0.0, 0.0) : v[s][cc]);
+    }
+#pragma unroll
+    for (int s = 0; s < RS; ++s)
+      if (slot == s && owner) {
+#pragma unroll
+        for (int cc = 0; cc < kPanel; ++cc) v[s][cc] = pv[cc];
+      }
   }
 #pragma unroll
   for (int s = 0; s < RS; ++s) {
@@ -157,16 +207,20 @@ __device__ __forceinline__ bool factor_panel(double2* A, double2* Xb, double2* p
 #pragma unroll
       for (int c = 0; c < kPanel; ++c) {
         Xb[r * kPanel + c] = v[s][c];
-        A[r * D::S + k0 + c] = v[s][c];   // (columns past N of the last panel stay zero)
+        if (N % kPanel == 0 || k0 + c < N) A[r * D::S + k0 + c] = v[s][c];
       }
     }
   }
   return ok;
 }
 
-// A <- A' + X A_P on the J column blocks jf, jf + step, ..; the panel's own four columns keep X
+// A <- A' + X A_P on the J column blocks jf, jf + step, ..; the four columns of panel t (they
+// hold X) and those of panel t + 1 (left to warp 0) are not stored.  Fragment rows and columns
+// past N read whatever lies there (clamped rows, the next row's first columns) and are not
+// stored either.
 template <int N, int J>
-__device__ __forceinline__ void update_blocks(double2* A, const double2* Xb, const int* piv, int t, int jf, int step) {
+__device__ __forceinline__ void update_blocks(double2* A, const double2* Xb, const int* piv, int t, int ahead, int jf,
+                                              int step) {
   using D = MmaDim<N>;
   const int lane = threadIdx.x & 31;
   const int g8 = lane >> 2, t4 = lane & 3;
@@ -178,26 +232,32 @@ __device__ __forceinline__ void update_blocks(double2* A, const double2* Xb, con
 #pragma unroll
   for (int i = 0; i < J; ++i) {
     const int j = jf + i * step;
-    b[i] = (N % kPanel == 0 || pr >= 0) ? A[pr * D::S + 8 * j + g8] : make_double2(0.0, 0.0);
-    keep[i] = j == (t >> 1) && (t4 >> 1) == (t & 1);   // this lane's two columns belong to the panel
+    const int panel = 2 * j + (t4 >> 1);   // panel of this lane's two columns of block j
+    const int bp = 2 * j + (g8 >> 2);      // panel of the column of A_P that this lane holds
+    const bool col = bp != t && !(ahead && bp == t + 1) && (N % 8 == 0 || 8 * j + g8 < N);
+    b[i] = col && (N % kPanel == 0 || pr >= 0) ? A[pr * D::S + 8 * j + g8] : make_double2(0.0, 0.0);
+    keep[i] = panel == t || (ahead && panel == t + 1) || (N % 8 != 0 && 8 * j + 2 * t4 >= N);
   }
   __syncwarp();   // A_P is read before any lane overwrites it
-  double2* Ap = A + g8 * D::S + 8 * jf + 2 * t4;
 #pragma unroll 2
   for (int bi = 0; bi < D::NB; ++bi) {
     const int r = 8 * bi + g8;
-    const double2 x = Xb[r * kPanel + t4];
+    const int rc = N % 8 == 0 ? r : min(r, N - 1);
+    const double2 x = Xb[rc * kPanel + t4];
     const bool zero = r == p0 || r == p1 || r == p2 || r == p3;
 #pragma unroll
     for (int i = 0; i < J; ++i) {
-      double2* c = Ap + bi * 8 * D::S + 8 * i * step;
-      double2 c0 = c[0], c1 = c[1];
-      if (zero) c0 = c1 = make_double2(0.0, 0.0);
+      double2* c = A + rc * D::S + 8 * (jf + i * step) + 2 * t4;
+      double2 c0 = make_double2(0.0, 0.0), c1 = c0;
+      if (!zero && !keep[i]) {
+        c0 = c[0];
+        c1 = c[1];
+      }
       dmma(c0.x, c1.x, x.x, b[i].x);
       dmma(c0.y, c1.y, x.x, b[i].y);
       dmma(c0.x, c1.x, -x.y, b[i].y);
       dmma(c0.y, c1.y, x.y, b[i].x);
-      if (!keep[i]) {
+      if (!keep[i] && (N % 8 == 0 || r < N)) {
         c[0] = c0;
         c[1] = c1;
       }
@@ -205,26 +265,14 @@ __device__ __forceinline__ void update_blocks(double2* A, const double2* Xb, con
   }
 }
 
+// every column block first, first + step, .. in pairs
 template <int N>
-__device__ __forceinline__ void update_list(double2* A, const double2* Xb, const int* piv, int t, int first, int step,
-                                            int skip) {
+__device__ __forceinline__ void update_list(double2* A, const double2* Xb, const int* piv, int t, int ahead, int first,
+                                            int step) {
   using D = MmaDim<N>;
-  // column blocks first, first + step, .. without `skip`, in pairs
   int j = first;
-  while (j < D::NB) {
-    if (j == skip) {
-      j += step;
-      continue;
-    }
-    const int j2 = j + step;
-    if (j2 < D::NB && j2 != skip) {
-      update_blocks<N, 2>(A, Xb, piv, t, j, step);
-      j = j2 + step;
-    } else {
-      update_blocks<N, 1>(A, Xb, piv, t, j, step);
-      j = j2;
-    }
-  }
+  for (; j + step < D::NB; j += 2 * step) update_blocks<N, 2>(A, Xb, piv, t, ahead, j, step);
+  if (j < D::NB) update_blocks<N, 1>(A, Xb, piv, t, ahead, j, step);
 }
 
 // OUT: 0 = operand / raw outputs, 1 = MODE_EXPECT, 2 = MODE_HK
@@ -241,10 +289,26 @@ __global__ void __launch_bounds__(32 * W, MINB) green_mma_kernel(GreenArgs a) {
   double2* eacc = reinterpret_cast<double2*>(smem + L.acc);
   int* piv = reinterpret_cast<int*>(smem + L.piv);
   int* pinv = reinterpret_cast<int*>(smem + L.pinv);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x;
+  // Warp 0 factors; the others update.  The scalar FP64 of the panel and the DMMAs share a
+  // sub-partition's pipe (warp id mod 4), so with W = 8 the fourth warp, its neighbour, takes no
+  // column blocks; with W = 2 every second pair of CTAs exchanges the two roles, or all the
+  // updates of an SM would sit on two of its four pipes.
+  int role = tid >> 5;
+  if (W == 2) {
+    if (tid == 0) {
+      unsigned wid;
+      asm volatile("mov.u32 %0, %%warpid;" : "=r"(wid));
+      piv[0] = (int)(wid >> 2) & 1;
+    }
+    __syncthreads();
+    role ^= piv[0];   // one choice for the CTA
+    __syncthreads();
+  }
+  constexpr int NU = W == 1 ? 1 : W == 8 ? 6 : W - 1;   // updating warps
+  const int mine = W == 8 ? (role == 4 ? -1 : role > 4 ? role - 2 : role - 1) : role - 1;
 
-  for (int e = tid; e < D::ROWS * D::S; e += T) A[e] = make_double2(0.0, 0.0);
-  for (int e = tid; e < 2 * D::ROWS * kPanel; e += T) X[e] = make_double2(0.0, 0.0);
+  for (int e = tid; e < N * D::S; e += T) A[e] = make_double2(0.0, 0.0);
   if (OUT == 1)
     for (int e = tid; e < 2 * N; e += T) eacc[e] = make_double2(0.0, 0.0);
   cta_sync<W>();
@@ -328,30 +392,25 @@ __global__ void __launch_bounds__(32 * W, MINB) green_mma_kernel(GreenArgs a) {
     // ---- blocked Gauss-Jordan ------------------------------------------------------
     unsigned used = 0u;
     bool ok = true;
-    if (warp == 0) ok = factor_panel<N>(A, X, prow, piv, 0, used);
+    if (role == 0) ok = factor_panel<N, false>(A, nullptr, X, prow, piv, 0, used);
     cta_sync<W>();
 #pragma unroll 1
     for (int t = 0; t < D::NP; ++t) {
-      const double2* Xt = X + (t & 1) * D::ROWS * kPanel;
-      double2* Xn = X + ((t + 1) & 1) * D::ROWS * kPanel;
+      const double2* Xt = X + (t & 1) * D::X_SIZE;
+      double2* Xn = X + ((t + 1) & 1) * D::X_SIZE;
       const bool more = t + 1 < D::NP;
-      const int jn = more ? (t + 1) >> 1 : -1;
       if (W == 1) {
-        update_list<N>(A, Xt, piv, t, 0, 1, -1);
+        update_list<N>(A, Xt, piv, t, 0, 0, 1);
         __syncwarp();
-        if (more) ok &= factor_panel<N>(A, Xn, prow, piv, t + 1, used);
-      } else if (warp == 0) {
-        if (more) {
-          update_blocks<N, 1>(A, Xt, piv, t, jn, 1);
-          __syncwarp();
-          ok &= factor_panel<N>(A, Xn, prow, piv, t + 1, used);
-        }
-      } else {
-        update_list<N>(A, Xt, piv, t, warp - 1, W - 1, jn);
+        if (more) ok &= factor_panel<N, false>(A, nullptr, Xn, prow, piv, t + 1, used);
+      } else if (role == 0) {
+        if (more) ok &= factor_panel<N, true>(A, Xt, Xn, prow, piv, t + 1, used);
+      } else if (mine >= 0) {
+        update_list<N>(A, Xt, piv, t, more ? 1 : 0, mine, NU);
       }
       cta_sync<W>();
     }
-    if (tid == 0 && !ok && a.status) {
+    if (role == 0 && (tid & 31) == 0 && !ok && a.status) {
       const int64_t pidx = a.p0 + pl + 1;
       atomicMin(a.status, (int)(pidx < 0x7fffffff ? pidx : 0x7fffffff));
     }
@@ -452,7 +511,7 @@ cudaError_t launch_green_mma(const GreenArgs& a, int num_sms, cudaStream_t s, in
   switch (a.n) {
     case 18: return launch_n<18, 1, 15>(a, num_sms, s, grid_used);
     case 36: return launch_n<36, 2, 8>(a, num_sms, s, grid_used);
-    case 40: return launch_n<40, 2, 7>(a, num_sms, s, grid_used);
+    case 40: return launch_n<40, 2, 6>(a, num_sms, s, grid_used);
     case 54: return launch_n<54, 4, 3>(a, num_sms, s, grid_used);
     case 72: return launch_n<72, 4, 2>(a, num_sms, s, grid_used);
     case 90: return launch_n<90, 8, 1>(a, num_sms, s, grid_used);
