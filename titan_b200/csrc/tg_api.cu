@@ -379,8 +379,8 @@ int build_eig(tg_ctx* c, int slot, int64_t nk) {
   const size_t nn = (size_t)c->dimH * c->dimH;
   TG_CHECK(c, c->d_eigU[slot].ensure((size_t)nk * nn), "alloc eigenvectors");
   TG_CHECK(c, c->d_eigL[slot].ensure((size_t)nk * c->dimH), "alloc eigenvalues");
-  KindTimer kt(c, 0);
   TG_CHECK(c, c->d_eigws.ensure(eig_ws_bytes(c->dimH, nk)), "alloc rotations");
+  KindTimer kt(c, 0);
   TG_CHECK(c, launch_eig(c->d_htab[slot].p, nk, c->dimH, c->d_eigU[slot].p, c->d_eigL[slot].p, c->d_eigws.p,
                          c->d_eig_status.p, c->num_sms, c->stream),
            "eigendecomposition");
@@ -397,8 +397,8 @@ int build_eig_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
   TG_CHECK(c, c->d_eigL[slot].ensure((size_t)nk * n), "alloc eigenvalues");
   TG_CHECK(c, c->d_hchunk.ensure((size_t)kc * nn), "alloc H chunk");
   TG_CHECK(c, c->d_hphase.ensure((size_t)kc * std::max(c->n_neigh, 1)), "alloc phases");
-  TG_CHECK(c, c->d_qvec.upload(q, 3, c->stream), "upload q");
   TG_CHECK(c, c->d_eigws.ensure(eig_ws_bytes((int)n, kc)), "alloc rotations");
+  TG_CHECK(c, c->d_qvec.upload(q, 3, c->stream), "upload q");
   const GreenArgs a = base_args(c);
   KindTimer kt(c, 0);
   for (int64_t k0 = 0; k0 < nk; k0 += kc) {
@@ -428,9 +428,9 @@ bool eig_room(tg_ctx* c, int64_t nk, int s0, int s1) {
   }
   const size_t kc = std::min<size_t>((size_t)nk, std::max<size_t>(1, ((size_t)2 << 30) / (nn * 16)));
   if (c->d_hchunk.n < kc * nn) need += (double)(kc * nn - c->d_hchunk.n) * sizeof(double2);
-  return need <= 0.5 * (double)fr;
   const size_t ws = eig_ws_bytes(c->dimH, kc);
   if (c->d_eigws.n < ws) need += (double)(ws - c->d_eigws.n);
+  return need <= 0.5 * (double)fr;
 }
 
 // Householder tridiagonalisation of H(k + q) for a k list into slot `slot`: T and the rows
