@@ -699,11 +699,11 @@ int split_quantize_operand(tg_ctx* c, const ChiView& v, int which, const double2
   else
     TG_CHECK(c, split_rowmax(X, ld, pd, m64, c->stream), "split rowmax");
   if (which == 0)
-    TG_CHECK(c, split_quantize(X, ld, pd, v.sgA, (int)v.split->groupsA.size(), kSplitRowsA, m64, c->d_EA.p,
+    TG_CHECK(c, split_quantize(X, ld, pd, v.sgA, (int)v.split->groupsA.size(), kSplitRowsA, false, m64, c->d_EA.p,
                                c->d_digA.p, c->stream),
              "split quantize A");
   else
-    TG_CHECK(c, split_quantize(X, ld, pd, v.sgB, (int)v.split->groupsB.size(), kSplitColsB, m64, c->d_EB.p,
+    TG_CHECK(c, split_quantize(X, ld, pd, v.sgB, (int)v.split->groupsB.size(), kSplitColsB, true, m64, c->d_EB.p,
                                c->d_digB.p, c->stream),
              "split quantize B");
   c->launches += 2;

@@ -146,8 +146,8 @@ __global__ void split_bound_kernel(const unsigned long long* __restrict__ m64A,
 __global__ void __launch_bounds__(256) split_quantize_kernel(
     const double2* __restrict__ X, int64_t ld, int stride, int n_ksteps, const int* __restrict__ kchunk,
     const int* __restrict__ kstart, const int* __restrict__ slot0, const int* __restrict__ count,
-    const SplitGroup* __restrict__ groups, int n_groups, int rows, const unsigned long long* __restrict__ M64,
-    int* __restrict__ E, int8_t* __restrict__ dig) {
+    const SplitGroup* __restrict__ groups, int n_groups, int rows, int slice_stride, int half_stride,
+    const unsigned long long* __restrict__ M64, int* __restrict__ E, int8_t* __restrict__ dig) {
   const int64_t per_t = (int64_t)2 * n_groups * rows;
   const int64_t total = (int64_t)n_ksteps * per_t;
   const int64_t block_bytes = (int64_t)kSplitSlices * 2 * rows * kSplitK;
@@ -183,16 +183,16 @@ __global__ void __launch_bounds__(256) split_quantize_kernel(
       xr[k] = __double2ll_rn(v.x * scale);
       xi[k] = __double2ll_rn(v.y * scale);
     }
-    int8_t* blk = dig + ((int64_t)t * n_groups + g) * block_bytes + (int64_t)kc * 2 * rows * 16;
+    int8_t* blk = dig + ((int64_t)t * n_groups + g) * block_bytes + (int64_t)kc * half_stride;
     uint4 d[kSplitSlices];
     digits16(xr, d);
 #pragma unroll
     for (int i = 0; i < kSplitSlices; ++i)
-      *reinterpret_cast<uint4*>(blk + (int64_t)i * 2 * rows * kSplitK + (int64_t)r * 16) = d[i];
+      *reinterpret_cast<uint4*>(blk + (int64_t)i * slice_stride + (int64_t)r * 16) = d[i];
     digits16(xi, d);
 #pragma unroll
     for (int i = 0; i < kSplitSlices; ++i)
-      *reinterpret_cast<uint4*>(blk + (int64_t)i * 2 * rows * kSplitK + (int64_t)(rows + r) * 16) = d[i];
+      *reinterpret_cast<uint4*>(blk + (int64_t)i * slice_stride + (int64_t)(rows + r) * 16) = d[i];
   }
 }
 
@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(256) split_quantize_kernel(
 // ----------------------------------------------------------------------------
 
 constexpr int kMmaM = 128;
-constexpr int kMmaN = 2 * kSplitColsB;     // 80
+constexpr int kMmaN = 2 * kSplitColsB;     // 80 rows of one digit of B
+constexpr int kMmaDigits = 3;              // digits of B per MMA (N <= 256)
 constexpr int kLevels = 6;                 // L = 2..7
 constexpr int kStages = 5;
 constexpr int kStageBytes = kSplitABlock + kSplitBBlock;   // 39936
@@ -216,9 +217,9 @@ constexpr size_t kSplitSmem = 1024 + kBarOff + kNumBars * 8 + 16;
 static_assert(kSplitSmem <= 232448, "the stage ring must fit the 227 KB of shared memory per CTA");
 constexpr unsigned long long kWaitNs = 2000000000ull;        // 2 s per wait
 
-__host__ __device__ constexpr uint32_t idesc_i8() {
+__host__ __device__ constexpr uint32_t idesc_i8(int n) {
   // c_format S32 (2), a/b format signed int8 (1), both K-major, N >> 3, M >> 4
-  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kMmaN >> 3) << 17) | ((uint32_t)(kMmaM >> 4) << 24);
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kMmaM >> 4) << 24);
 }
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -416,7 +417,6 @@ __global__ void __launch_bounds__(kThreads, 1) split_contract_kernel(SplitContra
   } else if (warp == 1) {
     // ---------------- MMA issuer: one lane ----------------
     if (lane == 0) {
-      const uint32_t idesc = idesc_i8();
       uint32_t it = 0, d = 0;
       bool ok = true, issued = false;
       for (int un = blockIdx.x; un < nunits && ok; un += gridDim.x) {
@@ -435,19 +435,22 @@ __global__ void __launch_bounds__(kThreads, 1) split_contract_kernel(SplitContra
             tc_fence_after();
             const uint32_t sa = base + (uint32_t)s * kStageBytes;
             const uint32_t sb = sa + kSplitABlock;
-            // digit pairs (i, j) (0-based) with level l = i + j <= 5, grouped by level: 21 MMAs
+            // digit pairs (i, j) (0-based) with level l = i + j <= 5: digit i of A against up to
+            // three consecutive digits j0 .. of B, whose products belong to consecutive levels,
+            // i.e. to consecutive accumulator columns: 21 products in 9 MMAs of N = 240, 160 or
+            // 80, which read A's digit once for up to three of them
 #pragma unroll
-            for (int l = 0; l < kLevels; ++l) {
+            for (int i = 0; i < kSplitSlices; ++i) {
+              const uint64_t ad =
+                  smem_desc(sa + (uint32_t)i * (2 * kSplitRowsA * kSplitK), 2 * kSplitRowsA * 16, 128);
 #pragma unroll
-              for (int i = 0; i < kSplitSlices; ++i) {
-                const int j = l - i;
-                if (j < 0 || j >= kSplitSlices) continue;
-                const bool first = i == (l > kSplitSlices - 1 ? l - (kSplitSlices - 1) : 0);
-                const uint64_t ad =
-                    smem_desc(sa + (uint32_t)i * (2 * kSplitRowsA * kSplitK), 2 * kSplitRowsA * 16, 128);
+              for (int j0 = 0; j0 < kLevels - i; j0 += kMmaDigits) {
+                const int nd = kLevels - i - j0 < kMmaDigits ? kLevels - i - j0 : kMmaDigits;
                 const uint64_t bd =
-                    smem_desc(sb + (uint32_t)j * (2 * kSplitColsB * kSplitK), 2 * kSplitColsB * 16, 128);
-                umma_i8(tmem + (uint32_t)(l * kMmaN), ad, bd, idesc, (tt != t || !first) ? 1u : 0u);
+                    smem_desc(sb + (uint32_t)j0 * (kMmaN * 16), kSplitSlices * kMmaN * 16, 128);
+                // (digit 0 of A touches every level, so it starts the chunk's accumulators)
+                umma_i8(tmem + (uint32_t)((i + j0) * kMmaN), ad, bd, idesc_i8(nd * kMmaN),
+                        (tt != t || i > 0) ? 1u : 0u);
               }
             }
             umma_commit(bar0 + 8u * (kStages + s));
@@ -637,13 +640,17 @@ cudaError_t split_bound(const unsigned long long* m64A, const unsigned long long
 }
 
 cudaError_t split_quantize(const double2* X, int64_t ld, const SplitPassDev& p, const SplitGroup* groups,
-                           int n_groups, int rows, const unsigned long long* M64, int* E, int8_t* dig,
+                           int n_groups, int rows, bool b_layout, const unsigned long long* M64, int* E, int8_t* dig,
                            cudaStream_t s) {
   if (p.n_ksteps <= 0) return cudaSuccess;
   const int64_t total = (int64_t)p.n_ksteps * 2 * n_groups * rows;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
+  // A blocks [slice][k half][row], B blocks [k half][slice][row]: consecutive slices of B are
+  // consecutive rows of one MMA operand
+  const int plane = 2 * rows * 16;
+  const int slice_stride = b_layout ? plane : 2 * plane, half_stride = b_layout ? kSplitSlices * plane : plane;
   split_quantize_kernel<<<blocks, 256, 0, s>>>(X, ld, p.stride, p.n_ksteps, p.kchunk, p.kstart, p.slot0, p.count, groups,
-                                               n_groups, rows, M64, E, dig);
+                                               n_groups, rows, slice_stride, half_stride, M64, E, dig);
   return cudaGetLastError();
 }
 

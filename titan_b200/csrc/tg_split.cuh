@@ -16,12 +16,12 @@
 //
 // Operand digits live in HBM as K-step blocks (32 points), K-major in the
 // canonical no-swizzle core-matrix layout, so one bulk copy stages a block:
-//   A block (t, gA): [slice 5][k half 2][row 128][16 B], rows 0..63 Re and
+//   A block (t, gA): [slice 6][k half 2][row 128][16 B], rows 0..63 Re and
 //                    64..127 Im of 64 complex rows u of one site pair
-//   B block (t, gB): [slice 5][k half 2][row 80][16 B], rows 0..39 Re and
+//   B block (t, gB): [k half 2][slice 6][row 80][16 B], rows 0..39 Re and
 //                    40..79 Im of 40 complex columns v of one site pair
-// One M=128 x N=80 x K=32 MMA per digit pair gives, for the 64 x 40 complex
-// tile, the four real products Ar Br, Ar Bi, Ai Br, Ai Bi at once.
+// An M=128 x K=32 MMA of digit i of A against N=80 rows per digit of B gives, for the
+// 64 x 40 complex tile, the four real products Ar Br, Ar Bi, Ai Br, Ai Bi at once.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -98,9 +98,9 @@ cudaError_t split_bound(const unsigned long long* m64A, const unsigned long long
                         const SplitPassDev& p, const int* pair_M, const int* pair_aoff, int n_pairs, double* bnd,
                         cudaStream_t s);
 
-// digits of one operand for a pass; writes E[c * ld + e] for every valid element
+// digits of one operand for a pass (b_layout: blocks of B);  writes E[c * ld + e] for every valid element
 cudaError_t split_quantize(const double2* X, int64_t ld, const SplitPassDev& p, const SplitGroup* groups,
-                           int n_groups, int rows, const unsigned long long* M64, int* E, int8_t* dig,
+                           int n_groups, int rows, bool b_layout, const unsigned long long* M64, int* E, int8_t* dig,
                            cudaStream_t s);
 
 struct SplitContractArgs {
