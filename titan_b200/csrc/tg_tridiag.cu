@@ -31,118 +31,219 @@ __device__ __forceinline__ double2 warp_sum2(double2 v) {
   return v;
 }
 
-// sum over the block, returned to every thread (red: 2 doubles per warp)
-__device__ double2 block_sum2(double2 v, double* red) {
-  v = warp_sum2(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) {
-    red[2 * warp] = v.x;
-    red[2 * warp + 1] = v.y;
-  }
-  __syncthreads();
-  double2 t = make_double2(0.0, 0.0);
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-    t.x += red[2 * w];
-    t.y += red[2 * w + 1];
-  }
-  return t;
-}
-
-// A: [nk][n][n] row-major H(k) table rows, overwritten; rows[ns]: the rows S of Q to form.
-// Out: D[k][i] = T(i, i), E[k][i] = T(i + 1, i) (E[k][n - 1] = 0), Q[k][s][c] = Q(rows[s], c).
-// One CTA per k; a warp per row for the matrix-vector products and rank-2 updates.
-__global__ void __launch_bounds__(kTriThreads) hh_tridiag_kernel(double2* __restrict__ A, int64_t nk, int n,
-                                                                 const int* __restrict__ rows, int ns,
-                                                                 double* __restrict__ D, double* __restrict__ E,
-                                                                 double2* __restrict__ Q) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  double2* v = reinterpret_cast<double2*>(smem);      // [n] reflector
-  double2* w = v + n;                                 // [n] p, then w
-  double* red = reinterpret_cast<double*>(w + n);     // [2 * warps]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
-    double2* Ak = A + k * (int64_t)n * n;
-    double2* Qk = Q + k * (int64_t)ns * n;
-    for (int64_t e = threadIdx.x; e < (int64_t)ns * n; e += blockDim.x) {
-      const int s = (int)(e / n), col = (int)(e % n);
-      Qk[e] = make_double2(col == rows[s] ? 1.0 : 0.0, 0.0);
-    }
-    for (int j = 0; j + 1 < n; ++j) {
-      const int m = n - j - 1;
-      // x = A(j+1:, j) into v; |x(1:)|^2
-      double part = 0.0;
-      for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const double2 x = Ak[(int64_t)(j + 1 + i) * n + j];
-        v[i] = x;
-        if (i > 0) part += x.x * x.x + x.y * x.y;
-      }
-      const double xn2 = block_sum2(make_double2(part, 0.0), red).x;   // its barriers publish v
-      const double2 alpha = v[0];
-      const bool refl = !(xn2 == 0.0 && alpha.y == 0.0);
-      // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
-      const double beta = refl ? -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x) : alpha.x;
-      if (threadIdx.x == 0) {
-        D[k * n + j] = Ak[(int64_t)j * n + j].x;
-        E[k * n + j] = beta;
-      }
-      __syncthreads();   // alpha read by every thread before v changes
-      if (!refl) continue;
-      const double2 tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-      {
-        const double dr = alpha.x - beta, di = alpha.y;
-        const double inv = 1.0 / (dr * dr + di * di);
-        const double2 sc = make_double2(dr * inv, -di * inv);
-        for (int i = threadIdx.x; i < m; i += blockDim.x) v[i] = i == 0 ? make_double2(1.0, 0.0) : cmul(v[i], sc);
-      }
-      __syncthreads();
-      // p = tau A22 v into w: a warp per row, lanes along the row
-      for (int r = warp; r < m; r += nw) {
-        const double2* Ar = Ak + (int64_t)(j + 1 + r) * n + (j + 1);
-        double2 acc = make_double2(0.0, 0.0);
-        for (int col = lane; col < m; col += 32) acc = cfma(Ar[col], v[col], acc);
-        acc = warp_sum2(acc);
-        if (lane == 0) w[r] = cmul(tau, acc);
-      }
-      __syncthreads();
-      // w = p - (tau / 2) (p^H v) v
-      double2 dp = make_double2(0.0, 0.0);
-      for (int i = threadIdx.x; i < m; i += blockDim.x) dp = cfma(cconj(w[i]), v[i], dp);
-      dp = block_sum2(dp, red);
-      const double2 a2 = cscale(cmul(tau, dp), -0.5);
-      for (int i = threadIdx.x; i < m; i += blockDim.x) w[i] = cfma(a2, v[i], w[i]);
-      __syncthreads();
-      // A22 -= v w^H + w v^H
-      for (int r = warp; r < m; r += nw) {
-        double2* Ar = Ak + (int64_t)(j + 1 + r) * n + (j + 1);
-        const double2 vr = v[r], wr = w[r];
-        for (int col = lane; col < m; col += 32)
-          Ar[col] = csub(Ar[col], cadd(cmul(vr, cconj(w[col])), cmul(wr, cconj(v[col]))));
-      }
-      // Q_S <- Q_S H_j on columns j+1..: y = Q_S(:, j+1:) v, Q_S(:, j+1:) -= tau y v^H
-      for (int s = warp; s < ns; s += nw) {
-        double2* Qs = Qk + (int64_t)s * n + (j + 1);
-        double2 acc = make_double2(0.0, 0.0);
-        for (int col = lane; col < m; col += 32) acc = cfma(Qs[col], v[col], acc);
-        const double2 ty = cmul(tau, warp_sum2(acc));
-        for (int col = lane; col < m; col += 32) Qs[col] = csub(Qs[col], cmul(ty, cconj(v[col])));
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      D[k * n + n - 1] = Ak[(int64_t)(n - 1) * n + n - 1].x;
-      E[k * n + n - 1] = 0.0;
-    }
-    __syncthreads();
-  }
-}
-
 // not volatile: the scheduler may interleave the MMAs of independent accumulators (a chain on
 // one accumulator keeps its order through the data dependence, so results do not change)
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(c0), "+d"(c1)
                : "d"(a), "d"(b));
+}
+
+// Reduction of one H(k) per CTA for dimensions whose matrix does not fit in shared memory.
+//
+// A: [nk][n][n] row-major H(k) table rows, overwritten; rows[ns]: the rows S of Q to form.
+// Out: D[k][i] = T(i, i), E[k][i] = T(i + 1, i) (E[k][n - 1] = 0), Q[k][s][c] = Q(rows[s], c).
+// Panels of 8 reflectors, as in LAPACK's zlatrd: inside a panel the trailing matrix is only
+// read (once per reflector, A v), with the panel's own changes V W^H + W V^H applied to the
+// vectors; it is rewritten once per panel, by FP64 tensor-core products of depth 8, and the
+// rows of Q pass through registers once per panel.  Bound by the reads of A v from L2 / HBM
+// (16 n^3 / 3 bytes per matrix, two rows and all their loads in flight per warp).
+constexpr int kPanThreads = 512;
+constexpr int kPanNb = 8;              // reflectors per panel
+constexpr int kPanS = kPanNb + 4;      // row stride of V and W: 4 mod 8, fragment reads apart
+constexpr int kPanSeg = 9;             // 32-column segments of a row: n <= 288
+
+__host__ __device__ inline size_t hh_panel_smem(int n) {
+  return sizeof(double2) * ((size_t)n * kPanS * 2 + (size_t)n * kPanNb + 2 * (size_t)n + 4 * kPanNb);
+}
+
+__global__ void __launch_bounds__(kPanThreads, 1) hh_panel_kernel(double2* __restrict__ A, int64_t nk, int n,
+                                                                const int* __restrict__ rows, int ns,
+                                                                double* __restrict__ D, double* __restrict__ E,
+                                                                double2* __restrict__ Q) {
+  extern __shared__ __align__(16) double2 psm[];
+  double2* V = psm;                          // [n][kPanS] reflectors of the panel
+  double2* W = V + (size_t)n * kPanS;        // [n][kPanS]
+  double2* Vt = W + (size_t)n * kPanS;       // [kPanNb][n] V again, contiguous along a reflector
+  double2* x = Vt + (size_t)n * kPanNb;      // [n] current column
+  double2* p = x + n;                        // [n] A v, then tau (A v - ..)
+  double2* cw = p + n;                       // [kPanNb] W^H v
+  double2* cv = cw + kPanNb;                 // [kPanNb] V^H v
+  double2* taus = cv + kPanNb;               // [kPanNb]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = kPanThreads / 32;
+  const double2 zero = make_double2(0.0, 0.0);
+  for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
+    double2* Ak = A + k * (int64_t)n * n;
+    double2* Qk = Q + k * (int64_t)ns * n;
+    for (int e = tid; e < ns * n; e += kPanThreads)
+      Qk[e] = make_double2(e % n == rows[e / n] ? 1.0 : 0.0, 0.0);
+    for (int j0 = 0; j0 + 1 < n; j0 += kPanNb) {
+      const int nb = min(kPanNb, n - 1 - j0);
+      for (int jj = 0; jj < nb; ++jj) {
+        const int j = j0 + jj;
+        // column j with the panel's changes (A is Hermitian: its row j, conjugated)
+        for (int i = j + tid; i < n; i += kPanThreads) {
+          double2 a = cconj(Ak[(int64_t)j * n + i]);
+          for (int t = 0; t < jj; ++t)
+            a = cfms(V[i * kPanS + t], cconj(W[j * kPanS + t]), cfms(W[i * kPanS + t], cconj(V[j * kPanS + t]), a));
+          x[i] = a;
+        }
+        __syncthreads();
+        double part = 0.0;
+        for (int i = j + 2 + lane; i < n; i += 32) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        const double2 alpha = x[j + 1];
+        const bool refl = !(part == 0.0 && alpha.y == 0.0);
+        // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
+        const double beta =
+            refl ? -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, part))), alpha.x) : alpha.x;
+        double2 tau = zero, sc = zero;
+        if (refl) {
+          tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
+          const double dr = alpha.x - beta, di = alpha.y;
+          const double inv = 1.0 / fma(dr, dr, di * di);
+          sc = make_double2(dr * inv, -di * inv);
+        }
+        if (tid == 0) {
+          D[k * n + j] = x[j].x;
+          E[k * n + j] = beta;
+          taus[jj] = tau;
+        }
+        // v (zero up to row j; all zero without a reflector)
+        for (int i = tid; i < n; i += kPanThreads) {
+          const double2 vi = !refl || i <= j ? zero : i == j + 1 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
+          V[i * kPanS + jj] = vi;
+          Vt[jj * n + i] = vi;
+        }
+        __syncthreads();
+        const double2* v = Vt + (size_t)jj * n;
+        if (refl) {
+          // A v, two rows per warp
+          for (int r = j + 1 + 2 * warp; r < n; r += 2 * nw) {
+            const double2* A0 = Ak + (int64_t)r * n;
+            const bool two = r + 1 < n;
+            double2 a0[kPanSeg], a1[kPanSeg];
+#pragma unroll
+            for (int u = 0; u < kPanSeg; ++u) {
+              const int c = lane + 32 * u;
+              const bool in = c > j && c < n;
+              a0[u] = in ? A0[c] : zero;
+              a1[u] = in && two ? A0[n + c] : zero;
+            }
+            double2 s0 = zero, s1 = zero;
+#pragma unroll
+            for (int u = 0; u < kPanSeg; ++u) {
+              const int c = lane + 32 * u;
+              if (c > j && c < n) {
+                const double2 vc = v[c];
+                s0 = cfma(a0[u], vc, s0);
+                s1 = cfma(a1[u], vc, s1);
+              }
+            }
+            s0 = warp_sum2(s0);
+            s1 = warp_sum2(s1);
+            if (lane == 0) {
+              p[r] = s0;
+              if (two) p[r + 1] = s1;
+            }
+          }
+          for (int t = warp; t < 2 * jj; t += nw) {
+            const double2* M = t < jj ? W + t : V + (t - jj);
+            double2 s = zero;
+            for (int c = j + 1 + lane; c < n; c += 32) s = cfma(cconj(M[c * kPanS]), v[c], s);
+            s = warp_sum2(s);
+            if (lane == 0) (t < jj ? cw[t] : cv[t - jj]) = s;
+          }
+        }
+        __syncthreads();
+        for (int r = j + 1 + tid; r < n && refl; r += kPanThreads) {
+          double2 a = p[r];
+          for (int t = 0; t < jj; ++t)
+            a = cfms(V[r * kPanS + t], cw[t], cfms(W[r * kPanS + t], cv[t], a));
+          p[r] = cmul(tau, a);
+        }
+        __syncthreads();
+        // w = p - (tau / 2) (p^H v) v
+        double2 dot = zero;
+        if (refl)
+          for (int r = j + 1 + lane; r < n; r += 32) dot = cfma(cconj(p[r]), v[r], dot);
+        dot = warp_sum2(dot);
+        const double2 a2 = cscale(cmul(tau, dot), -0.5);
+        for (int r = tid; r < n; r += kPanThreads)
+          W[r * kPanS + jj] = refl && r > j ? cfma(a2, v[r], p[r]) : zero;
+        __syncthreads();
+      }
+      // columns of V and W past the panel's reflectors count as zero below
+      for (int e = tid; e < n * (kPanNb - nb); e += kPanThreads) {
+        const int i = e / (kPanNb - nb), t = nb + e % (kPanNb - nb);
+        V[i * kPanS + t] = W[i * kPanS + t] = zero;
+      }
+      __syncthreads();
+      // A22 -= V W^H + W V^H in 8 x 8 fragments (rows and columns from the first 8-block boundary
+      // at or below the panel's end: what lies before it is not read again)
+      const int b0 = (j0 + nb) / 8, nbk = (n + 7) / 8, side = nbk - b0;
+      const int g8 = lane >> 2, t4 = lane & 3;
+      for (int f = warp; f < side * side; f += nw) {
+        const int r = 8 * (b0 + f / side) + g8, c = 8 * (b0 + f % side) + 2 * t4;
+        const int cb = 8 * (b0 + f % side) + g8;
+        double2* Ap = Ak + (int64_t)r * n + c;
+        const bool in0 = r < n && c < n, in1 = r < n && c + 1 < n;
+        double2 c0 = in0 ? Ap[0] : zero, c1 = in1 ? Ap[1] : zero;
+#pragma unroll
+        for (int h = 0; h < kPanNb; h += 4) {
+          const double2 av = r < n ? V[r * kPanS + h + t4] : zero, aw = r < n ? W[r * kPanS + h + t4] : zero;
+          const double2 bw = cb < n ? W[cb * kPanS + h + t4] : zero, bv = cb < n ? V[cb * kPanS + h + t4] : zero;
+          // -(a conj(b)): real part -ar br - ai bi, imaginary part -ai br + ar bi
+          dmma(c0.x, c1.x, -av.x, bw.x);
+          dmma(c0.y, c1.y, -av.y, bw.x);
+          dmma(c0.x, c1.x, -av.y, bw.y);
+          dmma(c0.y, c1.y, av.x, bw.y);
+          dmma(c0.x, c1.x, -aw.x, bv.x);
+          dmma(c0.y, c1.y, -aw.y, bv.x);
+          dmma(c0.x, c1.x, -aw.y, bv.y);
+          dmma(c0.y, c1.y, aw.x, bv.y);
+        }
+        if (in0) Ap[0] = c0;
+        if (in1) Ap[1] = c1;
+      }
+      // Q_S <- Q_S H_j0 H_j0+1 ..: a row per warp in registers, y = q v, q -= tau y v^H
+      for (int s = warp; s < ns; s += nw) {
+        double2* Qs = Qk + (int64_t)s * n;
+        double2 q[kPanSeg];
+#pragma unroll
+        for (int u = 0; u < kPanSeg; ++u) {
+          const int c = lane + 32 * u;
+          q[u] = c < n ? Qs[c] : zero;
+        }
+        for (int t = 0; t < nb; ++t) {
+          const double2* v = Vt + (size_t)t * n;
+          double2 y = zero;
+#pragma unroll
+          for (int u = 0; u < kPanSeg; ++u) {
+            const int c = lane + 32 * u;
+            if (c < n) y = cfma(q[u], v[c], y);
+          }
+          const double2 ty = cmul(taus[t], warp_sum2(y));
+#pragma unroll
+          for (int u = 0; u < kPanSeg; ++u) {
+            const int c = lane + 32 * u;
+            if (c < n) q[u] = cfms(ty, cconj(v[c]), q[u]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kPanSeg; ++u) {
+          const int c = lane + 32 * u;
+          if (c < n) Qs[c] = q[u];
+        }
+      }
+      __syncthreads();   // (orders this CTA's writes of A before the next panel's reads)
+    }
+    if (tid == 0) {
+      D[k * n + n - 1] = Ak[(int64_t)(n - 1) * n + n - 1].x;
+      E[k * n + n - 1] = 0.0;
+    }
+    __syncthreads();
+  }
 }
 
 // G of S x S per point (k, z) of a k-major pass.  z - T = L D L^T (complex symmetric, no pivoting),
@@ -367,9 +468,12 @@ cudaError_t launch_tridiag(double2* H, int64_t nk, int n, const int* rows, int n
   if (n < 2 || ns <= 0 || ns > n) return cudaErrorInvalidValue;
   // the matrix in shared memory where it fits (no pass over it goes to L2)
   if (hh_small_supported(n)) return launch_hh_small(H, nk, n, rows, ns, D, E, Q, num_sms, s);
-  const size_t smem = sizeof(double2) * 2 * (size_t)n + sizeof(double) * 2 * (kTriThreads / 32);
-  const int64_t grid = std::min<int64_t>(nk, (int64_t)num_sms * 4);
-  hh_tridiag_kernel<<<(unsigned)grid, kTriThreads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
+  if (n > 32 * kPanSeg) return cudaErrorInvalidValue;
+  const size_t smem = hh_panel_smem(n);
+  cudaError_t e = cudaFuncSetAttribute(hh_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int64_t grid = std::min<int64_t>(nk, (int64_t)num_sms);
+  hh_panel_kernel<<<(unsigned)grid, kPanThreads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
   return cudaGetLastError();
 }
 
