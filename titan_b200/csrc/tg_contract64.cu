@@ -9,7 +9,7 @@
 // A_p = w_p (G1 - G1^dagger)_ij, B_p = conj(G2)_ij on the real axis
 // (eintshechi.F90:146-164).  The chi element is then picked out of C in the
 // epilogue (chi = C_ij + conj(C_ji) with permuted indices, Fint = -i D_ij).
-// This file holds the FP64 SIMT GEMM (the plain-precision GPU path), the
+// This file holds the FP64 tensor-core GEMM (the plain-precision GPU path) and the
 // chi assembly epilogue.
 #include "tg_internal.cuh"
 
@@ -19,19 +19,43 @@ namespace tg {
 
 namespace {
 
-constexpr int TT = 16;            // thread grid side (TT x TT = 256 threads)
-constexpr int PT = 7;             // complex entries per thread and dimension
-constexpr int TILE = TT * PT;     // 112: three tiles cover 4*9*9 = 324 (sp-d sites)
+// One CTA per output tile and K-range: WM x WN warps of FM x FN fragments (8 x 8 complex, four
+// real DMMAs m8n8k4 per fragment and four points), points in stages of KC through a cp.async
+// ring.  A stage's row of one point is 2 mod 8 complex longer than the tile, so the fragment
+// reads of a quarter warp (four points, two rows) fall into distinct banks.
+//   112 x 112 (7 x 2 warps of 2 x 7): three tiles cover the 324 = 4 9^2 rows of two spd sites
+//     (93 % of the tile area used)
+//   104 x 104 (13 x 1 warps of 1 x 13): the 100 = 4 5^2 rows of the d orbitals (92 %)
+// Bound by the FP64 tensor pipe: 56 (52) DMMAs per warp, four points and 9 (14) shared-memory
+// reads.
 constexpr int KC = 8;             // points per shared-memory stage
-constexpr size_t kSmem = sizeof(double2) * 2 * 2 * KC * TILE;
+constexpr int kStages = 3;
 
-__global__ void __launch_bounds__(TT * TT, 1)
+template <int WM, int WN, int FM, int FN>
+struct Gemm64 {
+  static constexpr int TILE = 8 * WM * FM;
+  static_assert(TILE == 8 * WN * FN, "square tiles");
+  static constexpr int THREADS = 32 * WM * WN;
+  static constexpr int S = TILE + (TILE % 8 == 0 ? 2 : 0);
+  static constexpr size_t smem = sizeof(double2) * kStages * 2 * KC * S;
+};
+using GemmWide = Gemm64<7, 2, 2, 7>;
+using GemmD = Gemm64<13, 1, 1, 13>;
+
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+
+template <int WM, int WN, int FM, int FN>
+__global__ void __launch_bounds__(32 * WM * WN, 1)
 gemm64_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int64_t ld, int64_t np, int nsplit,
               const PairTile* __restrict__ tiles, const int* __restrict__ pair_M, const int* __restrict__ pair_aoff,
               const int64_t* __restrict__ pair_coff, double2* __restrict__ Cpart, int64_t cstride) {
-  extern __shared__ __align__(16) double2 smem64[];
-  double2 (*As)[KC][TILE] = reinterpret_cast<double2 (*)[KC][TILE]>(smem64);
-  double2 (*Bs)[KC][TILE] = reinterpret_cast<double2 (*)[KC][TILE]>(smem64 + 2 * KC * TILE);
+  using G = Gemm64<WM, WN, FM, FN>;
+  constexpr int TILE = G::TILE, S = G::S, T = G::THREADS;
+  extern __shared__ __align__(16) double2 smem64[];   // [stage][A, B][KC][S]
   const int tile_id = blockIdx.x / nsplit;
   const int split = blockIdx.x % nsplit;
   const PairTile t = tiles[tile_id];
@@ -39,73 +63,92 @@ gemm64_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int6
   const int aoff = pair_aoff[t.pair];
   const int64_t p_begin = np * split / nsplit;
   const int64_t p_end = np * (split + 1) / nsplit;
-  const int tid = threadIdx.x;
-  const int ty = tid / TT, tx = tid % TT;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g8 = lane >> 2, t4 = lane & 3;
+  const int wm = (warp % WM) * 8 * FM, wn = (warp / WM) * 8 * FN;
 
-  double2 acc[PT][PT];
+  double cr[FM][FN][2], ci[FM][FN][2];
 #pragma unroll
-  for (int i = 0; i < PT; ++i)
+  for (int i = 0; i < FM; ++i)
 #pragma unroll
-    for (int j = 0; j < PT; ++j) acc[i][j] = make_double2(0.0, 0.0);
+    for (int j = 0; j < FN; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
 
-  auto load_stage = [&](int buf, int64_t p0) {
-    // KC x TILE complex for A and for B; 16-byte cp.async per element
-    for (int e = tid; e < KC * TILE; e += TT * TT) {
-      const int kk = e / TILE, col = e % TILE;
-      const int64_t p = p0 + kk;
-      const int ua = t.u0 + col, vb = t.v0 + col;
-      double2* da = &As[buf][kk][col];
-      double2* db = &Bs[buf][kk][col];
-      const bool pa = (p < p_end) && (ua < M);
-      const bool pb = (p < p_end) && (vb < M);
-      const double2* sa = pa ? A + p * ld + aoff + ua : A;
-      const double2* sb = pb ? B + p * ld + aoff + vb : B;
-      const unsigned sda = (unsigned)__cvta_generic_to_shared(da);
-      const unsigned sdb = (unsigned)__cvta_generic_to_shared(db);
-      const int na = pa ? 16 : 0, nb = pb ? 16 : 0;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sda), "l"(sa), "r"(na));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sdb), "l"(sb), "r"(nb));
+  // a thread copies column `col` of the points kk and kk + 4 of every stage
+  static_assert(2 * T == KC * TILE, "two elements of either operand per thread and stage");
+  const int kk0 = tid / TILE, col = tid % TILE;
+  const bool ina = t.u0 + col < M, inb = t.v0 + col < M;
+  const double2* ga = A + (p_begin + kk0) * ld + aoff + (ina ? t.u0 + col : 0);
+  const double2* gb = B + (p_begin + kk0) * ld + aoff + (inb ? t.v0 + col : 0);
+  const unsigned sdst = (unsigned)__cvta_generic_to_shared(smem64 + kk0 * S + col);
+  int left = (int)(p_end - p_begin) - kk0;   // points from this thread's next one to the end
+  auto load_stage = [&](int buf) {
+    const unsigned d = sdst + (unsigned)(buf * 2 * KC * S * sizeof(double2));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool in = left > 4 * h;
+      const unsigned o = (unsigned)(4 * h * S * sizeof(double2));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d + o), "l"(in ? ga + 4 * h * ld : A),
+                   "r"(in && ina ? 16 : 0));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                       d + o + (unsigned)(KC * S * sizeof(double2))),
+                   "l"(in ? gb + 4 * h * ld : B), "r"(in && inb ? 16 : 0));
     }
-    asm volatile("cp.async.commit_group;\n" ::);
+    ga += KC * ld;
+    gb += KC * ld;
+    left -= KC;
   };
 
   const int64_t nstages = (p_end - p_begin + KC - 1) / KC;
-  if (nstages > 0) load_stage(0, p_begin);
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    if (s < nstages) load_stage(s);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  int buf = 0, fill = kStages - 1;   // stage to multiply, stage to load
   for (int64_t s = 0; s < nstages; ++s) {
-    const int buf = (int)(s & 1);
-    if (s + 1 < nstages) {
-      load_stage(buf ^ 1, p_begin + (s + 1) * KC);
-      asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2));
+    __syncthreads();   // stage s has landed, and every warp is done with the one loaded next
+    if (s + kStages - 1 < nstages) load_stage(fill);
+    fill = fill + 1 == kStages ? 0 : fill + 1;
+    asm volatile("cp.async.commit_group;\n" ::);
+    const double2* as = smem64 + (size_t)buf * 2 * KC * S + t4 * S + wm + g8;
+    const double2* bs = smem64 + (size_t)buf * 2 * KC * S + (KC + t4) * S + wn + g8;
+    buf = buf + 1 == kStages ? 0 : buf + 1;
+#pragma unroll 1
+    for (int kk = 0; kk < KC; kk += 4) {
+      double2 av[FM];
+#pragma unroll
+      for (int i = 0; i < FM; ++i) av[i] = as[kk * S + 8 * i];
+#pragma unroll
+      for (int j = 0; j < FN; ++j) {
+        const double2 bv = bs[kk * S + 8 * j];
+#pragma unroll
+        for (int i = 0; i < FM; ++i) {
+          dmma(cr[i][j][0], cr[i][j][1], av[i].x, bv.x);
+          dmma(ci[i][j][0], ci[i][j][1], av[i].x, bv.y);
+        }
+#pragma unroll
+        for (int i = 0; i < FM; ++i) {
+          dmma(cr[i][j][0], cr[i][j][1], -av[i].y, bv.y);
+          dmma(ci[i][j][0], ci[i][j][1], av[i].y, bv.x);
+        }
+      }
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < KC; ++kk) {
-      double2 a[PT], b[PT];
-#pragma unroll
-      for (int i = 0; i < PT; ++i) a[i] = As[buf][kk][ty + TT * i];
-#pragma unroll
-      for (int j = 0; j < PT; ++j) b[j] = Bs[buf][kk][tx + TT * j];
-#pragma unroll
-      for (int i = 0; i < PT; ++i)
-#pragma unroll
-        for (int j = 0; j < PT; ++j) acc[i][j] = cfma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
   }
   double2* C = Cpart + (int64_t)split * cstride + pair_coff[t.pair];
 #pragma unroll
-  for (int i = 0; i < PT; ++i) {
-    const int u = t.u0 + ty + TT * i;
+  for (int i = 0; i < FM; ++i) {
+    const int u = t.u0 + wm + 8 * i + g8;
     if (u >= M) continue;
 #pragma unroll
-    for (int j = 0; j < PT; ++j) {
-      const int v = t.v0 + tx + TT * j;
-      if (v >= M) continue;
-      double2* c = C + (int64_t)u * M + v;
-      *c = cadd(*c, acc[i][j]);
-    }
+    for (int j = 0; j < FN; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int v = t.v0 + wn + 8 * j + 2 * t4 + h;
+        if (v >= M) continue;
+        double2* c = C + (int64_t)u * M + v;
+        *c = cadd(*c, make_double2(cr[i][j][h], ci[i][j][h]));
+      }
   }
 }
 
@@ -151,19 +194,32 @@ __global__ void chi_epilogue_kernel(const double2* __restrict__ Cpart, const dou
 
 }  // namespace
 
-cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit,
+namespace {
+
+template <int WM, int WN, int FM, int FN>
+cudaError_t launch_gemm64_t(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit,
+                            const PairTile* tiles, int ntiles, const int* pair_M, const int* pair_aoff,
+                            const int64_t* pair_coff, double2* Cpart, int64_t cstride, cudaStream_t s) {
+  using G = Gemm64<WM, WN, FM, FN>;
+  auto kernel = gemm64_kernel<WM, WN, FM, FN>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
+  if (e != cudaSuccess) return e;
+  kernel<<<ntiles * nsplit, G::THREADS, G::smem, s>>>(A, B, ld, np, nsplit, tiles, pair_M, pair_aoff, pair_coff, Cpart,
+                                                     cstride);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit, int tile,
                           const PairTile* tiles, int ntiles, const int* pair_M, const int* pair_aoff,
                           const int64_t* pair_coff, double2* Cpart, int64_t cstride, cudaStream_t s) {
   if (np <= 0 || ntiles <= 0) return cudaSuccess;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  gemm64_kernel<<<ntiles * nsplit, TT * TT, kSmem, s>>>(A, B, ld, np, nsplit, tiles, pair_M, pair_aoff, pair_coff,
-                                                    Cpart, cstride);
-  return cudaGetLastError();
+  if (tile == GemmD::TILE)
+    return launch_gemm64_t<13, 1, 1, 13>(A, B, ld, np, nsplit, tiles, ntiles, pair_M, pair_aoff, pair_coff, Cpart,
+                                         cstride, s);
+  return launch_gemm64_t<7, 2, 2, 7>(A, B, ld, np, nsplit, tiles, ntiles, pair_M, pair_aoff, pair_coff, Cpart, cstride,
+                                     s);
 }
 
 cudaError_t launch_chi_epilogue(const double2* Cpart, const double2* Dpart, int nsplit, int64_t cstride,
@@ -176,6 +232,17 @@ cudaError_t launch_chi_epilogue(const double2* Cpart, const double2* Dpart, int 
   return cudaGetLastError();
 }
 
-int gemm64_tile() { return TILE; }
+// tile side for the site pairs of a layout (pair_M[n_pairs] rows each): the one whose tiles
+// cover the smaller area (DMMAs of the padding cost as much as the others), 112 on ties
+int gemm64_tile(int n_pairs, const int* pair_M) {
+  double wide = 0.0, d = 0.0;
+  for (int i = 0; i < n_pairs; ++i) {
+    const double a = (pair_M[i] + GemmWide::TILE - 1) / GemmWide::TILE * GemmWide::TILE;
+    const double b = (pair_M[i] + GemmD::TILE - 1) / GemmD::TILE * GemmD::TILE;
+    wide += a * a;
+    d += b * b;
+  }
+  return d < wide ? GemmD::TILE : GemmWide::TILE;
+}
 
 }  // namespace tg
