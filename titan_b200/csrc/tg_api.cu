@@ -74,7 +74,6 @@ struct ChiLayout {
   std::vector<int> pair_M, pair_aoff;
   std::vector<int64_t> pair_coff;
   std::vector<PairTile> tiles;
-  int tile = 0;                       // side of the FP64 contraction's tiles
   SplitLayout split;
   DevArray<int> d_rows;               // the nsel rows of G that enter chi, site by site
   DevArray<int> d_outmap, d_decode, d_norb, d_pair_M, d_pair_aoff;
@@ -93,7 +92,7 @@ struct ChiView {
   const int *outmap = nullptr, *decode = nullptr, *norb = nullptr, *pair_M = nullptr, *pair_aoff = nullptr;
   const int64_t* pair_coff = nullptr;
   const PairTile* tiles = nullptr;
-  int ntiles = 0, tile = 0;
+  int ntiles = 0;
   const SplitLayout* split = nullptr;
   const SplitGroup *sgA = nullptr, *sgB = nullptr;
   const SplitTile* stiles = nullptr;
@@ -115,7 +114,6 @@ struct tg_ctx {
   std::vector<int> pair_M, pair_aoff;   // per pair (i*nat + j)
   std::vector<int64_t> pair_coff;
   std::vector<PairTile> tiles;
-  int tile = 0;
   DevArray<double> d_R;
   DevArray<int> d_pair_start, d_pair_neigh, d_row_atom, d_row_orb, d_row_spin, d_outmap, d_decode, d_norb,
       d_pair_M, d_pair_aoff, d_exp_rows, d_gg_desc;
@@ -516,7 +514,7 @@ ChiView chi_view(tg_ctx* c) {
   v.gather = true;
   v.outmap = L.d_outmap.p; v.decode = L.d_decode.p; v.norb = L.d_norb.p;
   v.pair_M = L.d_pair_M.p; v.pair_aoff = L.d_pair_aoff.p; v.pair_coff = L.d_pair_coff.p;
-  v.tiles = L.d_tiles.p; v.ntiles = (int)L.tiles.size(); v.tile = L.tile; v.split = &L.split;
+  v.tiles = L.d_tiles.p; v.ntiles = (int)L.tiles.size(); v.split = &L.split;
   v.sgA = L.d_sgA.p; v.sgB = L.d_sgB.p; v.stiles = L.d_stiles.p;
   v.rows = L.d_rows.p; v.nrows = L.nsel;
   return v;
@@ -545,7 +543,7 @@ int build_chi_layout(tg_ctx* c, const std::vector<std::vector<int>>& orbs, ChiLa
   int64_t coff = 0;
   for (int i = 0; i < nat; ++i)
     for (int j = 0; j < nat; ++j) L.pair_M[i * nat + j] = 4 * L.nc[i] * L.nc[j];
-  const int T = L.tile = gemm64_tile(np2, L.pair_M.data());
+  const int T = gemm64_tile();
   for (int i = 0; i < nat; ++i)
     for (int j = 0; j < nat; ++j) {
       const int p = i * nat + j;
@@ -595,7 +593,7 @@ ChiView full_view(tg_ctx* c) {
   v.gather = !green_supported(c->dimH);
   v.outmap = c->d_outmap.p; v.decode = c->d_decode.p; v.norb = c->d_norb.p;
   v.pair_M = c->d_pair_M.p; v.pair_aoff = c->d_pair_aoff.p; v.pair_coff = c->d_pair_coff.p;
-  v.tiles = c->d_tiles.p; v.ntiles = (int)c->tiles.size(); v.tile = c->tile; v.split = &c->split;
+  v.tiles = c->d_tiles.p; v.ntiles = (int)c->tiles.size(); v.split = &c->split;
   v.sgA = c->d_sgA.p; v.sgB = c->d_sgB.p; v.stiles = c->d_stiles.p;
   v.rows = c->d_allrows.p; v.nrows = c->dimH;
   return v;
@@ -610,7 +608,7 @@ int nsplit_view(tg_ctx* c, const ChiView& v) {
 int contract(tg_ctx* c, const ChiView& v, const double2* A, const double2* B, int64_t np, double2* Cpart, int nsplit,
              int64_t cstride) {
   c->launches += 1;
-  TG_CHECK(c, launch_gemm64(A, B, v.ld, np, nsplit, v.tile, v.tiles, v.ntiles, v.pair_M, v.pair_aoff, v.pair_coff, Cpart,
+  TG_CHECK(c, launch_gemm64(A, B, v.ld, np, nsplit, v.tiles, v.ntiles, v.pair_M, v.pair_aoff, v.pair_coff, Cpart,
                             cstride, c->stream),
            "contraction (fp64)");
   return TG_OK;
@@ -1029,7 +1027,7 @@ int tg_set_system(tg_ctx* c, int n_atoms, const int* norb, int norb_max, int n_n
   c->tiles.clear();
   for (int i = 0; i < n_atoms; ++i)
     for (int j = 0; j < n_atoms; ++j) c->pair_M[i * n_atoms + j] = 4 * c->norb[i] * c->norb[j];
-  const int T = c->tile = gemm64_tile(np2, c->pair_M.data());
+  const int T = gemm64_tile();
   for (int i = 0; i < n_atoms; ++i)
     for (int j = 0; j < n_atoms; ++j) {
       const int p = i * n_atoms + j;

@@ -19,28 +19,24 @@ namespace tg {
 
 namespace {
 
-// One CTA per output tile and K-range: WM x WN warps of FM x FN fragments (8 x 8 complex, four
-// real DMMAs m8n8k4 per fragment and four points), points in stages of KC through a cp.async
-// ring.  A stage's row of one point is 2 mod 8 complex longer than the tile, so the fragment
-// reads of a quarter warp (four points, two rows) fall into distinct banks.
-//   112 x 112 (7 x 2 warps of 2 x 7): three tiles cover the 324 = 4 9^2 rows of two spd sites
-//     (93 % of the tile area used)
-//   104 x 104 (13 x 1 warps of 1 x 13): the 100 = 4 5^2 rows of the d orbitals (92 %)
-// Bound by the FP64 tensor pipe: 56 (52) DMMAs per warp, four points and 9 (14) shared-memory
-// reads.
-constexpr int KC = 8;             // points per shared-memory stage
+// One CTA per output tile of 112 x 112 and K-range; points in stages of KC through a cp.async
+// ring.  A stage's row of one point is 2 mod 8 complex long, so the fragment reads of a quarter
+// warp (four points, two rows) fall into distinct banks.
+//
+// 112 = 14 fragments: three tiles cover the 324 = 4 9^2 rows of two spd sites to 93 %.  Each of
+// the four sub-partitions of the SM (warp id mod 4) takes one 56 x 56 quadrant, 7 x 7 fragments
+// of 8 x 8 complex (four real DMMAs m8n8k4 per fragment and four points) dealt to its four
+// warps in columns of 2, 2, 2 and 1, so that the four FP64 pipes, which bound the kernel, have
+// equal work.  Fragments past the site pair's rows or columns are skipped.
+constexpr int KC = 16;            // points per shared-memory stage
 constexpr int kStages = 3;
-
-template <int WM, int WN, int FM, int FN>
-struct Gemm64 {
-  static constexpr int TILE = 8 * WM * FM;
-  static_assert(TILE == 8 * WN * FN, "square tiles");
-  static constexpr int THREADS = 32 * WM * WN;
-  static constexpr int S = TILE + (TILE % 8 == 0 ? 2 : 0);
-  static constexpr size_t smem = sizeof(double2) * kStages * 2 * KC * S;
-};
-using GemmWide = Gemm64<7, 2, 2, 7>;
-using GemmD = Gemm64<13, 1, 1, 13>;
+constexpr int kTile = 112;
+constexpr int kQuad = kTile / 2;
+constexpr int kFM = 7, kFN = 2;   // fragments of a warp
+constexpr int kThreads = 512;
+constexpr int kLoaders = 4 * kTile;   // threads that copy KC / 4 elements of either operand per stage
+constexpr int kS = kTile + 2;
+constexpr size_t kSmem = sizeof(double2) * kStages * 2 * KC * kS;
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -48,14 +44,11 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
       : "d"(a), "d"(b));
 }
 
-template <int WM, int WN, int FM, int FN>
-__global__ void __launch_bounds__(32 * WM * WN, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 gemm64_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int64_t ld, int64_t np, int nsplit,
               const PairTile* __restrict__ tiles, const int* __restrict__ pair_M, const int* __restrict__ pair_aoff,
               const int64_t* __restrict__ pair_coff, double2* __restrict__ Cpart, int64_t cstride) {
-  using G = Gemm64<WM, WN, FM, FN>;
-  constexpr int TILE = G::TILE, S = G::S, T = G::THREADS;
-  extern __shared__ __align__(16) double2 smem64[];   // [stage][A, B][KC][S]
+  extern __shared__ __align__(16) double2 smem64[];   // [stage][A, B][KC][kS]
   const int tile_id = blockIdx.x / nsplit;
   const int split = blockIdx.x % nsplit;
   const PairTile t = tiles[tile_id];
@@ -65,37 +58,42 @@ gemm64_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int6
   const int64_t p_end = np * (split + 1) / nsplit;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g8 = lane >> 2, t4 = lane & 3;
-  const int wm = (warp % WM) * 8 * FM, wn = (warp / WM) * 8 * FN;
+  const int wm = (warp & 1) * kQuad, wn = ((warp >> 1) & 1) * kQuad + (warp >> 2) * 8 * kFN;
+  // this warp's fragments inside the site pair
+  const int fm = max(0, min(kFM, (M - t.u0 - wm + 7) / 8));
+  const int fn = max(0, min((warp >> 2) == 3 ? 1 : kFN, (M - t.v0 - wn + 7) / 8));
 
-  double cr[FM][FN][2], ci[FM][FN][2];
+  double cr[kFM][kFN][2], ci[kFM][kFN][2];
 #pragma unroll
-  for (int i = 0; i < FM; ++i)
+  for (int i = 0; i < kFM; ++i)
 #pragma unroll
-    for (int j = 0; j < FN; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
+    for (int j = 0; j < kFN; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
 
-  // a thread copies column `col` of the points kk and kk + 4 of every stage
-  static_assert(2 * T == KC * TILE, "two elements of either operand per thread and stage");
-  const int kk0 = tid / TILE, col = tid % TILE;
+  // a loader copies column `col` of the points kk0, kk0 + 4, .. of every stage
+  const int kk0 = tid / kTile, col = tid % kTile;
+  const bool loads = tid < kLoaders;
   const bool ina = t.u0 + col < M, inb = t.v0 + col < M;
   const double2* ga = A + (p_begin + kk0) * ld + aoff + (ina ? t.u0 + col : 0);
   const double2* gb = B + (p_begin + kk0) * ld + aoff + (inb ? t.v0 + col : 0);
-  const unsigned sdst = (unsigned)__cvta_generic_to_shared(smem64 + kk0 * S + col);
+  const unsigned sdst = (unsigned)__cvta_generic_to_shared(smem64 + kk0 * kS + col);
   int left = (int)(p_end - p_begin) - kk0;   // points from this thread's next one to the end
   auto load_stage = [&](int buf) {
-    const unsigned d = sdst + (unsigned)(buf * 2 * KC * S * sizeof(double2));
+    if (loads) {
+      const unsigned d = sdst + (unsigned)(buf * 2 * KC * kS * sizeof(double2));
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool in = left > 4 * h;
-      const unsigned o = (unsigned)(4 * h * S * sizeof(double2));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d + o), "l"(in ? ga + 4 * h * ld : A),
-                   "r"(in && ina ? 16 : 0));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                       d + o + (unsigned)(KC * S * sizeof(double2))),
-                   "l"(in ? gb + 4 * h * ld : B), "r"(in && inb ? 16 : 0));
+      for (int h = 0; h < KC / 4; ++h) {
+        const bool in = left > 4 * h;
+        const unsigned o = (unsigned)(4 * h * kS * sizeof(double2));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d + o), "l"(in ? ga + 4 * h * ld : A),
+                     "r"(in && ina ? 16 : 0));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         d + o + (unsigned)(KC * kS * sizeof(double2))),
+                     "l"(in ? gb + 4 * h * ld : B), "r"(in && inb ? 16 : 0));
+      }
+      ga += KC * ld;
+      gb += KC * ld;
+      left -= KC;
     }
-    ga += KC * ld;
-    gb += KC * ld;
-    left -= KC;
   };
 
   const int64_t nstages = (p_end - p_begin + KC - 1) / KC;
@@ -111,41 +109,52 @@ gemm64_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int6
     if (s + kStages - 1 < nstages) load_stage(fill);
     fill = fill + 1 == kStages ? 0 : fill + 1;
     asm volatile("cp.async.commit_group;\n" ::);
-    const double2* as = smem64 + (size_t)buf * 2 * KC * S + t4 * S + wm + g8;
-    const double2* bs = smem64 + (size_t)buf * 2 * KC * S + (KC + t4) * S + wn + g8;
+    const double2* as = smem64 + (size_t)buf * 2 * KC * kS + t4 * kS + wm + g8;
+    const double2* bs = smem64 + (size_t)buf * 2 * KC * kS + (KC + t4) * kS + wn + g8;
     buf = buf + 1 == kStages ? 0 : buf + 1;
+    if (fn == 0) continue;
 #pragma unroll 1
     for (int kk = 0; kk < KC; kk += 4) {
-      double2 av[FM];
+      const double2 b0 = bs[kk * kS];
+      if (fn == kFN) {
+        const double2 b1 = bs[kk * kS + 8];
 #pragma unroll
-      for (int i = 0; i < FM; ++i) av[i] = as[kk * S + 8 * i];
-#pragma unroll
-      for (int j = 0; j < FN; ++j) {
-        const double2 bv = bs[kk * S + 8 * j];
-#pragma unroll
-        for (int i = 0; i < FM; ++i) {
-          dmma(cr[i][j][0], cr[i][j][1], av[i].x, bv.x);
-          dmma(ci[i][j][0], ci[i][j][1], av[i].x, bv.y);
+        for (int i = 0; i < kFM; ++i) {
+          if (i >= fm) break;
+          const double2 av = as[kk * kS + 8 * i];
+          dmma(cr[i][0][0], cr[i][0][1], av.x, b0.x);
+          dmma(ci[i][0][0], ci[i][0][1], av.x, b0.y);
+          dmma(cr[i][1][0], cr[i][1][1], av.x, b1.x);
+          dmma(ci[i][1][0], ci[i][1][1], av.x, b1.y);
+          dmma(cr[i][0][0], cr[i][0][1], -av.y, b0.y);
+          dmma(ci[i][0][0], ci[i][0][1], av.y, b0.x);
+          dmma(cr[i][1][0], cr[i][1][1], -av.y, b1.y);
+          dmma(ci[i][1][0], ci[i][1][1], av.y, b1.x);
         }
+      } else {
 #pragma unroll
-        for (int i = 0; i < FM; ++i) {
-          dmma(cr[i][j][0], cr[i][j][1], -av[i].y, bv.y);
-          dmma(ci[i][j][0], ci[i][j][1], av[i].y, bv.x);
+        for (int i = 0; i < kFM; ++i) {
+          if (i >= fm) break;
+          const double2 av = as[kk * kS + 8 * i];
+          dmma(cr[i][0][0], cr[i][0][1], av.x, b0.x);
+          dmma(ci[i][0][0], ci[i][0][1], av.x, b0.y);
+          dmma(cr[i][0][0], cr[i][0][1], -av.y, b0.y);
+          dmma(ci[i][0][0], ci[i][0][1], av.y, b0.x);
         }
       }
     }
   }
   double2* C = Cpart + (int64_t)split * cstride + pair_coff[t.pair];
 #pragma unroll
-  for (int i = 0; i < FM; ++i) {
+  for (int i = 0; i < kFM; ++i) {
     const int u = t.u0 + wm + 8 * i + g8;
-    if (u >= M) continue;
+    if (i >= fm || u >= M) continue;
 #pragma unroll
-    for (int j = 0; j < FN; ++j)
+    for (int j = 0; j < kFN; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int v = t.v0 + wn + 8 * j + 2 * t4 + h;
-        if (v >= M) continue;
+        if (j >= fn || v >= M) continue;
         double2* c = C + (int64_t)u * M + v;
         *c = cadd(*c, make_double2(cr[i][j][h], ci[i][j][h]));
       }
@@ -194,32 +203,15 @@ __global__ void chi_epilogue_kernel(const double2* __restrict__ Cpart, const dou
 
 }  // namespace
 
-namespace {
-
-template <int WM, int WN, int FM, int FN>
-cudaError_t launch_gemm64_t(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit,
-                            const PairTile* tiles, int ntiles, const int* pair_M, const int* pair_aoff,
-                            const int64_t* pair_coff, double2* Cpart, int64_t cstride, cudaStream_t s) {
-  using G = Gemm64<WM, WN, FM, FN>;
-  auto kernel = gemm64_kernel<WM, WN, FM, FN>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
-  if (e != cudaSuccess) return e;
-  kernel<<<ntiles * nsplit, G::THREADS, G::smem, s>>>(A, B, ld, np, nsplit, tiles, pair_M, pair_aoff, pair_coff, Cpart,
-                                                     cstride);
-  return cudaGetLastError();
-}
-
-}  // namespace
-
-cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit, int tile,
+cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit,
                           const PairTile* tiles, int ntiles, const int* pair_M, const int* pair_aoff,
                           const int64_t* pair_coff, double2* Cpart, int64_t cstride, cudaStream_t s) {
   if (np <= 0 || ntiles <= 0) return cudaSuccess;
-  if (tile == GemmD::TILE)
-    return launch_gemm64_t<13, 1, 1, 13>(A, B, ld, np, nsplit, tiles, ntiles, pair_M, pair_aoff, pair_coff, Cpart,
-                                         cstride, s);
-  return launch_gemm64_t<7, 2, 2, 7>(A, B, ld, np, nsplit, tiles, ntiles, pair_M, pair_aoff, pair_coff, Cpart, cstride,
-                                     s);
+  cudaError_t e = cudaFuncSetAttribute(gemm64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  if (e != cudaSuccess) return e;
+  gemm64_kernel<<<ntiles * nsplit, kThreads, kSmem, s>>>(A, B, ld, np, nsplit, tiles, pair_M, pair_aoff, pair_coff,
+                                                         Cpart, cstride);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_chi_epilogue(const double2* Cpart, const double2* Dpart, int nsplit, int64_t cstride,
@@ -232,17 +224,6 @@ cudaError_t launch_chi_epilogue(const double2* Cpart, const double2* Dpart, int 
   return cudaGetLastError();
 }
 
-// tile side for the site pairs of a layout (pair_M[n_pairs] rows each): the one whose tiles
-// cover the smaller area (DMMAs of the padding cost as much as the others), 112 on ties
-int gemm64_tile(int n_pairs, const int* pair_M) {
-  double wide = 0.0, d = 0.0;
-  for (int i = 0; i < n_pairs; ++i) {
-    const double a = (pair_M[i] + GemmWide::TILE - 1) / GemmWide::TILE * GemmWide::TILE;
-    const double b = (pair_M[i] + GemmD::TILE - 1) / GemmD::TILE * GemmD::TILE;
-    wide += a * a;
-    d += b * b;
-  }
-  return d < wide ? GemmD::TILE : GemmWide::TILE;
-}
+int gemm64_tile() { return kTile; }
 
 }  // namespace tg

@@ -205,8 +205,7 @@ cudaError_t launch_entries(const GreenArgs& g, const double2* G, const int2* ent
 
 // FP64 pair-block contraction: Cpart[split][cpair_off + u*M + v] += sum_p A[p][off+u] B[p][off+v]
 struct PairTile { int pair; int u0; int v0; };
-// (tile: side of the tiles, a value of gemm64_tile)
-cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit, int tile,
+cudaError_t launch_gemm64(const double2* A, const double2* B, int64_t ld, int64_t np, int nsplit,
                           const PairTile* tiles, int ntiles, const int* pair_M, const int* pair_aoff,
                           const int64_t* pair_coff, double2* Cpart, int64_t cstride, cudaStream_t s);
 
@@ -215,7 +214,7 @@ cudaError_t launch_chi_epilogue(const double2* Cpart, const double2* Dpart, int 
                                 int dimens, const int* decode, const int* norb, const int64_t* pair_coff,
                                 int n_atoms, double scale, double2* chi, cudaStream_t s);
 
-int gemm64_tile(int n_pairs, const int* pair_M);
+int gemm64_tile();
 // H(k) table for a k list (plus q): H[k][r][c] = h0 + H_nl(k + q)
 cudaError_t launch_hk_table(const GreenArgs& a, const double* kp, int64_t nk, const double* d_q, double2* phase_ws,
                             double2* H, cudaStream_t s);
