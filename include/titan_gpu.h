@@ -228,6 +228,12 @@ int tg_system_shape(const tg_ctx* ctx, int* n_atoms, int* norb_max, int* norb);
  * (calculate_chi.F90:85-89).  All matrices (dimens, dimens) complex. */
 int tg_dyson(tg_ctx* ctx, int dimens, const double* chi_hf, const double* umat, double* chi);
 
+/* tg_dyson for hosts that hold matrices row by row: chi_rows / umat_rows != 0 say that chi_hf /
+ * umat are row-major (transposed on the device instead of by the host); chi is column-major as
+ * in tg_dyson.  No counterpart in the reference. */
+int tg_dyson_order(tg_ctx* ctx, int dimens, const double* chi_hf, int chi_rows, const double* umat, int umat_rows,
+                   double* chi);
+
 /* Disturbance response to an electric field: replaces eintshe(q, e)
  * (source/eintshe.F90:2-309) for one frequency e.
  *   tchi(dimens, 4) complex = prefactor . (1/2pi) sum_{k,E} w df1iikl(k, E)

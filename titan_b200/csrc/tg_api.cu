@@ -10,10 +10,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/titan_gpu.h"
@@ -25,6 +27,7 @@ using namespace tg;
 namespace tg {
 cudaError_t dyson_device(int n, const double2* chi_hf, const double2* U, double2* work, double2* chi, int* piv,
                          int* status, cudaStream_t s);
+cudaError_t launch_transpose(int n, const double2* in, double2* out, cudaStream_t s);
 }
 
 namespace {
@@ -192,6 +195,9 @@ struct tg_ctx {
   DevArray<double2> d_triQ[4 + kTriQSlots];
   DevArray<double2> d_triws;   // factors of z - T of a pass's points
   DevArray<unsigned char> d_clws;   // workspace of the thread-block-cluster Gauss-Jordan kernel
+  // pinned staging of large transfers between pageable host arrays and the device
+  char* stage = nullptr;
+  cudaEvent_t stage_ev[2 * 8] = {};
   // tg_expectation_noalloc: device address of the library's fixed scratch array on this
   // context's device (looked up by the context's first no-alloc call)
   double2* noalloc_ptr = nullptr;
@@ -268,6 +274,94 @@ int cuda_err(tg_ctx* c, cudaError_t e, const char* where) {
     cudaError_t _e = (call);                          \
     if (_e != cudaSuccess) return cuda_err(c, _e, where); \
   } while (0)
+
+// Large transfers of pageable host arrays.  cudaMemcpyAsync stages those through one thread of
+// the driver (and on a fresh result array that thread takes every page fault); here up to
+// kStageThreads threads of this call each move their part in pieces of kStagePiece through two
+// pinned buffers of the context, copying one piece while the other is on the link.  Transfers
+// below kStageLeast, and arrays that are pinned already, go to cudaMemcpyAsync.  The source of
+// an upload may be reused, and the destination of a download read, when copy_host returns.
+constexpr int kStageThreads = 8;
+constexpr size_t kStagePiece = (size_t)1 << 20;
+constexpr size_t kStageLeast = (size_t)4 << 20;
+
+cudaError_t copy_host(tg_ctx* c, void* dst, const void* src, size_t bytes, bool to_device) {
+  const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+  auto plain = [&]() {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, c->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
+  };
+  if (bytes < kStageLeast) return plain();
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, to_device ? src : dst) != cudaSuccess) cudaGetLastError();
+  else if (at.type != cudaMemoryTypeUnregistered) return plain();
+  if (!c->stage) {
+    void* p = nullptr;
+    if (cudaMallocHost(&p, 2 * kStageThreads * kStagePiece) != cudaSuccess) {
+      cudaGetLastError();
+      return plain();
+    }
+    c->stage = static_cast<char*>(p);
+    for (auto& ev : c->stage_ev) {
+      const cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  const size_t pieces = (bytes + kStagePiece - 1) / kStagePiece;
+  const int nt = (int)std::min<size_t>(std::min<size_t>(kStageThreads, pieces),
+                                       std::max(1u, std::thread::hardware_concurrency()));
+  std::atomic<int> err{(int)cudaSuccess};
+  auto work = [&](int t) {   // pieces t, t + nt, ..
+    auto fail = [&](cudaError_t e) {
+      if (e == cudaSuccess) return false;
+      err.store((int)e);
+      return true;
+    };
+    if (fail(cudaSetDevice(c->device))) return;
+    char* buf[2] = {c->stage + (size_t)(2 * t) * kStagePiece, c->stage + (size_t)(2 * t + 1) * kStagePiece};
+    cudaEvent_t* ev = c->stage_ev + 2 * t;
+    auto part = [&](size_t i) { return std::min(kStagePiece, bytes - i * kStagePiece); };
+    size_t turn = 0;
+    if (to_device) {
+      for (size_t i = t; i < pieces; i += nt, ++turn) {
+        const int b = (int)(turn & 1);
+        if (turn >= 2 && fail(cudaEventSynchronize(ev[b]))) return;
+        std::memcpy(buf[b], static_cast<const char*>(src) + i * kStagePiece, part(i));
+        if (fail(cudaMemcpyAsync(static_cast<char*>(dst) + i * kStagePiece, buf[b], part(i), kind, c->stream))) return;
+        if (fail(cudaEventRecord(ev[b], c->stream))) return;
+      }
+      for (int b = 0; b < 2 && b < (int)turn; ++b)
+        if (fail(cudaEventSynchronize(ev[b]))) return;
+    } else {
+      auto fetch = [&](size_t i, int b) {
+        return fail(cudaMemcpyAsync(buf[b], static_cast<const char*>(src) + i * kStagePiece, part(i), kind, c->stream)) ||
+               fail(cudaEventRecord(ev[b], c->stream));
+      };
+      if (fetch(t, 0)) return;
+      for (size_t i = t; i < pieces; i += nt, ++turn) {
+        const int b = (int)(turn & 1);
+        if (i + nt < pieces && fetch(i + nt, b ^ 1)) return;
+        if (fail(cudaEventSynchronize(ev[b]))) return;
+        std::memcpy(static_cast<char*>(dst) + i * kStagePiece, buf[b], part(i));
+      }
+    }
+  };
+  std::vector<std::thread> threads;
+  int started = 0;
+  try {
+    threads.reserve(nt);
+    for (int t = 1; t < nt; ++t) {
+      threads.emplace_back(work, t);
+      ++started;
+    }
+  } catch (...) {   // no more threads to be had: their parts are done here
+  }
+  work(0);
+  for (int t = started + 1; t < nt; ++t) work(t);
+  for (auto& th : threads) th.join();
+  if (err.load() != (int)cudaSuccess) cudaStreamSynchronize(c->stream);   // no copy still reads the buffers
+  return (cudaError_t)err.load();
+}
 
 GreenArgs base_args(tg_ctx* c) {
   GreenArgs a;
@@ -780,9 +874,12 @@ int bound_finish(tg_ctx* c, bool split, int n_res, int64_t cstride, const double
       sd += bd * bd;
     }
     const double err = kappa * (2.0 * std::sqrt(sc) + std::sqrt(sd));
-    double nrm = 0.0;
+    double part[8] = {};   // independent sums: one chain of additions would bound the loop
     const double* x = chiorb + 2 * (size_t)r * cstride;
-    for (int64_t i = 0; i < 2 * cstride; ++i) nrm += x[i] * x[i];
+    for (int64_t i = 0; i < 2 * cstride; i += 8)   // (cstride is a square of a multiple of 4)
+      for (int j = 0; j < 8; ++j) part[j] += x[i + j] * x[i + j];
+    double nrm = 0.0;
+    for (double y : part) nrm += y;
     nrm = std::sqrt(nrm);
     c->err_bound[r] = err == 0.0 ? 0.0 : (nrm > 0.0 ? err / nrm : HUGE_VAL);
   }
@@ -936,6 +1033,9 @@ int tg_destroy(tg_ctx* c) {
     cudaEventDestroy(u.second.first);
     cudaEventDestroy(u.second.second);
   }
+  if (c->stage) cudaFreeHost(c->stage);
+  for (cudaEvent_t e : c->stage_ev)
+    if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;   // every DevArray member frees what the calls above did not
   return TG_OK;
@@ -1512,8 +1612,7 @@ int tg_chi0_batch(tg_ctx* c, const double* q, int n_omega, const double* e, doub
                                     nsplit, cstride, v.dimens, v.decode, v.norb, v.pair_coff,
                                     c->n_atoms, 1.0 / (2.0 * kPi), c->d_chi.p, s),
              "epilogue");
-    TG_CHECK(c, cudaMemcpyAsync(chiorb_hf + 2 * (size_t)w * cstride, c->d_chi.p, sizeof(double2) * cstride,
-                                cudaMemcpyDeviceToHost, s),
+    TG_CHECK(c, copy_host(c, chiorb_hf + 2 * (size_t)w * cstride, c->d_chi.p, sizeof(double2) * cstride, false),
              "copy chi");
   }
   cudaEventRecord(ev[6], s);
@@ -1830,8 +1929,8 @@ int chi0_qshared(tg_ctx* c, int n_q, const double* qs, int n_omega, const double
       TG_CHECK(c, launch_chi_epilogue(acc_at(c->d_C.p, iq, w), acc_at(c->d_D.p, iq, w), nsplit, cstride, v.dimens,
                                       v.decode, v.norb, v.pair_coff, c->n_atoms, 1.0 / (2.0 * kPi), c->d_chi.p, s),
                "epilogue");
-      TG_CHECK(c, cudaMemcpyAsync(chiorb_hf + 2 * ((size_t)iq * n_omega + w) * cstride, c->d_chi.p,
-                                  sizeof(double2) * cstride, cudaMemcpyDeviceToHost, s),
+      TG_CHECK(c, copy_host(c, chiorb_hf + 2 * ((size_t)iq * n_omega + w) * cstride, c->d_chi.p,
+                            sizeof(double2) * cstride, false),
                "copy chi");
     }
   TG_CHECK(c, cudaEventRecord(ev[6], s), "event");
@@ -2468,7 +2567,7 @@ int tg_chi0_linear_soc(tg_ctx* c, const double* q, double e, double Ef, double e
                                       c->d_pair_coff.p, c->n_atoms, 1.0 / (2.0 * kPi), c->d_chi.p, s),
                "epilogue");
     }
-    TG_CHECK(c, cudaMemcpyAsync(outs[k], c->d_chi.p, sizeof(double2) * cstride, cudaMemcpyDeviceToHost, s), "copy");
+    TG_CHECK(c, copy_host(c, outs[k], c->d_chi.p, sizeof(double2) * cstride, false), "copy");
   }
   profile_end(c);
   return read_status(c);
@@ -2690,6 +2789,11 @@ int tg_ldos(tg_ctx* c, int n_e, const double* e, double eta, double* ldosu, doub
 }
 
 int tg_dyson(tg_ctx* c, int dimens, const double* chi_hf, const double* umat, double* chi) {
+  return tg_dyson_order(c, dimens, chi_hf, 0, umat, 0, chi);
+}
+
+int tg_dyson_order(tg_ctx* c, int dimens, const double* chi_hf, int chi_rows, const double* umat, int umat_rows,
+                   double* chi) {
   if (!c) return TG_ERR_ARG;
   if (dimens <= 0 || !chi_hf || !umat || !chi) return set_err(c, TG_ERR_ARG, "tg_dyson: bad args");
   cudaSetDevice(c->device);
@@ -2701,12 +2805,15 @@ int tg_dyson(tg_ctx* c, int dimens, const double* chi_hf, const double* umat, do
   double2* U = X + nn;
   double2* W = U + nn;
   double2* R = W + nn;
-  TG_CHECK(c, cudaMemcpyAsync(X, chi_hf, sizeof(double2) * nn, cudaMemcpyHostToDevice, s), "upload");
-  TG_CHECK(c, cudaMemcpyAsync(U, umat, sizeof(double2) * nn, cudaMemcpyHostToDevice, s), "upload");
   int rc = reset_status(c);
   if (rc) return rc;
+  // a row-major matrix arrives in a free buffer and is transposed into its place
+  TG_CHECK(c, copy_host(c, chi_rows ? W : X, chi_hf, sizeof(double2) * nn, true), "upload");
+  if (chi_rows) TG_CHECK(c, launch_transpose(dimens, W, X, s), "transpose");
+  TG_CHECK(c, copy_host(c, umat_rows ? R : U, umat, sizeof(double2) * nn, true), "upload");
+  if (umat_rows) TG_CHECK(c, launch_transpose(dimens, R, U, s), "transpose");
   TG_CHECK(c, dyson_device(dimens, X, U, W, R, c->d_piv.p, c->d_status.p, s), "dyson");
-  TG_CHECK(c, cudaMemcpyAsync(chi, R, sizeof(double2) * nn, cudaMemcpyDeviceToHost, s), "copy");
+  TG_CHECK(c, copy_host(c, chi, R, sizeof(double2) * nn, false), "copy");
   return read_status(c);
 }
 

@@ -400,7 +400,26 @@ __global__ void __launch_bounds__(256) back_solve_kernel(int n, int k0, int nb, 
   }
 }
 
+// out = in^T, n x n
+__global__ void __launch_bounds__(256) transpose_kernel(int n, const double2* __restrict__ in,
+                                                        double2* __restrict__ out) {
+  __shared__ double2 t[32][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  for (int i = y; i < 32; i += 8)
+    if (r0 + i < n && c0 + x < n) t[i][x] = in[(size_t)(r0 + i) * n + c0 + x];
+  __syncthreads();
+  for (int i = y; i < 32; i += 8)
+    if (c0 + i < n && r0 + x < n) out[(size_t)(c0 + i) * n + r0 + x] = t[x][i];
+}
+
 }  // namespace
+
+cudaError_t launch_transpose(int n, const double2* in, double2* out, cudaStream_t s) {
+  const dim3 g((n + 31) / 32, (n + 31) / 32);
+  transpose_kernel<<<g, 256, 0, s>>>(n, in, out);
+  return cudaGetLastError();
+}
 
 // work (n x n) and chi (n x n) are overwritten; piv[n]
 cudaError_t dyson_device(int n, const double2* chi_hf, const double2* U, double2* work, double2* chi, int* piv,

@@ -52,6 +52,7 @@ SIGNATURES = {
     "tg_gg_tensor": (C.c_int, [C.c_void_p, C.c_double, C.c_double, C.c_int, _ip, _dp]),
     "tg_fermi_column": (C.c_int, [C.c_void_p, C.c_double, C.c_double, _dp]),
     "tg_dyson": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp, _dp]),
+    "tg_dyson_order": (C.c_int, [C.c_void_p, C.c_int, _dp, C.c_int, _dp, C.c_int, _dp]),
     "tg_set_green_method": (C.c_int, [C.c_void_p, C.c_int]),
     "tg_ldos": (C.c_int, [C.c_void_p, C.c_int, _dp, C.c_double, _dp, _dp]),
     "tg_smunu": (C.c_int, [C.c_void_p, C.c_double, C.c_double, _dp]),
@@ -165,6 +166,15 @@ def jacobian_assemble(system, T, D, fixEf=False):
 def _fortran_complex(m):
     """numpy [row, col] complex matrix -> Fortran-ordered complex128 buffer."""
     return np.ascontiguousarray(np.asarray(m, dtype=np.complex128).T)
+
+
+def _ordered_complex(m):
+    """numpy [row, col] complex matrix -> (contiguous complex128 buffer, 1 if it is row by row);
+    a Fortran-ordered matrix is passed as it lies."""
+    m = np.asarray(m, dtype=np.complex128)
+    if m.flags.f_contiguous:
+        return m.T, 0
+    return np.ascontiguousarray(m), 1
 
 
 class GreenGPU:
@@ -418,11 +428,11 @@ class GreenGPU:
 
     def dyson(self, chi_hf, U):
         n = chi_hf.shape[0]
-        a = _fortran_complex(chi_hf)
-        u = _fortran_complex(U)
+        a, a_rows = _ordered_complex(chi_hf)
+        u, u_rows = _ordered_complex(U)
         out = np.empty((n, n), np.complex128)
-        self._check(self.lib.tg_dyson(self.h, n, _p(a.view(np.float64)), _p(u.view(np.float64)),
-                                      _p(out.view(np.float64))))
+        self._check(self.lib.tg_dyson_order(self.h, n, _p(a.view(np.float64)), a_rows, _p(u.view(np.float64)), u_rows,
+                                            _p(out.view(np.float64))))
         return out.T
 
     def chi0_linear_soc(self, q, e, Ef, eta, etap, x2, p2, vsoc):
