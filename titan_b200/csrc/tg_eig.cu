@@ -24,7 +24,7 @@ namespace tg {
 namespace {
 
 constexpr int kHhMax = 96;          // largest dimension of hh_small_kernel (three rows per lane)
-constexpr int kHhThreads = 384;
+constexpr int kHhThreads = 480;
 constexpr int kQlIterations = 60;   // per eigenvalue
 
 __host__ __device__ inline int odd_stride(int n) { return n | 1; }
@@ -38,27 +38,17 @@ __device__ __forceinline__ double2 warp_sum2(double2 v) {
 }
 
 // --------------------------------------------------------------------------- 1. tridiagonalisation
-// B holds A column by column with an odd stride (A(r, c) at c S + r), both triangles; PT
-// threads per row (or, for Q, per column) share its sums.  Per reflector: norm (every warp on
-// its own, no barrier), product A v, update
+// B holds A column by column with an odd stride (A(r, c) at c S + r), both triangles.  The warps
+// share the trailing block by 32 rows (a lane per row, so the vector entry of a column is one
+// broadcast) and by columns; for Q by 32 columns and by rows.  Per reflector: norm and vector
+// (warp 0), product A v with the column parts added up through shared memory, update
 //   A <- A - v p^H - q v^H,  p = tau A v, q = p - Re(tau p^H v) v,
-// three barriers; per reflector of Q one.  The loops read four entries before they write the
-// first (the compiler cannot tell the stores from the next loads apart).  Bound by the latency
-// of these steps where one matrix fills the SM (n = 90), by shared memory where several share
-// it (15 + 14 wavefronts per 32 entries and step, n^3 / 3 entries in all).
+// four barriers; per reflector of Q two.  The loops read four entries before they write the
+// first (the compiler cannot tell the stores from the next loads apart).  Bound by shared
+// memory: 15 wavefronts per 32 entries and reflector for the reduction, 14 for Q (29 and 23
+// with neighbouring lanes on the columns of a row), n^3 / 3 entries each.
 constexpr int kHhBatch = 4;
 
-template <int PT>
-__device__ __forceinline__ double2 group_sum2(double2 v) {
-#pragma unroll
-  for (int o = 1; o < PT; o <<= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  return v;
-}
-
-template <int PT>
 __global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __restrict__ H, int64_t nk, int n,
                                                             const int* __restrict__ rows, int ns,
                                                             double* __restrict__ D, double* __restrict__ E,
@@ -69,8 +59,9 @@ __global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __r
   double2* v = B + n * S;
   double2* p = v + n;
   double2* taus = p + n;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rt = tid / PT, h = tid % PT;
+  double2* dots = taus + n;     // [3] per 32 rows, then tau of the step
+  double2* parts = dots + 4;    // [warps][32]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const double2 zero = make_double2(0.0, 0.0);
   for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
     const double2* Hk = H + k * (int64_t)n * n;
@@ -80,78 +71,91 @@ __global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __r
     for (int j = 0; j + 1 < n; ++j) {
       const int m = n - j - 1;
       double2* col = B + j * S + j + 1;
-      double2 x[3];
-      double part = 0.0;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const int r = lane + 32 * i;
-        x[i] = r < m ? col[r] : zero;
-        if (r > 0) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
-      }
-      const double2 alpha = col[0];
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      const bool refl = !(part == 0.0 && alpha.y == 0.0);
-      // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
-      const double beta =
-          refl ? -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, part))), alpha.x) : alpha.x;
-      double2 tau = zero;
-      if (refl) {
-        const double ib = 1.0 / beta;
-        tau = make_double2((beta - alpha.x) * ib, -alpha.y * ib);
-      }
       if (warp == 0) {
+        double2 x[3];
+        double part = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const int r = lane + 32 * i;
+          x[i] = r < m ? col[r] : zero;
+          if (r > 0) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
+        }
+        const double2 alpha = col[0];
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        const bool refl = !(part == 0.0 && alpha.y == 0.0);
+        // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
+        const double beta =
+            refl ? -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, part))), alpha.x) : alpha.x;
+        double2 tau = zero;
+        if (refl) {
+          const double ib = 1.0 / beta;
+          tau = make_double2((beta - alpha.x) * ib, -alpha.y * ib);
+          const double dr = alpha.x - beta, di = alpha.y;
+          const double inv = 1.0 / fma(dr, dr, di * di);
+          const double2 sc = make_double2(dr * inv, -di * inv);
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const int r = lane + 32 * i;
+            if (r < m) {
+              const double2 vr = r == 0 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
+              v[r] = vr;
+              col[r] = vr;   // kept for Q; the column is done with
+            }
+          }
+        }
         if (lane == 0) {
           D[k * n + j] = B[j * S + j].x;
           E[k * n + j] = beta;
           taus[j] = tau;
         }
-        if (refl) {
-          const double dr = alpha.x - beta, di = alpha.y;
-          const double inv = 1.0 / fma(dr, dr, di * di);
-          const double2 sc = make_double2(dr * inv, -di * inv);
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            const int r = lane + 32 * i;
-            if (r < m) v[r] = r == 0 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
-          }
-        }
       }
       __syncthreads();
-      if (!refl) continue;   // (uniform: every thread took the same sums)
-      if (warp == 0)
-        for (int r = lane; r < m; r += 32) col[r] = v[r];   // kept for Q; the column is done with
-      double2* Ar = B + (j + 1) * S + j + 1 + rt;
+      const double2 tau = taus[j];
+      if (tau.x == 0.0 && tau.y == 0.0) continue;   // no reflector (the same in every thread)
+      // row block and column part of this warp
+      const int nrb = (m + 31) >> 5, np = nw / nrb;
+      const int rb = warp % nrb, cp = warp / nrb, r = 32 * rb + lane;
+      double2* Ar = B + (j + 1) * S + j + 1 + r;
+      const bool mine = cp < np && r < m;
       double2 acc = zero, acc1 = zero;
-      if (rt < m) {
-        int c = h;
-        for (; c + 3 * PT < m; c += 4 * PT) {
+      if (mine) {
+        int c = cp;
+        for (; c + 3 * np < m; c += 4 * np) {
           acc = cfma(Ar[c * S], v[c], acc);
-          acc1 = cfma(Ar[(c + PT) * S], v[c + PT], acc1);
-          acc = cfma(Ar[(c + 2 * PT) * S], v[c + 2 * PT], acc);
-          acc1 = cfma(Ar[(c + 3 * PT) * S], v[c + 3 * PT], acc1);
+          acc1 = cfma(Ar[(c + np) * S], v[c + np], acc1);
+          acc = cfma(Ar[(c + 2 * np) * S], v[c + 2 * np], acc);
+          acc1 = cfma(Ar[(c + 3 * np) * S], v[c + 3 * np], acc1);
         }
-        for (; c < m; c += PT) acc = cfma(Ar[c * S], v[c], acc);
+        for (; c < m; c += np) acc = cfma(Ar[c * S], v[c], acc);
       }
-      acc = group_sum2<PT>(cadd(acc, acc1));
-      const double2 pr = cmul(tau, acc);
-      if (rt < m && h == 0) p[rt] = pr;
+      parts[32 * warp + lane] = cadd(acc, acc1);
       __syncthreads();
-      double2 dot = zero;
-      for (int r = lane; r < m; r += 32) dot = cfma(cconj(p[r]), v[r], dot);
-      dot = warp_sum2(dot);
-      const double t2 = -cmul(tau, dot).x;   // 2 Re(-tau (p^H v) / 2)
-      if (rt < m) {
-        const double2 vr = v[rt], qr = make_double2(fma(t2, vr.x, pr.x), fma(t2, vr.y, pr.y));
-        for (int c0 = h; c0 < m; c0 += kHhBatch * PT) {
+      if (cp == 0) {
+        double2 a = zero;
+        for (int q = 0; q < np; ++q) a = cadd(a, parts[32 * (q * nrb + rb) + lane]);
+        const double2 pr = cmul(tau, a);
+        if (r < m) p[r] = pr;
+        const double2 d = warp_sum2(r < m ? cmul(cconj(pr), v[r]) : zero);
+        if (lane == 0) dots[rb] = d;
+      }
+      __syncthreads();
+      if (mine) {
+        double2 dot = dots[0];
+        for (int q = 1; q < nrb; ++q) dot = cadd(dot, dots[q]);
+        const double t2 = -cmul(tau, dot).x;   // 2 Re(-tau (p^H v) / 2)
+        const double2 vr = v[r], pr = p[r];
+        const double2 qr = make_double2(fma(t2, vr.x, pr.x), fma(t2, vr.y, pr.y));
+        for (int c0 = cp; c0 < m; c0 += kHhBatch * np) {
           double2 a[kHhBatch];
 #pragma unroll
           for (int u = 0; u < kHhBatch; ++u) {
-            const int c = c0 + u * PT;
+            const int c = c0 + u * np;
             a[u] = c < m ? cfms(qr, cconj(v[c]), cfms(vr, cconj(p[c]), Ar[c * S])) : zero;
           }
 #pragma unroll
           for (int u = 0; u < kHhBatch; ++u)
-            if (c0 + u * PT < m) Ar[(c0 + u * PT) * S] = a[u];
+            if (c0 + u * np < m) Ar[(c0 + u * np) * S] = a[u];
         }
       }
       __syncthreads();
@@ -166,36 +170,45 @@ __global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __r
       const double2 tau = taus[j];
       const bool refl = tau.x != 0.0 || tau.y != 0.0;
       const double2* vj = B + j * S + j + 1;
-      double2* col = B + (j + 1 + rt) * S + j + 1;   // this thread's column
-      double2 y = zero, y1 = zero;
-      if (refl && rt > 0 && rt < m) {
-        int r = 1 + h;
-        for (; r + 3 * PT < m; r += 4 * PT) {
-          y = cfma(cconj(vj[r]), col[r], y);
-          y1 = cfma(cconj(vj[r + PT]), col[r + PT], y1);
-          y = cfma(cconj(vj[r + 2 * PT]), col[r + 2 * PT], y);
-          y1 = cfma(cconj(vj[r + 3 * PT]), col[r + 3 * PT], y1);
+      const int nrb = (m + 31) >> 5, np = nw / nrb;
+      const int rb = warp % nrb, rp = warp / nrb, ct = 32 * rb + lane;   // this thread's column, row part
+      const bool mine = rp < np && ct < m;
+      double2* col = B + (j + 1 + ct) * S + j + 1;
+      if (refl) {
+        double2 y = zero, y1 = zero;
+        if (mine && ct > 0) {
+          int r = 1 + rp;
+          for (; r + 3 * np < m; r += 4 * np) {
+            y = cfma(cconj(vj[r]), col[r], y);
+            y1 = cfma(cconj(vj[r + np]), col[r + np], y1);
+            y = cfma(cconj(vj[r + 2 * np]), col[r + 2 * np], y);
+            y1 = cfma(cconj(vj[r + 3 * np]), col[r + 3 * np], y1);
+          }
+          for (; r < m; r += np) y = cfma(cconj(vj[r]), col[r], y);
         }
-        for (; r < m; r += PT) y = cfma(cconj(vj[r]), col[r], y);
+        parts[32 * warp + lane] = cadd(y, y1);
       }
-      y = group_sum2<PT>(cadd(y, y1));
-      if (rt == 0) y = make_double2(1.0, 0.0);   // column j + 1 enters as a unit vector
-      const double2 ty = cmul(tau, y);
-      if (rt < m) {
-        if (refl || rt == 0)
-          for (int r0 = 1 + h; r0 < m; r0 += kHhBatch * PT) {
+      __syncthreads();
+      if (mine) {
+        double2 y = zero;
+        if (ct == 0) y = make_double2(1.0, 0.0);   // column j + 1 enters as a unit vector
+        else if (refl)
+          for (int q = 0; q < np; ++q) y = cadd(y, parts[32 * (q * nrb + rb) + lane]);
+        const double2 ty = cmul(tau, y);
+        if (refl || ct == 0)
+          for (int r0 = 1 + rp; r0 < m; r0 += kHhBatch * np) {
             double2 a[kHhBatch];
 #pragma unroll
             for (int u = 0; u < kHhBatch; ++u) {
-              const int r = r0 + u * PT;
+              const int r = r0 + u * np;
               const double2 vr = refl && r < m ? vj[r] : zero;   // (no reflector: the unit vector stays)
-              a[u] = cfms(ty, vr, rt > 0 && r < m ? col[r] : zero);
+              a[u] = cfms(ty, vr, ct > 0 && r < m ? col[r] : zero);
             }
 #pragma unroll
             for (int u = 0; u < kHhBatch; ++u)
-              if (r0 + u * PT < m) col[r0 + u * PT] = a[u];
+              if (r0 + u * np < m) col[r0 + u * np] = a[u];
           }
-        if (h == 0) col[0] = make_double2((rt == 0 ? 1.0 : 0.0) - ty.x, -ty.y);
+        if (rp == 0) col[0] = make_double2((ct == 0 ? 1.0 : 0.0) - ty.x, -ty.y);
       }
       __syncthreads();
     }
@@ -495,7 +508,13 @@ size_t fin_smem(int n, bool packed) {
 
 bool fin_packed(int n, int optin) { return fin_smem(n, false) > (size_t)optin; }
 
-size_t hh_smem(int n) { return sizeof(double2) * ((size_t)n * odd_stride(n) + 3 * (size_t)n); }
+// warps per matrix: 32 rows each, times the parts of the columns (few where several matrices
+// share an SM)
+int hh_warps(int n) { return n <= 32 ? 2 : n <= 40 ? 4 : n <= 64 ? 6 : n <= 76 ? 9 : 15; }
+
+size_t hh_smem(int n) {
+  return sizeof(double2) * ((size_t)n * odd_stride(n) + 3 * (size_t)n + 4 + 32 * (size_t)hh_warps(n));
+}
 
 // rotations and sweeps kept per k: the iteration takes about 1.3 n^2 rotations in 2.3 n sweeps
 int ql_cap(int n) { return 3 * n * n + 32; }
@@ -528,18 +547,15 @@ cudaError_t launch_hh_small(const double2* H, int64_t nk, int n, const int* rows
   if (nk <= 0) return cudaSuccess;
   if (!hh_small_supported(n) || ns <= 0 || ns > n) return cudaErrorInvalidValue;
   const size_t smem = hh_smem(n);
-  // two threads per row where several matrices share an SM, four where one fills it
-  const bool wide = smem > (size_t)optin_smem() / 2;
-  const int threads = ((wide ? 4 : 2) * n + 31) / 32 * 32;
-  auto kernel = wide ? hh_small_kernel<4> : hh_small_kernel<2>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int threads = 32 * hh_warps(n);
+  cudaError_t e = cudaFuncSetAttribute(hh_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hh_small_kernel, threads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm <= 0) return cudaErrorInvalidValue;
   const int64_t grid = std::min<int64_t>(nk, (int64_t)num_sms * per_sm);
-  kernel<<<(unsigned)grid, threads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
+  hh_small_kernel<<<(unsigned)grid, threads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
   return cudaGetLastError();
 }
 
