@@ -139,6 +139,16 @@ cudaError_t zgemm(int m, int n, int k, const double2* A, int64_t lda, const doub
   return cudaGetLastError();
 }
 
+// largest key of the warp and the first row that has it, by integer reductions on the key's two
+// words
+__device__ __forceinline__ void warp_best(unsigned long long& key, int& row) {
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+  row = (int)__reduce_min_sync(0xffffffffu, hi == mhi && lo == mlo ? (unsigned)row : 0x7fffffffu);
+  key = (unsigned long long)mhi << 32 | mlo;
+}
+
 // ---------------------------------------------------------------------------
 // panel: columns j0 .. j0 + nb - 1 of M, rows j0 .. n - 1
 // ---------------------------------------------------------------------------
@@ -152,7 +162,7 @@ __global__ void __launch_bounds__(kPanThreads, 1) panel_kernel(int n, int j0, in
   extern __shared__ __align__(16) double2 psm[];
   __shared__ unsigned long long skey[32];
   __shared__ int srow[32];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, T = blockDim.x, nw = T >> 5;
   const int rows = n - j0;
   double2* P = psm;
   auto at = [&](int r, int c) -> double2& {   // r relative to j0
@@ -160,14 +170,14 @@ __global__ void __launch_bounds__(kPanThreads, 1) panel_kernel(int n, int j0, in
   };
   if (STAGED) {
     for (int c = 0; c < nb; ++c)
-      for (int r = tid; r < rows; r += kPanThreads) P[r * (kPan + 1) + c] = M[(int64_t)(j0 + c) * n + j0 + r];
+      for (int r = tid; r < rows; r += T) P[r * (kPan + 1) + c] = M[(int64_t)(j0 + c) * n + j0 + r];
     __syncthreads();
   }
   for (int c = 0; c < nb; ++c) {
     // largest |Re| + |Im| of column c among rows >= c, first row on ties
     unsigned long long key = 0ull;
     int row = 0x7fffffff;
-    for (int r = tid; r < rows; r += kPanThreads) {
+    for (int r = tid; r < rows; r += T) {
       if (r < c) continue;
       const double2 v = at(r, c);
       const double m = fabs(v.x) + fabs(v.y);
@@ -177,29 +187,15 @@ __global__ void __launch_bounds__(kPanThreads, 1) panel_kernel(int n, int j0, in
         row = r;
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o);
-      const int r2 = __shfl_xor_sync(0xffffffffu, row, o);
-      if (k2 > key || (k2 == key && r2 < row)) {
-        key = k2;
-        row = r2;
-      }
-    }
+    warp_best(key, row);
     if (lane == 0) {
       skey[warp] = key;
       srow[warp] = row;
     }
     __syncthreads();
-    key = skey[lane];
-    row = srow[lane];
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o);
-      const int r2 = __shfl_xor_sync(0xffffffffu, row, o);
-      if (k2 > key || (k2 == key && r2 < row)) {
-        key = k2;
-        row = r2;
-      }
-    }
+    key = lane < nw ? skey[lane] : 0ull;
+    row = lane < nw ? srow[lane] : 0x7fffffff;
+    warp_best(key, row);
     const int p = key == 0ull ? c : row;
     if (tid == 0) {
       piv[j0 + c] = j0 + p;
@@ -219,7 +215,7 @@ __global__ void __launch_bounds__(kPanThreads, 1) panel_kernel(int n, int j0, in
     for (int cc = 1; cc < kPan; ++cc)
       if (cc == c) diag = u[cc];
     const double2 d = crecip(diag);
-    for (int r = tid; r < rows; r += kPanThreads) {
+    for (int r = tid; r < rows; r += T) {
       if (r <= c) continue;
       const double2 f = cmul(at(r, c), d);
       at(r, c) = f;
@@ -231,7 +227,7 @@ __global__ void __launch_bounds__(kPanThreads, 1) panel_kernel(int n, int j0, in
   }
   if (STAGED)
     for (int c = 0; c < nb; ++c)
-      for (int r = tid; r < rows; r += kPanThreads) M[(int64_t)(j0 + c) * n + j0 + r] = P[r * (kPan + 1) + c];
+      for (int r = tid; r < rows; r += T) M[(int64_t)(j0 + c) * n + j0 + r] = P[r * (kPan + 1) + c];
 }
 
 // Net effect of the row swaps piv[j0 .. j0 + nb) (rows relative to j0, nb <= kBlock): row j < nb
@@ -447,7 +443,9 @@ cudaError_t dyson_device(int n, const double2* chi_hf, const double2* U, double2
     for (int j0 = k0; j0 < k1; j0 += kPan) {
       const int nb = std::min(kPan, k1 - j0);
       const size_t pb = pan_bytes * (size_t)(n - j0);
-      if (pb + pan_static <= (size_t)optin) panel_kernel<true><<<1, kPanThreads, pb, s>>>(n, j0, nb, work, piv, status);
+      // a thread per row: fewer warps make the block-wide search cheaper
+      const int threads = std::min(kPanThreads, std::max(64, (n - j0 + 31) / 32 * 32));
+      if (pb + pan_static <= (size_t)optin) panel_kernel<true><<<1, threads, pb, s>>>(n, j0, nb, work, piv, status);
       else panel_kernel<false><<<1, kPanThreads, 0, s>>>(n, j0, nb, work, piv, status);
       const int others = k1 - k0 - nb;
       if (others > 0)
