@@ -768,6 +768,7 @@ int split_prepare(tg_ctx* c, const ChiView& v, const SplitChunks& ch, SplitPassD
   pd.n_chunks = nc;
   pd.n_ksteps = nks;
   pd.stride = ch.stride;
+  pd.max_count = nc > 0 ? *std::max_element(ch.count.begin(), ch.count.end()) : 0;
   pd.slot0 = c->d_chunks.p;
   pd.count = c->d_chunks.p + nc;
   pd.kstart = c->d_chunks.p + 2 * nc;

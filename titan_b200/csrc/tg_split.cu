@@ -36,8 +36,9 @@ __global__ void split_rowmax_kernel(const double2* __restrict__ X, int64_t ld, i
   if (s_begin >= cnt) return;
   const int s_end = min(cnt, s_begin + kRowmaxSlots);
   const int64_t base = (int64_t)slot0[c];
-  for (int64_t e = threadIdx.x; e < ld; e += blockDim.x) {
+  for (int64_t e = blockIdx.z * (int64_t)blockDim.x + threadIdx.x; e < ld; e += (int64_t)gridDim.z * blockDim.x) {
     double m = 0.0;
+#pragma unroll 4
     for (int s = s_begin; s < s_end; ++s) {
       const double2 v = X[(base + (int64_t)s * stride) * ld + e];
       m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
@@ -61,8 +62,9 @@ __global__ void split_rowmax_e16_kernel(const int16_t* __restrict__ E16, int64_t
   const int64_t base = (int64_t)slot0[c];
   const int64_t ld2 = ld / 2;
   const uint32_t* W = reinterpret_cast<const uint32_t*>(E16);
-  for (int64_t e2 = threadIdx.x; e2 < ld2; e2 += blockDim.x) {
+  for (int64_t e2 = blockIdx.z * (int64_t)blockDim.x + threadIdx.x; e2 < ld2; e2 += (int64_t)gridDim.z * blockDim.x) {
     int m0 = -32768, m1 = -32768;
+#pragma unroll 8
     for (int s = s_begin; s < s_end; ++s) {
       const uint32_t w = W[((base + (int64_t)s * stride) * ld) / 2 + e2];
       m0 = max(m0, (int)(int16_t)(w & 0xffffu));
@@ -612,11 +614,22 @@ int split_nsplit(int ntiles, int num_sms, int64_t ksteps_hint) {
   return best;
 }
 
+namespace {
+
+// blocks of kRowmaxSlots points of a chunk by 256 of its elements: a large system has few
+// points per chunk and many elements, a small one the other way round
+dim3 rowmax_grid(const SplitPassDev& p, int64_t elems) {
+  const int gx = (std::max(p.max_count, 1) + kRowmaxSlots - 1) / kRowmaxSlots;
+  const int gz = (int)std::max<int64_t>(1, std::min<int64_t>((elems + 255) / 256, 64));
+  return dim3(gx, p.n_chunks, gz);
+}
+
+}  // namespace
+
 cudaError_t split_rowmax(const double2* X, int64_t ld, const SplitPassDev& p, unsigned long long* M64,
                          cudaStream_t s) {
   if (p.n_chunks <= 0) return cudaSuccess;
-  const int gx = (kSplitMaxChunk + kRowmaxSlots - 1) / kRowmaxSlots;
-  split_rowmax_kernel<<<dim3(gx, p.n_chunks), 256, 0, s>>>(X, ld, p.stride, p.slot0, p.count, M64);
+  split_rowmax_kernel<<<rowmax_grid(p, ld), 256, 0, s>>>(X, ld, p.stride, p.slot0, p.count, M64);
   return cudaGetLastError();
 }
 
@@ -624,8 +637,7 @@ cudaError_t split_rowmax_e16(const int16_t* E16, int64_t ld, const SplitPassDev&
                              cudaStream_t s) {
   if (p.n_chunks <= 0) return cudaSuccess;
   if (ld % 2) return cudaErrorInvalidValue;
-  const int gx = (kSplitMaxChunk + kRowmaxSlots - 1) / kRowmaxSlots;
-  split_rowmax_e16_kernel<<<dim3(gx, p.n_chunks), 256, 0, s>>>(E16, ld, p.stride, p.slot0, p.count, M64);
+  split_rowmax_e16_kernel<<<rowmax_grid(p, ld / 2), 256, 0, s>>>(E16, ld, p.stride, p.slot0, p.count, M64);
   return cudaGetLastError();
 }
 

@@ -72,6 +72,7 @@ struct SplitChunks {
 // device views used by the kernels
 struct SplitPassDev {
   int n_chunks = 0, n_ksteps = 0;
+  int max_count = 0;   // points of the longest chunk
   int stride = 1;
   const int* slot0 = nullptr;
   const int* count = nullptr;
