@@ -928,8 +928,17 @@ int choose_nsplit(tg_ctx* c, const ChiView& v, bool split, int64_t P, int* out) 
   }
   float best_ms = 0.f;
   int best = model;
-  for (int ns = 1; ns <= 64; ns *= 2) {
-    if ((int64_t)ns * v.ntiles > (int64_t)64 * c->num_sms * 64) break;
+  // 1, 2, 4, .. 64 and the smallest count whose tiles fill every SM equally (37 for the 36 and
+  // 216 tiles of two spd sites on 148 SMs)
+  const int tiles = split ? (int)v.split->tiles.size() : v.ntiles;
+  std::vector<int> counts = {1, 2, 4, 8, 16, 32, 64};
+  for (int ns = 1; ns <= 64; ++ns)
+    if ((int64_t)tiles * ns % c->num_sms == 0) {
+      if (std::find(counts.begin(), counts.end(), ns) == counts.end()) counts.push_back(ns);
+      break;
+    }
+  for (int ns : counts) {
+    if ((int64_t)ns * v.ntiles > (int64_t)64 * c->num_sms * 64) continue;
     TG_CHECK(c, c->d_tune.ensure((size_t)ns * cstride), "alloc tuning accumulators");
     float ms = 0.f;
     for (int rep = 0; rep < 2; ++rep) {   // the first launch warms up
