@@ -59,6 +59,11 @@ __device__ __forceinline__ uint32_t exponent_pair(double2 a, double2 b) {
   return (uint32_t)(uint16_t)exponent_code16(a) | (uint32_t)(uint16_t)exponent_code16(b) << 16;
 }
 
+// two adjacent complex numbers, 32-byte aligned, in one store (a whole sector)
+__device__ __forceinline__ void store_pair(double2* p, double2 a, double2 b) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
+}
+
 // G = X + i Y with X = sum_a Re(D_a) P_a and Y = sum_a Im(D_a) P_a, both Hermitian because every
 // P_a = u_a u_a^H is: only the entries r <= c are formed, G(r, c) = X + i Y and
 // G(c, r) = conj(X) + i conj(Y).  One task is a k and 16 energies; a warp takes tiles of two
@@ -205,8 +210,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
             v1 = cconj(v1);
           }
           const int64_t o = (int64_t)pt * nn + pos;
-          out[o] = v0;
-          out[o + 1] = v1;
+          store_pair(out + o, v0, v1);
           if (eout) *reinterpret_cast<uint32_t*>(eout + o) = exponent_pair(v0, v1);
         };
         if (c == r) {
