@@ -18,6 +18,8 @@ __host__ __device__ inline int pair_stride(int n) { return (n + 6) / 8 * 8 + 1; 
 // A pair is an orbital a of one site and an orbital b of another (or the same), as the rows
 // (a up, a down, b up, b down); per pair and point p
 //   acc[s' + 2 t + 4 t' + 8 s] += w_p Ga(a s', b t) Gb(b t', a s)
+// and, where Ga and Gb differ, the same with the two exchanged in the second half of the npairs =
+// 2 nlist sums (both from one reading of the matrices),
 // into the CTA's slice of acc (zeroed before the first pass of a call).
 // A thread owns one pair for the whole launch, its 16 sums in registers; tpm threads share a
 // point (blockDim / tpm points at a time), blockIdx.y takes tpm pairs each.  STAGED: the
@@ -27,7 +29,8 @@ __host__ __device__ inline int pair_stride(int n) { return (n + 6) / 8 * 8 + 1; 
 template <bool STAGED>
 __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(GreenArgs g, const double2* __restrict__ Ga,
                                                             const double2* __restrict__ Gb,
-                                                            const int4* __restrict__ pairs, int npairs, int tpm,
+                                                            const int4* __restrict__ pairs, int nlist, int npairs,
+                                                            int tpm,
                                                             double2* __restrict__ acc) {
   extern __shared__ __align__(16) double2 psm[];
   const int n = g.n, S = STAGED ? pair_stride(n) : n;
@@ -38,7 +41,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(GreenArgs g, cons
   const bool two = Ga != Gb;
   const int64_t mat = (int64_t)n * S;
   const bool mine = m < slots && pi < npairs;
-  const int4 pr = mine ? pairs[pi] : make_int4(0, 0, 0, 0);
+  const int4 pr = mine ? pairs[pi % nlist] : make_int4(0, 0, 0, 0);
+  const bool swapped = pi >= nlist;   // second half of a two-matrix call: Gb in the first factor
   double2 s16[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) s16[q] = make_double2(0.0, 0.0);
@@ -68,6 +72,11 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(GreenArgs g, cons
     }
     if (mine && pl < g.np) {
       const double w = point_weight(g, pl);
+      if (swapped) {
+        const double2* t = xa;
+        xa = xb;
+        xb = t;
+      }
       const int ra[2] = {pr.x, pr.y}, rb[2] = {pr.z, pr.w};
       double2 u[2][2], v[2][2];
 #pragma unroll
@@ -158,15 +167,17 @@ cudaError_t pair_plan(int n, int npairs, bool two, int num_sms, int64_t np, Pair
 
 }  // namespace
 
-size_t pair_partials(int n, int npairs, bool two, int num_sms, int64_t np) {
+size_t pair_partials(int n, int nlist, bool two, int num_sms, int64_t np) {
   PairPlan p;
+  const int npairs = two ? 2 * nlist : nlist;
   if (npairs <= 0 || pair_plan(n, npairs, two, num_sms, np, p) != cudaSuccess) return 1;
   return (size_t)p.grid * p.slots;
 }
 
-cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* Gb, const int4* pairs, int npairs,
+cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* Gb, const int4* pairs, int nlist,
                          int num_sms, double2* acc, cudaStream_t s) {
-  if (npairs <= 0 || g.np <= 0) return cudaSuccess;
+  if (nlist <= 0 || g.np <= 0) return cudaSuccess;
+  const int npairs = Ga != Gb ? 2 * nlist : nlist;
   PairPlan p;
   cudaError_t e = pair_plan(g.n, npairs, Ga != Gb, num_sms, g.np, p);
   if (e != cudaSuccess) return e;
@@ -174,9 +185,9 @@ cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* G
   if (p.staged) {
     e = cudaFuncSetAttribute(pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return e;
-    pair_kernel<true><<<grid, p.tpm * p.slots, p.smem, s>>>(g, Ga, Gb, pairs, npairs, p.tpm, acc);
+    pair_kernel<true><<<grid, p.tpm * p.slots, p.smem, s>>>(g, Ga, Gb, pairs, nlist, npairs, p.tpm, acc);
   } else {
-    pair_kernel<false><<<grid, p.tpm * p.slots, 0, s>>>(g, Ga, Gb, pairs, npairs, p.tpm, acc);
+    pair_kernel<false><<<grid, p.tpm * p.slots, 0, s>>>(g, Ga, Gb, pairs, nlist, npairs, p.tpm, acc);
   }
   return cudaGetLastError();
 }

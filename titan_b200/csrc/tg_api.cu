@@ -2145,17 +2145,12 @@ int imag_pairs(tg_ctx* c, double Ef, double eta, const double* q, const std::vec
       TG_CHECK(c, launch_green(b, c->num_sms, s, nullptr), "green (k - q)");
     }
     KindTimer kt(c, 1);
-    for (int x = 0; x < sets; ++x) {
-      c->launches += 1;
-      TG_CHECK(c, launch_pairs(a, x ? b.out : a.out, x ? a.out : b.out, dp, npairs, c->num_sms,
-                               c->d_acc.p + x * parts * len, s),
-               "pair sums");
-    }
+    c->launches += 1;
+    TG_CHECK(c, launch_pairs(a, a.out, b.out, dp, npairs, c->num_sms, c->d_acc.p, s), "pair sums");
   }
-  for (int x = 0; x < sets; ++x) {
+  {
     KindTimer kt(c, 2);
-    TG_CHECK(c, launch_reduce_blocks(c->d_acc.p + x * parts * len, (int)parts, len, c->d_acc_red.p + (size_t)x * len, s),
-             "reduce");
+    TG_CHECK(c, launch_reduce_blocks(c->d_acc.p, (int)parts, sets * len, c->d_acc_red.p, s), "reduce");
   }
   TG_CHECK(c, cudaMemcpyAsync(h.data(), c->d_acc_red.p, sizeof(double2) * len, cudaMemcpyDeviceToHost, s), "copy");
   if (hs && q)

@@ -195,9 +195,10 @@ __device__ __forceinline__ double point_weight(const GreenArgs& g, int64_t pl) {
 
 // Weighted sums over the column-major Green functions of a pass, added into per-CTA slices of
 // acc: products of the spin blocks of orbital pairs (16 sums each, rows (a up, a down, b up,
-// b down) per pair; pair_partials slices), and single entries (row, column) (entry_partials)
-size_t pair_partials(int n, int npairs, bool two, int num_sms, int64_t np);
-cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* Gb, const int4* pairs, int npairs,
+// b down) per pair; pair_partials slices; with two matrices also the sums with the two
+// exchanged, after the others), and single entries (row, column) (entry_partials)
+size_t pair_partials(int n, int nlist, bool two, int num_sms, int64_t np);
+cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* Gb, const int4* pairs, int nlist,
                          int num_sms, double2* acc, cudaStream_t s);
 int entry_partials(int64_t np, int num_sms);
 cudaError_t launch_entries(const GreenArgs& g, const double2* G, const int2* entries, int ne, int num_sms,
