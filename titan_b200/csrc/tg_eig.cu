@@ -342,6 +342,35 @@ struct HermA {
 constexpr int kEigCols = 3;   // columns per lane of the post-pass row products: n <= 96
 constexpr int kFinThreads = 256;
 
+constexpr int kEigFrags = 9;   // 8-column fragments of a row block in registers: n <= 72
+
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+
+// c += X Y (or X^H Y) for the 8 x 8 fragment at (i0, j0) of two n x n matrices in shared memory
+// (stride S), on the FP64 tensor cores: the lane's columns j0 + 2 t4, j0 + 2 t4 + 1 of row i0 + g8
+template <bool HERM>
+__device__ __forceinline__ void frag_product(const double2* X, const double2* Y, int n, int S, int i0, int j0,
+                                             double2& c0, double2& c1) {
+  const int lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+  const int i = min(i0 + g8, n - 1), j = min(j0 + g8, n - 1);   // clamped: those results are not used
+#pragma unroll 2
+  for (int k0 = 0; k0 < n; k0 += 4) {
+    const int k = k0 + t4;
+    const bool in = k < n;
+    double2 a = in ? (HERM ? X[k * S + i] : X[i * S + k]) : make_double2(0.0, 0.0);
+    const double2 b = in ? Y[k * S + j] : make_double2(0.0, 0.0);
+    if (HERM) a.y = -a.y;
+    dmma(c0.x, c1.x, a.x, b.x);
+    dmma(c0.y, c1.y, a.x, b.y);
+    dmma(c0.x, c1.x, -a.y, b.y);
+    dmma(c0.y, c1.y, a.y, b.x);
+  }
+}
+
 // H: [nk][n][n] row-major; U: in Q (row-major), out the eigenvectors U[r][a]; lam: [nk][n]
 template <bool PACKED>
 __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* __restrict__ H, int64_t nk, int n,
@@ -356,6 +385,7 @@ __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* 
   const int na = HermA<PACKED>::entries(n);
   const int room = (int)HermA<PACKED>::storage(n);   // rotations that the scratch holds
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+  const int g8 = lane >> 2, t4 = lane & 3;
   for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
     const double2* Hk = H + k * (int64_t)n * n;
     double2* Uk = Uio + k * (int64_t)n * n;
@@ -412,31 +442,76 @@ __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* 
     }
     // Post-pass: re-orthonormalised vectors and Rayleigh-quotient eigenvalues.
     //  (1) E = U^H U - 1 (Hermitian)
-    for (int e = tid; e < na; e += blockDim.x) {
-      int i, j;
-      A.ij(e, i, j);
-      double2 acc = make_double2(i == j ? -1.0 : 0.0, 0.0);
-      for (int r = 0; r < n; ++r) acc = cfma(cconj(U[r * S + i]), U[r * S + j], acc);
-      A.a[A.at(i, j)] = acc;
+    if (!PACKED) {
+      const int nf = (n + 7) / 8;
+      for (int f = warp; f < nf * nf; f += nwarps) {
+        const int fi = f / nf, fj = f % nf;
+        if (fj < fi) continue;   // its transpose is written with the upper fragment
+        double2 c0 = make_double2(0.0, 0.0), c1 = c0;
+        frag_product<true>(U, U, n, S, 8 * fi, 8 * fj, c0, c1);
+        const int i = 8 * fi + g8, j = 8 * fj + 2 * t4;
+        if (i < n && j < n) {   // (n is even: j + 1 < n too)
+          if (i == j) c0.x -= 1.0;
+          if (i == j + 1) c1.x -= 1.0;
+          A.a[i * S + j] = c0;
+          A.a[i * S + j + 1] = c1;
+          if (fj > fi) {
+            A.a[j * S + i] = cconj(c0);
+            A.a[(j + 1) * S + i] = cconj(c1);
+          }
+        }
+      }
+    } else {
+      for (int e = tid; e < na; e += blockDim.x) {
+        int i, j;
+        A.ij(e, i, j);
+        double2 acc = make_double2(i == j ? -1.0 : 0.0, 0.0);
+        for (int r = 0; r < n; ++r) acc = cfma(cconj(U[r * S + i]), U[r * S + j], acc);
+        A.a[A.at(i, j)] = acc;
+      }
     }
     __syncthreads();
-    //  (2) one Newton-Schulz step U <- U (1 - E / 2): a warp per row, the row read before written
-    for (int r = warp; r < n; r += nwarps) {
-      double2 x[kEigCols];
+    //  (2) one Newton-Schulz step U <- U (1 - E / 2): a warp per 8 rows (or per row), the rows
+    //  read before they are written
+    if (!PACKED) {
+      const int nf = (n + 7) / 8;
+      for (int fi = warp; fi < nf; fi += nwarps) {
+        double2 c[2 * kEigFrags];
 #pragma unroll
-      for (int m = 0; m < kEigCols; ++m) {
-        x[m] = make_double2(0.0, 0.0);
-        const int j = lane + 32 * m;
-        if (j < n)
-          for (int i = 0; i < n; ++i) x[m] = cfma(U[r * S + i], A.get(i, j), x[m]);
-      }
-      __syncwarp();
+        for (int fj = 0; fj < kEigFrags; ++fj) {
+          c[2 * fj] = c[2 * fj + 1] = make_double2(0.0, 0.0);
+          if (fj < nf) frag_product<false>(U, A.a, n, S, 8 * fi, 8 * fj, c[2 * fj], c[2 * fj + 1]);
+        }
+        __syncwarp();
+        const int i = 8 * fi + g8;
 #pragma unroll
-      for (int m = 0; m < kEigCols; ++m) {
-        const int j = lane + 32 * m;
-        if (j < n) U[r * S + j] = csub(U[r * S + j], cscale(x[m], 0.5));
+        for (int fj = 0; fj < kEigFrags; ++fj) {
+          const int j = 8 * fj + 2 * t4;
+          if (fj < nf && i < n && j < n) {
+            U[i * S + j] = csub(U[i * S + j], cscale(c[2 * fj], 0.5));
+            U[i * S + j + 1] = csub(U[i * S + j + 1], cscale(c[2 * fj + 1], 0.5));
+          }
+        }
+        __syncwarp();
       }
-      __syncwarp();
+    } else {
+      for (int r = warp; r < n; r += nwarps) {
+        double2 x[kEigCols];
+#pragma unroll
+        for (int m = 0; m < kEigCols; ++m) {
+          x[m] = make_double2(0.0, 0.0);
+          const int j = lane + 32 * m;
+          if (j < n)
+            for (int i = 0; i < n; ++i) x[m] = cfma(U[r * S + i], A.get(i, j), x[m]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < kEigCols; ++m) {
+          const int j = lane + 32 * m;
+          if (j < n) U[r * S + j] = csub(U[r * S + j], cscale(x[m], 0.5));
+        }
+        __syncwarp();
+      }
     }
     __syncthreads();
     //  (3) lambda_a = Re u_a^H Hs u_a with Hs = (H + H^H) / 2 from the table
@@ -449,21 +524,24 @@ __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* 
     __syncthreads();
     for (int e = tid; e < n * n; e += blockDim.x) Uk[e] = U[(e / n) * S + e % n];
     if (!PACKED) {
-      // W = Hs U row by row in place (a warp per row), then one thread per eigenvalue
-      for (int r = warp; r < n; r += nwarps) {
-        double2 x[kEigCols];
+      // W = Hs U in place (a warp per 8 rows), then one thread per eigenvalue
+      const int nf = (n + 7) / 8;
+      for (int fi = warp; fi < nf; fi += nwarps) {
+        double2 c[2 * kEigFrags];
 #pragma unroll
-        for (int m = 0; m < kEigCols; ++m) {
-          x[m] = make_double2(0.0, 0.0);
-          const int j = lane + 32 * m;
-          if (j < n)
-            for (int c = 0; c < n; ++c) x[m] = cfma(A.a[r * S + c], U[c * S + j], x[m]);
+        for (int fj = 0; fj < kEigFrags; ++fj) {
+          c[2 * fj] = c[2 * fj + 1] = make_double2(0.0, 0.0);
+          if (fj < nf) frag_product<false>(A.a, U, n, S, 8 * fi, 8 * fj, c[2 * fj], c[2 * fj + 1]);
         }
         __syncwarp();
+        const int i = 8 * fi + g8;
 #pragma unroll
-        for (int m = 0; m < kEigCols; ++m) {
-          const int j = lane + 32 * m;
-          if (j < n) A.a[r * S + j] = x[m];
+        for (int fj = 0; fj < kEigFrags; ++fj) {
+          const int j = 8 * fj + 2 * t4;
+          if (fj < nf && i < n && j < n) {
+            A.a[i * S + j] = c[2 * fj];
+            A.a[i * S + j + 1] = c[2 * fj + 1];
+          }
         }
         __syncwarp();
       }
@@ -506,7 +584,8 @@ size_t fin_smem(int n, bool packed) {
          ((size_t)n * odd_stride(n) + (packed ? HermA<true>::storage(n) : HermA<false>::storage(n)));
 }
 
-bool fin_packed(int n, int optin) { return fin_smem(n, false) > (size_t)optin; }
+// the post-pass with the packed scratch: beyond the fragments of a row block, or the memory
+bool fin_packed(int n, int optin) { return n > 8 * kEigFrags || fin_smem(n, false) > (size_t)optin; }
 
 // warps per matrix: 32 rows each, times the parts of the columns (few where several matrices
 // share an SM)
@@ -527,11 +606,11 @@ int64_t ql_chunk(int n, int64_t nk) {
 
 }  // namespace
 
-// the unpacked post-pass (U and its scratch both whole in shared memory): cheap enough to
-// diagonalise per k even where few energies share a k list
+// U and a scratch matrix both whole in shared memory: cheap enough to diagonalise per k even
+// where few energies share a k list
 int eig_fast(int n) {
   if (n % 2 != 0 || n < 2 || n > 32 * kEigCols) return 0;
-  return !fin_packed(n, optin_smem());
+  return fin_smem(n, false) <= (size_t)optin_smem();
 }
 
 int eig_supported(int n) {
