@@ -407,7 +407,9 @@ __global__ void __launch_bounds__(kTriThreads, 1) tri_green_kernel(GreenArgs a, 
     for (int ck = 0; ck < nch; ++ck) {
       asm volatile("cp.async.wait_group 1;\n" ::);
       __syncthreads();   // operands of chunk ck and the factors of chunk ck + 1 are in place
-      if (ck + 1 < nch) advance(q != nullptr, ck + 1);
+      // the two warps of a sub-partition (w and w + 4) sweep one before and one after their
+      // products, so that its FP64 pipe always has one of them multiplying
+      if (warp < 4 && ck + 1 < nch) advance(q != nullptr, ck + 1);
       if (ck + 3 < nch) fetch(item, q, ck + 3);
       else asm volatile("cp.async.commit_group;\n" ::);
       const double2* A = As + (ck & 1) * kTriK * SA;
@@ -429,6 +431,7 @@ __global__ void __launch_bounds__(kTriThreads, 1) tri_green_kernel(GreenArgs a, 
           }
         }
       }
+      if (warp >= 4 && ck + 1 < nch) advance(q != nullptr, ck + 1);
     }
     // the next item's first chunks travel while this one's results leave
     __syncthreads();
