@@ -1,6 +1,6 @@
 // Eigendecompositions and tridiagonalisations of an H(k) table, one Hermitian matrix per k.
 //
-// Three kernels, each parallel over the k in its own way:
+// Four kernels, each parallel over the k in its own way:
 //   1. hh_small_kernel: H = Q T Q^H, T real symmetric tridiagonal (the Householder reduction of
 //      LAPACK's zhetd2, lower form, with zlarfg's reflectors), one CTA per k with the matrix in
 //      shared memory; Q is accumulated backwards in place.  Also used for the resolvents of
@@ -9,10 +9,10 @@
 //      Martin, Reinsch and Wilkinson, 1968), one thread per k with d and e in shared memory.
 //      The iteration is a serial chain of n^2 plane rotations, so only the number of k hides
 //      it; its rotations go to global memory.
-//   3. eig_finish_kernel: U = Q Z, one CTA per k with Q in shared memory and a thread per real
-//      row (rotations of columns act on every row alone, without any barrier), then one
-//      Newton-Schulz step U <- U (1 - (U^H U - 1) / 2) and Rayleigh quotients of H for the
-//      eigenvalues.
+//   3. eig_apply_kernel: U = Q Z, one CTA per k with Q in shared memory and a thread per real
+//      row (rotations of columns act on every row alone, without any barrier).
+//   4. eig_finish_kernel: one Newton-Schulz step U <- U (1 - (U^H U - 1) / 2) and Rayleigh
+//      quotients of H for the eigenvalues, its products on the FP64 tensor cores.
 // About 20 n^3 flops per matrix against the 10 sweeps of 24 n^3 of a cyclic Jacobi iteration,
 // whose rotations also need a CTA barrier per round.
 #include "tg_internal.cuh"
@@ -342,7 +342,7 @@ struct HermA {
 constexpr int kEigCols = 3;   // columns per lane of the post-pass row products: n <= 96
 constexpr int kFinThreads = 256;
 
-constexpr int kEigFrags = 9;   // 8-column fragments of a row block in registers: n <= 72
+constexpr int kEigFrags = 9;   // largest NF of the post-pass: n <= 72 without packing
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -371,75 +371,93 @@ __device__ __forceinline__ void frag_product(const double2* X, const double2* Y,
   }
 }
 
-// H: [nk][n][n] row-major; U: in Q (row-major), out the eigenvectors U[r][a]; lam: [nk][n]
-template <bool PACKED>
+// U <- Q Z for every k: U holds Q on entry (row-major).  A thread per real row (Re or Im part of a
+// row of Q), which the rotations of columns combine with nothing else; they are staged through
+// shared memory as many whole sweeps at a time as kRotRoom holds.  Bound by shared memory: one
+// 8-byte load and store per row and rotation.
+constexpr int kRotRoom = 512;
+
+__global__ void __launch_bounds__(192) eig_apply_kernel(int64_t nk, int n, const double2* __restrict__ rot, int cap,
+                                                        const int* __restrict__ sweep, int scap,
+                                                        const int* __restrict__ nsweep, double2* __restrict__ Uio) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int S = odd_stride(n);
+  double2* U = reinterpret_cast<double2*>(smem);   // [n][S]
+  double2* stage = U + n * S;                      // [kRotRoom]
+  const int tid = threadIdx.x;
+  for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
+    double2* Uk = Uio + k * (int64_t)n * n;
+#pragma unroll 4
+    for (int e = tid; e < n * n; e += blockDim.x) U[(e / n) * S + e % n] = Uk[e];
+    double* row = reinterpret_cast<double*>(U + (tid >> 1) * S) + (tid & 1);
+    const double2* rk = rot + k * cap;
+    const int* sk = sweep + k * scap;
+    const int nsw = nsweep[k];
+    __syncthreads();
+    for (int w0 = 0; w0 < nsw;) {
+      int w1 = w0, cnt = 0;
+      while (w1 < nsw) {
+        const int lm = sk[w1], len = (lm >> 16) - (lm & 0xffff);
+        if (w1 > w0 && cnt + len > kRotRoom) break;   // (one sweep, n - 1 rotations, always fits)
+        cnt += len;
+        ++w1;
+      }
+      for (int e = tid; e < cnt; e += blockDim.x) stage[e] = rk[e];
+      __syncthreads();
+      if (tid < 2 * n) {
+        const double2* t = stage;
+        for (int w = w0; w < w1; ++w) {
+          const int lm = sk[w], l = lm & 0xffff, m = lm >> 16;
+          double x = row[2 * m];
+          int i = m - 1;
+          for (; i >= l + 3; i -= 4, t += 4) {
+            const double f0 = row[2 * i], f1 = row[2 * i - 2], f2 = row[2 * i - 4], f3 = row[2 * i - 6];
+            const double2 r0 = t[0], r1 = t[1], r2 = t[2], r3 = t[3];
+            row[2 * i + 2] = fma(r0.y, f0, r0.x * x);
+            x = fma(r0.x, f0, -(r0.y * x));
+            row[2 * i] = fma(r1.y, f1, r1.x * x);
+            x = fma(r1.x, f1, -(r1.y * x));
+            row[2 * i - 2] = fma(r2.y, f2, r2.x * x);
+            x = fma(r2.x, f2, -(r2.y * x));
+            row[2 * i - 4] = fma(r3.y, f3, r3.x * x);
+            x = fma(r3.x, f3, -(r3.y * x));
+          }
+          for (; i >= l; --i, ++t) {
+            const double f = row[2 * i];
+            row[2 * i + 2] = fma(t->y, f, t->x * x);
+            x = fma(t->x, f, -(t->y * x));
+          }
+          row[2 * l] = x;
+        }
+      }
+      __syncthreads();
+      rk += cnt;
+      w0 = w1;
+    }
+#pragma unroll 4
+    for (int e = tid; e < n * n; e += blockDim.x) Uk[e] = U[(e / n) * S + e % n];
+    __syncthreads();
+  }
+}
+
+// Post-pass: H: [nk][n][n] row-major; U: in Q Z, out the eigenvectors U[r][a]; lam: [nk][n].
+// NF: 8-column fragments of a row block in registers (n <= 8 NF)
+template <bool PACKED, int NF>
 __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* __restrict__ H, int64_t nk, int n,
-                                                                 const double2* __restrict__ rot, int cap,
-                                                                 const int* __restrict__ sweep, int scap,
-                                                                 const int* __restrict__ nsweep,
                                                                  double2* __restrict__ Uio, double* __restrict__ lam) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int S = odd_stride(n);
   double2* U = reinterpret_cast<double2*>(smem);   // [n][S]
   const HermA<PACKED> A{U + n * S, n, S};
   const int na = HermA<PACKED>::entries(n);
-  const int room = (int)HermA<PACKED>::storage(n);   // rotations that the scratch holds
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
   const int g8 = lane >> 2, t4 = lane & 3;
   for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
     const double2* Hk = H + k * (int64_t)n * n;
     double2* Uk = Uio + k * (int64_t)n * n;
+#pragma unroll 4
     for (int e = tid; e < n * n; e += blockDim.x) U[(e / n) * S + e % n] = Uk[e];
     __syncthreads();
-    // U <- Q Z: real row 2 r + part of thread tid, the rotations in their order, staged through
-    // the scratch of the post-pass as many whole sweeps at a time as it holds
-    {
-      double* row = reinterpret_cast<double*>(U + (tid >> 1) * S) + (tid & 1);
-      const double2* rk = rot + k * cap;
-      const int* sk = sweep + k * scap;
-      const int nsw = nsweep[k];
-      for (int w0 = 0; w0 < nsw;) {
-        int w1 = w0, cnt = 0;
-        while (w1 < nsw) {
-          const int lm = sk[w1], len = (lm >> 16) - (lm & 0xffff);
-          if (w1 > w0 && cnt + len > room) break;   // (one sweep, n - 1 rotations, always fits)
-          cnt += len;
-          ++w1;
-        }
-#pragma unroll 4
-        for (int e = tid; e < cnt; e += blockDim.x) A.a[e] = rk[e];
-        __syncthreads();
-        if (tid < 2 * n) {
-          const double2* t = A.a;
-          for (int w = w0; w < w1; ++w) {
-            const int lm = sk[w], l = lm & 0xffff, m = lm >> 16;
-            double x = row[2 * m];
-            int i = m - 1;
-            for (; i >= l + 3; i -= 4, t += 4) {
-              const double f0 = row[2 * i], f1 = row[2 * i - 2], f2 = row[2 * i - 4], f3 = row[2 * i - 6];
-              const double2 r0 = t[0], r1 = t[1], r2 = t[2], r3 = t[3];
-              row[2 * i + 2] = fma(r0.y, f0, r0.x * x);
-              x = fma(r0.x, f0, -(r0.y * x));
-              row[2 * i] = fma(r1.y, f1, r1.x * x);
-              x = fma(r1.x, f1, -(r1.y * x));
-              row[2 * i - 2] = fma(r2.y, f2, r2.x * x);
-              x = fma(r2.x, f2, -(r2.y * x));
-              row[2 * i - 4] = fma(r3.y, f3, r3.x * x);
-              x = fma(r3.x, f3, -(r3.y * x));
-            }
-            for (; i >= l; --i, ++t) {
-              const double f = row[2 * i];
-              row[2 * i + 2] = fma(t->y, f, t->x * x);
-              x = fma(t->x, f, -(t->y * x));
-            }
-            row[2 * l] = x;
-          }
-        }
-        __syncthreads();
-        rk += cnt;
-        w0 = w1;
-      }
-    }
     // Post-pass: re-orthonormalised vectors and Rayleigh-quotient eigenvalues.
     //  (1) E = U^H U - 1 (Hermitian)
     if (!PACKED) {
@@ -476,16 +494,16 @@ __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* 
     if (!PACKED) {
       const int nf = (n + 7) / 8;
       for (int fi = warp; fi < nf; fi += nwarps) {
-        double2 c[2 * kEigFrags];
+        double2 c[2 * NF];
 #pragma unroll
-        for (int fj = 0; fj < kEigFrags; ++fj) {
+        for (int fj = 0; fj < NF; ++fj) {
           c[2 * fj] = c[2 * fj + 1] = make_double2(0.0, 0.0);
           if (fj < nf) frag_product<false>(U, A.a, n, S, 8 * fi, 8 * fj, c[2 * fj], c[2 * fj + 1]);
         }
         __syncwarp();
         const int i = 8 * fi + g8;
 #pragma unroll
-        for (int fj = 0; fj < kEigFrags; ++fj) {
+        for (int fj = 0; fj < NF; ++fj) {
           const int j = 8 * fj + 2 * t4;
           if (fj < nf && i < n && j < n) {
             U[i * S + j] = csub(U[i * S + j], cscale(c[2 * fj], 0.5));
@@ -527,16 +545,16 @@ __global__ void __launch_bounds__(kFinThreads) eig_finish_kernel(const double2* 
       // W = Hs U in place (a warp per 8 rows), then one thread per eigenvalue
       const int nf = (n + 7) / 8;
       for (int fi = warp; fi < nf; fi += nwarps) {
-        double2 c[2 * kEigFrags];
+        double2 c[2 * NF];
 #pragma unroll
-        for (int fj = 0; fj < kEigFrags; ++fj) {
+        for (int fj = 0; fj < NF; ++fj) {
           c[2 * fj] = c[2 * fj + 1] = make_double2(0.0, 0.0);
           if (fj < nf) frag_product<false>(A.a, U, n, S, 8 * fi, 8 * fj, c[2 * fj], c[2 * fj + 1]);
         }
         __syncwarp();
         const int i = 8 * fi + g8;
 #pragma unroll
-        for (int fj = 0; fj < kEigFrags; ++fj) {
+        for (int fj = 0; fj < NF; ++fj) {
           const int j = 8 * fj + 2 * t4;
           if (fj < nf && i < n && j < n) {
             A.a[i * S + j] = c[2 * fj];
@@ -662,22 +680,33 @@ cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* 
   if (e != cudaSuccess) return e;
   const bool packed = fin_packed(n, optin_smem());
   const size_t fsmem = fin_smem(n, packed);
-  auto fin = packed ? eig_finish_kernel<true> : eig_finish_kernel<false>;
+  auto fin = packed            ? eig_finish_kernel<true, 1>
+             : n <= 24         ? eig_finish_kernel<false, 3>
+             : n <= 40         ? eig_finish_kernel<false, 5>
+             : n <= 56         ? eig_finish_kernel<false, 7>
+                               : eig_finish_kernel<false, kEigFrags>;
   e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fin, kFinThreads, fsmem);
+  const size_t asmem = sizeof(double2) * ((size_t)n * odd_stride(n) + kRotRoom);
+  const int athreads = (2 * n + 31) / 32 * 32;
+  e = cudaFuncSetAttribute(eig_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asmem);
   if (e != cudaSuccess) return e;
-  if (per_sm <= 0) return cudaErrorInvalidValue;
+  int per_sm = 0, aper_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fin, kFinThreads, fsmem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&aper_sm, eig_apply_kernel, athreads, asmem);
+  if (e != cudaSuccess) return e;
+  if (per_sm <= 0 || aper_sm <= 0) return cudaErrorInvalidValue;
   for (int64_t k0 = 0; k0 < nk; k0 += chunk) {
     const int64_t m = std::min(chunk, nk - k0);
     int lanes = 32;
     while (lanes > 2 && (m + lanes - 1) / lanes < 4 * num_sms) lanes /= 2;
     ql_kernel<<<(unsigned)((m + lanes - 1) / lanes), 32, qsmem, s>>>(D, E, k0, m, n, lam, rot, cap, sweep, scap,
                                                                     nsweep, lanes, status);
-    const int64_t grid = std::min<int64_t>(m, (int64_t)num_sms * per_sm);
-    fin<<<(unsigned)grid, kFinThreads, fsmem, s>>>(H + k0 * (int64_t)n * n, m, n, rot, cap, sweep, scap, nsweep,
-                                                   U + k0 * (int64_t)n * n, lam + k0 * n);
+    double2* Uk = U + k0 * (int64_t)n * n;
+    eig_apply_kernel<<<(unsigned)std::min<int64_t>(m, (int64_t)num_sms * aper_sm), athreads, asmem, s>>>(
+        m, n, rot, cap, sweep, scap, nsweep, Uk);
+    fin<<<(unsigned)std::min<int64_t>(m, (int64_t)num_sms * per_sm), kFinThreads, fsmem, s>>>(
+        H + k0 * (int64_t)n * n, m, n, Uk, lam + k0 * n);
   }
   return cudaGetLastError();
 }
