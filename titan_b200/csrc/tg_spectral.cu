@@ -22,7 +22,8 @@ namespace tg {
 
 namespace {
 
-constexpr int kSpecZ = 16;          // energies per task (two m8 fragments)
+constexpr int kSpecZ = 16;          // energies of a tile (two m8 fragments)
+constexpr int kSpecGroups = 4;      // largest number of 16-energy groups of a task
 constexpr int kSpecThreads = 256;
 
 // --------------------------------------------------------------------------- G from (U, lambda)
@@ -40,16 +41,17 @@ struct SpecArgs {
   const double* lam = nullptr;  // [nk][n]
   const int* outinv = nullptr;  // [n*n] pair-block slot of (r, c) = r * n + c
   int kp = 0;                   // K padded to a multiple of 4
+  int nz = kSpecZ;              // energies per task, a multiple of 16
 };
 
 // row stride of U and D in shared memory: 4 mod 8 complex, so that the fragment reads of a
 // quarter warp (two rows, four columns) fall into distinct banks
 __host__ __device__ inline int spec_stride(int kp) { return kp % 8 == 4 ? kp : kp + 4; }
 
-__host__ __device__ inline size_t spec_smem(int n, int kp) {
+__host__ __device__ inline size_t spec_smem(int n, int kp, int nz) {
   const int S = spec_stride(kp);
-  const int tiles = ((n + 1) / 2) * ((n + 7) / 8 + 1);   // more than the tiles of the upper triangle
-  return sizeof(double2) * ((size_t)n * S + (size_t)kSpecZ * S) + sizeof(double) * kSpecZ + sizeof(int) * kSpecZ +
+  const int nb = (n + 3) / 4, tiles = nb * (nb + 1) / 2;
+  return sizeof(double2) * ((size_t)n * S + (size_t)nz * S) + sizeof(double) * nz + sizeof(int) * nz +
          sizeof(int) * (size_t)tiles;
 }
 
@@ -66,30 +68,31 @@ __device__ __forceinline__ void store_pair(double2* p, double2 a, double2 b) {
 
 // G = X + i Y with X = sum_a Re(D_a) P_a and Y = sum_a Im(D_a) P_a, both Hermitian because every
 // P_a = u_a u_a^H is: only the entries r <= c are formed, G(r, c) = X + i Y and
-// G(c, r) = conj(X) + i conj(Y).  One task is a k and 16 energies; a warp takes tiles of two
-// rows (r, r + 1) and eight columns from r on, four real DMMAs per 8 pairs, 8 energies and 4
-// eigenvalues, and writes the four 2 x 2 blocks (32 bytes each) of both triangles.
+// G(c, r) = conj(X) + i conj(Y).  One task is a k and up to 64 energies; a warp takes tiles of
+// 16 energies and 4 x 4 pairs of the upper triangle (90 % of the tiles' pairs are needed at n = 36,
+// 83 % in tiles of 2 x 8), four real DMMAs per 8 pairs, 8 energies and 4 eigenvalues, and a lane
+// writes a 2 x 2 block and its mirror image, four runs of 32 bytes.
 // Im(D) alone (ANTI: w (G - G^+) = w 2 i Y) takes half of them.  Bound by the FP64 tensor pipe
 // up to n = 36 or so by the G output as well (16 n^2 bytes per point).
 template <bool ANTI>
 __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa) {
   extern __shared__ __align__(16) unsigned char smem[];
   const GreenArgs& a = sa.g;
-  const int n = a.n, kp = sa.kp, nn = n * n, S = spec_stride(kp);
+  const int n = a.n, kp = sa.kp, nn = n * n, S = spec_stride(kp), nz = sa.nz;
   double2* Us = reinterpret_cast<double2*>(smem);          // [n][S]
-  double2* Ds = Us + (size_t)n * S;                         // [kSpecZ][S]
-  double* ws = reinterpret_cast<double*>(Ds + (size_t)kSpecZ * S);
-  int* item = reinterpret_cast<int*>(ws + kSpecZ);          // pass-local point of each row, -1 = none
-  int* tiles = item + kSpecZ;                               // r | c0 << 16
+  double2* Ds = Us + (size_t)n * S;                         // [nz][S]
+  double* ws = reinterpret_cast<double*>(Ds + (size_t)nz * S);
+  int* item = reinterpret_cast<int*>(ws + nz);              // pass-local point of each row, -1 = none
+  int* tiles = item + nz;                                   // r | c0 << 16
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarp = blockDim.x >> 5;
   const int g8 = lane >> 2, t4 = lane & 3;
   int ntile = 0;
-  for (int r = 0; r < n; r += 2)
-    for (int c0 = r; c0 < n; c0 += 8, ++ntile)
-      if (ntile % (int)blockDim.x == (int)threadIdx.x) tiles[ntile] = r | c0 << 16;
+  for (int r0 = 0; r0 < n; r0 += 4)
+    for (int c0 = r0; c0 < n; c0 += 4, ++ntile)
+      if (ntile % (int)blockDim.x == (int)threadIdx.x) tiles[ntile] = r0 | c0 << 16;
   const int64_t ne = a.n_e;
-  const int64_t per_k = (ne + kSpecZ - 1) / kSpecZ;
+  const int64_t per_k = (ne + nz - 1) / nz;
   const int64_t ik0 = a.p0 / ne, ik1 = (a.p0 + a.np - 1) / ne;
   const int64_t ntask = (ik1 - ik0 + 1) * per_k;
   // position (p, q) of the output holds G(p, q), or G(q, p) (G^T, and column-major raw G)
@@ -99,9 +102,10 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
   const bool conj = a.mode == MODE_B_REAL;
   for (int64_t t = blockIdx.x; t < ntask; t += gridDim.x) {
     const int64_t ik = ik0 + t / per_k;
-    const int64_t ie0 = (t % per_k) * kSpecZ;
+    const int64_t ie0 = (t % per_k) * nz;
+    const int groups = (int)((min((int64_t)nz, ne - ie0) + kSpecZ - 1) / kSpecZ);
     // rows of this task
-    if (threadIdx.x < kSpecZ) {
+    if (threadIdx.x < nz) {
       const int64_t ie = ie0 + threadIdx.x;
       const int64_t wi = ik * ne + ie;
       const bool kept = a.y_side <= 0 || a.pts.kind != 0 || (ie < ne && a.zi + a.ylist[ie] >= a.y_split);
@@ -110,12 +114,19 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
     const double2* Uk = sa.U + ik * (int64_t)nn;
     for (int e = threadIdx.x; e < n * kp; e += blockDim.x) {
       const int r = e / kp, aa = e % kp;
-      Us[r * S + aa] = aa < n ? Uk[r * n + aa] : make_double2(0.0, 0.0);
+      if (aa < n) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(Us + r * S + aa)),
+                     "l"(Uk + r * n + aa)
+                     : "memory");
+      } else {
+        Us[r * S + aa] = make_double2(0.0, 0.0);
+      }
     }
     __syncthreads();
     // D[z][a] and the weights
     const double* lk = sa.lam + ik * n;
-    for (int e = threadIdx.x; e < kSpecZ * kp; e += blockDim.x) {
+    for (int e = threadIdx.x; e < groups * kSpecZ * kp; e += blockDim.x) {
       const int zr = e / kp, aa = e % kp;
       double2 dv = make_double2(0.0, 0.0);
       if (item[zr] >= 0 && aa < n) {
@@ -142,7 +153,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
       }
       Ds[zr * S + aa] = dv;
     }
-    if (threadIdx.x < kSpecZ) {
+    if (threadIdx.x < nz) {
       double w = 0.0;
       if (item[threadIdx.x] >= 0) {
         const int64_t ie = ie0 + threadIdx.x;
@@ -150,14 +161,32 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
       }
       ws[threadIdx.x] = w;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // U, under way while D was formed
     __syncthreads();
-    for (int tl = warp; tl < ntile; tl += nwarp) {
-      const int r = tiles[tl] & 0xffff, c0 = tiles[tl] >> 16;
-      const double2* u0 = Us + (size_t)r * S + t4;
-      const double2* u1 = r + 1 < n ? u0 + S : u0;
-      const double2* uc = Us + (size_t)min(c0 + g8, n - 1) * S + t4;
-      const double2* dp = Ds + (size_t)g8 * S + t4;
-      double xr[2][2][2], xi[2][2][2], yr[2][2][2], yi[2][2][2];   // [row][energy block][column]
+    for (int tl = warp, z0 = 0;; tl += nwarp) {
+      while (tl >= ntile) {
+        tl -= ntile;
+        z0 += kSpecZ;
+      }
+      if (z0 >= groups * kSpecZ) break;
+      const int r0 = tiles[tl] & 0xffff, c0 = tiles[tl] >> 16;
+      // the lane's block of the output: rows r, r + 1 and columns c, c + 1 (n is even, so they
+      // exist together); the positions of (r + i, c) and (c + i, r), each starting a pair of
+      // adjacent ones, are looked up before the products, which hide the latency
+      const int r = r0 + 2 * (t4 & 1), c = c0 + 2 * (t4 >> 1);
+      const bool mine = r <= c && c < n;   // (below the diagonal of a diagonal tile: a lane above it has the pair)
+      int pu[2] = {0, 0}, pl_[2] = {0, 0};
+      if (mine)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          pu[i] = a.mode == MODE_RAW ? (r + i) * n + c : sa.outinv[(r + i) * n + c];
+          pl_[i] = a.mode == MODE_RAW ? (c + i) * n + r : sa.outinv[(c + i) * n + r];
+        }
+      // column j of a product's B fragment: row r0 + j % 4 and column c0 + 2 (j / 4) + f
+      const double2* ur = Us + (size_t)min(r0 + (g8 & 3), n - 1) * S + t4;
+      const double2* uc = Us + (size_t)min(c0 + 2 * (g8 >> 2), n - 2) * S + t4;
+      const double2* dp = Ds + (size_t)(z0 + g8) * S + t4;
+      double xr[2][2][2], xi[2][2][2], yr[2][2][2], yi[2][2][2];   // [column f][energy block][row h]
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -165,8 +194,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
 #pragma unroll
           for (int h = 0; h < 2; ++h) xr[i][m][h] = xi[i][m][h] = yr[i][m][h] = yi[i][m][h] = 0.0;
       for (int k0 = 0; k0 < kp; k0 += 4) {
-        const double2 cc = cconj(uc[k0]);
-        const double2 pv[2] = {cmul(u0[k0], cc), cmul(u1[k0], cc)};
+        const double2 uv = ur[k0];
+        const double2 pv[2] = {cmul(uv, cconj(uc[k0])), cmul(uv, cconj(uc[S + k0]))};
         const double2 dv[2] = {dp[k0], dp[8 * S + k0]};
 #pragma unroll
         for (int m = 0; m < 2; ++m)
@@ -178,18 +207,10 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
             dmma(yi[i][m][0], yi[i][m][1], dv[m].y, pv[i].y);
           }
       }
-      // the lane's columns c, c + 1 (n is even, so they exist together) against rows r, r + 1
-      const int c = c0 + 2 * t4;
-      if (c >= n) continue;
-      int pu[2], pl_[2];   // positions (r + i, c) and (c + i, r): each starts a pair of adjacent ones
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        pu[i] = a.mode == MODE_RAW ? (r + i) * n + c : sa.outinv[(r + i) * n + c];
-        pl_[i] = a.mode == MODE_RAW ? (c + i) * n + r : sa.outinv[(c + i) * n + r];
-      }
+      if (!mine) continue;
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const int zr = m * 8 + g8;
+        const int zr = z0 + m * 8 + g8;
         const int pt = item[zr];
         if (pt < 0) continue;
         const double w = ws[zr];
@@ -198,8 +219,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_green_kernel(SpecArgs sa
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            up[i][h] = make_double2(xr[i][m][h] - yi[i][m][h], xi[i][m][h] + yr[i][m][h]);
-            lo[h][i] = make_double2(xr[i][m][h] + yi[i][m][h], yr[i][m][h] - xi[i][m][h]);
+            up[h][i] = make_double2(xr[i][m][h] - yi[i][m][h], xi[i][m][h] + yr[i][m][h]);
+            lo[i][h] = make_double2(xr[i][m][h] + yi[i][m][h], yr[i][m][h] - xi[i][m][h]);
           }
         auto put = [&](double2* out, int16_t* eout, int pos, double2 v0, double2 v1, bool sc) {
           if (sc) {
@@ -408,16 +429,30 @@ cudaError_t launch_green_spectral(const GreenArgs& g, const double2* U, const do
   sa.lam = lam;
   sa.outinv = outinv;
   sa.kp = (g.n + 3) / 4 * 4;
-  const size_t smem = spec_smem(g.n, sa.kp);
   auto kernel = g.mode == MODE_A_REAL ? spec_green_kernel<true> : spec_green_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int dev = 0, optin = 0, smax = 0, per_sm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSpecThreads, smem);
+  // energies of a task: the more, the fewer loads of U and barriers, as long as two blocks share
+  // an SM (one where two could not do with 16 either) and every block has a few tasks
+  const int64_t ne = g.n_e;
+  const int64_t nks = (g.p0 + g.np - 1) / ne - g.p0 / ne + 1;
+  auto tasks = [&](int nz) { return nks * ((ne + nz - 1) / nz); };
+  auto blocks = [&](int nz) { return std::min<int64_t>(2, smax / ((int64_t)spec_smem(g.n, sa.kp, nz) + 1024)); };
+  for (int nz = kSpecZ * kSpecGroups; nz > kSpecZ; nz /= 2)
+    if (spec_smem(g.n, sa.kp, nz) <= (size_t)optin && blocks(nz) == blocks(kSpecZ) &&
+        nz - kSpecZ < ne && tasks(nz) >= 4 * blocks(nz) * num_sms) {
+      sa.nz = nz;
+      break;
+    }
+  const size_t smem = spec_smem(g.n, sa.kp, sa.nz);
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSpecThreads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm <= 0) return cudaErrorInvalidValue;
-  const int64_t ne = g.n_e;
-  const int64_t ntask = ((g.p0 + g.np - 1) / ne - g.p0 / ne + 1) * ((ne + kSpecZ - 1) / kSpecZ);
+  const int64_t ntask = tasks(sa.nz);
   const int64_t grid = std::min<int64_t>(ntask, (int64_t)num_sms * per_sm);
   kernel<<<(unsigned)grid, kSpecThreads, smem, s>>>(sa);
   return cudaGetLastError();
