@@ -103,3 +103,20 @@ def test_dyson_reports_a_singular_system(gpu):
     with pytest.raises(TitanGPUError) as err:
         gpu.dyson(x, 0.5 * u - 0.5 * np.diag(np.arange(70) == 66))
     assert err.value.code == 67
+
+
+@pytest.mark.parametrize("shape,nk,n_neighbour_stages", [("bcc1", (2, 3, 2), 2), ("sq2", (3, 2, 1), 1), ("slab3", (2, 2, 1), 2)])
+def test_disturbance_fragments(gpu, shape, nk, n_neighbour_stages):
+    """The vertex products in 8 x 8 fragments: one site (25 fragments for eight warps, a last column
+    block of two orbitals), two sites (50), and three (75, more than the warps hold: the staged
+    kernel).  Both axes, one after the other into the same sums, q and frequency nonzero; within
+    1e-10 of the oracle, the bound of the plain test."""
+    deck = synthetic.make_deck(shape, nk=nk, n1gl=5, parts=1, n3gl=3)
+    s = deck.system
+    h0 = s.h0(initial_state(s))
+    gpu.setup(deck, h0)
+    e, q, ue = 0.04, np.array([0.1, 0.05, 0.0]), np.array([0.6, 0.0, 0.8])
+    x2, p2 = deck.real_points(e, s.Ef)
+    ref = O.eintshe(O.Model(s, h0), deck.ek, (deck.real_kp, deck.real_w), q, e, s.Ef, s.eta, s.etap, x2, p2, ue)
+    got = gpu.she(q, e, s.Ef, s.eta, s.etap, x2, p2, ue)
+    assert np.max(np.abs(got - ref)) <= 1e-10 * np.max(np.abs(ref)), shape

@@ -2880,9 +2880,9 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
   cudaStream_t s = c->stream;
   const int n = c->dimH, no = n / 2, D = c->dimens;
   const int64_t nn = (int64_t)n * n;
-  int n_tiles = 0;
-  for (int i = 0; i < c->n_atoms; ++i) n_tiles += 16 * ((c->norb[i] + 2) / 3) * ((c->norb[i] + 2) / 3);
-  const int grid = she_grid(n, D, c->n_neigh, n_tiles, c->num_sms);
+  int n_frags = 0;
+  for (int i = 0; i < c->n_atoms; ++i) n_frags += ((c->norb[i] + 1) / 2) * ((c->norb[i] + 1) / 2);
+  const int grid = she_grid(n, D, c->n_neigh, n_frags, c->num_sms);
   if (grid <= 0) return set_err(c, TG_ERR_ARG, "tg_she: dimH / dimens too large for the shared-memory vertex kernel");
   // orbital tables of the kernel
   std::vector<int> tab((size_t)4 * no);
@@ -2987,6 +2987,7 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
   l.rowoff = c->d_she_rowoff.p;
   for (int i = 0; i < 3; ++i) l.ue[i] = efield[i];
   she_spin_codes(l.spins);
+  l.n_frags = n_frags;
   l.partial = c->d_she_part.p;
   l.grid = grid;
   // one pass: G2 = G(k, E), G1 = G(k + q, E + e), both column-major per point, then the

@@ -136,7 +136,7 @@ struct GreenArgs {
   const double2* eigU = nullptr;
   const double* eigL = nullptr;
   // optional Householder tridiagonalisation of every k of the k-major traversal (dimensions
-  // beyond the Jacobi kernel): T's diagonal triD[k][n] and off-diagonal triE[k][n], the rows
+  // where G from eigenvectors is not used): T's diagonal triD[k][n] and off-diagonal triE[k][n], the rows
   // trirows[tri_ns] of Q as triQ[k][s][c]; the output is G over those rows and columns
   const double* triD = nullptr;
   const double* triE = nullptr;
@@ -289,6 +289,7 @@ struct SheLaunch {
   // sigma | s' << 2 | site << 4 | x0 << 14 | y0 << 20, and the first df row of each site
   const int* ztiles = nullptr;
   int n_ztiles = 0;
+  int n_frags = 0;                // sum_i ceil(n_i / 2)^2: 8 x 8 fragments of the sites' entries
   const int* rowoff = nullptr;
   double ue[3] = {0, 0, 0};
   unsigned char spins[3][16] = {};
@@ -299,10 +300,8 @@ struct SheLaunch {
   int64_t n_e = 0, nk_tab = 0;
   const double* klist = nullptr;
 };
-// (n_ztiles: second-stage tiles of the system, 16 sum_i ceil(n_i / 3)^2)
-size_t she_smem_bytes(int n, int dimens, int n_neigh, int n_ztiles);
 // CTAs of one vertex launch (SMs x resident CTAs); 0 when the shared memory does not fit
-int she_grid(int n, int dimens, int n_neigh, int n_ztiles, int num_sms);
+int she_grid(int n, int dimens, int n_neigh, int n_frags, int num_sms);
 cudaError_t launch_she(const SheLaunch& l, cudaStream_t s);
 cudaError_t launch_she_prefactor(const double2* P, const double2* df, int dimens, double scale, double2* out,
                                  cudaStream_t s);
