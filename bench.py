@@ -396,14 +396,14 @@ def run_ours(args, rank, world, local_rank):
     roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": (achieved / peak) if achieved else None, "traffic": traffic,
             "kernel": "chi0 contraction (" + ("tcgen05 int8-sliced split_contract_kernel" if args.precision == "split"
-                                              else "fp64 SIMT gemm64_kernel") + ")",
+                                              else "fp64 DMMA gemm64_kernel") + ")",
             "peak_source": ("of measured bf16 dense sustained (MEASURED_PEAKS.json)" if pk_kind == "measured"
                             else "of fallback 1.4 PF sustained"),
             "flops_per_unit": 8.0 * D ** 2,
             "launches_in_last_step": int(con_n), "avg_launch_ms": (con_ms / con_n) if con_n else None,
             "quantize_ms_last_step": q_ms if args.precision == "split" else None}
     if args.precision == "split" and con_n:
-        # what the tensor pipe executes: 21 int8 MMAs of 128 x 80 x 32 per 64 x 40 complex tile
+        # what the tensor pipe executes: 21 int8 products of 128 x 80 x 32 per 64 x 40 complex tile
         # and K-step of 32 points (tiles: ceil(M/64) x ceil(M/40) per site pair, M = 4 n_i n_j)
         nc = s.norbs if sel is None else [len(x) for x in sel]
         tiles = sum(-(-4 * a * b // 64) * -(-4 * a * b // 40) for a in nc for b in nc)
@@ -421,8 +421,8 @@ def run_ours(args, rank, world, local_rank):
     dfma, dmma = fp64_peak()
     native_n = s.dimH in (4, 8, 16, 18, 20, 36, 40, 54, 72, 90)
     tabulated = len(set(np.bincount(deck.ek.energy_index).tolist())) == 1   # every energy on the same k list
-    # chi0's Green functions on meshes whose energies share a k list: spectral from the unpacked
-    # Jacobi kernel (even dimH <= 72), else under AUTO from a Householder tridiagonalisation per k
+    # chi0's Green functions on meshes whose energies share a k list: spectral from one
+    # eigendecomposition per k (even dimH <= 72), else under AUTO from a Householder tridiagonalisation per k
     # (G over the rows chi needs: 8 |S|^2 n flops per point, a DMMA GEMM); adaptive imaginary axes
     # (shared G2 across q) keep Gauss-Jordan there and use these on the real axis only
     eig_fast = args.green != "gauss-jordan" and s.dimH % 2 == 0 and s.dimH <= 72
@@ -436,12 +436,13 @@ def run_ours(args, rank, world, local_rank):
     n_inv = inversions_of(deck, per, reals, start + args.warmup * per + (args.steps - 1) * per, nq, shared,
                           spectral_real and shared)
     ns = sum(2 * len(o) for o in sel) if sel is not None else s.dimH
-    tri_name = ("hh_tridiag_kernel + tri_green_kernel (Householder tridiagonalisation per k, G over the %d rows "
+    tri_name = (("hh_small_kernel" if s.dimH <= 96 else "hh_panel_kernel") + " + tri_green_kernel (Householder tridiagonalisation per k, G over the %d rows "
                 "of chi per point: tridiagonal solves + FP64 DMMA GEMM) + gather_kernel" % ns)
-    gj_name = ("green_w1_kernel / green_team_kernel (fused H(k) + Gauss-Jordan)" if native_n else
+    gj_name = (("green_team_kernel" if s.dimH in (4, 8, 16, 20) else "green_mma_kernel") +
+               " (fused H(k) + Gauss-Jordan)" if native_n else
                "green_cluster_kernel (thread-block-cluster Gauss-Jordan) + gather_kernel")
-    kname = ("eig_jacobi_kernel + spec_green_kernel (spectral G, FP64 DMMA)" if spectral else
-             gj_name + " on the imaginary axis; eig_jacobi_kernel + spec_green_kernel (spectral) on the real axis"
+    kname = ("hh_small / ql / eig_apply / eig_finish + spec_green_kernel (spectral G, FP64 DMMA)" if spectral else
+             gj_name + " on the imaginary axis; eigensolver + spec_green_kernel (spectral) on the real axis"
              if spectral_real else
              tri_name if tri_all else
              gj_name + " on the imaginary axis; " + tri_name + " on the real axis" if tri_real else gj_name)
@@ -477,7 +478,7 @@ def run_ours(args, rank, world, local_rank):
                                       step0=args.warmup + args.steps - 1)
         line["fp64_path"] = {"value": u64 / (sum(ms64) / 1e3), "unit": UNIT, "ms_per_step": sum(ms64),
                              "step": "one chi0 call over the frequencies and wave vectors of the last timed step, "
-                                     "TG_PREC_FP64 (FP64 SIMT contraction), same Green functions"}
+                                     "TG_PREC_FP64 (FP64 contraction), same Green functions"}
         line["split_over_fp64"] = (value / world) / line["fp64_path"]["value"]
     if args.precision == "split" and not args.no_check:
         line["split_rel_err"] = split_accuracy(gpu, deck, omegas, reals, per)

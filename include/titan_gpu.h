@@ -33,7 +33,7 @@ extern "C" {
 #define TG_ERR_NUMERIC  (-6)   /* an iterative device solver did not converge */
 
 /* Precision of the chi0 contraction (tg_chi0). */
-#define TG_PREC_FP64     0     /* FP64 SIMT contraction */
+#define TG_PREC_FP64     0     /* FP64 contraction (FP64 tensor cores) */
 #define TG_PREC_SPLIT    1     /* INT8-sliced tensor-core contraction (tcgen05), FP64 recombination */
 
 typedef struct tg_ctx tg_ctx;
@@ -299,7 +299,7 @@ int tg_ldos(tg_ctx* ctx, int n_e, const double* e, double eta, double* ldosu, do
 
 /* How G(k, z) is computed.  Spectral: on meshes where every energy uses the same
  * k list (uniform imaginary axis, the real-axis BZ) H(k) is diagonalised once per k
- * (Jacobi, FP64) and G(k, z) = U diag(1/(z - lambda)) U^+ is formed for all energies
+ * (Householder and implicit QL, FP64) and G(k, z) = U diag(1/(z - lambda)) U^+ is formed for all energies
  * with FP64 tensor-core GEMMs.  Gauss-Jordan: one inversion per (k, z), the
  * reference's invers (mod_tools.F90:796-829).  Near the real axis the spectral G
  * carries errors up to eps |H| / Im z relative (1e-13 at Im z = 1e-3): the mixing of
@@ -326,10 +326,10 @@ int tg_ldos(tg_ctx* ctx, int n_e, const double* e, double eta, double* ldosu, do
 #define TG_GREEN_SPECTRAL      2
 int tg_set_green_method(tg_ctx* ctx, int method);
 
-/* Test hook: eigenvalues lam(dimH, nk) and eigenvectors of h0 + H(k) from the Jacobi
- * kernel behind TG_GREEN_AUTO, U(dimH, dimH, nk) with U(a, :, k) = eigenvector a (the
- * device's row-major [k][r][a] layout); TG_ERR_NUMERIC if a matrix did not converge in
- * 30 sweeps. */
+/* Test hook: eigenvalues lam(dimH, nk) and eigenvectors of h0 + H(k) from the eigensolver
+ * behind TG_GREEN_AUTO, U(dimH, dimH, nk) with U(a, :, k) = eigenvector a (the
+ * device's row-major [k][r][a] layout); TG_ERR_NUMERIC if an eigenvalue did not converge in
+ * 60 QL iterations. */
 int tg_eig_batch(tg_ctx* ctx, int64_t nk, const double* kp, double* lam, double* U);
 
 /* Test hooks.  G(dimH, dimH, nz) = (z - h0 - H(k))^-1 for nz (k, z) pairs,

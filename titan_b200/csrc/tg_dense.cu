@@ -12,7 +12,9 @@
 //
 // What bounds it: at dimension 1600 the GEMMs (8 n^3 for chi_hf U, 8/3 n^3 for the LU, 8 n^3
 // for the solve) take most of the time, the panels (one SM at a time, about a microsecond a
-// column) the rest; small matrices are bound by the panels.
+// column) the rest; small matrices are bound by the panels.  Dimension 1600, one call with its
+// host copies: 54 ms with panels of 8 and these GEMMs, 18.6 ms with row-major operands transposed
+// on the device and staged copies as well (157 ms with column by column elimination).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -14,7 +14,9 @@
 //   4. eig_finish_kernel: one Newton-Schulz step U <- U (1 - (U^H U - 1) / 2) and Rayleigh
 //      quotients of H for the eigenvalues, its products on the FP64 tensor cores.
 // About 20 n^3 flops per matrix against the 10 sweeps of 24 n^3 of a cyclic Jacobi iteration,
-// whose rotations also need a CTA barrier per round.
+// whose rotations also need a CTA barrier per round.  Measured: 9801 matrices of dimension 36 in
+// 24 ms with Jacobi rotations, 3.7 ms now (1.5, 0.5, 1.1 and 0.6 ms for the four kernels); 1331 of
+// dimension 72 in 45 ms and 5.4 ms, of which the serial chains of ql_kernel take 1.7 ms.
 #include "tg_internal.cuh"
 
 #include <algorithm>
@@ -606,7 +608,7 @@ size_t fin_smem(int n, bool packed) {
 bool fin_packed(int n, int optin) { return n > 8 * kEigFrags || fin_smem(n, false) > (size_t)optin; }
 
 // warps per matrix: 32 rows each, times the parts of the columns (few where several matrices
-// share an SM)
+// share an SM, as many as there are registers for where one fills it)
 int hh_warps(int n) { return n <= 32 ? 2 : n <= 40 ? 4 : n <= 64 ? 6 : n <= 76 ? 9 : 15; }
 
 size_t hh_smem(int n) {
@@ -624,8 +626,10 @@ int64_t ql_chunk(int n, int64_t nk) {
 
 }  // namespace
 
-// U and a scratch matrix both whole in shared memory: cheap enough to diagonalise per k even
-// where few energies share a k list
+// U and a scratch matrix both whole in shared memory (dimensions up to 72 or so): there G from
+// (U, lambda) costs 8 n^3 flops per point like the tridiagonal resolvents, without their sweeps;
+// beyond, the packed post-pass runs one matrix per SM and the tridiagonalisation alone is
+// cheaper per k
 int eig_fast(int n) {
   if (n % 2 != 0 || n < 2 || n > 32 * kEigCols) return 0;
   return fin_smem(n, false) <= (size_t)optin_smem();

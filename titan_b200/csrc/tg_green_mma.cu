@@ -19,6 +19,12 @@
 // writes the operand layouts (w G, G^T, w (G - G^+), conj G), raw G, H(k) or the
 // expectation sums.
 //
+// What bounds it: shared memory (the A fragments of the updates; L1 at 59 to 69 % of its rate, the
+// FP64 tensor pipe at 44 to 49 %) and, at the small dimensions, warp 0's chain of four pivots per
+// panel (about 3500 cycles).  Cycles per matrix and SM on one B200, before (Gauss-Jordan steps of
+// rank one, matrix in registers) and now: dimension 18: 4400 and 2500, 36: 17500 and 10400, 54:
+// 73600 and 29000, 72: 180000 and 62000, 90: 357000 and 118000.  Panels of 8 were slower (36:
+// 19800, 72: 81500, 90: 212000): the factorisation grows faster than the updates shrink.
 #include "tg_internal.cuh"
 
 #include <algorithm>
@@ -508,6 +514,9 @@ cudaError_t launch_green_mma(const GreenArgs& a, int num_sms, cudaStream_t s, in
     if (grid_used) *grid_used = 0;
     return cudaSuccess;
   }
+  // warps per matrix, resident CTAs: enough matrices per SM to hide the factoring warp where the
+  // matrix is small, enough warps to update beside it where few matrices fit.  Neighbouring
+  // choices measured slower (36: 1, 3 and 4 warps; 54: 3, 5 and 7; 72: 5 to 9; 90: 7 to 13).
   switch (a.n) {
     case 18: return launch_n<18, 1, 15>(a, num_sms, s, grid_used);
     case 36: return launch_n<36, 2, 8>(a, num_sms, s, grid_used);

@@ -473,10 +473,14 @@ __global__ void __launch_bounds__(kSheMmaThreads, 2) she_mma_kernel(SheArgs a, S
       acc[j][h] = v.x;
       acc[j][2 + h] = v.y;
     }
-  for (int64_t pl = blockIdx.x; pl < a.np; pl += gridDim.x) {
+  // a run of points per CTA: in k-major order most have the k of the one before, and its V
+  double vx = 0.0, vy = 0.0, vz = 0.0;
+  bool have = false;
+  const int64_t end = a.np * (blockIdx.x + 1) / gridDim.x;
+  for (int64_t pl = a.np * blockIdx.x / gridDim.x; pl < end; ++pl) {
     double kx, ky, kz, w;
     she_point(a, a.p0 + pl, kx, ky, kz, w);
-    she_phases(a, kx, ky, kz, ph);
+    const bool fresh = !have || kx != vx || ky != vy || kz != vz;
     const double2* g1 = a.G1 + pl * (int64_t)n * n;
     const double2* g2 = a.G2 + pl * (int64_t)n * n;
     // Green functions of the point, spin-major; real axis: S1 = G1 - G1^+, S2 = G2^+
@@ -496,10 +500,17 @@ __global__ void __launch_bounds__(kSheMmaThreads, 2) she_mma_kernel(SheArgs a, S
         S2[perm[c] * L.sg + perm[r]] = make_double2(y.x, -y.y);
       }
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < no * no; e += blockDim.x) {
-      const int rr = e / no, cc = e - rr * no;
-      M[rr * L.sm + cc] = she_vertex(a, ph, site[rr], site[cc], orb[rr], orb[cc]);
+    if (fresh) {
+      she_phases(a, kx, ky, kz, ph);
+      __syncthreads();
+      for (int e = threadIdx.x; e < no * no; e += blockDim.x) {
+        const int rr = e / no, cc = e - rr * no;
+        M[rr * L.sm + cc] = she_vertex(a, ph, site[rr], site[cc], orb[rr], orb[cc]);
+      }
+      have = true;
+      vx = kx;
+      vy = ky;
+      vz = kz;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();

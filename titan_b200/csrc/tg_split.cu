@@ -5,12 +5,18 @@
 // element, the largest |Re|, |Im|), split_quantize_kernel (FP64 operand ->
 // six int8 digit planes, K-step blocks) and split_contract_kernel (warp-
 // specialised: one producer warp stages digit blocks with bulk copies into a
-// five-stage shared-memory ring, one warp issues the 21 MMAs per K-step, eight
-// warps drain the six int32 level accumulators from TMEM at every chunk end
-// into FP64 sums held in registers until the unit ends).
+// five-stage shared-memory ring, one warp issues the 21 digit products of a
+// K-step as nine MMAs, eight warps drain the six int32 level accumulators from
+// TMEM at every chunk end into FP64 sums held in registers until the unit ends).
 // Every wait on an mbarrier is bounded (2 s of %globaltimer); on a timeout the
 // kernel records an error code, waits (bounded) for its own copies and MMAs in
 // flight, frees its TMEM and returns.
+//
+// What bounds the contraction: the shared-memory reads of the MMA operands.  A
+// product of one digit pair reads 128 rows of A for 80 of B, one MMA of a digit of
+// A with three neighbouring digits of B reads them for 240: 1874 cycles per K-step
+// with 21 MMAs, 1053 with nine (970 without the draining warps, 840 at the nominal
+// int8 rate).  The quantisation is bound by HBM (90 % of the measured copy rate).
 #include "tg_internal.cuh"
 #include "tg_split.cuh"
 

@@ -20,8 +20,9 @@
 //                    64..127 Im of 64 complex rows u of one site pair
 //   B block (t, gB): [k half 2][slice 6][row 80][16 B], rows 0..39 Re and
 //                    40..79 Im of 40 complex columns v of one site pair
-// An M=128 x K=32 MMA of digit i of A against N=80 rows per digit of B gives, for the
-// 64 x 40 complex tile, the four real products Ar Br, Ar Bi, Ai Br, Ai Bi at once.
+// An M=128 x K=32 MMA of digit i of A against N=80 rows per digit of B (one, two or
+// three neighbouring digits) gives, for the 64 x 40 complex tile, the four real products
+// Ar Br, Ar Bi, Ai Br, Ai Bi of each at once.
 #pragma once
 
 #include <cuda_runtime.h>

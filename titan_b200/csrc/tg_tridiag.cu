@@ -47,7 +47,9 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
 // read (once per reflector, A v), with the panel's own changes V W^H + W V^H applied to the
 // vectors; it is rewritten once per panel, by FP64 tensor-core products of depth 8, and the
 // rows of Q pass through registers once per panel.  Bound by the reads of A v from L2 / HBM
-// (16 n^3 / 3 bytes per matrix, two rows and all their loads in flight per warp).
+// (16 n^3 / 3 bytes per matrix, two rows and all their loads in flight per warp) and by shared
+// memory (71 % of its rate).  196 matrices of dimension 288: 55 ms with a row pass per
+// reflector, 13.5 ms now.
 constexpr int kPanThreads = 512;
 constexpr int kPanNb = 8;              // reflectors per panel
 constexpr int kPanS = kPanNb + 4;      // row stride of V and W: 4 mod 8, fragment reads apart
@@ -299,7 +301,9 @@ __global__ void __launch_bounds__(64) tri_lu_kernel(GreenArgs a, double2* __rest
 // (tile 32 FM x 16 FN).  Per chunk of 8 steps i every sweeping thread fetches its 8 entries of
 // Q_S two chunks ahead (cp.async, its own 128 bytes, so no barrier), advances its state and
 // leaves w_i / d_i or v_i in the double-buffered operand tiles; one barrier per chunk.  The
-// DMMAs bound it: 4 FM FN per warp and 4 steps against FM + FN shared-memory reads.
+// DMMAs bound it: 4 FM FN per warp and 4 steps against FM + FN shared-memory reads.  At 288 with
+// 160 rows: 74 ms when a thread swept a whole column before the products, 58 ms now (75 % of the
+// FP64 tensor pipe); 62 ms with all warps sweeping at the same time.
 constexpr int kTriK = 8, kTriStages = 3;
 
 template <int FM, int FN>
@@ -513,7 +517,9 @@ cudaError_t launch_green_tri(const GreenArgs& g, int num_sms, cudaStream_t s) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // the tile shape whose tiles cover the fewest entries of G beyond ns x ns (the DMMAs of the
-  // padding cost as much as the others); larger ones first, for their operand reuse
+  // padding cost as much as the others); larger ones first, for their operand reuse and because
+  // every tile of a point sweeps its own rows and columns again (160 rows: 160 x 80 twice, 90 rows:
+  // 96 x 96 once)
   struct Shape {
     int m, n;
   };
