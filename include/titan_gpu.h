@@ -152,7 +152,7 @@ int tg_expectation(tg_ctx* ctx, double Ef, double eta, double* rho, double* mx, 
  * default method; this call always inverts per (k, z) point (Gauss-Jordan),
  * whatever tg_set_green_method chose.  H(k) is summed inside the kernel and the
  * partial sums live in a fixed 8 MiB device array of the library:
- * (16 x SMs + 1) x 2 dimH complex must fit (dimH <= 90 on a B200), else
+ * (16 x SMs + 1) x 2 dimH complex (25 x SMs up to dimH 18) must fit (dimH <= 90 on a B200), else
  * TG_ERR_ARG before any work.  The first call on a context looks the array's
  * address up on the context's device (make it before any stream capture);
  * nothing has to start at zero; calls that overlap in time on one device race

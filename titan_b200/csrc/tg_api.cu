@@ -2195,7 +2195,7 @@ int tg_expectation(tg_ctx* c, double Ef, double eta, double* rho, double* mx, do
     a.nk_tab = c->nk_u;
     a.ylist = c->d_ylist.p;
   }
-  const int maxgrid = c->num_sms * (kGreenMaxCtas + 1);
+  const int maxgrid = c->num_sms * (green_max_ctas(n) + 1);
   TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * len), "alloc acc");
   TG_CHECK(c, c->d_acc_red.ensure(len), "alloc acc");
   a.acc = c->d_acc.p;
@@ -3118,7 +3118,7 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
 // sums in a fixed 8 MiB device array compiled into the library and sums H(k)
 // inside the inversion kernel instead of tabulating it.
 //
-// * Size limit: (16 x SMs + 1) x 2 dimH complex doubles must fit in 8 MiB
+// * Size limit: (16 x SMs + 1) x 2 dimH complex doubles (25 x SMs up to dimH 18) must fit in 8 MiB
 //   (dimH <= 90 on a 148-SM B200 needs 6.8 MB); larger requests, and dimensions
 //   that only the general-dimension kernel handles, return TG_ERR_ARG before
 //   any work.
@@ -3166,8 +3166,9 @@ extern "C" int tg_expectation_noalloc(tg_ctx* c, double Ef, double eta, double* 
   if (!rho || !mx || !my || !mz || !mp) return set_err(c, TG_ERR_ARG, "tg_expectation_noalloc: null output");
   const int n = c->dimH;
   const int len = 2 * n;
-  // partial slots: the team kernel runs at most 15 teams per SM (per-SM CTAs x teams <= 8 + teams - 1)
-  const size_t slots = (size_t)c->num_sms * 16;
+  // partial slots: the team kernel runs at most 15 teams per SM (per-SM CTAs x teams <= 8 + teams - 1),
+  // the blocked one green_max_ctas
+  const size_t slots = (size_t)c->num_sms * (green_max_ctas(n) + 1);
   const size_t need = (slots + 1) * (size_t)len * sizeof(double2);
   if (!green_supported(n))
     return set_err(c, TG_ERR_ARG, "tg_expectation_noalloc: this dimension needs the general-dimension kernel, "

@@ -22,7 +22,7 @@
 // What bounds it: shared memory (the A fragments of the updates; L1 at 59 to 69 % of its rate, the
 // FP64 tensor pipe at 44 to 49 %) and, at the small dimensions, warp 0's chain of four pivots per
 // panel (about 3500 cycles).  Cycles per matrix and SM on one B200, before (Gauss-Jordan steps of
-// rank one, matrix in registers) and now: dimension 18: 4400 and 2500, 36: 17500 and 10400, 54:
+// rank one, matrix in registers) and now: dimension 18: 4400 and 2300, 36: 17500 and 10400, 54:
 // 73600 and 29000, 72: 180000 and 62000, 90: 357000 and 118000.  Panels of 8 were slower (36:
 // 19800, 72: 81500, 90: 212000): the factorisation grows faster than the updates shrink.
 #include "tg_internal.cuh"
@@ -486,7 +486,7 @@ cudaError_t launch_o(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * W, smem);
   if (err != cudaSuccess) return err;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  per_sm = std::min(per_sm, kGreenMaxCtas);   // per-CTA partial sums of MODE_EXPECT are sized for these
+  per_sm = std::min(per_sm, green_max_ctas(N));   // per-CTA partial sums of MODE_EXPECT are sized for these
   int64_t grid = std::min<int64_t>((int64_t)num_sms * per_sm, a.np);
   if (grid_used) *grid_used = (int)grid;
   kern<<<(unsigned)grid, 32 * W, smem, s>>>(a);
@@ -517,8 +517,10 @@ cudaError_t launch_green_mma(const GreenArgs& a, int num_sms, cudaStream_t s, in
   // warps per matrix, resident CTAs: enough matrices per SM to hide the factoring warp where the
   // matrix is small, enough warps to update beside it where few matrices fit.  Neighbouring
   // choices measured slower (36: 1, 3 and 4 warps; 54: 3, 5 and 7; 72: 5 to 9; 90: 7 to 13).
+  // At 18 the 24 matrices of an SM take 80 registers a lane (one Newton step of a bulk cell 16.6 ms;
+  // 20 matrices 16.8, 16 matrices 17.5).
   switch (a.n) {
-    case 18: return launch_n<18, 1, 15>(a, num_sms, s, grid_used);
+    case 18: return launch_n<18, 1, 24>(a, num_sms, s, grid_used);
     case 36: return launch_n<36, 2, 8>(a, num_sms, s, grid_used);
     case 40: return launch_n<40, 2, 6>(a, num_sms, s, grid_used);
     case 54: return launch_n<54, 4, 3>(a, num_sms, s, grid_used);

@@ -171,8 +171,8 @@ int green_supported(int n);
 int green_warp_supported(int n, int mode);
 cudaError_t launch_green_warp(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used);
 // blocked Gauss-Jordan on the FP64 tensor cores (dimensions 18, 36, 40, 54, 72, 90): one CTA per
-// matrix, at most kGreenMaxCtas CTAs per SM (per-CTA partial sums of MODE_EXPECT)
-constexpr int kGreenMaxCtas = 15;
+// matrix, at most green_max_ctas(n) CTAs per SM (per-CTA partial sums of MODE_EXPECT)
+constexpr int green_max_ctas(int n) { return n <= 18 ? 24 : 15; }
 int green_mma_supported(int n, int mode);
 cudaError_t launch_green_mma(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used);
 // any dimension up to 288, MODE_RAW only: one thread-block cluster per matrix
