@@ -16,7 +16,7 @@
 // About 20 n^3 flops per matrix against the 10 sweeps of 24 n^3 of a cyclic Jacobi iteration,
 // whose rotations also need a CTA barrier per round.  Measured: 9801 matrices of dimension 36 in
 // 24 ms with Jacobi rotations, 3.7 ms now (1.5, 0.5, 1.1 and 0.6 ms for the four kernels); 1331 of
-// dimension 72 in 45 ms and 5.4 ms, of which the serial chains of ql_kernel take 1.7 ms.
+// dimension 72 in 45 ms and 5.5 ms, of which the serial chains of ql_kernel take 1.7 ms.
 #include "tg_internal.cuh"
 
 #include <algorithm>

@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kSheThreads) she_kernel(SheArgs a) {
 // 16-byte reads of a quarter warp fall apart.  Bound by the FP64 tensor pipe: 2 (2 n no^2 + 16 sum_i n_i^2 no) complex products per
 // imaginary point, and 25 % more in padded fragments for sites of nine orbitals.  Two such
 // sites: 28.4 ms for 0.36 M points of both axes with register-tiled products on the scalar units,
-// 22.5 ms here.
+// 22.1 ms here (61 % of the pipe at the imaginary points).
 constexpr int kSheMmaThreads = 256;
 constexpr int kSheFrags = 7;   // fragments of a warp
 
