@@ -1,6 +1,7 @@
 """Blocked FP64 tensor-core solvers at the sizes where their tiling can go wrong (needs a B200):
 the Gauss-Jordan inversion (panels of 4 columns, blocks of 8), the pair sums over its Green
-functions and the Dyson LU (panels of 8, blocks of 64)."""
+functions, the Dyson LU (panels of 8, blocks of 64), the disturbance vertex, the tridiagonal
+resolvents and the eigensolver."""
 import numpy as np
 import pytest
 
@@ -120,3 +121,51 @@ def test_disturbance_fragments(gpu, shape, nk, n_neighbour_stages):
     ref = O.eintshe(O.Model(s, h0), deck.ek, (deck.real_kp, deck.real_w), q, e, s.Ef, s.eta, s.etap, x2, p2, ue)
     got = gpu.she(q, e, s.Ef, s.eta, s.etap, x2, p2, ue)
     assert np.max(np.abs(got - ref)) <= 1e-10 * np.max(np.abs(ref)), shape
+
+
+# 60 of 108 rows (tiles of 64 x 64), all 126 rows (128 x 64; no multiple of the reduction's panels
+# of 8), 50 of 90 rows (reduction in shared memory)
+@pytest.mark.parametrize("shape,d_only", [("slab6", True), ("slab7", False), ("slab5", True)])
+def test_tridiagonal_tiles_equal_gauss_jordan(gpu, shape, d_only):
+    """chi0 from tridiagonalised Green functions at every tile shape of their products equals the
+    Gauss-Jordan path to 1e-12, the bound of the plain test (which has the 160 x 80 tiles)."""
+    deck = synthetic.make_deck(shape, nk=(2, 2, 1), n1gl=3, parts=1, n3gl=3)
+    s = deck.system
+    gpu.setup(deck, s.h0(initial_state(s)))
+    gpu.set_chi_orbitals([list(d) for d in s.dorbs] if d_only else None)
+    e, q = 0.05, np.array([0.1, 0.0, 0.0])
+    x2, p2 = deck.real_points(e, s.Ef)
+    try:
+        auto = gpu.chi0(q, e, s.Ef, s.eta, s.etap, x2, p2, precision="fp64")
+        gpu.set_green_method("gauss-jordan")
+        gj = gpu.chi0(q, e, s.Ef, s.eta, s.etap, x2, p2, precision="fp64")
+    finally:
+        gpu.set_green_method("auto")
+        gpu.set_chi_orbitals(None)
+    assert np.linalg.norm(auto - gj) < 1e-12 * np.linalg.norm(gj)
+
+
+@pytest.mark.parametrize("shape", ["bcc1", "sq2", "slab3", "bcc4", "slab5"])
+@pytest.mark.parametrize("kind", ["model", "two_levels", "diagonal"])
+def test_eigensolver_edges(gpu, shape, kind):
+    """Eigenpairs at the dimensions of the solver's variants, also of matrices that are diagonal
+    already or have two eigenvalues only: residual, orthogonality and eigenvalues within
+    10 n eps (times |H|), the backward error of a reduction of n reflectors."""
+    deck = synthetic.make_deck(shape, mesh=False)
+    s = deck.system
+    n = s.dimH
+    h0 = s.h0(initial_state(s))
+    kp = np.random.default_rng(3).uniform(-2, 2, (1 if kind != "model" else 37, 3))
+    gpu.set_system(s)
+    gpu.set_h0(h0)
+    if kind != "model":   # h0 such that H(k) is the wanted matrix up to roundoff
+        want = np.diag(np.arange(n) - 0.5 * n) if kind == "diagonal" else np.kron(np.diag([1.0, -1.0]), np.eye(n // 2))
+        gpu.set_h0(want.astype(complex) - (gpu.hamiltk_batch(kp)[0] - h0))
+    H = gpu.hamiltk_batch(kp)
+    lam, U = gpu.eig_batch(kp)
+    tol = 10 * n * EPS
+    for k in range(len(kp)):
+        h = np.linalg.norm(H[k], 2)
+        assert np.max(np.abs(U[k].conj().T @ U[k] - np.eye(n))) <= tol
+        assert np.max(np.abs((U[k] * lam[k]) @ U[k].conj().T - H[k])) <= tol * h
+        assert np.max(np.abs(np.sort(lam[k]) - np.linalg.eigvalsh(H[k]))) <= tol * h
