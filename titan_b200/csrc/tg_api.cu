@@ -197,6 +197,7 @@ struct tg_ctx {
   DevArray<unsigned char> d_clws;   // workspace of the thread-block-cluster Gauss-Jordan kernel
   // pinned staging of large transfers between pageable host arrays and the device
   char* stage = nullptr;
+  size_t stage_moved = 0;   // bytes of large pageable transfers so far
   cudaEvent_t stage_ev[2 * 8] = {};
   // tg_expectation_noalloc: device address of the library's fixed scratch array on this
   // context's device (looked up by the context's first no-alloc call)
@@ -281,11 +282,14 @@ int cuda_err(tg_ctx* c, cudaError_t e, const char* where) {
 // pinned buffers of the context, copying one piece while the other is on the link.  Transfers
 // below kStageLeast (a few pieces, the least that several threads can share), and arrays that are
 // pinned already, go to cudaMemcpyAsync.  A call with a result of 41 MB took 108 ms with plain
-// copies and takes 101 ms with these, one with four results of 6.7 MB 215 and 211 ms.  The source of
+// copies and takes 101 ms with these, one with four results of 6.7 MB 215 and 211 ms.  Pinning the
+// buffers takes about 10 ms, what they save on 64 MB (kStagePays): a context makes them when
+// it has been asked to move that much.  The source of
 // an upload may be reused, and the destination of a download read, when copy_host returns.
 constexpr int kStageThreads = 8;
 constexpr size_t kStagePiece = (size_t)1 << 20;
 constexpr size_t kStageLeast = (size_t)4 << 20;
+constexpr size_t kStagePays = (size_t)64 << 20;
 
 cudaError_t copy_host(tg_ctx* c, void* dst, const void* src, size_t bytes, bool to_device) {
   const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
@@ -297,7 +301,9 @@ cudaError_t copy_host(tg_ctx* c, void* dst, const void* src, size_t bytes, bool 
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, to_device ? src : dst) != cudaSuccess) cudaGetLastError();
   else if (at.type != cudaMemoryTypeUnregistered) return plain();
+  c->stage_moved += bytes;
   if (!c->stage) {
+    if (c->stage_moved < kStagePays) return plain();
     void* p = nullptr;
     if (cudaMallocHost(&p, 2 * kStageThreads * kStagePiece) != cudaSuccess) {
       cudaGetLastError();
