@@ -389,9 +389,9 @@ def run_ours(args, rank, world, local_rank):
     # the contraction runs inside a seconds-long step: the sustained (power-capped) GEMM peak
     peak = pk.get("bf16_tflops_sustained", pk.get("bf16_tflops"))
     # DRAM traffic per contraction launch from the ncu capture in
-    # profiles/split_contract_sq2_small.md (2.188 GB over 1984 K-steps of 32 points),
+    # profiles/split_contract_sq2_small.md (2.618 GB over 1984 K-steps of 32 points),
     # scaled by the K-steps one launch of this run processes
-    kstep_bytes = 2.188e9 / 1984
+    kstep_bytes = 2.618e9 / 1984
     traffic = kstep_bytes * (last_units / 32.0) / con_n if (con_n and args.precision == "split") else None
     roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": (achieved / peak) if achieved else None, "traffic": traffic,

@@ -22,7 +22,7 @@
 // What bounds it: shared memory (the A fragments of the updates; L1 at 59 to 69 % of its rate, the
 // FP64 tensor pipe at 44 to 49 %) and, at the small dimensions, warp 0's chain of four pivots per
 // panel (about 3500 cycles).  Cycles per matrix and SM on one B200, before (Gauss-Jordan steps of
-// rank one, matrix in registers) and now: dimension 18: 4400 and 2300, 36: 17500 and 10400, 54:
+// rank one, matrix in registers) and now: dimension 18: 4400 and 2240, 36: 17500 and 10400, 54:
 // 73600 and 29000, 72: 180000 and 62000, 90: 357000 and 118000.  Panels of 8 were slower (36:
 // 19800, 72: 81500, 90: 212000): the factorisation grows faster than the updates shrink.
 #include "tg_internal.cuh"

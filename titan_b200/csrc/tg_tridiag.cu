@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(64) tri_lu_kernel(GreenArgs a, double2* __rest
 // Q_S two chunks ahead (cp.async, its own 128 bytes, so no barrier), advances its state and
 // leaves w_i / d_i or v_i in the double-buffered operand tiles; one barrier per chunk.  The
 // DMMAs bound it: 4 FM FN per warp and 4 steps against FM + FN shared-memory reads.  At 288 with
-// 160 rows: 74 ms when a thread swept a whole column before the products, 59 ms now (73 % of the
+// 160 rows: 74 ms when a thread swept a whole column before the products, 59 ms now (69 % of the
 // FP64 tensor pipe); 62 ms with all warps sweeping at the same time.
 constexpr int kTriK = 8, kTriStages = 3;
 
