@@ -14,7 +14,8 @@
 // for the solve) take most of the time, the panels (one SM at a time, about a microsecond a
 // column) the rest; small matrices are bound by the panels.  Dimension 1600, one call with its
 // host copies: 54 ms with panels of 8 and these GEMMs, 18.6 ms with row-major operands transposed
-// on the device and staged copies as well (157 ms with column by column elimination).
+// on the device and staged copies as well (157 ms with column by column elimination), 17.2 ms
+// with panel rows in registers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -232,6 +233,65 @@ __global__ void __launch_bounds__(kPanThreads, 1) panel_kernel(int n, int j0, in
       for (int r = tid; r < rows; r += T) M[(int64_t)(j0 + c) * n + j0 + r] = P[r * (kPan + 1) + c];
 }
 
+// The same for at most kPanThreads rows, a thread per row with the row's panel columns in
+// registers: rows are exchanged by exchanging their positions, and only the pivot row passes
+// through shared memory, so a column costs two barriers.  Bound by its chain of reductions,
+// barriers and the reciprocal: 11.7 us for a panel of 320 rows (21.9 us with the panel in shared
+// memory), 17 us for 1024 (40 us for the 1600 that stay there; two rows per thread would not fit
+// the registers of 1024 threads).
+__global__ void __launch_bounds__(kPanThreads, 1) panel_rows_kernel(int n, int j0, int nb, double2* __restrict__ M,
+                                                                    int* __restrict__ piv, int* status) {
+  __shared__ unsigned long long skey[32];
+  __shared__ int spos[32];
+  __shared__ double2 u[kPan];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+  const int rows = n - j0;
+  int pos = tid < rows ? tid : -1;   // position of this thread's row
+  double2 v[kPan];
+#pragma unroll
+  for (int c = 0; c < kPan; ++c)
+    v[c] = tid < rows && c < nb ? M[(int64_t)(j0 + c) * n + j0 + tid] : make_double2(0.0, 0.0);
+#pragma unroll
+  for (int c = 0; c < kPan; ++c) {
+    if (c >= nb) break;
+    // largest |Re| + |Im| of column c among positions >= c, first position on ties
+    const double m = fabs(v[c].x) + fabs(v[c].y);
+    unsigned long long key = pos >= c && m > 0.0 ? (unsigned long long)__double_as_longlong(m) : 0ull;
+    int at = key != 0ull ? pos : 0x7fffffff;
+    warp_best(key, at);
+    if (lane == 0) {
+      skey[warp] = key;
+      spos[warp] = at;
+    }
+    __syncthreads();
+    key = lane < nw ? skey[lane] : 0ull;
+    at = lane < nw ? spos[lane] : 0x7fffffff;
+    warp_best(key, at);
+    const int p = key == 0ull ? c : at;
+    if (tid == 0) {
+      piv[j0 + c] = j0 + p;
+      if (key == 0ull) atomicMin(status, j0 + c + 1);
+    }
+    const bool pivot = pos == p;
+    if (pivot) {
+#pragma unroll
+      for (int cc = c; cc < kPan; ++cc) u[cc] = v[cc];
+    }
+    pos = pivot ? c : pos == c ? p : pos;
+    __syncthreads();
+    if (pos > c) {
+      const double2 f = cmul(v[c], crecip(u[c]));
+      v[c] = f;
+#pragma unroll
+      for (int cc = c + 1; cc < kPan; ++cc) v[cc] = cfms(f, u[cc], v[cc]);
+    }
+  }
+  if (pos >= 0)
+#pragma unroll
+    for (int c = 0; c < kPan; ++c)
+      if (c < nb) M[(int64_t)(j0 + c) * n + j0 + pos] = v[c];
+}
+
 // Net effect of the row swaps piv[j0 .. j0 + nb) (rows relative to j0, nb <= kBlock): row j < nb
 // receives the old row top[j], row row[j] = piv[j0 + j] - j0, when >= nb, the old row
 // ext[first[j]] (first[j]: the first of the swaps with that row).  Every thread calls it.
@@ -445,9 +505,10 @@ cudaError_t dyson_device(int n, const double2* chi_hf, const double2* U, double2
     for (int j0 = k0; j0 < k1; j0 += kPan) {
       const int nb = std::min(kPan, k1 - j0);
       const size_t pb = pan_bytes * (size_t)(n - j0);
-      // a thread per row: fewer warps make the block-wide search cheaper
-      const int threads = std::min(kPanThreads, std::max(64, (n - j0 + 31) / 32 * 32));
-      if (pb + pan_static <= (size_t)optin) panel_kernel<true><<<1, threads, pb, s>>>(n, j0, nb, work, piv, status);
+      if (n - j0 <= kPanThreads)
+        panel_rows_kernel<<<1, std::max(64, (n - j0 + 31) / 32 * 32), 0, s>>>(n, j0, nb, work, piv, status);
+      else if (pb + pan_static <= (size_t)optin)
+        panel_kernel<true><<<1, kPanThreads, pb, s>>>(n, j0, nb, work, piv, status);
       else panel_kernel<false><<<1, kPanThreads, 0, s>>>(n, j0, nb, work, piv, status);
       const int others = k1 - k0 - nb;
       if (others > 0)
