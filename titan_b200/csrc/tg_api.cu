@@ -265,6 +265,7 @@ int set_err(tg_ctx* c, int code, const std::string& msg) {
 
 int cuda_err(tg_ctx* c, cudaError_t e, const char* where) {
   if (e == cudaSuccess) return TG_OK;
+  cudaGetLastError();   // reported here; else the next call's first launch would report it again
   std::string m = std::string(where) + ": " + cudaGetErrorString(e);
   if (e == cudaErrorMemoryAllocation) return set_err(c, TG_ERR_NOMEM, m);
   return set_err(c, TG_ERR_CUDA, m);
