@@ -51,3 +51,32 @@ def test_a_call_after_one_that_ran_out_of_memory():
         assert err.value.code == -5
         assert np.allclose(g.dyson(x, x), want, rtol=0, atol=1e-12 * np.abs(want).max())
     g.close()
+
+
+def calls_of(deck):
+    s = deck.system
+    ev = np.tile([[0.6, 0.0, 0.8]], (s.n_atoms, 1))
+    return {"smunu": lambda g: g.smunu(s.Ef, s.eta), "gs_orbital": lambda g: g.gs_orbital(s.Ef, s.eta),
+            "gg_tensor": lambda g: g.gg_tensor(s.Ef, s.eta), "fermi_column": lambda g: g.fermi_column(s.Ef, s.eta),
+            "jacobian": lambda g: g.jacobian(s.Ef, s.eta), "adjoint_vb": lambda g: g.adjoint_vb(s.Ef, s.eta),
+            "jij": lambda g: g.jij(np.array([0.1, 0.05, 0.0]), s.Ef, s.eta, ev, s.Um())}
+
+
+@pytest.mark.parametrize("free,names", [(640, ("smunu", "gs_orbital", "gg_tensor", "fermi_column", "jacobian",
+                                                "adjoint_vb")), (2600, ("jij",))])
+def test_sums_without_room_for_their_tables(free, names):
+    """31329 k of two spd sites: an H(k) table is 650 MB and the Green functions of a pass are up to
+    1 GiB.  With `free` MiB left the sums form H(k) in the inversion and take shorter passes; they
+    differ from the others by the order of the sum only (1e-12)."""
+    deck = synthetic.make_deck("sq2", nk=(177, 177, 1), n1gl=2, parts=1, n3gl=2)
+    h0 = deck.system.h0(initial_state(deck.system))
+    calls = calls_of(deck)
+    for name in names:
+        g = context(deck, h0)
+        want = calls[name](g)   # (also loads the kernels)
+        g.close()
+        g = context(deck, h0)
+        with filled_device(free * MIB):
+            got = calls[name](g)
+            g.close()
+        assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want)), name

@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2051,9 +2052,23 @@ struct PairRef {
   int block;   // output block of an orbital pair
 };
 
-// the imaginary-axis points at Ef + i (y + eta); on a uniform mesh (and when `table`) with the
-// H(k) table of its k list in slot 0
-int imag_points(tg_ctx* c, double Ef, double eta, bool table, GreenArgs& a) {
+// room for the H(k) tables of nk points in slots 0 .. slots - 1; without it both are given back and
+// the inversion kernels form H(k) themselves
+bool htab_room(tg_ctx* c, int slots, int64_t nk) {
+  const size_t nn = (size_t)c->dimH * c->dimH;
+  if (nk * (int64_t)nn * 16 > ((int64_t)8 << 30)) return false;
+  bool ok = c->d_hphase.ensure((size_t)nk * std::max(c->n_neigh, 1)) == cudaSuccess;
+  for (int i = 0; i < slots && ok; ++i) ok = c->d_htab[i].ensure((size_t)nk * nn) == cudaSuccess;
+  if (ok) return true;
+  cudaGetLastError();
+  c->d_hphase.free_();
+  for (int i = 0; i < slots; ++i) c->d_htab[i].free_();
+  return false;
+}
+
+// the imaginary-axis points at Ef + i (y + eta) in a, and with q those of G(k - q) in b; on a
+// uniform mesh with H(k) tables of its k list in the slots 0 and 1, or neither of them
+int imag_points(tg_ctx* c, double Ef, double eta, const double* q, GreenArgs& a, GreenArgs* b) {
   a = base_args(c);
   a.pts.kind = 0;
   a.pts.y = c->d_y.p;
@@ -2061,35 +2076,62 @@ int imag_points(tg_ctx* c, double Ef, double eta, bool table, GreenArgs& a) {
   a.pts.w = c->d_w.p;
   a.zr = Ef;
   a.zi = eta;
-  if (table && c->imag_uniform && (int64_t)c->nk_u * c->dimH * c->dimH * 16 <= ((int64_t)8 << 30)) {
-    const double zero3[3] = {0.0, 0.0, 0.0};
-    int rc = build_htab(c, 0, c->d_klist_u.p, c->nk_u, zero3);
-    if (rc) return rc;
+  const double zero3[3] = {0.0, 0.0, 0.0};
+  const bool table = c->imag_uniform && htab_room(c, q ? 2 : 1, c->nk_u);
+  int rc;
+  if (table) {
+    if ((rc = build_htab(c, 0, c->d_klist_u.p, c->nk_u, zero3))) return rc;
     a.htab = c->d_htab[0].p;
     a.n_e = c->n_e_u;
     a.nk_tab = c->nk_u;
     a.ylist = c->d_ylist.p;
   }
+  if (!q) return TG_OK;
+  *b = a;
+  const double mq[3] = {-q[0], -q[1], -q[2]};
+  if (table) {
+    if ((rc = build_htab(c, 1, c->d_klist_u.p, c->nk_u, mq))) return rc;
+    b->htab = c->d_htab[1].p;
+  } else {
+    for (int i = 0; i < 3; ++i) b->q[i] = mq[i];
+  }
   return TG_OK;
 }
 
-// out[e] = sum over the np points of a of w G(ent[e].x, ent[e].y): raw Green functions of at
-// most 1 GiB per pass, summed by the entry kernel
-int entry_sums(tg_ctx* c, GreenArgs a, int64_t np, const std::vector<int2>& ent, std::vector<double2>& out,
-               const char* what) {
+// raw Green functions of P points in each of the buffers; P is halved while the device memory does
+// not hold them
+int ensure_pass(tg_ctx* c, std::initializer_list<DevArray<double2>*> bufs, int64_t& P) {
+  for (;;) {
+    cudaError_t e = cudaSuccess;
+    for (auto* b : bufs)
+      if (e == cudaSuccess) e = b->ensure((size_t)P * c->dimH * c->dimH);
+    if (e != cudaErrorMemoryAllocation || P <= 64) return cuda_err(c, e, "alloc G");
+    cudaGetLastError();
+    for (auto* b : bufs) b->free_();
+    P = std::max<int64_t>(64, P / 2);
+  }
+}
+
+// out[e] = sum over the np points that points(a) sets of w G(ent[e].x, ent[e].y): raw Green functions
+// of at most 1 GiB per pass, summed by the entry kernel (their buffer is taken before the tables of
+// points(a), which can be done without)
+template <class Points>
+int entry_sums(tg_ctx* c, int64_t np, const std::vector<int2>& ent, std::vector<double2>& out, const char* what,
+               Points points) {
   cudaStream_t s = c->stream;
-  const int64_t nn = (int64_t)c->dimH * c->dimH;
   const int ne = (int)ent.size();
   out.assign(ent.size(), make_double2(0.0, 0.0));
-  const int64_t P = pass_size(c, np, (int64_t)1 << 30);
+  int64_t P = pass_size(c, np, (int64_t)1 << 30);
   const int parts = entry_partials(P, c->num_sms);
   TG_CHECK(c, c->d_gg_desc.upload(reinterpret_cast<const int*>(ent.data()), 2 * ent.size(), s), "upload");
-  TG_CHECK(c, c->d_graw.ensure((size_t)P * nn), "alloc G");
   TG_CHECK(c, c->d_acc.ensure((size_t)parts * ne), "alloc acc");
   TG_CHECK(c, c->d_acc_red.ensure(ne), "alloc acc");
-  TG_CHECK(c, cudaMemsetAsync(c->d_acc.p, 0, sizeof(double2) * (size_t)parts * ne, s), "memset");
-  int rc = reset_status(c);
+  int rc = ensure_pass(c, {&c->d_graw}, P);
   if (rc) return rc;
+  GreenArgs a;
+  if ((rc = points(a))) return rc;
+  TG_CHECK(c, cudaMemsetAsync(c->d_acc.p, 0, sizeof(double2) * (size_t)parts * ne, s), "memset");
+  if ((rc = reset_status(c))) return rc;
   a.mode = MODE_RAW;
   a.out = c->d_graw.p;
   for (int64_t p0 = 0; p0 < np; p0 += P) {
@@ -2111,32 +2153,21 @@ int entry_sums(tg_ctx* c, GreenArgs a, int64_t np, const std::vector<int2>& ent,
 int imag_pairs(tg_ctx* c, double Ef, double eta, const double* q, const std::vector<int4>& pairs,
                std::vector<double2>& h, std::vector<double2>* hs) {
   cudaStream_t s = c->stream;
-  const int64_t nn = (int64_t)c->dimH * c->dimH;
   const int npairs = (int)pairs.size(), len = 16 * npairs, sets = q ? 2 : 1;
   h.assign(len, make_double2(0.0, 0.0));
   if (hs) hs->assign(len, make_double2(0.0, 0.0));
   if (npairs == 0) return TG_OK;
-  GreenArgs a;
-  int rc = imag_points(c, Ef, eta, true, a);
-  if (rc) return rc;
-  GreenArgs b = a;   // the points of G(k - q)
-  if (q) {
-    const double mq[3] = {-q[0], -q[1], -q[2]};
-    if (a.htab) {
-      if ((rc = build_htab(c, 1, c->d_klist_u.p, c->nk_u, mq))) return rc;
-      b.htab = c->d_htab[1].p;
-    } else {
-      for (int i = 0; i < 3; ++i) b.q[i] = mq[i];
-    }
-  }
-  const int64_t P = pass_size(c, c->n_imag, (int64_t)1 << 30);
+  int64_t P = pass_size(c, c->n_imag, (int64_t)1 << 30);
   const size_t parts = pair_partials(c->dimH, npairs, q != nullptr, c->num_sms, P);
   TG_CHECK(c, c->d_gg_desc.upload(reinterpret_cast<const int*>(pairs.data()), 4 * pairs.size(), s), "upload pairs");
   const int4* dp = reinterpret_cast<const int4*>(c->d_gg_desc.p);
-  TG_CHECK(c, c->d_A.ensure((size_t)P * nn), "alloc G");
-  if (q) TG_CHECK(c, c->d_B.ensure((size_t)P * nn), "alloc G");
   TG_CHECK(c, c->d_acc.ensure(sets * parts * len), "alloc acc");
   TG_CHECK(c, c->d_acc_red.ensure((size_t)sets * len), "alloc acc");
+  int rc = q ? ensure_pass(c, {&c->d_A, &c->d_B}, P) : ensure_pass(c, {&c->d_A}, P);
+  if (rc) return rc;
+  GreenArgs a, b;
+  if ((rc = imag_points(c, Ef, eta, q, a, &b))) return rc;
+  if (!q) b = a;
   TG_CHECK(c, cudaMemsetAsync(c->d_acc.p, 0, sizeof(double2) * sets * parts * len, s), "memset");
   if ((rc = reset_status(c))) return rc;
   profile_begin(c);
@@ -2183,28 +2214,15 @@ int tg_expectation(tg_ctx* c, double Ef, double eta, double* rho, double* mx, do
   cudaStream_t s = c->stream;
   const int n = c->dimH;
   const int len = 2 * n;   // 4 complex per orbital, n/2 orbitals
-  GreenArgs a = base_args(c);
-  a.pts.kind = 0;
-  a.pts.y = c->d_y.p;
-  a.pts.kp = c->d_kp.p;
-  a.pts.w = c->d_w.p;
-  a.p0 = 0;
-  a.np = c->n_imag;
-  a.zr = Ef;
-  a.zi = eta;
-  a.mode = MODE_EXPECT;
-  a.exp_rows = c->d_exp_rows.p;
-  if (c->imag_uniform && (int64_t)c->nk_u * c->dimH * c->dimH * 16 <= ((int64_t)8 << 30)) {
-    const double zero3[3] = {0.0, 0.0, 0.0};
-    if ((rc = build_htab(c, 0, c->d_klist_u.p, c->nk_u, zero3))) return rc;
-    a.htab = c->d_htab[0].p;
-    a.n_e = c->n_e_u;
-    a.nk_tab = c->nk_u;
-    a.ylist = c->d_ylist.p;
-  }
   const int maxgrid = c->num_sms * (green_max_ctas(n) + 1);
   TG_CHECK(c, c->d_acc.ensure((size_t)maxgrid * len), "alloc acc");
   TG_CHECK(c, c->d_acc_red.ensure(len), "alloc acc");
+  GreenArgs a;
+  if ((rc = imag_points(c, Ef, eta, nullptr, a, nullptr))) return rc;
+  a.p0 = 0;
+  a.np = c->n_imag;
+  a.mode = MODE_EXPECT;
+  a.exp_rows = c->d_exp_rows.p;
   a.acc = c->d_acc.p;
   rc = reset_status(c);
   if (rc) return rc;
@@ -2333,17 +2351,20 @@ int tg_fermi_column(tg_ctx* c, double Ef, double eta, double* D) {
       ent.push_back(make_int2(u, d));
       ent.push_back(make_int2(d, u));
     }
-  GreenArgs a = base_args(c);
-  a.pts.kind = 1;
-  a.pts.kp = c->d_rkp.p;
-  a.pts.w = c->d_rw.p;
-  a.pts.x2 = c->d_x2.p;
-  a.pts.p2 = c->d_p2.p;
-  a.pts.nk = c->n_realk;
-  a.zr = 0.0;
-  a.zi = eta;
+  auto points = [&](GreenArgs& a) {
+    a = base_args(c);
+    a.pts.kind = 1;
+    a.pts.kp = c->d_rkp.p;
+    a.pts.w = c->d_rw.p;
+    a.pts.x2 = c->d_x2.p;
+    a.pts.p2 = c->d_p2.p;
+    a.pts.nk = c->n_realk;
+    a.zr = 0.0;
+    a.zi = eta;
+    return TG_OK;
+  };
   std::vector<double2> g, h(ent.size());
-  if ((rc = entry_sums(c, a, c->n_realk, ent, g, "green (fermi column)"))) return rc;
+  if ((rc = entry_sums(c, c->n_realk, ent, g, "green (fermi column)", points))) return rc;
   for (size_t o = 0; o + 3 < g.size(); o += 4) {   // traces with 1, sigma_x, sigma_y, sigma_z
     const double2 uu = g[o], dd = g[o + 1], ud = g[o + 2], du = g[o + 3];
     h[o] = cadd(uu, dd);
@@ -2678,10 +2699,9 @@ int tg_smunu(tg_ctx* c, double Ef, double eta, double* S) {
   }
   std::vector<int2> ent;
   for (size_t e = 0; e + 1 < desc.size(); e += 2) ent.push_back(make_int2(desc[e], desc[e + 1]));
-  GreenArgs a;
-  if ((rc = imag_points(c, Ef, eta, true, a))) return rc;
   std::vector<double2> h;
-  if ((rc = entry_sums(c, a, c->n_imag, ent, h, "green (on-site blocks)"))) return rc;
+  auto points = [&](GreenArgs& a) { return imag_points(c, Ef, eta, nullptr, a, nullptr); };
+  if ((rc = entry_sums(c, c->n_imag, ent, h, "green (on-site blocks)", points))) return rc;
   // calcSmunu: imgXY(mu, nu) = (A(nu X, mu Y) + conj(A(mu Y, nu X))) / 2 pi, 1/2 on the uu / dd diagonals
   const double tpi = 2.0 * kPi;
   std::fill(S, S + (size_t)2 * nmax * nmax * 3 * nat, 0.0);
@@ -2733,10 +2753,9 @@ int tg_gs_orbital(tg_ctx* c, double Ef, double eta, double* gupgd) {
   }
   std::vector<int2> ent;
   for (size_t e = 0; e + 1 < desc.size(); e += 2) ent.push_back(make_int2(desc[e], desc[e + 1]));
-  GreenArgs a;
-  if ((rc = imag_points(c, Ef, eta, true, a))) return rc;
   std::vector<double2> h;
-  if ((rc = entry_sums(c, a, c->n_imag, ent, h, "green (on-site spin blocks)"))) return rc;
+  auto points = [&](GreenArgs& a) { return imag_points(c, Ef, eta, nullptr, a, nullptr); };
+  if ((rc = entry_sums(c, c->n_imag, ent, h, "green (on-site spin blocks)", points))) return rc;
   // gupgd(nu, mu, i) = (1/pi) sum w (G(i mu up, i nu up) + G(i mu dn, i nu dn))  (mod_expectation.F90:957-975)
   std::fill(gupgd, gupgd + (size_t)2 * nmax * nmax * nat, 0.0);
   for (int i = 0; i < nat; ++i) {
