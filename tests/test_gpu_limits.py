@@ -80,3 +80,21 @@ def test_sums_without_room_for_their_tables(free, names):
             got = calls[name](g)
             g.close()
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want)), name
+
+
+def test_ldos_without_room_for_every_rotation():
+    """The LDOS of 16900 k of two spd sites keeps 700 MB of matrices and eigenvectors; the list of
+    their rotations, 1 GiB where there is room, is worked off in shorter parts with 1 GiB left."""
+    deck = synthetic.make_deck("sq2", nk=(130, 130, 1), n1gl=2, parts=1, n3gl=2)
+    s = deck.system
+    h0 = s.h0(initial_state(s))
+    es = s.Ef + np.linspace(-1.0, 1.0, 5)
+    g = context(deck, h0)
+    want = g.ldos(es, s.eta)
+    g.close()
+    g = context(deck, h0)
+    with filled_device(1024 * MIB):
+        got = g.ldos(es, s.eta)
+        g.close()
+    for a, b in zip(got, want):
+        assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))

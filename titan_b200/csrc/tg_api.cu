@@ -462,7 +462,6 @@ int build_htab(tg_ctx* c, int slot, const double* d_k, int64_t nk, const double*
   return TG_OK;
 }
 
-// eigendecomposition of every row of H table `slot` (spectral Green functions)
 // chi0 and the LDOS use spectral Green functions unless Gauss-Jordan is forced; the
 // disturbance integral and the occupations only when TG_GREEN_SPECTRAL asks for them (see
 // tg_set_green_method)
@@ -479,13 +478,26 @@ bool chi_tridiag(tg_ctx* c) {
   return !chi_spectral(c) && c->green_method == TG_GREEN_AUTO && tri_supported(c->dimH);
 }
 
+// workspace of launch_eig for tables of nk matrices, `chunk` of them at a time: fewer where the
+// device memory does not hold the rotations of all that 1 GiB would
+int ensure_eig_ws(tg_ctx* c, int64_t nk, int64_t& chunk) {
+  for (chunk = eig_chunk(c->dimH, nk);; chunk = (chunk + 1) / 2) {
+    const cudaError_t e = c->d_eigws.ensure(eig_ws_bytes(c->dimH, nk, chunk));
+    if (e != cudaErrorMemoryAllocation || chunk <= 64) return cuda_err(c, e, "alloc rotations");
+    cudaGetLastError();
+  }
+}
+
+// eigendecomposition of every row of H table `slot` (spectral Green functions)
 int build_eig(tg_ctx* c, int slot, int64_t nk) {
   const size_t nn = (size_t)c->dimH * c->dimH;
   TG_CHECK(c, c->d_eigU[slot].ensure((size_t)nk * nn), "alloc eigenvectors");
   TG_CHECK(c, c->d_eigL[slot].ensure((size_t)nk * c->dimH), "alloc eigenvalues");
-  TG_CHECK(c, c->d_eigws.ensure(eig_ws_bytes(c->dimH, nk)), "alloc rotations");
+  int64_t chunk = 0;
+  int rc = ensure_eig_ws(c, nk, chunk);
+  if (rc) return rc;
   KindTimer kt(c, 0);
-  TG_CHECK(c, launch_eig(c->d_htab[slot].p, nk, c->dimH, c->d_eigU[slot].p, c->d_eigL[slot].p, c->d_eigws.p,
+  TG_CHECK(c, launch_eig(c->d_htab[slot].p, nk, c->dimH, c->d_eigU[slot].p, c->d_eigL[slot].p, c->d_eigws.p, chunk,
                          c->d_eig_status.p, c->num_sms, c->stream),
            "eigendecomposition");
   return TG_OK;
@@ -501,7 +513,9 @@ int build_eig_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
   TG_CHECK(c, c->d_eigL[slot].ensure((size_t)nk * n), "alloc eigenvalues");
   TG_CHECK(c, c->d_hchunk.ensure((size_t)kc * nn), "alloc H chunk");
   TG_CHECK(c, c->d_hphase.ensure((size_t)kc * std::max(c->n_neigh, 1)), "alloc phases");
-  TG_CHECK(c, c->d_eigws.ensure(eig_ws_bytes((int)n, kc)), "alloc rotations");
+  int64_t chunk = 0;
+  int rc = ensure_eig_ws(c, kc, chunk);
+  if (rc) return rc;
   TG_CHECK(c, c->d_qvec.upload(q, 3, c->stream), "upload q");
   const GreenArgs a = base_args(c);
   KindTimer kt(c, 0);
@@ -510,7 +524,7 @@ int build_eig_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
     TG_CHECK(c, launch_hk_table(a, d_k + 3 * k0, m, c->d_qvec.p, c->d_hphase.p, c->d_hchunk.p, c->stream),
              "H table");
     TG_CHECK(c, launch_eig(c->d_hchunk.p, m, (int)n, c->d_eigU[slot].p + k0 * nn, c->d_eigL[slot].p + k0 * n,
-                           c->d_eigws.p, c->d_eig_status.p, c->num_sms, c->stream),
+                           c->d_eigws.p, std::min(chunk, m), c->d_eig_status.p, c->num_sms, c->stream),
              "eigendecomposition");
     c->launches += 5;
   }
@@ -532,7 +546,7 @@ bool eig_room(tg_ctx* c, int64_t nk, int s0, int s1) {
   }
   const size_t kc = std::min<size_t>((size_t)nk, std::max<size_t>(1, ((size_t)2 << 30) / (nn * 16)));
   if (c->d_hchunk.n < kc * nn) need += (double)(kc * nn - c->d_hchunk.n) * sizeof(double2);
-  const size_t ws = eig_ws_bytes(c->dimH, kc);
+  const size_t ws = eig_ws_bytes(c->dimH, kc, eig_chunk(c->dimH, kc));
   if (c->d_eigws.n < ws) need += (double)(ws - c->d_eigws.n);
   return need <= 0.5 * (double)fr;
 }

@@ -619,11 +619,6 @@ size_t hh_smem(int n) {
 int ql_cap(int n) { return 3 * n * n + 32; }
 int ql_sweeps(int n) { return 8 * n + 16; }
 
-// k per chunk: at most 1 GiB of rotations
-int64_t ql_chunk(int n, int64_t nk) {
-  return std::max<int64_t>(1, std::min<int64_t>(nk, ((int64_t)1 << 30) / ((int64_t)ql_cap(n) * 16)));
-}
-
 }  // namespace
 
 // U and a scratch matrix both whole in shared memory (dimensions up to 72 or so): there G from
@@ -660,17 +655,20 @@ cudaError_t launch_hh_small(const double2* H, int64_t nk, int n, const int* rows
   return cudaGetLastError();
 }
 
-size_t eig_ws_bytes(int n, int64_t nk) {
-  const int64_t c = ql_chunk(n, nk);
-  return (size_t)c * ((size_t)ql_cap(n) * sizeof(double2) + (size_t)ql_sweeps(n) * sizeof(int) + sizeof(int)) +
+// at most 1 GiB of rotations
+int64_t eig_chunk(int n, int64_t nk) {
+  return std::max<int64_t>(1, std::min<int64_t>(nk, ((int64_t)1 << 30) / ((int64_t)ql_cap(n) * 16)));
+}
+
+size_t eig_ws_bytes(int n, int64_t nk, int64_t chunk) {
+  return (size_t)chunk * ((size_t)ql_cap(n) * sizeof(double2) + (size_t)ql_sweeps(n) * sizeof(int) + sizeof(int)) +
          (size_t)nk * n * 2 * sizeof(double) + 256;
 }
 
-cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int* status,
-                       int num_sms, cudaStream_t s) {
+cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int64_t chunk,
+                       int* status, int num_sms, cudaStream_t s) {
   if (nk <= 0) return cudaSuccess;
-  if (!eig_supported(n)) return cudaErrorInvalidValue;
-  const int64_t chunk = ql_chunk(n, nk);
+  if (!eig_supported(n) || chunk <= 0) return cudaErrorInvalidValue;
   const int cap = ql_cap(n), scap = ql_sweeps(n);
   double2* rot = static_cast<double2*>(ws);
   double* D = reinterpret_cast<double*>(rot + chunk * cap);

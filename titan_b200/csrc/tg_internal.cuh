@@ -222,12 +222,14 @@ cudaError_t launch_hk_table(const GreenArgs& a, const double* kp, int64_t nk, co
 cudaError_t launch_reduce_blocks(const double2* part, int nblocks, int len, double2* out, cudaStream_t s);
 
 // Spectral Green functions: eigendecomposition of an H(k) table (ws: eig_ws_bytes of device
-// memory) and G from (U, lambda)
+// memory for the rotations of `chunk` matrices at a time, eig_chunk where there is room) and G from
+// (U, lambda)
 int eig_supported(int n);
 int eig_fast(int n);
-size_t eig_ws_bytes(int n, int64_t nk);
-cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int* status,
-                       int num_sms, cudaStream_t s);
+int64_t eig_chunk(int n, int64_t nk);
+size_t eig_ws_bytes(int n, int64_t nk, int64_t chunk);
+cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int64_t chunk,
+                       int* status, int num_sms, cudaStream_t s);
 // Householder tridiagonalisation of an H(k) table in shared memory, dimensions up to 96 (H is
 // kept; rows null: every row of Q)
 int hh_small_supported(int n);
