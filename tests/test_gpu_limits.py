@@ -1,4 +1,5 @@
-"""Calls where device memory is short (needs a B200)."""
+"""Calls where device memory is short, and on Hamiltonians with entries whose squares underflow
+(needs a B200)."""
 import numpy as np
 import pytest
 
@@ -98,3 +99,63 @@ def test_ldos_without_room_for_every_rotation():
         g.close()
     for a, b in zip(got, want):
         assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
+
+
+def without_hoppings(shape):
+    s = synthetic.make_system(shape)
+    cv, bi, ish, t = s.neighbor_table()
+    s.neighbor_table = lambda: (cv, bi, ish, 0.0 * t)
+    return s
+
+
+def weakly_coupled(n, tiny, rng):
+    """Random Hermitian matrix whose first three rows couple to each other and to the rest by
+    imaginary entries of size `tiny` alone."""
+    h = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    h = 0.5 * (h + h.conj().T)
+    for r in range(3):
+        d = h[r, r]
+        h[r, :], h[:, r] = 1j * tiny, -1j * tiny
+        h[r, r] = d
+    for r in range(3):
+        h[r, :r], h[:r, r] = -1j * tiny, 1j * tiny
+    return h
+
+
+@pytest.mark.parametrize("tiny", [1e-145, 1e-158, 1e-170])
+@pytest.mark.parametrize("shape", ["bcc1", "sq2", "bcc4", "slab5"])
+def test_eigenvectors_of_couplings_that_underflow(shape, tiny):
+    """A reflector of a column whose squares are denormal or zero is unitary all the same:
+    orthogonality and residual within 10 n eps (times |H|)."""
+    from titan_b200.native import GreenGPU
+    s = without_hoppings(shape)
+    h = weakly_coupled(s.dimH, tiny, np.random.default_rng(4))
+    g = GreenGPU(0)
+    g.set_system(s)
+    g.set_h0(h)
+    lam, U = g.eig_batch(np.zeros((3, 3)))
+    g.close()
+    tol = 10 * s.dimH * EPS
+    for l, u in zip(lam, U):
+        assert np.max(np.abs(u.conj().T @ u - np.eye(s.dimH))) <= tol
+        assert np.max(np.abs((u * l) @ u.conj().T - h)) <= tol * np.linalg.norm(h, 2)
+
+
+@pytest.mark.parametrize("shape", ["slab5", "slab7"])
+def test_resolvents_of_couplings_that_underflow(shape):
+    """The same for the resolvents from tridiagonalised H(k) (in shared memory, and in panels
+    beyond dimension 96): chi0 equals the Gauss-Jordan path to 1e-12."""
+    from titan_b200.native import GreenGPU
+    deck = synthetic.make_deck(shape, nk=(2, 2, 1), n1gl=3, parts=1, n3gl=3)
+    s = without_hoppings(shape)
+    g = GreenGPU(0)
+    g.set_system(s)
+    g.set_h0(weakly_coupled(s.dimH, 1e-158, np.random.default_rng(4)))
+    g.set_imag_mesh(deck.ek)
+    g.set_chi_orbitals([list(d) for d in s.dorbs])
+    q = np.array([0.1, 0.0, 0.0])
+    auto = g.chi0(q, 0.0, s.Ef, s.eta, s.etap)
+    g.set_green_method("gauss-jordan")
+    gj = g.chi0(q, 0.0, s.Ef, s.eta, s.etap)
+    g.close()
+    assert np.linalg.norm(auto - gj) < 1e-12 * np.linalg.norm(gj)

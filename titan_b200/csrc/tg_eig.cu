@@ -82,25 +82,28 @@ __global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __r
           x[i] = r < m ? col[r] : zero;
           if (r > 0) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
         }
-        const double2 alpha = col[0];
+        double2 alpha = col[0];
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        const bool refl = !(part == 0.0 && alpha.y == 0.0);
-        // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
-        const double beta =
-            refl ? -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, part))), alpha.x) : alpha.x;
-        double2 tau = zero;
-        if (refl) {
-          const double ib = 1.0 / beta;
-          tau = make_double2((beta - alpha.x) * ib, -alpha.y * ib);
-          const double dr = alpha.x - beta, di = alpha.y;
-          const double inv = 1.0 / fma(dr, dr, di * di);
-          const double2 sc = make_double2(dr * inv, -di * inv);
+        double down = 1.0;
+        if (reflector_norm2(alpha, part) < kReflectorTiny) {   // (the same in every lane)
+          part = 0.0;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            x[i] = cscale(x[i], kReflectorUp);
+            if (lane + 32 * i > 0) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
+          }
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          alpha = cscale(alpha, kReflectorUp);
+          down = kReflectorDown;
+        }
+        const Reflector h = reflector(alpha, part);
+        if (h.any) {
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             const int r = lane + 32 * i;
             if (r < m) {
-              const double2 vr = r == 0 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
+              const double2 vr = r == 0 ? make_double2(1.0, 0.0) : cmul(x[i], h.sc);
               v[r] = vr;
               col[r] = vr;   // kept for Q; the column is done with
             }
@@ -108,8 +111,8 @@ __global__ void __launch_bounds__(kHhThreads) hh_small_kernel(const double2* __r
         }
         if (lane == 0) {
           D[k * n + j] = B[j * S + j].x;
-          E[k * n + j] = beta;
-          taus[j] = tau;
+          E[k * n + j] = h.beta * down;
+          taus[j] = h.tau;
         }
       }
       __syncthreads();

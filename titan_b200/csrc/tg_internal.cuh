@@ -230,6 +230,33 @@ int64_t eig_chunk(int n, int64_t nk);
 size_t eig_ws_bytes(int n, int64_t nk, int64_t chunk);
 cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int64_t chunk,
                        int* status, int num_sms, cudaStream_t s);
+// Reflector I - tau v v^H of LAPACK's zlarfg that takes the vector (alpha, x) to (beta, 0), from
+// rest = |x|^2: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = (1, sc x); none
+// (tau = 0) when x = 0 and alpha is real.  A vector whose squares may underflow, |(alpha, x)|^2 below
+// kReflectorTiny, is passed times kReflectorUp (tau and v are the same for it): the reflector of one
+// with denormal squares would not be unitary.
+constexpr double kReflectorTiny = 1e-270, kReflectorUp = 0x1p600, kReflectorDown = 0x1p-600;
+struct Reflector {
+  bool any;
+  double beta;
+  double2 tau, sc;
+};
+__device__ __forceinline__ double reflector_norm2(double2 alpha, double rest) {
+  return fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, rest));
+}
+__device__ __forceinline__ Reflector reflector(double2 alpha, double rest) {
+  Reflector h{!(rest == 0.0 && alpha.y == 0.0), alpha.x, make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+  if (h.any) {
+    h.beta = -copysign(sqrt(reflector_norm2(alpha, rest)), alpha.x);
+    const double ib = 1.0 / h.beta;
+    h.tau = make_double2((h.beta - alpha.x) * ib, -alpha.y * ib);
+    const double dr = alpha.x - h.beta, di = alpha.y;
+    const double inv = 1.0 / fma(dr, dr, di * di);
+    h.sc = make_double2(dr * inv, -di * inv);
+  }
+  return h;
+}
+
 // Householder tridiagonalisation of an H(k) table in shared memory, dimensions up to 96 (H is
 // kept; rows null: every row of Q)
 int hh_small_supported(int n);

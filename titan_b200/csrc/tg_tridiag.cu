@@ -94,26 +94,30 @@ __global__ void __launch_bounds__(kPanThreads, 1) hh_panel_kernel(double2* __res
         double part = 0.0;
         for (int i = j + 2 + lane; i < n; i += 32) part = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, part));
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        const double2 alpha = x[j + 1];
-        const bool refl = !(part == 0.0 && alpha.y == 0.0);
-        // zlarfg: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
-        const double beta =
-            refl ? -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, part))), alpha.x) : alpha.x;
-        double2 tau = zero, sc = zero;
-        if (refl) {
-          tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-          const double dr = alpha.x - beta, di = alpha.y;
-          const double inv = 1.0 / fma(dr, dr, di * di);
-          sc = make_double2(dr * inv, -di * inv);
+        double2 alpha = x[j + 1];
+        double up = 1.0, down = 1.0;
+        if (reflector_norm2(alpha, part) < kReflectorTiny) {   // (the same in every thread)
+          up = kReflectorUp;
+          down = kReflectorDown;
+          alpha = cscale(alpha, up);
+          part = 0.0;
+          for (int i = j + 2 + lane; i < n; i += 32) {
+            const double2 xi = cscale(x[i], up);
+            part = fma(xi.x, xi.x, fma(xi.y, xi.y, part));
+          }
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
         }
+        const Reflector h = reflector(alpha, part);
+        const bool refl = h.any;
+        const double2 tau = h.tau;
         if (tid == 0) {
           D[k * n + j] = x[j].x;
-          E[k * n + j] = beta;
+          E[k * n + j] = h.beta * down;
           taus[jj] = tau;
         }
         // v (zero up to row j; all zero without a reflector)
         for (int i = tid; i < n; i += kPanThreads) {
-          const double2 vi = !refl || i <= j ? zero : i == j + 1 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
+          const double2 vi = !refl || i <= j ? zero : i == j + 1 ? make_double2(1.0, 0.0) : cmul(cscale(x[i], up), h.sc);
           V[i * kPanS + jj] = vi;
           Vt[jj * n + i] = vi;
         }
