@@ -10,18 +10,17 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/titan_gpu.h"
 #include "tg_internal.cuh"
 #include "tg_split.cuh"
+#include "tg_stage.cuh"
 
 using namespace tg;
 
@@ -196,10 +195,7 @@ struct tg_ctx {
   DevArray<double2> d_triQ[4 + kTriQSlots];
   DevArray<double2> d_triws;   // factors of z - T of a pass's points
   DevArray<unsigned char> d_clws;   // workspace of the thread-block-cluster Gauss-Jordan kernel
-  // pinned staging of large transfers between pageable host arrays and the device
-  char* stage = nullptr;
-  size_t stage_moved = 0;   // bytes of large pageable transfers so far
-  cudaEvent_t stage_ev[2 * 8] = {};
+  HostStage stage;   // large transfers between pageable host arrays and the device
   // tg_expectation_noalloc: device address of the library's fixed scratch array on this
   // context's device (looked up by the context's first no-alloc call)
   double2* noalloc_ptr = nullptr;
@@ -278,99 +274,9 @@ int cuda_err(tg_ctx* c, cudaError_t e, const char* where) {
     if (_e != cudaSuccess) return cuda_err(c, _e, where); \
   } while (0)
 
-// Large transfers of pageable host arrays.  cudaMemcpyAsync stages those through one thread of
-// the driver (and on a fresh result array that thread takes every page fault); here up to
-// kStageThreads threads of this call each move their part in pieces of kStagePiece through two
-// pinned buffers of the context, copying one piece while the other is on the link.  Transfers
-// below kStageLeast (a few pieces, the least that several threads can share), and arrays that are
-// pinned already, go to cudaMemcpyAsync.  A call with a result of 41 MB took 108 ms with plain
-// copies and takes 101 ms with these, one with four results of 6.7 MB 215 and 211 ms.  Pinning the
-// buffers takes about 10 ms, what they save on 64 MB (kStagePays): a context makes them when
-// it has been asked to move that much.  The source of
-// an upload may be reused, and the destination of a download read, when copy_host returns.
-constexpr int kStageThreads = 8;
-constexpr size_t kStagePiece = (size_t)1 << 20;
-constexpr size_t kStageLeast = (size_t)4 << 20;
-constexpr size_t kStagePays = (size_t)64 << 20;
-
+// a transfer between a host array and the device, complete on return
 cudaError_t copy_host(tg_ctx* c, void* dst, const void* src, size_t bytes, bool to_device) {
-  const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-  auto plain = [&]() {
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, c->stream);
-    return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
-  };
-  if (bytes < kStageLeast) return plain();
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, to_device ? src : dst) != cudaSuccess) cudaGetLastError();
-  else if (at.type != cudaMemoryTypeUnregistered) return plain();
-  c->stage_moved += bytes;
-  if (!c->stage) {
-    if (c->stage_moved < kStagePays) return plain();
-    void* p = nullptr;
-    if (cudaMallocHost(&p, 2 * kStageThreads * kStagePiece) != cudaSuccess) {
-      cudaGetLastError();
-      return plain();
-    }
-    c->stage = static_cast<char*>(p);
-    for (auto& ev : c->stage_ev) {
-      const cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-      if (e != cudaSuccess) return e;
-    }
-  }
-  const size_t pieces = (bytes + kStagePiece - 1) / kStagePiece;
-  const int nt = (int)std::min<size_t>(std::min<size_t>(kStageThreads, pieces),
-                                       std::max(1u, std::thread::hardware_concurrency()));
-  std::atomic<int> err{(int)cudaSuccess};
-  auto work = [&](int t) {   // pieces t, t + nt, ..
-    auto fail = [&](cudaError_t e) {
-      if (e == cudaSuccess) return false;
-      err.store((int)e);
-      return true;
-    };
-    if (fail(cudaSetDevice(c->device))) return;
-    char* buf[2] = {c->stage + (size_t)(2 * t) * kStagePiece, c->stage + (size_t)(2 * t + 1) * kStagePiece};
-    cudaEvent_t* ev = c->stage_ev + 2 * t;
-    auto part = [&](size_t i) { return std::min(kStagePiece, bytes - i * kStagePiece); };
-    size_t turn = 0;
-    if (to_device) {
-      for (size_t i = t; i < pieces; i += nt, ++turn) {
-        const int b = (int)(turn & 1);
-        if (turn >= 2 && fail(cudaEventSynchronize(ev[b]))) return;
-        std::memcpy(buf[b], static_cast<const char*>(src) + i * kStagePiece, part(i));
-        if (fail(cudaMemcpyAsync(static_cast<char*>(dst) + i * kStagePiece, buf[b], part(i), kind, c->stream))) return;
-        if (fail(cudaEventRecord(ev[b], c->stream))) return;
-      }
-      for (int b = 0; b < 2 && b < (int)turn; ++b)
-        if (fail(cudaEventSynchronize(ev[b]))) return;
-    } else {
-      auto fetch = [&](size_t i, int b) {
-        return fail(cudaMemcpyAsync(buf[b], static_cast<const char*>(src) + i * kStagePiece, part(i), kind, c->stream)) ||
-               fail(cudaEventRecord(ev[b], c->stream));
-      };
-      if (fetch(t, 0)) return;
-      for (size_t i = t; i < pieces; i += nt, ++turn) {
-        const int b = (int)(turn & 1);
-        if (i + nt < pieces && fetch(i + nt, b ^ 1)) return;
-        if (fail(cudaEventSynchronize(ev[b]))) return;
-        std::memcpy(static_cast<char*>(dst) + i * kStagePiece, buf[b], part(i));
-      }
-    }
-  };
-  std::vector<std::thread> threads;
-  int started = 0;
-  try {
-    threads.reserve(nt);
-    for (int t = 1; t < nt; ++t) {
-      threads.emplace_back(work, t);
-      ++started;
-    }
-  } catch (...) {   // no more threads to be had: their parts are done here
-  }
-  work(0);
-  for (int t = started + 1; t < nt; ++t) work(t);
-  for (auto& th : threads) th.join();
-  if (err.load() != (int)cudaSuccess) cudaStreamSynchronize(c->stream);   // no copy still reads the buffers
-  return (cudaError_t)err.load();
+  return c->stage.copy(c->device, c->stream, dst, src, bytes, to_device);
 }
 
 GreenArgs base_args(tg_ctx* c) {
@@ -1068,9 +974,7 @@ int tg_destroy(tg_ctx* c) {
     cudaEventDestroy(u.second.first);
     cudaEventDestroy(u.second.second);
   }
-  if (c->stage) cudaFreeHost(c->stage);
-  for (cudaEvent_t e : c->stage_ev)
-    if (e) cudaEventDestroy(e);
+  c->stage.release();
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;   // every DevArray member frees what the calls above did not
   return TG_OK;
