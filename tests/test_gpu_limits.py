@@ -1,5 +1,8 @@
-"""Calls where device memory is short, and on Hamiltonians with entries whose squares underflow
-(needs a B200)."""
+"""Calls where device memory is short, from several threads, and on Hamiltonians with entries whose
+squares underflow (needs a B200)."""
+import threading
+import time
+
 import numpy as np
 import pytest
 
@@ -159,3 +162,32 @@ def test_resolvents_of_couplings_that_underflow(shape):
     gj = g.chi0(q, 0.0, s.Ef, s.eta, s.etap)
     g.close()
     assert np.linalg.norm(auto - gj) < 1e-12 * np.linalg.norm(gj)
+
+
+def test_threads_with_different_shared_memory():
+    """Six contexts of one process whose kernels need different amounts of shared memory (dimensions
+    36, 54 and 72, one or two shells of neighbours): every call of every thread is carried out."""
+    from titan_b200.native import GreenGPU
+    errors = []
+
+    def work(shape, n_stages, seconds=3.0):
+        try:
+            s = synthetic.make_system(shape, n_stages=n_stages)
+            g = GreenGPU(0)
+            g.set_system(s)
+            g.set_h0(s.h0(initial_state(s)))
+            kp, z = np.random.default_rng(1).uniform(-2, 2, (4, 3)), s.Ef + 0.1j * np.arange(1, 5)
+            end = time.monotonic() + seconds
+            while time.monotonic() < end:
+                g.eig_batch(kp)
+                g.green_batch(z, kp)
+            g.close()
+        except Exception as ex:
+            errors.append(ex)
+
+    threads = [threading.Thread(target=work, args=a) for a in (("sq2", 1), ("bcc4", 2), ("slab3", 1)) * 2]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors

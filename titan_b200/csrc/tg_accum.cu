@@ -185,7 +185,7 @@ cudaError_t launch_pairs(const GreenArgs& g, const double2* Ga, const double2* G
   if (e != cudaSuccess) return e;
   const dim3 grid(p.grid, p.tiles);
   if (p.staged) {
-    e = cudaFuncSetAttribute(pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    e = allow_smem(pair_kernel<true>, p.smem);
     if (e != cudaSuccess) return e;
     pair_kernel<true><<<grid, p.tpm * p.slots, p.smem, s>>>(g, Ga, Gb, pairs, nlist, npairs, p.tpm, acc);
   } else {

@@ -647,7 +647,7 @@ cudaError_t launch_hh_small(const double2* H, int64_t nk, int n, const int* rows
   if (!hh_small_supported(n) || ns <= 0 || ns > n) return cudaErrorInvalidValue;
   const size_t smem = hh_smem(n);
   const int threads = 32 * hh_warps(n);
-  cudaError_t e = cudaFuncSetAttribute(hh_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(hh_small_kernel, smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hh_small_kernel, threads, smem);
@@ -681,7 +681,7 @@ cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* 
   cudaError_t e = launch_hh_small(H, nk, n, nullptr, n, D, E, U, num_sms, s);
   if (e != cudaSuccess) return e;
   const size_t qsmem = sizeof(double) * 64 * (size_t)n;
-  e = cudaFuncSetAttribute(ql_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsmem);
+  e = allow_smem(ql_kernel, qsmem);
   if (e != cudaSuccess) return e;
   const bool packed = fin_packed(n, optin_smem());
   const size_t fsmem = fin_smem(n, packed);
@@ -690,11 +690,11 @@ cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* 
              : n <= 40         ? eig_finish_kernel<false, 5>
              : n <= 56         ? eig_finish_kernel<false, 7>
                                : eig_finish_kernel<false, kEigFrags>;
-  e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
+  e = allow_smem(fin, fsmem);
   if (e != cudaSuccess) return e;
   const size_t asmem = sizeof(double2) * ((size_t)n * odd_stride(n) + kRotRoom);
   const int athreads = (2 * n + 31) / 32 * 32;
-  e = cudaFuncSetAttribute(eig_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asmem);
+  e = allow_smem(eig_apply_kernel, asmem);
   if (e != cudaSuccess) return e;
   int per_sm = 0, aper_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fin, kFinThreads, fsmem);

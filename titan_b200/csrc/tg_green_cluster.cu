@@ -382,7 +382,7 @@ cudaError_t launch_green_cluster(const GreenArgs& a, int num_sms, cudaStream_t s
   if (((a.n + kPB - 1) / kPB + cs - 1) / cs * kPB > kNLC) return cudaErrorInvalidValue;
   const int threads = (a.n + 31) / 32 * 32;
   const size_t smem = cl_smem(a.n, a.n_neigh).total;
-  cudaError_t e = cudaFuncSetAttribute(green_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(green_cluster_kernel, smem);
   if (e != cudaSuccess) return e;
   if (cs > 8) {
     e = cudaFuncSetAttribute(green_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

@@ -480,7 +480,7 @@ cudaError_t launch_o(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (smem > (size_t)max_smem) return cudaErrorInvalidValue;
   auto kern = green_mma_kernel<N, W, MINB, OUT>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allow_smem(kern, smem);
   if (err != cudaSuccess) return err;
   int per_sm = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * W, smem);

@@ -380,7 +380,7 @@ cudaError_t launch_t3(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid
   const size_t smem = L.per_team * teams;
   if (smem > (size_t)max_smem) return cudaErrorInvalidValue;
   auto kern = green_team_kernel<N, W, TC, OUT>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allow_smem(kern, smem);
   if (err != cudaSuccess) return err;
   const int threads = teams * T::LANES;
   int per_sm = 0;

@@ -4,10 +4,27 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
 namespace tg {
+
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit belongs to the function,
+// for all threads of the process, not to a launch: every call sets the largest that the device allows,
+// so that no thread lowers it between another one's call and launch.
+template <class K>
+inline cudaError_t allow_smem(K kernel, size_t bytes) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes at{};
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, kernel);
+  if (e != cudaSuccess) return e;
+  const int most = optin - (int)at.sharedSizeBytes;
+  if (bytes > (size_t)std::max(most, 0)) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
 
 // ---------------------------------------------------------------------------
 // complex FP64 helpers (double2 = re, im)

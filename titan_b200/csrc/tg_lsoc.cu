@@ -164,7 +164,7 @@ cudaError_t launch_gvg(const double2* G, const double2* V, int n, int64_t np, do
                        cudaStream_t s) {
   if (np <= 0) return cudaSuccess;
   const size_t smem = gvg_smem_bytes(n);
-  cudaError_t e = cudaFuncSetAttribute(gvg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(gvg_kernel, smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gvg_kernel, 256, smem);

@@ -622,7 +622,7 @@ ShePlan she_plan(int n, int dimens, int n_neigh, int n_frags) {
 int she_grid(int n, int dimens, int n_neigh, int n_frags, int num_sms) {
   const ShePlan p = she_plan(n, dimens, n_neigh, n_frags);
   if (p.bytes == 0) return 0;
-  if (cudaFuncSetAttribute(p.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes) != cudaSuccess) return 0;
+  if (allow_smem(p.fn, p.bytes) != cudaSuccess) return 0;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.fn, p.threads, p.bytes) != cudaSuccess) return 0;
   return num_sms * std::max(per_sm, 1);
@@ -663,7 +663,7 @@ cudaError_t launch_she(const SheLaunch& l, cudaStream_t s) {
   a.klist = l.klist;
   const ShePlan p = she_plan(a.n, a.dimens, a.n_neigh, l.n_frags);
   if (p.bytes == 0) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(p.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes);
+  cudaError_t e = allow_smem(p.fn, p.bytes);
   if (e != cudaSuccess) return e;
   if (p.v == SHE_MMA)
     she_mma_kernel<<<l.grid, p.threads, p.bytes, s>>>(a, p.mma, l.n_frags);

@@ -395,7 +395,7 @@ cudaError_t launch_spec_ldos(const double2* U, const double* lam, const double* 
                 : nf <= 6 ? spec_ldos_kernel<6>
                 : nf <= 9 ? spec_ldos_kernel<9>
                           : spec_ldos_kernel<12>;
-  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allow_smem(kernel, smem);
   if (err != cudaSuccess) return err;
   err = cudaMemsetAsync(out, 0, sizeof(double) * (size_t)n_e * n, s);
   if (err != cudaSuccess) return err;
@@ -451,7 +451,7 @@ cudaError_t launch_green_spectral(const GreenArgs& g, const double2* U, const do
       break;
     }
   const size_t smem = spec_smem(g.n, sa.kp, sa.nz);
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = allow_smem(kernel, smem);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSpecThreads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm <= 0) return cudaErrorInvalidValue;

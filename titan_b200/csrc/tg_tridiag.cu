@@ -481,7 +481,7 @@ cudaError_t launch_tridiag(double2* H, int64_t nk, int n, const int* rows, int n
   if (hh_small_supported(n)) return launch_hh_small(H, nk, n, rows, ns, D, E, Q, num_sms, s);
   if (n > 32 * kPanSeg) return cudaErrorInvalidValue;
   const size_t smem = hh_panel_smem(n);
-  cudaError_t e = cudaFuncSetAttribute(hh_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(hh_panel_kernel, smem);
   if (e != cudaSuccess) return e;
   const int64_t grid = std::min<int64_t>(nk, (int64_t)num_sms);
   hh_panel_kernel<<<(unsigned)grid, kPanThreads, smem, s>>>(H, nk, n, rows, ns, D, E, Q);
@@ -494,7 +494,7 @@ template <int FM, int FN>
 cudaError_t launch_tri_tile(const GreenArgs& g, int num_sms, cudaStream_t s) {
   using TT = TriTile<FM, FN>;
   auto kernel = tri_green_kernel<FM, FN>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT::smem);
+  cudaError_t e = allow_smem(kernel, TT::smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTriThreads, TT::smem);
