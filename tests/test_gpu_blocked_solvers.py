@@ -169,3 +169,27 @@ def test_eigensolver_edges(gpu, shape, kind):
         assert np.max(np.abs(U[k].conj().T @ U[k] - np.eye(n))) <= tol
         assert np.max(np.abs((U[k] * lam[k]) @ U[k].conj().T - H[k])) <= tol * h
         assert np.max(np.abs(np.sort(lam[k]) - np.linalg.eigvalsh(H[k]))) <= tol * h
+
+
+@pytest.mark.parametrize("shape,d_only,counts", [("bcc1", False, (9, 19, 29)), ("slab6", True, (9, 21, 31))])
+def test_launches_are_counted(gpu, shape, d_only, counts):
+    """tg_last_timing's number of kernels of chi0 (static; at finite q and frequency, FP64 and split):
+    two per H(k) table; four per eigendecomposition, then one launch per Green function (or pair of
+    operands), or one per tridiagonalisation, then two launches and a gather per operand; the
+    contraction one per axis, in split precision two more per operand and one per axis; the epilogue."""
+    deck = synthetic.make_deck(shape, nk=(3, 3, 3) if shape == "bcc1" else (3, 3, 1), n1gl=4, parts=1, n3gl=3)
+    s = deck.system
+    gpu.setup(deck, s.h0(initial_state(s)))
+    gpu.set_chi_orbitals([list(d) for d in s.dorbs] if d_only else None)
+    x2, p2 = deck.real_points(0.05, s.Ef)
+    q = np.array([0.1, 0.0, 0.0])
+    got = []
+    try:
+        gpu.chi0(0.0 * q, 0.0, s.Ef, s.eta, s.etap)
+        got.append(int(gpu.last_timing()[10]))
+        for precision in ("fp64", "split"):
+            gpu.chi0(q, 0.05, s.Ef, s.eta, s.etap, x2, p2, precision)
+            got.append(int(gpu.last_timing()[10]))
+    finally:
+        gpu.set_chi_orbitals(None)
+    assert tuple(got) == counts

@@ -402,7 +402,8 @@ int build_eig(tg_ctx* c, int slot, int64_t nk) {
   int64_t chunk = 0;
   int rc = ensure_eig_ws(c, nk, chunk);
   if (rc) return rc;
-  KindTimer kt(c, 0);
+  KindTimer kt(c, 0);   // (counts one launch)
+  c->launches += eig_launches(nk, chunk) - 1;
   TG_CHECK(c, launch_eig(c->d_htab[slot].p, nk, c->dimH, c->d_eigU[slot].p, c->d_eigL[slot].p, c->d_eigws.p, chunk,
                          c->d_eig_status.p, c->num_sms, c->stream),
            "eigendecomposition");
@@ -432,8 +433,9 @@ int build_eig_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
     TG_CHECK(c, launch_eig(c->d_hchunk.p, m, (int)n, c->d_eigU[slot].p + k0 * nn, c->d_eigL[slot].p + k0 * n,
                            c->d_eigws.p, std::min(chunk, m), c->d_eig_status.p, c->num_sms, c->stream),
              "eigendecomposition");
-    c->launches += 5;
+    c->launches += 2 + eig_launches(m, chunk);
   }
+  c->launches -= 1;   // (the timer counts one)
   return TG_OK;
 }
 
@@ -479,6 +481,7 @@ int build_tri_chunked(tg_ctx* c, int slot, const double* d_k, int64_t nk, const 
              "tridiagonalisation");
     c->launches += 3;
   }
+  c->launches -= 1;   // (the timer counts one)
   return TG_OK;
 }
 
@@ -2083,12 +2086,12 @@ int imag_pairs(tg_ctx* c, double Ef, double eta, const double* q, const std::vec
   TG_CHECK(c, c->d_acc_red.ensure((size_t)sets * len), "alloc acc");
   int rc = q ? ensure_pass(c, {&c->d_A, &c->d_B}, P) : ensure_pass(c, {&c->d_A}, P);
   if (rc) return rc;
+  profile_begin(c);
   GreenArgs a, b;
   if ((rc = imag_points(c, Ef, eta, q, a, &b))) return rc;
   if (!q) b = a;
   TG_CHECK(c, cudaMemsetAsync(c->d_acc.p, 0, sizeof(double2) * sets * parts * len, s), "memset");
   if ((rc = reset_status(c))) return rc;
-  profile_begin(c);
   a.mode = b.mode = MODE_RAW;
   a.out = c->d_A.p;
   b.out = q ? c->d_B.p : c->d_A.p;

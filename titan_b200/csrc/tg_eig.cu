@@ -668,6 +668,8 @@ size_t eig_ws_bytes(int n, int64_t nk, int64_t chunk) {
          (size_t)nk * n * 2 * sizeof(double) + 256;
 }
 
+int64_t eig_launches(int64_t nk, int64_t chunk) { return nk > 0 ? 1 + 3 * ((nk + chunk - 1) / chunk) : 0; }
+
 cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int64_t chunk,
                        int* status, int num_sms, cudaStream_t s) {
   if (nk <= 0) return cudaSuccess;

@@ -245,6 +245,7 @@ int eig_supported(int n);
 int eig_fast(int n);
 int64_t eig_chunk(int n, int64_t nk);
 size_t eig_ws_bytes(int n, int64_t nk, int64_t chunk);
+int64_t eig_launches(int64_t nk, int64_t chunk);   // kernels of launch_eig
 cudaError_t launch_eig(const double2* H, int64_t nk, int n, double2* U, double* lam, void* ws, int64_t chunk,
                        int* status, int num_sms, cudaStream_t s);
 // Reflector I - tau v v^H of LAPACK's zlarfg that takes the vector (alpha, x) to (beta, 0), from
