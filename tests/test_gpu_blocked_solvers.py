@@ -97,17 +97,33 @@ def test_dyson_at_the_edges_of_its_panels(gpu, n, order):
     assert np.linalg.norm(got - ref) <= 10.0 * n * EPS * np.linalg.cond(M) * np.linalg.norm(ref)
 
 
-def test_dyson_reports_a_singular_system(gpu):
+@pytest.mark.parametrize("n", [1024, 1025, 1300, 1620])
+def test_dyson_exchanges_rows_in_every_panel_kernel(gpu, n):
+    """Random chi and U where panels have up to 1024 rows (a row per thread in registers), up to 1607
+    (shared memory) and more (global memory), with the switches between them inside one solve: the
+    backward error of the solution and its distance from LAPACK's, each within 10 n eps (times the
+    condition)."""
+    rng = np.random.default_rng(n)
+    x, u = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) for _ in range(2))
+    got = gpu.dyson(x, u)
+    M = np.eye(n) + x @ u
+    assert np.linalg.norm(M @ got - x) <= 10.0 * n * EPS * np.linalg.norm(M) * np.linalg.norm(got)
+    ref = np.linalg.solve(M, x)
+    assert np.linalg.norm(got - ref) <= 10.0 * n * EPS * np.linalg.cond(M, 1) * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [70, 1300, 1700])   # column 67 in a panel of each of the three kernels
+def test_dyson_reports_a_singular_system(gpu, n):
     from titan_b200.native import TitanGPUError
-    x = np.eye(70, dtype=complex)
-    u = -np.eye(70, dtype=complex)
+    x = np.eye(n, dtype=complex)
+    u = -np.eye(n, dtype=complex)
     with pytest.raises(TitanGPUError) as err:
-        gpu.dyson(x, 0.5 * u - 0.5 * np.diag(np.arange(70) == 66))
+        gpu.dyson(x, 0.5 * u - 0.5 * np.diag(np.arange(n) == 66))
     assert err.value.code == 67
 
 
-@pytest.mark.parametrize("shape,nk,n_neighbour_stages", [("bcc1", (2, 3, 2), 2), ("sq2", (3, 2, 1), 1), ("slab3", (2, 2, 1), 2)])
-def test_disturbance_fragments(gpu, shape, nk, n_neighbour_stages):
+@pytest.mark.parametrize("shape,nk", [("bcc1", (2, 3, 2)), ("sq2", (3, 2, 1)), ("slab3", (2, 2, 1))])
+def test_disturbance_fragments(gpu, shape, nk):
     """The vertex products in 8 x 8 fragments: one site (25 fragments for eight warps, a last column
     block of two orbitals), two sites (50), and three (75, more than the warps hold: the staged
     kernel).  Both axes, one after the other into the same sums, q and frequency nonzero; within
@@ -124,10 +140,10 @@ def test_disturbance_fragments(gpu, shape, nk, n_neighbour_stages):
 
 
 # 60 of 108 rows (tiles of 64 x 64), all 126 rows (128 x 64; no multiple of the reduction's panels
-# of 8), 50 of 90 rows (reduction in shared memory)
-@pytest.mark.parametrize("shape,d_only", [("slab6", True), ("slab7", False), ("slab5", True)])
+# of 8), 50 of 90 rows (64 x 64, reduction in shared memory), all 90 rows (96 x 96)
+@pytest.mark.parametrize("shape,d_only", [("slab6", True), ("slab7", False), ("slab5", True), ("slab5", False)])
 def test_tridiagonal_tiles_equal_gauss_jordan(gpu, shape, d_only):
-    """chi0 from tridiagonalised Green functions at every tile shape of their products equals the
+    """chi0 from tridiagonalised Green functions at the tile shapes of their products equals the
     Gauss-Jordan path to 1e-12, the bound of the plain test (which has the 160 x 80 tiles)."""
     deck = synthetic.make_deck(shape, nk=(2, 2, 1), n1gl=3, parts=1, n3gl=3)
     s = deck.system

@@ -35,11 +35,12 @@ def test_nb_ldos_golden_through_gpu(gpu, method):
     np.testing.assert_allclose(dn[:, 0], md[:, 1:], rtol=2e-9, atol=0)
 
 
-@pytest.mark.parametrize("shape", ["bcc1", "sq2", "bcc4"])
-def test_ldos_matches_oracle(gpu, shape):
-    """Spectral and Gauss-Jordan LDOS against the oracle on seeded cells (dimH 18, 36, 72),
-    energies across the bands, eta = 1e-3."""
-    deck = synthetic.make_deck(shape, nk=(6, 6, 6) if shape != "sq2" else (12, 12, 1), n1gl=4, parts=1, n3gl=4)
+@pytest.mark.parametrize("shape,nk", [("bcc1", (6, 6, 6)), ("sq2", (12, 12, 1)), ("bcc4", (6, 6, 6)),
+                                      ("slab5", (5, 5, 1))])
+def test_ldos_matches_oracle(gpu, shape, nk):
+    """Spectral and Gauss-Jordan LDOS against the oracle on seeded cells (dimH 18, 36, 72, 90: the
+    last with the packed post-pass of the eigensolver), energies across the bands, eta = 1e-3."""
+    deck = synthetic.make_deck(shape, nk=nk, n1gl=4, parts=1, n3gl=4)
     s = deck.system
     h0 = s.h0(initial_state(s))
     gpu.setup(deck, h0)
