@@ -107,3 +107,37 @@ def test_two_pass_chi0_equals_single_pass_shards(gpu, precision, tol):
         gpu.setup(deck, s.h0(initial_state(s)))
         ref = gpu.chi0(q, e, s.Ef, s.eta, s.etap, x2, p2, precision="fp64")
         assert rel(full, ref) < 1e-9
+
+
+@pytest.mark.parametrize("norbs", [(2,), (4,), (4, 4), (5, 5), (9,), (9, 9), (5, 5, 5, 5), (9, 9, 9), (9,) * 4,
+                                   (9,) * 5, (9,) * 6], ids=lambda x: "dim%d" % (2 * sum(x)))
+def test_hamiltonian_that_is_not_a_number_is_an_error(norbs):
+    """One NaN on the diagonal, and NaN alone, at every dimension of the inversion kernels: no row is
+    a pivot by size, the point is reported as singular, and the context goes on working."""
+    from types import SimpleNamespace
+
+    from titan_b200.native import GreenGPU
+    nat, n = len(norbs), 2 * sum(norbs)
+    s = SimpleNamespace(n_atoms=nat, norbs=norbs, dimH=n, dimens=4 * sum(x * x for x in norbs))
+    s.neighbor_table = lambda: (np.zeros((1, 3)), np.zeros(1, np.int32), np.zeros((1, nat), np.int32),
+                                np.zeros((1, nat, max(norbs), max(norbs)), complex))
+    rng = np.random.default_rng(n)
+    h = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    h = h + h.conj().T
+    one = h.copy()
+    one[0, 0] = np.nan
+    z, kp = np.full(3, 0.1 + 0.2j), np.zeros((3, 3))
+    want = np.linalg.inv(z[0] * np.eye(n) - h)
+    g = GreenGPU(0)
+    try:
+        g.set_system(s)
+        for bad in (one, np.full((n, n), np.nan + 0j)):
+            g.set_h0(bad)
+            with pytest.raises(TitanGPUError) as ex:
+                g.green_batch(z, kp)
+            assert ex.value.code == 1   # the first point
+            g.set_h0(h)
+            for G in g.green_batch(z, kp):
+                assert np.max(np.abs(G - want)) <= 1e-12 * n * np.max(np.abs(want))
+    finally:
+        g.close()

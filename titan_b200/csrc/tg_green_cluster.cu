@@ -100,7 +100,8 @@ __device__ __forceinline__ void factor_panel(ClState& st, double2* blk, int s0, 
     if (j < nb) {
       const double2 v = x[j];
       if (t < n) F[(size_t)j * n + t] = v;
-      double best = (t < n && !st.used) ? fabs(v.x) + fabs(v.y) : -1.0;
+      // (NaN counts as zero: every lane compares alike, and there is a pivot row for every column)
+      double best = (t < n && !st.used) ? fmax(fabs(v.x) + fabs(v.y), 0.0) : -1.0;
       int bi = t;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
@@ -133,7 +134,7 @@ __device__ __forceinline__ void factor_panel(ClState& st, double2* blk, int s0, 
       }
       const double2* pr = candrow + (size_t)(pb * kMaxWarps + wbest) * (kPB + 1) + 1;
       const double2 pv = pr[j];
-      if (pv.x == 0.0 && pv.y == 0.0 && t == 0) atomicMin(status, (int)(point + 1));
+      if (!(vb > 0.0) && t == 0) atomicMin(status, (int)(point + 1));
       const double2 inv = crecip_fast(pv);
       if (t == 0) {
         INV[j] = inv;

@@ -217,7 +217,8 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
 #pragma unroll
           for (int rr = 0; rr < RB; ++rr) {
             const int r = tr + TR * rr;
-            const double v = fabs(A[rr][kk].x) + fabs(A[rr][kk].y);
+            // (NaN counts as zero: there is a pivot row, a valid index, for every column)
+            const double v = fmax(fabs(A[rr][kk].x) + fabs(A[rr][kk].y), 0.0);
             if (r < N && !((used >> rr) & 1u) && (v > best || (v == best && r < brow))) {
               best = v;
               brow = r;
