@@ -438,7 +438,7 @@ def run_ours(args, rank, world, local_rank):
     ns = sum(2 * len(o) for o in sel) if sel is not None else s.dimH
     tri_name = (("hh_small_kernel" if s.dimH <= 96 else "hh_panel_kernel") + " + tri_green_kernel (Householder tridiagonalisation per k, G over the %d rows "
                 "of chi per point: tridiagonal solves + FP64 DMMA GEMM) + gather_kernel" % ns)
-    gj_name = (("green_team_kernel" if s.dimH in (4, 8, 16, 20) else "green_mma_kernel") +
+    gj_name = (("green_warp_kernel" if s.dimH in (4, 8, 16, 20) else "green_mma_kernel") +
                " (fused H(k) + Gauss-Jordan)" if native_n else
                "green_cluster_kernel (thread-block-cluster Gauss-Jordan) + gather_kernel")
     kname = ("hh_small / ql / eig_apply / eig_finish + spec_green_kernel (spectral G, FP64 DMMA)" if spectral else

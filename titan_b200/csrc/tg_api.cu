@@ -568,13 +568,12 @@ int build_chi_layout(tg_ctx* c, const std::vector<std::vector<int>>& orbs, ChiLa
   auto row_of = [&](int i, int x) { return c->ia[i] + (x / L.nc[i]) * c->norb[i] + orbs[i][x % L.nc[i]]; };
   int aoff = 0;
   int64_t coff = 0;
-  for (int i = 0; i < nat; ++i)
-    for (int j = 0; j < nat; ++j) L.pair_M[i * nat + j] = 4 * L.nc[i] * L.nc[j];
   const int T = gemm64_tile();
   for (int i = 0; i < nat; ++i)
     for (int j = 0; j < nat; ++j) {
       const int p = i * nat + j;
-      const int M = L.pair_M[p];
+      const int M = 4 * L.nc[i] * L.nc[j];
+      L.pair_M[p] = M;
       L.pair_aoff[p] = aoff;
       L.pair_coff[p] = coff;
       const int ni2 = 2 * L.nc[i], nj2 = 2 * L.nc[j];
@@ -1067,13 +1066,12 @@ int tg_set_system(tg_ctx* c, int n_atoms, const int* norb, int norb_max, int n_n
   int aoff = 0;
   int64_t coff = 0;
   c->tiles.clear();
-  for (int i = 0; i < n_atoms; ++i)
-    for (int j = 0; j < n_atoms; ++j) c->pair_M[i * n_atoms + j] = 4 * c->norb[i] * c->norb[j];
   const int T = gemm64_tile();
   for (int i = 0; i < n_atoms; ++i)
     for (int j = 0; j < n_atoms; ++j) {
       const int p = i * n_atoms + j;
-      const int M = c->pair_M[p];
+      const int M = 4 * c->norb[i] * c->norb[j];
+      c->pair_M[p] = M;
       c->pair_aoff[p] = aoff;
       c->pair_coff[p] = coff;
       const int ni2 = 2 * c->norb[i], nj2 = 2 * c->norb[j];
@@ -1969,10 +1967,6 @@ int tg_profile(tg_ctx* c, int enable) {
 
 namespace {
 
-struct PairRef {
-  int block;   // output block of an orbital pair
-};
-
 // room for the H(k) tables of nk points in slots 0 .. slots - 1; without it both are given back and
 // the inversion kernels form H(k) themselves
 bool htab_room(tg_ctx* c, int slots, int64_t nk) {
@@ -2227,8 +2221,8 @@ int tg_gg_tensor(tg_ctx* c, double Ef, double eta, int orbital_resolved, const i
   }
   // every orbital pair (row orbital of any site, column orbital of any site) is summed on the
   // device; the groups of several orbitals are added up here
-  std::vector<PairRef> refs;
   std::vector<int4> pairs;
+  std::vector<int> block;   // output block of a pair
   for (int i = 0; i < nat; ++i)
     for (int j = 0; j < nat; ++j)
       for (int h = 0; h < (int)colg[j].size(); ++h)
@@ -2237,15 +2231,15 @@ int tg_gg_tensor(tg_ctx* c, double Ef, double eta, int orbital_resolved, const i
             for (int mu : rowg[i][g]) {
               pairs.push_back(make_int4(c->ia[i] + mu, c->ia[i] + c->norb[i] + mu, c->ia[j] + nu,
                                         c->ia[j] + c->norb[j] + nu));
-              refs.push_back(PairRef{((i * nat + j) * nrow + g) * ncol + h});
+              block.push_back(((i * nat + j) * nrow + g) * ncol + h);
             }
   std::vector<double2> h;
   if ((rc = imag_pairs(c, Ef, eta, nullptr, pairs, h, nullptr))) return rc;
   const size_t total = (size_t)nat * nat * nrow * ncol * 16;
   std::memset(T, 0, sizeof(double) * 2 * total);
-  for (size_t b = 0; b < refs.size(); ++b)
+  for (size_t b = 0; b < block.size(); ++b)
     for (int q = 0; q < 16; ++q) {
-      const size_t dst = (size_t)refs[b].block * 16 + q;
+      const size_t dst = (size_t)block[b] * 16 + q;
       T[2 * dst] += h[16 * b + q].x;
       T[2 * dst + 1] += h[16 * b + q].y;
     }
@@ -2931,7 +2925,6 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
   l.tab = c->d_she_tab.p;
   l.ia = c->d_ia.p;
   l.norb = c->d_norb.p;
-  l.decode = c->d_decode.p;
   l.ztiles = c->d_she_ztiles.p;
   l.n_ztiles = n_ztiles;
   l.n_frags = n_frags;
@@ -3060,7 +3053,7 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
 // For callers that cannot let a library call allocate device memory: a host
 // that hands the GPU's memory to its own pool or to another solver up front and
 // budgets every byte of HBM itself, so that a cudaMalloc inside a library call
-// would fail or break that budget.  tg_expectation allocates its per-team
+// would fail or break that budget.  tg_expectation allocates its
 // partial sums (and an H(k) table) on first use; this variant keeps the partial
 // sums in a fixed 8 MiB device array compiled into the library and sums H(k)
 // inside the inversion kernel instead of tabulating it.
@@ -3113,8 +3106,7 @@ extern "C" int tg_expectation_noalloc(tg_ctx* c, double Ef, double eta, double* 
   if (!rho || !mx || !my || !mz || !mp) return set_err(c, TG_ERR_ARG, "tg_expectation_noalloc: null output");
   const int n = c->dimH;
   const int len = 2 * n;
-  // partial slots: the team kernel runs at most 15 teams per SM (per-SM CTAs x teams <= 8 + teams - 1),
-  // the blocked one green_max_ctas
+  // partial slots: the one-warp kernel runs at most 15 matrices per SM, the blocked one green_max_ctas
   const size_t slots = (size_t)c->num_sms * (green_max_ctas(n) + 1);
   const size_t need = (slots + 1) * (size_t)len * sizeof(double2);
   if (!green_supported(n))

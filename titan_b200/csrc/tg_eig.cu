@@ -321,8 +321,7 @@ template <bool PACKED>
 struct HermA {
   double2* a;
   int n, S;
-  __device__ __forceinline__ double2 get(int i, int j) const {
-    if (!PACKED) return a[i * S + j];
+  __device__ __forceinline__ double2 get(int i, int j) const {   // (PACKED)
     return i <= j ? a[j * (j + 1) / 2 + i] : cconj(a[i * (i + 1) / 2 + j]);
   }
   __host__ __device__ static int entries(int n) { return PACKED ? n * (n + 1) / 2 : n * n; }

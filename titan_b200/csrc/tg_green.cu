@@ -3,7 +3,7 @@
 //     (tg_spectral.cu) where the launch carries one;
 //   * else an inversion per (k, z) point, replacing invers = zgetrf + zgetri
 //     (mod_tools.F90:796-829): blocked Gauss-Jordan on the FP64 tensor cores
-//     (tg_green_mma.cu) for the dimensions it is instantiated for; the one-warp team kernel
+//     (tg_green_mma.cu) for the dimensions it is instantiated for; the one-warp kernel
 //     (tg_green_warp.cu) for dimensions of at most 20, whose panels would be mostly padding;
 //     the thread-block-cluster kernel (tg_green_cluster.cu) for every other one up to 288.
 #include "tg_internal.cuh"

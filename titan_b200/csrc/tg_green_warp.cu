@@ -1,56 +1,53 @@
-// Team-per-matrix fused H(k) + complex Gauss-Jordan inversion, FP64.
+// Warp-per-matrix fused H(k) + complex Gauss-Jordan inversion, FP64, for dimensions 4, 8, 16, 20.
 //
-// A team of W warps (32 W lanes) owns one (k, z) matrix at a time.  Lanes
-// form a TR x TC grid (TR * TC = 32 W, TC = 8 or 16 divides 32); lane
-// (tr, tc) keeps rows r = tr + TR*rr and columns c = tc + TC*cc in registers
-// (cyclic distribution, padded slots are an inert identity).  Per elimination
-// step k = tck + TC*kk (slot kk compile-time, lane column tck runtime):
-//   * the lanes owning column k pick the largest |Re|+|Im| among the rows not
-//     yet used (the zgetrf/izamax choice): shuffles inside each warp, shared
-//     memory + one named barrier across the team's warps;
-//   * the owners of row p publish the scaled pivot row a_p/a_pk, the owners of
-//     column k the multipliers (a_pk - 1 for row p itself, so the update below
-//     needs no branch), both in team-private shared memory, double-buffered by
-//     step parity: one more barrier (W > 1) or __syncwarp (W = 1) per step;
+// A warp owns one (k, z) matrix at a time.  Its lanes form a 4 x 8 grid; lane (tr, tc) keeps rows
+// r = tr + 4 rr and columns c = tc + 8 cc in registers (cyclic distribution, padded slots are an
+// inert identity).  Per elimination step k = tck + 8 kk (slot kk compile-time, lane column tck
+// runtime):
+//   * the lanes owning column k pick the largest |Re|+|Im| among the rows not yet used (the
+//     zgetrf/izamax choice) by shuffles;
+//   * the owners of row p publish the scaled pivot row a_p/a_pk, the owners of column k the
+//     multipliers (a_pk - 1 for row p itself, so the update below needs no branch), both in the
+//     warp's shared memory, double-buffered by step parity: one __syncwarp per step;
 //   * every lane applies  a <- a - f * pvd  to its register block.
-// Rows are never swapped; G[r][s] = X[piv[r]][pinv[s]] is applied when the
-// result leaves through the output stage.  Teams are persistent and
-// independent; H(k) comes either from a precomputed table (k-major walk,
-// so each table row is reused from L2 across energies) or is summed here.
+// Rows are never swapped; G[r][s] = X[piv[r]][pinv[s]] is applied when the result leaves through
+// the output stage.  The warps are persistent and independent; H(k) comes either from a
+// precomputed table (k-major walk, so each table row is reused from L2 across energies) or is
+// summed here.
 #include "tg_internal.cuh"
 
 namespace tg {
 
 namespace {
 
-template <int N, int W, int TC>
-struct Team {
-  static constexpr int LANES = 32 * W;
-  static constexpr int TR = LANES / TC;
+constexpr int kWarps = 8;        // largest number of matrices of a CTA
+constexpr int TR = 4, TC = 8;    // lane grid
+
+template <int N>
+struct WarpDim {
   static constexpr int RB = (N + TR - 1) / TR;
   static constexpr int CB = (N + TC - 1) / TC;
   static constexpr int NR = TR * RB;
   static constexpr int NC = TC * CB;
 };
 
-struct TeamSmem {
-  size_t stage, bufs, cand, phase, piv, pinv, zw, acc, per_team;
+struct WarpSmem {
+  size_t stage, bufs, phase, piv, pinv, zw, acc, per_warp;
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15); }
 
-__host__ __device__ inline TeamSmem team_smem(int n, int nr, int nc, int w, int n_neigh) {
-  TeamSmem L;
+__host__ __device__ inline WarpSmem warp_smem(int n, int nr, int nc, int n_neigh) {
+  WarpSmem L;
   size_t o = 0;
   L.stage = o; o = al16(o + sizeof(double2) * (size_t)n * n);
   L.bufs = o;  o = al16(o + sizeof(double2) * 2 * (size_t)(nr + nc));
-  L.cand = o;  o = al16(o + sizeof(double2) * 2 * 2 * (size_t)w);        // [buf][warp] {value,row}, pivot
   L.phase = o; o = al16(o + sizeof(double2) * (size_t)(n_neigh > 0 ? n_neigh : 1));
   L.piv = o;   o = al16(o + sizeof(int) * (size_t)n);
   L.pinv = o;  o = al16(o + sizeof(int) * (size_t)n);
   L.zw = o;    o = al16(o + sizeof(double) * 8);
   L.acc = o;   o = al16(o + sizeof(double2) * 2 * (size_t)n);           // MODE_EXPECT sums (4 per orbital)
-  L.per_team = o;
+  L.per_warp = o;
   return L;
 }
 
@@ -60,49 +57,35 @@ __device__ __forceinline__ double2 shfl_d2(double2 v, int src) {
   return v;
 }
 
-template <int W>
-__device__ __forceinline__ void team_sync(int team) {
-  if (W == 1) {
-    __syncwarp();
-  } else {
-    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * W) : "memory");
-  }
-}
-
 // OUT: 0 = operand / raw outputs, 1 = MODE_EXPECT, 2 = MODE_HK
-template <int N, int W, int TC, int OUT>
-__global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
-  using T = Team<N, W, TC>;
-  constexpr int TR = T::TR, RB = T::RB, CB = T::CB, NR = T::NR, NC = T::NC, LANES = T::LANES;
+template <int N, int OUT>
+__global__ void __launch_bounds__(32 * kWarps, 1) green_warp_kernel(GreenArgs a) {
+  using D = WarpDim<N>;
+  constexpr int RB = D::RB, CB = D::CB, NR = D::NR, NC = D::NC;
   extern __shared__ __align__(16) unsigned char smem[];
-  const TeamSmem L = team_smem(N, NR, NC, W, a.n_neigh);
-  const int teams = blockDim.x / LANES;
-  const int team = threadIdx.x / LANES;
-  const int tl = threadIdx.x % LANES;          // lane within the team
-  const int lane = threadIdx.x & 31;
-  const int wt = tl >> 5;                      // warp within the team
-  unsigned char* base = smem + (size_t)team * L.per_team;
+  const WarpSmem L = warp_smem(N, NR, NC, a.n_neigh);
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char* base = smem + (size_t)warp * L.per_warp;
   double2* X = reinterpret_cast<double2*>(base + L.stage);
   double2* bufs = reinterpret_cast<double2*>(base + L.bufs);
-  double2* cand = reinterpret_cast<double2*>(base + L.cand);
   double2* phase = reinterpret_cast<double2*>(base + L.phase);
   int* piv = reinterpret_cast<int*>(base + L.piv);
   int* pinv = reinterpret_cast<int*>(base + L.pinv);
   double* zw = reinterpret_cast<double*>(base + L.zw);
   double2* eacc = reinterpret_cast<double2*>(base + L.acc);
-  const int tr = tl / TC, tc = tl % TC;
+  const int tr = lane / TC, tc = lane % TC;
 
   if (OUT == 1) {
-    for (int e = tl; e < 2 * N; e += LANES) eacc[e] = make_double2(0, 0);
+    for (int e = lane; e < 2 * N; e += 32) eacc[e] = make_double2(0, 0);
   }
-  team_sync<W>(team);
+  __syncwarp();
 
-  const int64_t nteams = (int64_t)gridDim.x * teams;
-  for (int64_t pl = (int64_t)blockIdx.x * teams + team; pl < a.np; pl += nteams) {
+  const int64_t nwarps = (int64_t)gridDim.x * warps;
+  for (int64_t pl = (int64_t)blockIdx.x * warps + warp; pl < a.np; pl += nwarps) {
     // ---- point data ------------------------------------------------------------
     int64_t ktab = -1;
     if (a.htab) ktab = (a.p0 + pl) / a.n_e;
-    if (tl == 0) {
+    if (lane == 0) {
       double zr, zi, kx = 0, ky = 0, kz = 0, w;
       if (a.htab) {
         const int64_t wi = a.p0 + pl;
@@ -138,16 +121,16 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
       }
       zw[0] = zr; zw[1] = zi; zw[2] = kx + a.q[0]; zw[3] = ky + a.q[1]; zw[4] = kz + a.q[2]; zw[5] = w;
     }
-    team_sync<W>(team);
+    __syncwarp();
     if (ktab < 0) {
       const double kx = zw[2], ky = zw[3], kz = zw[4];
-      for (int nb = tl; nb < a.n_neigh; nb += LANES) {
+      for (int nb = lane; nb < a.n_neigh; nb += 32) {
         const double th = kx * a.R[3 * nb] + ky * a.R[3 * nb + 1] + kz * a.R[3 * nb + 2];
         double s, c;
         sincos(th, &s, &c);
         phase[nb] = make_double2(c, s);
       }
-      team_sync<W>(team);
+      __syncwarp();
     }
 
     // ---- A = z 1 - H(k) into registers ------------------------------------------
@@ -195,12 +178,13 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
             a.out[pl * N * N + (size_t)c * N + r] = make_double2(-v.x, -v.y);
           }
         }
-      team_sync<W>(team);
+      __syncwarp();
       continue;
     }
 
     // ---- Gauss-Jordan with implicit partial pivoting -----------------------------
     unsigned used = 0u;     // bit rr: row tr + TR*rr already used as a pivot row
+    for (int k = lane; k < N; k += 32) pinv[k] = k;   // (stays valid where rows are used twice, see below)
     bool singular = false;
 #pragma unroll
     for (int kk = 0; kk < CB; ++kk) {
@@ -217,8 +201,7 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
 #pragma unroll
           for (int rr = 0; rr < RB; ++rr) {
             const int r = tr + TR * rr;
-            // (NaN counts as zero: there is a pivot row, a valid index, for every column)
-            const double v = fmax(fabs(A[rr][kk].x) + fabs(A[rr][kk].y), 0.0);
+            const double v = fabs(A[rr][kk].x) + fabs(A[rr][kk].y);
             if (r < N && !((used >> rr) & 1u) && (v > best || (v == best && r < brow))) {
               best = v;
               brow = r;
@@ -226,7 +209,7 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
             }
           }
         }
-        // reduce over the lanes of lane column tck inside this warp
+        // reduce over the lanes of lane column tck
 #pragma unroll
         for (int m = TC; m < 32; m <<= 1) {
           const double ob = __shfl_xor_sync(0xffffffffu, best, m);
@@ -238,32 +221,10 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
             bval = oval;
           }
         }
-        int p;
-        double2 apk = make_double2(0, 0);
-        if (W == 1) {
-          best = __shfl_sync(0xffffffffu, best, tck);
-          p = __shfl_sync(0xffffffffu, brow, tck);
-          apk = shfl_d2(bval, tck);
-        } else {
-          double2* cb = cand + buf * 2 * W;
-          if (lane == tck) {
-            cb[2 * wt] = make_double2(best, __longlong_as_double((long long)brow));
-            cb[2 * wt + 1] = bval;
-          }
-          team_sync<W>(team);
-          best = -1.0;
-          p = 0x7fffffff;
-#pragma unroll
-          for (int ww = 0; ww < W; ++ww) {
-            const double2 e = cb[2 * ww];
-            const int row = (int)__double_as_longlong(e.y);
-            if (e.x > best || (e.x == best && row < p)) {
-              best = e.x;
-              p = row;
-              apk = cb[2 * ww + 1];
-            }
-          }
-        }
+        best = __shfl_sync(0xffffffffu, best, tck);
+        // (a column of nothing but NaN: any row will do, the point is flagged and its result not used)
+        const int p = min(__shfl_sync(0xffffffffu, brow, tck), N - 1);
+        const double2 apk = shfl_d2(bval, tck);
         if (!(best > 0.0)) singular = true;
         const double2 d = crecip_fast(apk);
         const int ptr = p % TR, prr = p / TR;
@@ -289,8 +250,8 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
             fcol[r] = f;
           }
         }
-        if (tl == 0) piv[k] = p;
-        team_sync<W>(team);
+        if (lane == 0) piv[k] = p;
+        __syncwarp();
         double2 pv[CB];
 #pragma unroll
         for (int cc = 0; cc < CB; ++cc) pv[cc] = pvd[tc + TC * cc];
@@ -304,7 +265,7 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
         }
       }
     }
-    if (tl == 0 && singular && a.status) {
+    if (lane == 0 && singular && a.status) {
       const int64_t pidx = a.p0 + pl + 1;
       atomicMin(a.status, (int)(pidx < 0x7fffffff ? pidx : 0x7fffffff));
     }
@@ -316,9 +277,9 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
         const int r = tr + TR * rr, c = tc + TC * cc;
         if (r < N && c < N) X[r * N + c] = A[rr][cc];
       }
-    team_sync<W>(team);
-    for (int k = tl; k < N; k += LANES) pinv[piv[k]] = k;
-    team_sync<W>(team);
+    __syncwarp();
+    for (int k = lane; k < N; k += 32) pinv[piv[k]] = k;
+    __syncwarp();
 
     // ---- output stage -----------------------------------------------------------
     const int NN = N * N;
@@ -328,7 +289,7 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
       for (int slot = 0; slot < nout; ++slot) {
         const int mode = slot == 0 ? a.mode : a.mode2;
         double2* dst = (slot == 0 ? a.out : a.out2) + pl * (int64_t)NN;
-        for (int o = tl; o < NN; o += LANES) {
+        for (int o = lane; o < NN; o += 32) {
           double2 v;
           if (mode == MODE_RAW) {
             const int r = o % N, c = o / N;
@@ -350,7 +311,7 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
         }
       }
     } else if (OUT == 1) {
-      for (int o = tl; o < N / 2; o += LANES) {
+      for (int o = lane; o < N / 2; o += 32) {
         const int ru = a.exp_rows[2 * o], rd = a.exp_rows[2 * o + 1];
         eacc[4 * o + 0] = cadd(eacc[4 * o + 0], cscale(X[piv[ru] * N + pinv[ru]], w));
         eacc[4 * o + 1] = cadd(eacc[4 * o + 1], cscale(X[piv[rd] * N + pinv[rd]], w));
@@ -358,57 +319,57 @@ __global__ void __launch_bounds__(256, 1) green_team_kernel(GreenArgs a) {
         eacc[4 * o + 3] = cadd(eacc[4 * o + 3], cscale(X[piv[rd] * N + pinv[ru]], w));
       }
     }
-    team_sync<W>(team);
+    __syncwarp();
   }
 
   if (OUT == 1) {
-    team_sync<W>(team);
-    double2* dst = a.acc + ((size_t)blockIdx.x * teams + team) * (2 * N);
-    for (int e = tl; e < 2 * N; e += LANES) dst[e] = eacc[e];
+    __syncwarp();
+    double2* dst = a.acc + ((size_t)blockIdx.x * warps + warp) * (2 * N);
+    for (int e = lane; e < 2 * N; e += 32) dst[e] = eacc[e];
   }
 }
 
-template <int N, int W, int TC, int OUT>
-cudaError_t launch_t3(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used) {
-  using T = Team<N, W, TC>;
-  const TeamSmem L = team_smem(N, T::NR, T::NC, W, a.n_neigh);
+template <int N, int OUT>
+cudaError_t launch_o(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used) {
+  using D = WarpDim<N>;
+  const WarpSmem L = warp_smem(N, D::NR, D::NC, a.n_neigh);
   int dev = 0;
   cudaGetDevice(&dev);
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  int teams = 256 / T::LANES;
-  while (teams > 1 && L.per_team * teams > (size_t)max_smem) --teams;
-  const size_t smem = L.per_team * teams;
+  int warps = kWarps;
+  while (warps > 1 && L.per_warp * warps > (size_t)max_smem) --warps;
+  const size_t smem = L.per_warp * warps;
   if (smem > (size_t)max_smem) return cudaErrorInvalidValue;
-  auto kern = green_team_kernel<N, W, TC, OUT>;
+  auto kern = green_warp_kernel<N, OUT>;
   cudaError_t err = allow_smem(kern, smem);
   if (err != cudaSuccess) return err;
-  const int threads = teams * T::LANES;
+  const int threads = 32 * warps;
   int per_sm = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
   if (err != cudaSuccess) return err;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  if (per_sm * teams > 8) per_sm = (8 + teams - 1) / teams;   // partial buffers: <= 8 teams per SM
-  if (per_sm < 1) per_sm = 1;
+  // partial sums of MODE_EXPECT: at most 8 + warps - 1 matrices per SM at a time
+  if (per_sm * warps > kWarps) per_sm = (kWarps + warps - 1) / warps;
   int64_t grid = (int64_t)num_sms * per_sm;
-  const int64_t need = (a.np + teams - 1) / teams;
+  const int64_t need = (a.np + warps - 1) / warps;
   if (grid > need) grid = need;
   if (grid < 1) grid = 1;
-  if (grid_used) *grid_used = (int)grid * teams;   // partial slots (one per team)
+  if (grid_used) *grid_used = (int)grid * warps;   // partial slots (one per warp)
   kern<<<(unsigned)grid, threads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
-template <int N, int W, int TC>
-cudaError_t launch_t(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used) {
-  if (a.mode == MODE_EXPECT) return launch_t3<N, W, TC, 1>(a, num_sms, s, grid_used);
-  if (a.mode == MODE_HK) return launch_t3<N, W, TC, 2>(a, num_sms, s, grid_used);
-  return launch_t3<N, W, TC, 0>(a, num_sms, s, grid_used);
+template <int N>
+cudaError_t launch_n(const GreenArgs& a, int num_sms, cudaStream_t s, int* grid_used) {
+  if (a.mode == MODE_EXPECT) return launch_o<N, 1>(a, num_sms, s, grid_used);
+  if (a.mode == MODE_HK) return launch_o<N, 2>(a, num_sms, s, grid_used);
+  return launch_o<N, 0>(a, num_sms, s, grid_used);
 }
 
 }  // namespace
 
-// Team-per-matrix path: raw / operand / expectation / H(k) modes.
+// Warp-per-matrix path: raw / operand / expectation / H(k) modes.
 int green_warp_supported(int n, int mode) {
   const bool nok = n == 4 || n == 8 || n == 16 || n == 20;
   const bool mok = mode == MODE_RAW || mode == MODE_A_IMAG || mode == MODE_B_IMAG || mode == MODE_A_REAL ||
@@ -422,10 +383,10 @@ cudaError_t launch_green_warp(const GreenArgs& a, int num_sms, cudaStream_t s, i
     return cudaSuccess;
   }
   switch (a.n) {
-    case 4: return launch_t<4, 1, 8>(a, num_sms, s, grid_used);
-    case 8: return launch_t<8, 1, 8>(a, num_sms, s, grid_used);
-    case 16: return launch_t<16, 1, 8>(a, num_sms, s, grid_used);
-    case 20: return launch_t<20, 1, 8>(a, num_sms, s, grid_used);
+    case 4: return launch_n<4>(a, num_sms, s, grid_used);
+    case 8: return launch_n<8>(a, num_sms, s, grid_used);
+    case 16: return launch_n<16>(a, num_sms, s, grid_used);
+    case 20: return launch_n<20>(a, num_sms, s, grid_used);
   }
   return cudaErrorInvalidValue;
 }

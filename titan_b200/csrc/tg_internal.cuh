@@ -331,7 +331,6 @@ struct SheLaunch {
   const int* tab = nullptr;       // [4][n / 2]
   const int* ia = nullptr;
   const int* norb = nullptr;
-  const int* decode = nullptr;
   // register-tiled second stage: 3 x 3 tiles of the (sigma, s', site) output blocks, code
   // sigma | s' << 2 | site << 4 | x0 << 14 | y0 << 20, and the first df row of each site
   const int* ztiles = nullptr;

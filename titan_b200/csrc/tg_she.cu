@@ -45,7 +45,6 @@ struct SheArgs {
   const int* tab = nullptr;       // [4][no]: full row (spin up), full row (spin down), site, orbital in site
   const int* ia = nullptr;        // first row of each site
   const int* norb = nullptr;
-  const int* decode = nullptr;    // [dimens] sigma | i << 2 | mu << 12 | nu << 18
   const int* ztiles = nullptr;    // second-stage tiles: sigma | s' << 2 | i << 4 | x0 << 14 | y0 << 20
   int n_ztiles = 0;
   const int* rowoff = nullptr;    // first df row of each site
@@ -649,7 +648,6 @@ cudaError_t launch_she(const SheLaunch& l, cudaStream_t s) {
   a.tab = l.tab;
   a.ia = l.ia;
   a.norb = l.norb;
-  a.decode = l.decode;
   a.ztiles = l.ztiles;
   a.n_ztiles = l.n_ztiles;
   a.rowoff = l.rowoff;
