@@ -316,8 +316,10 @@ int tg_ldos(tg_ctx* ctx, int n_e, const double* e, double eta, double* ldosu, do
  *                            Gauss-Jordan below and on the real axis (dimH 36; elsewhere
  *                            Gauss-Jordan)
  *   TG_GREEN_GAUSS_JORDAN    Gauss-Jordan everywhere
- *   TG_GREEN_SPECTRAL        spectral wherever the mesh allows (tg_she ~4x faster,
- *                            tg_expectation one eigendecomposition per k for all energies)
+ *   TG_GREEN_SPECTRAL        spectral wherever the mesh allows in chi0, tg_ldos, tg_she and
+ *                            tg_expectation (61 x 61 k of two spd sites, 64 imaginary and
+ *                            32 real energies: tg_she 31.9 ms against 44.9 under AUTO,
+ *                            tg_expectation 2.1 against 8.5)
  * The eigendecomposition handles even dimH up to 96 and the tridiagonalisation any dimH up
  * to 288; meshes whose energies do not share a k list (adaptive imaginary axes) always use
  * Gauss-Jordan there.  No counterpart in the reference. */

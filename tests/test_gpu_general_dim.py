@@ -146,7 +146,7 @@ def test_dyson_at_the_d_only_dimension_of_the_16_layer_slab(gpu):
 @pytest.mark.parametrize("shape,sel_d,precision", [("slab6", False, "fp64"), ("slab16", True, "fp64"),
                                                    ("slab16", True, "split")])
 def test_tridiagonal_resolvents_equal_gauss_jordan(gpu, shape, sel_d, precision):
-    """Uniform meshes beyond the Jacobi kernel's dimensions: chi0 from G over the rows chi
+    """Uniform meshes beyond the dimensions of spectral G: chi0 from G over the rows chi
     needs, formed from a Householder tridiagonalisation per k (the default there), equals the
     cluster Gauss-Jordan path, at q != 0 with the real axis."""
     deck = synthetic.make_deck(shape, nk=(3, 3, 1), n1gl=4, parts=1, n3gl=3)

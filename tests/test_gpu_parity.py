@@ -274,7 +274,7 @@ def test_nanoribbon_golden_through_gpu(gpu, precision):
 
 @pytest.mark.parametrize("shape", ["bcc1", "sq2", "bcc4", "slab5"])
 def test_eig_batch_matches_eigh(gpu, shape):
-    """Jacobi eigendecomposition of H(k) behind the spectral Green functions (at dimH 90 on
+    """Eigendecomposition of H(k) behind the spectral Green functions (at dimH 90 on
     the packed upper triangle of the rotated matrix)."""
     deck = synthetic.make_deck(shape, mesh=False)
     s = deck.system

@@ -26,8 +26,8 @@ __host__ __device__ inline int pair_stride(int n) { return (n + 6) / 8 * 8 + 1; 
 // point's matrices are copied to shared memory first, where the 8 entries of a pair-point (64
 // FMAs) cost as many cycles as its arithmetic; otherwise (two matrices beyond the shared
 // memory) they are read through L1.  Bound by the reading of G (16 n^2 bytes per matrix): the
-// GG tensor of 72 x 72 matrices takes 1.6 ms beside 13.2 ms for their inversion (46 ms when the
-// inversion kernel formed the products itself, from one CTA's registers).
+// GG tensor of 29160 matrices of dimension 72 takes 1.5 ms beside 6.6 ms for their inversion (46 ms
+// together when the inversion kernel formed the products itself, from one CTA's registers).
 template <bool STAGED>
 __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(GreenArgs g, const double2* __restrict__ Ga,
                                                             const double2* __restrict__ Gb,

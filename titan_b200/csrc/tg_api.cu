@@ -2883,7 +2883,12 @@ extern "C" int tg_she(tg_ctx* c, const double* q, double e, double Ef, double et
   const bool spec = spectral_forced(c);
   // AUTO at n = 36 on a tabulated imaginary axis: spectral G for the energies with
   // Im z >= 10 eta (its eps |H| / Im z error is negligible there; the nanoribbon goldens
-  // hold with the split at 10 eta), the one-warp Gauss-Jordan kernel below and on the real axis
+  // hold with the split at 10 eta), the blocked Gauss-Jordan kernel below and on the real axis.
+  // Measured against Gauss-Jordan alone (ms, 64 and 20 imaginary energies, 8 real ones): 36, 61 x 61 k:
+  // 34.3 / 37.8 and 15.8 / 14.5, 13 x 13 k: 3.0 / 2.0 and 2.2 / 0.9; the split on at the other
+  // dimensions: 18, 14^3 k: 8.2 / 8.6 and 3.9 / 3.4; 54, 30 x 30 k: 32.2 / 36.4 and 16.5 / 13.8; 72,
+  // 8^3 k: 59.7 / 64.9 and 29.1 / 24.2.  It pays by the energies per k and the number of k rather
+  // than by the dimension; it is kept to the dimension it was brought in for.
   const bool hybrid = !spec && c->green_method == TG_GREEN_AUTO && tab_imag && eig_supported(n) &&
                       n == 36 && green_mma_supported(n, MODE_RAW);
   const double y_split = 10.0 * eta;

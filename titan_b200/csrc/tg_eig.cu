@@ -5,16 +5,17 @@
 //      LAPACK's zhetd2, lower form, with zlarfg's reflectors), one CTA per k with the matrix in
 //      shared memory; Q is accumulated backwards in place.  Also used for the resolvents of
 //      tg_tridiag.cu at dimensions up to 96.
-//   2. ql_kernel: T = Z diag(lambda) Z^T by the implicitly shifted QL iteration (Bowdler,
-//      Martin, Reinsch and Wilkinson, 1968), one thread per k with d and e in shared memory.
+//   2. ql_kernel: T = Z diag(lambda) Z^T by the implicitly shifted QL iteration (Martin and
+//      Wilkinson, 1968; Dubrulle, 1970), one thread per k with d and e in shared memory.
 //      The iteration is a serial chain of n^2 plane rotations, so only the number of k hides
 //      it; its rotations go to global memory.
 //   3. eig_apply_kernel: U = Q Z, one CTA per k with Q in shared memory and a thread per real
 //      row (rotations of columns act on every row alone, without any barrier).
 //   4. eig_finish_kernel: one Newton-Schulz step U <- U (1 - (U^H U - 1) / 2) and Rayleigh
 //      quotients of H for the eigenvalues, its products on the FP64 tensor cores.
-// About 20 n^3 flops per matrix against the 10 sweeps of 24 n^3 of a cyclic Jacobi iteration,
-// whose rotations also need a CTA barrier per round.  Measured: 9801 matrices of dimension 36 in
+// About 46 n^3 flops per matrix (reduction and Q 16/3 n^3 each, 1.3 n^2 rotations of 2 n real rows
+// 16 n^3, post-pass 20 n^3) against the 10 sweeps of 24 n^3 of a cyclic Jacobi iteration, whose
+// rotations also need a CTA barrier per round.  Measured: 9801 matrices of dimension 36 in
 // 24 ms with Jacobi rotations, 3.7 ms now (1.5, 0.5, 1.1 and 0.6 ms for the four kernels); 1331 of
 // dimension 72 in 45 ms and 5.5 ms, of which the serial chains of ql_kernel take 1.7 ms.
 #include "tg_internal.cuh"
