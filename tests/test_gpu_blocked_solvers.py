@@ -209,3 +209,73 @@ def test_launches_are_counted(gpu, shape, d_only, counts):
     finally:
         gpu.set_chi_orbitals(None)
     assert tuple(got) == counts
+
+
+class MixedSites:
+    """A chain of sites of `norbs` orbitals with random Hermitian hoppings to two cells: what the
+    binding and the oracle read of a system."""
+
+    def __init__(self, norbs, rng):
+        self.norbs, self.n_atoms = list(norbs), len(norbs)
+        self.dimH, self.dimens = 2 * sum(norbs), 4 * sum(n * n for n in norbs)
+        nat, nm = self.n_atoms, max(norbs)
+        cells, basis, t = [], [], []
+        for R in (np.array([1.0, 0.2, 0.0]), np.array([0.1, 1.1, 0.0])):
+            b = {(j, i): 0.3 * (rng.standard_normal((norbs[j], norbs[i])) + 1j * rng.standard_normal((norbs[j], norbs[i])))
+                 for j in range(nat) for i in range(nat)}
+            for sign in (1, -1):
+                for j in range(nat):
+                    blk = np.zeros((nat, nm, nm), complex)
+                    for i in range(nat):
+                        blk[i, :norbs[j], :norbs[i]] = b[j, i] if sign > 0 else b[i, j].conj().T
+                    cells.append(sign * R)
+                    basis.append(j)
+                    t.append(blk)
+        self.table = (np.array(cells), np.array(basis, np.int32), np.ones((len(t), nat), np.int32), np.array(t))
+
+    def neighbor_table(self):
+        return self.table
+
+    def ia(self):
+        from titan_b200.host import onsite
+        return onsite.site_offsets(self.norbs)
+
+    def sigmaimunu2i(self):
+        from titan_b200.host.system import TBSystem
+        return TBSystem.sigmaimunu2i(self)
+
+
+@pytest.mark.parametrize("norbs", [(4, 5), (2, 3, 4), (9, 4, 5), (1, 8, 9), (9, 9, 2), (9, 5, 9, 4), (5, 9, 9, 9, 4),
+                                   (10, 9, 8, 9, 9), (13, 9, 9, 9, 8)])
+def test_sites_of_different_orbital_counts(gpu, norbs):
+    """chi0 (spectral, tridiagonalised from 90 on, and Gauss-Jordan) and, up to 90, the disturbance
+    integral on both axes where no site starts or ends at a fragment's or a tile's edge: dimensions
+    18 to 96 with a kernel of their own, within 1e-10 of the oracle, the bound of the plain tests."""
+    from titan_b200.host.mesh import EKMesh
+    rng = np.random.default_rng(sum(norbs) * 31 + len(norbs))
+    s = MixedSites(norbs, rng)
+    h = rng.standard_normal((s.dimH, s.dimH)) + 1j * rng.standard_normal((s.dimH, s.dimH))
+    h = 0.5 * (h + h.conj().T)
+    nk, y, wy = 5, np.array([0.01, 0.2, 3.0]), rng.uniform(0.2, 1.0, 3)
+    k = rng.uniform(-2, 2, (nk, 3))
+    ek = EKMesh(y, wy, np.repeat(np.arange(3), nk), np.tile(k, (3, 1)), np.repeat(wy, nk) / nk)
+    Ef, eta, etap, e, q, ue = 0.1, 2e-3, 1e-3, 0.07, np.array([0.2, 0.1, 0.0]), np.array([0.6, 0.3, 0.0])
+    x2, p2 = np.linspace(Ef - e, Ef, 3), np.full(3, 0.02)
+    gpu.set_system(s)
+    gpu.set_h0(h)
+    gpu.set_imag_mesh(ek)
+    gpu.set_real_mesh(k, np.full(nk, 1.0 / nk))
+    m, bz = O.Model(s, h), (k, np.full(nk, 1.0 / nk))
+    ref = O.eintshechi(m, ek, bz, q, e, Ef, eta, etap, x2, p2)
+    single = s.dimH in (18, 36, 40, 54, 72, 90)   # (the cluster kernel has no disturbance integral)
+    try:
+        for method in ("auto", "gauss-jordan"):
+            gpu.set_green_method(method)
+            got = gpu.chi0(q, e, Ef, eta, etap, x2, p2)
+            assert np.linalg.norm(got - ref) <= 1e-10 * np.linalg.norm(ref), method
+            if single:
+                she = gpu.she(q, e, Ef, eta, etap, x2, p2, ue)
+                sref = O.eintshe(m, ek, bz, q, e, Ef, eta, etap, x2, p2, ue)
+                assert np.max(np.abs(she - sref)) <= 1e-10 * np.max(np.abs(sref)), method
+    finally:
+        gpu.set_green_method("auto")
